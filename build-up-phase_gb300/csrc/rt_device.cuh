@@ -92,9 +92,32 @@ struct Ray {
     float d[3];
     float invd[3];
     float sx, sy, sz;
-    uint32_t oct;   // bit a set: invd[a] < 0
+    uint32_t prio;  // visiting order of a node's slots, see child_priority
     uint32_t kxyz;  // kx | ky << 2 | kz << 4
 };
+
+// Children are visited in ascending (slot ^ octant), bit a of the octant set
+// where invd[a] < 0.  Byte a of the word holds the slots whose bit a equals the
+// octant's, i.e. those that come first as far as axis a decides, so the next of
+// a set of slots is found by narrowing it with the z byte, then y, then x.
+__device__ __forceinline__ uint32_t child_priority(uint32_t oct) {
+    return (0x55u << (oct & 1u)) | (0x3300u << (oct & 2u)) | (0x0f0000u << (oct & 4u));
+}
+// The octant's bits back from the word.
+__device__ __forceinline__ bool prio_neg_x(uint32_t prio) { return (prio & 1u) == 0u; }
+__device__ __forceinline__ bool prio_neg_y(uint32_t prio) { return (prio & 0x100u) == 0u; }
+__device__ __forceinline__ bool prio_neg_z(uint32_t prio) { return (prio & 0x10000u) == 0u; }
+
+// The first slot of the non-empty set `slots` (bits 0-7) in visiting order, as
+// a one-bit mask.
+__device__ __forceinline__ uint32_t first_slot(uint32_t slots, uint32_t prio) {
+    uint32_t t = slots & (prio >> 16);
+    slots = t ? t : slots;
+    t = slots & (prio >> 8);
+    slots = t ? t : slots;
+    t = slots & prio;
+    return t ? t : slots;
+}
 
 __device__ __forceinline__ float sel3(uint32_t k, float x, float y, float z) {
     return k == 0 ? x : (k == 1 ? y : z);
@@ -110,7 +133,7 @@ __device__ __forceinline__ void ray_setup(Ray &r, const float o[3], const float 
         r.invd[a] = 1.0f / dd;
         oct |= (r.invd[a] < 0.0f ? 1u : 0u) << a;
     }
-    r.oct = oct;
+    r.prio = child_priority(oct);
     float ax = fabsf(d[0]), ay = fabsf(d[1]), az = fabsf(d[2]);
     uint32_t kz = ax >= ay ? (ax >= az ? 0u : 2u) : (ay >= az ? 1u : 2u);
     uint32_t kx = kz == 2u ? 0u : kz + 1u;
@@ -120,7 +143,9 @@ __device__ __forceinline__ void ray_setup(Ray &r, const float o[3], const float 
     r.kxyz = kx | (ky << 2) | (kz << 4);
     r.sx = sel3(kx, d[0], d[1], d[2]) / dkz;
     r.sy = sel3(ky, d[0], d[1], d[2]) / dkz;
-    r.sz = 1.0f / dkz;
+    // the largest component's reciprocal, computed above unless the whole
+    // direction is below RT_DIR_EPS
+    r.sz = fabsf(dkz) < RT_DIR_EPS ? 1.0f / dkz : sel3(kz, r.invd[0], r.invd[1], r.invd[2]);
 }
 
 // Returns true and (t, u, v) when the triangle is hit with t in [tmin, tmax].
@@ -215,26 +240,31 @@ __device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
     return d;
 }
-// Byte b of wx and of wy as the pair (2^23 + qx, 2^23 + qy); adding
+// Bytes b and b + 1 of w as the pair (2^23 + q, 2^23 + q'); adding
 // (-2^23, -2^23) leaves the exact byte values.
-__device__ __forceinline__ uint64_t qpair2_biased(uint32_t wx, uint32_t wy, int b) {
-    const uint32_t lo = __byte_perm(wx, 0x4B000000u, 0x7540u | (uint32_t)b);
-    const uint32_t hi = __byte_perm(wy, 0x4B000000u, 0x7540u | (uint32_t)b);
+__device__ __forceinline__ uint64_t qpair_biased(uint32_t w, int b) {
+    const uint32_t lo = __byte_perm(w, 0x4B000000u, 0x7540u | (uint32_t)b);
+    const uint32_t hi = __byte_perm(w, 0x4B000000u, 0x7541u + (uint32_t)b);
     uint64_t d;
     asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(hi));
     return d;
 }
 
-// Box test of a node's 8 children against [tmin, tcur].
-//   node_hits: bit (slot ^ oct) for every internal child hit
-//   prim_hits: leaf-record mask relative to the node's prim_base
-// An internal child's meta byte is 0x20 | (24 + slot) and a leaf's offset is
-// below 24, so XOR-ing the octant into the internal bytes (four at a time)
-// lets one shift-or per hit slot build both masks: internal children land on
-// bit 24 + (slot ^ oct), leaf records on their offsets.
-template <bool PAIR_Z = false>
-__device__ __forceinline__ void isect_node(const Ray &r, const NodeWords &n, float tmin, float tcur,
-                                           uint32_t &node_hits, uint32_t &prim_hits) {
+// Box test of a node's 8 children against [tmin, tcur]: bit s set where the
+// box of slot s is hit (an unused slot may show a hit: its meta byte is 0 and
+// it is not an internal child, so it leads nowhere).
+//
+// The kernels that call it are bound by issue slots, so it is laid out for
+// instruction count: two neighbouring children share every .f32x2 add and fma
+// (plane distance fma(q, scale, adj), each half rounded as the scalar
+// instruction).  Their bytes come out of one word, so the pairs form in place;
+// pairing the x and y planes of one child instead cost a register move for
+// nearly every pair.  A child is missed when tfar * scale - tnear is negative,
+// and the eight sign bits are shifted into one mask: the scale goes on by an
+// fma with +0, which leaves no -0 whose difference to +0 would carry a sign,
+// and an inf - inf carries none either (a hit, as inf <= inf is).  Measured on one node per lane: 175 instructions,
+// 301 with the planes of one child paired and a mask bit or-ed in per child.
+__device__ __forceinline__ uint32_t isect_node(const Ray &r, const NodeWords &n, float tmin, float tcur) {
     const float px = __uint_as_float(n.w0.x), py = __uint_as_float(n.w0.y), pz = __uint_as_float(n.w0.z);
     const int ex = (int)(int8_t)(n.w0.w & 0xffu);
     const int ey = (int)(int8_t)((n.w0.w >> 8) & 0xffu);
@@ -246,45 +276,60 @@ __device__ __forceinline__ void isect_node(const Ray &r, const NodeWords &n, flo
     // qlo/qhi words for slots 0-3 (lo) and 4-7 (hi), per axis
     const uint32_t lox[2] = {n.w2.x, n.w2.y}, loy[2] = {n.w2.z, n.w2.w}, loz[2] = {n.w3.x, n.w3.y};
     const uint32_t hix[2] = {n.w3.z, n.w3.w}, hiy[2] = {n.w4.x, n.w4.y}, hiz[2] = {n.w4.z, n.w4.w};
-    const uint32_t meta[2] = {n.w1.z, n.w1.w};
-    const bool nx = r.oct & 1u, ny = r.oct & 2u, nz = r.oct & 4u;
-    // a child's x and y plane distances as one .f32x2 add and fma and, with
-    // PAIR_Z (kernels with registers to spare), its near and far z distances
-    // as another; each half equals the scalar fma(q, scale, adj)
-    const uint64_t bias2 = f2_pack(-8388608.0f, -8388608.0f);
-    const uint64_t scxy = f2_pack(scx, scy), adjxy = f2_pack(adjx, adjy);
-    uint32_t hits = 0;
+    const bool nx = prio_neg_x(r.prio), ny = prio_neg_y(r.prio), nz = prio_neg_z(r.prio);
+    const uint64_t bias = f2_pack(-8388608.0f, -8388608.0f), far_scale = f2_pack(kTfarScale, kTfarScale);
+    const uint64_t zero = f2_pack(0.0f, 0.0f);
+    const uint64_t sx = f2_pack(scx, scx), sy = f2_pack(scy, scy), sz = f2_pack(scz, scz);
+    const uint64_t ax = f2_pack(adjx, adjx), ay = f2_pack(adjy, adjy), az = f2_pack(adjz, adjz);
+    uint32_t miss = 0u;
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
+    for (int h = 1; h >= 0; --h) {
         const uint32_t nearx = nx ? hix[h] : lox[h], farx = nx ? lox[h] : hix[h];
         const uint32_t neary = ny ? hiy[h] : loy[h], fary = ny ? loy[h] : hiy[h];
         const uint32_t nearz = nz ? hiz[h] : loz[h], farz = nz ? loz[h] : hiz[h];
-        const uint32_t inner4 = (meta[h] >> 3) & (meta[h] >> 4) & 0x01010101u;
-        const uint32_t mx4 = meta[h] ^ (inner4 * r.oct);
 #pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            float nxv, nyv, fxv, fyv, tn, tf;
-            f2_unpack(f2_fma(f2_add(qpair2_biased(nearx, neary, b), bias2), scxy, adjxy), nxv, nyv);
-            f2_unpack(f2_fma(f2_add(qpair2_biased(farx, fary, b), bias2), scxy, adjxy), fxv, fyv);
-            if constexpr (PAIR_Z) {
-                float nzv, fzv;
-                f2_unpack(f2_fma(f2_add(qpair2_biased(nearz, farz, b), bias2), f2_pack(scz, scz),
-                                 f2_pack(adjz, adjz)),
-                          nzv, fzv);
-                tn = fmaxf(fmax3(tmin, nxv, nyv), nzv);
-                tf = fminf(fmin3(tcur, fxv, fyv), fzv);
-            } else {
-                tn = fmaxf(fmax3(tmin, nxv, nyv), __fmaf_rn(qbyte(nearz, b), scz, adjz));
-                tf = fminf(fmin3(tcur, fxv, fyv), __fmaf_rn(qbyte(farz, b), scz, adjz));
-            }
-            if (tn <= tf * kTfarScale) {
-                const uint32_t m = byte_of(mx4, b);
-                hits |= (m >> 5) << (m & 31u);
-            }
+        for (int b = 2; b >= 0; b -= 2) {
+            float nx0, nx1, ny0, ny1, nz0, nz1, fx0, fx1, fy0, fy1, fz0, fz1, d0, d1;
+            f2_unpack(f2_fma(f2_add(qpair_biased(nearx, b), bias), sx, ax), nx0, nx1);
+            f2_unpack(f2_fma(f2_add(qpair_biased(neary, b), bias), sy, ay), ny0, ny1);
+            f2_unpack(f2_fma(f2_add(qpair_biased(nearz, b), bias), sz, az), nz0, nz1);
+            f2_unpack(f2_fma(f2_add(qpair_biased(farx, b), bias), sx, ax), fx0, fx1);
+            f2_unpack(f2_fma(f2_add(qpair_biased(fary, b), bias), sy, ay), fy0, fy1);
+            f2_unpack(f2_fma(f2_add(qpair_biased(farz, b), bias), sz, az), fz0, fz1);
+            const float tn0 = fmaxf(fmax3(tmin, nx0, ny0), nz0), tn1 = fmaxf(fmax3(tmin, nx1, ny1), nz1);
+            const float tf0 = fminf(fmin3(tcur, fx0, fy0), fz0), tf1 = fminf(fmin3(tcur, fx1, fy1), fz1);
+            f2_unpack(f2_add(f2_fma(f2_pack(tf0, tf1), far_scale, zero), f2_pack(-tn0, -tn1)), d0, d1);
+            miss = __funnelshift_l(__float_as_uint(d1), miss, 1);
+            miss = __funnelshift_l(__float_as_uint(d0), miss, 1);
         }
     }
-    node_hits = hits >> 24;
-    prim_hits = hits & 0x00ffffffu;
+    return ~miss & 0xffu;
+}
+
+// Leaf records of the hit slots, as a mask relative to the node's prim_base (a
+// leaf's meta byte: its record count in unary, then its first record's offset).
+__device__ __forceinline__ uint32_t leaf_records(const NodeWords &n, uint32_t hits) {
+    uint32_t leaf = hits & ~(n.w0.w >> 24), recs = 0u;
+    while (leaf) {
+        const uint32_t m = __byte_perm(n.w1.z, n.w1.w, (uint32_t)__ffs((int)leaf) - 1u) & 0xffu;
+        leaf &= leaf - 1u;
+        recs |= (m >> 5) << (m & 31u);
+    }
+    return recs;
+}
+
+// The hit internal children of a node as a traversal group: first child's
+// index, hit slots (bits 0-7) and all internal slots (bits 8-15).
+__device__ __forceinline__ uint2 child_group(const NodeWords &n, uint32_t hits) {
+    const uint32_t inner = n.w0.w >> 24;
+    return make_uint2(n.w1.x, (hits & inner) | (inner << 8));
+}
+__device__ __forceinline__ bool group_left(const uint2 &g) { return (g.y & 0xffu) != 0u; }
+// Takes the next child of a group with children left; returns its node.
+__device__ __forceinline__ uint32_t take_child(uint2 &g, uint32_t prio) {
+    const uint32_t bit = first_slot(g.y & 0xffu, prio);
+    g.y ^= bit;
+    return g.x + __popc((g.y >> 8) & (bit - 1u));
 }
 
 // Device-side error reporting: the first error code wins.

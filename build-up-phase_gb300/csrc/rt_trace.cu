@@ -14,12 +14,13 @@
 //                   structure in the header is not its kind.
 //   k_pipeline      the sample's raygen + traceRayEXT + closest-hit / miss +
 //                   imageStore, one thread per launch id.
+//   k_trace_stats   node visits and triangle tests, one thread per ray.
 //
-// Visiting order (identical in the CPU restatement, so hits and statistics
-// agree exactly): a node's leaf records first, in ascending record order,
-// then its internal children in ascending (slot ^ ray octant); remaining
-// siblings are pushed as one group.  Closest hit = smallest t, ties broken by
-// the smallest (instance, triangle) key.
+// Visiting order: a node's leaf records first, in ascending record order, then
+// its internal children in ascending (slot ^ ray octant); remaining siblings
+// are pushed as one group (identical in the CPU restatement, whose statistics
+// k_trace_stats equals; k_trace_blas tests records in batches).  Closest hit =
+// smallest t, ties broken by the smallest (instance, triangle) key.
 #include <cmath>
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -68,8 +69,8 @@ __device__ bool traverse_blas_simple(const uint8_t *accel, const Ray &r, float t
             return h.found;
         }
         NodeWords nd = load_node(nodes, node);
-        uint32_t nh, ph;
-        isect_node(r, nd, tmin, h.t, nh, ph);
+        const uint32_t hits = isect_node(r, nd, tmin, h.t);
+        uint32_t ph = leaf_records(nd, hits);
         if (stats) stats[0]++;
         const uint32_t pbase = nd.w1.y;
         while (ph) {
@@ -94,14 +95,11 @@ __device__ bool traverse_blas_simple(const uint8_t *accel, const Ray &r, float t
                 hkey = key;
             }
         }
-        uint2 g = make_uint2(nd.w1.x, nh | ((nd.w0.w >> 24) << 8));
+        uint2 g = child_group(nd, hits);
         for (;;) {
-            if (g.y & 0xffu) {
-                uint32_t k = __ffs(g.y & 0xffu) - 1;
-                g.y &= ~(1u << k);
-                uint32_t s = k ^ r.oct;
-                node = g.x + __popc((g.y >> 8) & ((1u << s) - 1u));
-                if (g.y & 0xffu) {
+            if (group_left(g)) {
+                node = take_child(g, r.prio);
+                if (group_left(g)) {
                     if (st.sp >= kMaxDepth) {
                         report_error(err, RT_ERR_BOUNDS, 0x70000000u);
                         return h.found;
@@ -174,8 +172,8 @@ __device__ bool trace_ray(const uint8_t *accel, const float o[3], const float d[
             break;
         }
         NodeWords nd = load_node(nodes, node);
-        uint32_t nh, ph;
-        isect_node(r, nd, tmin, h.t, nh, ph);
+        const uint32_t hits = isect_node(r, nd, tmin, h.t);
+        uint32_t ph = leaf_records(nd, hits);
         if (stats) stats[0]++;
         const uint32_t pbase = nd.w1.y;
         while (ph && !(ANY && h.found)) {
@@ -200,14 +198,11 @@ __device__ bool trace_ray(const uint8_t *accel, const float o[3], const float d[
             if (ANY && hit) break;
         }
         if (ANY && h.found) break;
-        uint2 g = make_uint2(nd.w1.x, nh | ((nd.w0.w >> 24) << 8));
+        uint2 g = child_group(nd, hits);
         for (;;) {
-            if (g.y & 0xffu) {
-                uint32_t k = __ffs(g.y & 0xffu) - 1;
-                g.y &= ~(1u << k);
-                uint32_t s = k ^ r.oct;
-                node = g.x + __popc((g.y >> 8) & ((1u << s) - 1u));
-                if (g.y & 0xffu) {
+            if (group_left(g)) {
+                node = take_child(g, r.prio);
+                if (group_left(g)) {
                     if (st.sp >= kMaxDepth) {
                         report_error(err, RT_ERR_BOUNDS, 0x71000000u);
                         done = true;
@@ -251,7 +246,7 @@ __device__ __forceinline__ bool inst_key_less(float t, uint32_t inst, uint32_t t
     return t < h.t || (t == h.t && (!h.found || inst < h.inst || (inst == h.inst && tri < h.tri)));
 }
 
-template <bool ANY, bool STATS>
+template <bool ANY>
 __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(const BatchArgs a) {
     const rt_accel_header *hd = reinterpret_cast<const rt_accel_header *>(a.accel);
     if (hd->kind != RT_ACCEL_KIND_TLAS) return;
@@ -277,7 +272,6 @@ __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(
     uint2 g = make_uint2(0u, 0u), ig = make_uint2(0u, 0u);
     int sp = 0, lo = 0;
     uint2 spill[kInstDepth];
-    unsigned long long n_nodes = 0, n_tris = 0;
     const uint32_t n_rays = a.n;
 
     auto push = [&](uint2 e) {
@@ -340,10 +334,9 @@ __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(
                         if (in_blas) ++visits_b;
                         else ++visits_t;
                         NodeWords nd = load_node(in_blas ? bnodes : tnodes, node);
-                        uint32_t nh, ph;
-                        isect_node<true>(r, nd, tmin, h.t, nh, ph);
-                        if (STATS) n_nodes++;
-                        g = make_uint2(nd.w1.x, nh | ((nd.w0.w >> 24) << 8));
+                        const uint32_t hits = isect_node(r, nd, tmin, h.t);
+                        uint32_t ph = leaf_records(nd, hits);
+                        g = child_group(nd, hits);
                         if (!in_blas) {
                             ig = make_uint2(nd.w1.y, ph);  // the node's instances, walked first
                         } else {
@@ -353,7 +346,6 @@ __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(
                                 ph &= ph - 1u;
                                 const uint4 *rec = bprims + (size_t)(pbase + i) * 3u;
                                 const uint4 q0 = ldg4(rec), q1 = ldg4(rec + 1), q2 = ldg4(rec + 2);
-                                if (STATS) n_tris++;
                                 float t, u, v;
                                 if (!isect_tri(r,
                                                make_float4(__uint_as_float(q0.x), __uint_as_float(q0.y),
@@ -394,7 +386,7 @@ __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(
                             break;
                         }
                         // save the TLAS node's remaining work under a return marker
-                        if (g.y & 0xffu) push(g);
+                        if (group_left(g)) push(g);
                         if (ig.y) push(make_uint2(ig.x, ig.y | kInstGroup));
                         push(make_uint2(0u, kReturnTop));
                         g = make_uint2(0u, 0u);
@@ -414,13 +406,10 @@ __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(
                         pending = true;
                         break;
                     }
-                    if (g.y & 0xffu) {
-                        const uint32_t k = __ffs(g.y & 0xffu) - 1;
-                        g.y &= ~(1u << k);
-                        const uint32_t s = k ^ r.oct;
-                        node = g.x + __popc((g.y >> 8) & ((1u << s) - 1u));
+                    if (group_left(g)) {
+                        node = take_child(g, r.prio);
                         pending = true;
-                        if (g.y & 0xffu) {
+                        if (group_left(g)) {
                             if (sp >= kInstDepth) {
                                 report_error(a.err, RT_ERR_BOUNDS, in_blas ? 0x70000000u : 0x71000000u);
                                 finish = true;
@@ -489,15 +478,29 @@ __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(
             if (!exhausted && (uint32_t)__popc(~act) >= a.refill) break;
         }
     }
-    if (STATS) {
-        for (int o = 16; o > 0; o >>= 1) {
-            n_nodes += __shfl_xor_sync(0xffffffffu, n_nodes, o);
-            n_tris += __shfl_xor_sync(0xffffffffu, n_tris, o);
-        }
-        if (lane == 0) {
-            atomicAdd(a.stats, n_nodes);
-            atomicAdd(a.stats + 1, n_tris);
-        }
+}
+
+// Traversal statistics (rt_trace_stats): node visits and triangle tests of
+// the per-thread walk, which tests a node's triangles as it visits the node,
+// in the order of the CPU restatement.
+template <bool ANY>
+__global__ void __launch_bounds__(kTraceThreads) k_trace_stats(const uint8_t *accel, const float4 *rays, uint32_t n,
+                                                                unsigned long long *counters, uint32_t *err) {
+    unsigned long long stats[2] = {0ull, 0ull};
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const float4 r0 = __ldg(rays + 2u * i), r1 = __ldg(rays + 2u * i + 1u);
+        const float o[3] = {r0.x, r0.y, r0.z}, d[3] = {r1.x, r1.y, r1.z};
+        Hit h;
+        HitIds ids;
+        trace_ray<ANY>(accel, o, d, r0.w, r1.w, 0xffu, h, ids, err, stats);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        stats[0] += __shfl_xor_sync(0xffffffffu, stats[0], o);
+        stats[1] += __shfl_xor_sync(0xffffffffu, stats[1], o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(counters, stats[0]);
+        atomicAdd(counters + 1, stats[1]);
     }
 }
 
@@ -531,7 +534,10 @@ __device__ __forceinline__ void raygen(const PipelineArgs &a, uint32_t x, uint32
     dir[2] = (p * 0.0f + q * 0.0f) + -1.0f;
 }
 
-__global__ void __launch_bounds__(128) k_pipeline(const PipelineArgs a) {
+// Six blocks per SM (80 registers): the walk is latency-bound (1200x800
+// pixels of the two-instance sample: 22.5 us; 24.3 at five blocks, 23.1 at
+// eight, 26.2 with the compiler's choice of 126 registers).
+__global__ void __launch_bounds__(128, 6) k_pipeline(const PipelineArgs a) {
     const uint32_t x = blockIdx.x * 16u + (threadIdx.x & 15u);
     const uint32_t y = blockIdx.y * 8u + (threadIdx.x >> 4);
     if (x >= a.width || y >= a.height) return;
@@ -582,7 +588,7 @@ __global__ void __launch_bounds__(128) k_pipeline(const PipelineArgs a) {
 // ---------------------------------------------------------------------------
 
 int launch_batch(rt_context *ctx, cudaStream_t st, uint64_t accel, const rt_ray *rays, rt_hit *hits,
-                 rt_hit_ext *hits_ext, uint8_t *occ, uint32_t n, bool any, unsigned long long *stats) {
+                 rt_hit_ext *hits_ext, uint8_t *occ, uint32_t n, bool any) {
     if (n == 0) return RT_OK;
     BatchArgs a{};
     a.accel = reinterpret_cast<const uint8_t *>(accel);
@@ -594,7 +600,6 @@ int launch_batch(rt_context *ctx, cudaStream_t st, uint64_t accel, const rt_ray 
     a.refill = ctx->tuning.batch_rays ? ctx->tuning.batch_rays : 4u;
     if (a.refill > 32u) a.refill = 32u;
     a.err = ctx->d_err;
-    a.stats = stats;
     a.n_dev = nullptr;
     a.out_rec = 0;
     a.counter = acquire_counter(ctx, st);
@@ -608,22 +613,12 @@ int launch_batch(rt_context *ctx, cudaStream_t st, uint64_t accel, const rt_ray 
     // kind returns immediately.
     uint32_t tl_blocks = kInstBlocksPerSm * (uint32_t)ctx->sm_count;
     if (tl_blocks > need) tl_blocks = need;
-    if (stats) {
-        if (any) {
-            k_trace_blas<true, true, false, kTraceThreads, kRing><<<blocks, kTraceThreads, 0, st>>>(a);
-            k_trace_inst<true, true><<<tl_blocks, kTraceThreads, 0, st>>>(a);
-        } else {
-            k_trace_blas<false, true, false, kTraceThreads, kRing><<<blocks, kTraceThreads, 0, st>>>(a);
-            k_trace_inst<false, true><<<tl_blocks, kTraceThreads, 0, st>>>(a);
-        }
+    if (any) {
+        k_trace_blas<true, false, kTraceThreads, kRing><<<blocks, kTraceThreads, 0, st>>>(a);
+        k_trace_inst<true><<<tl_blocks, kTraceThreads, 0, st>>>(a);
     } else {
-        if (any) {
-            k_trace_blas<true, false, false, kTraceThreads, kRing><<<blocks, kTraceThreads, 0, st>>>(a);
-            k_trace_inst<true, false><<<tl_blocks, kTraceThreads, 0, st>>>(a);
-        } else {
-            k_trace_blas<false, false, false, kTraceThreads, kRing><<<blocks, kTraceThreads, 0, st>>>(a);
-            k_trace_inst<false, false><<<tl_blocks, kTraceThreads, 0, st>>>(a);
-        }
+        k_trace_blas<false, false, kTraceThreads, kRing><<<blocks, kTraceThreads, 0, st>>>(a);
+        k_trace_inst<false><<<tl_blocks, kTraceThreads, 0, st>>>(a);
     }
     RT_CUDA_CTX(ctx, cudaGetLastError());
     return RT_OK;
@@ -656,7 +651,6 @@ int launch_queue_trace(rt_context *ctx, cudaStream_t st, const uint8_t *accel, c
     a.n = max_n;
     a.refill = kQueueRefill;
     a.err = ctx->d_err;
-    a.stats = nullptr;
     a.n_dev = n_dev;
     a.out_rec = 1;
     a.counter = counter;
@@ -665,8 +659,8 @@ int launch_queue_trace(rt_context *ctx, cudaStream_t st, const uint8_t *accel, c
     uint32_t blocks = per_sm * (uint32_t)ctx->sm_count;
     uint32_t need = (max_n + kTraceThreads - 1) / kTraceThreads;
     if (blocks > need) blocks = need;
-    if (any) k_trace_blas<true, false, false, kTraceThreads, kRing><<<blocks, kTraceThreads, 0, st>>>(a);
-    else k_trace_blas<false, false, false, kTraceThreads, kRing><<<blocks, kTraceThreads, 0, st>>>(a);
+    if (any) k_trace_blas<true, false, kTraceThreads, kRing><<<blocks, kTraceThreads, 0, st>>>(a);
+    else k_trace_blas<false, false, kTraceThreads, kRing><<<blocks, kTraceThreads, 0, st>>>(a);
     RT_CUDA_CTX(ctx, cudaGetLastError());
     return RT_OK;
 }
@@ -696,7 +690,7 @@ int launch_queue_trace_mixed(rt_context *ctx, cudaStream_t st, const uint8_t *ac
     uint32_t blocks = per_sm * (uint32_t)ctx->sm_count;
     const uint32_t need = (uint32_t)(((uint64_t)max_n * 2u + kTraceThreads - 1) / kTraceThreads);
     if (blocks > need) blocks = need;
-    k_trace_blas<false, false, false, kTraceThreads, kRing, true><<<blocks, kTraceThreads, 0, st>>>(a);
+    k_trace_blas<false, false, kTraceThreads, kRing, true><<<blocks, kTraceThreads, 0, st>>>(a);
     RT_CUDA_CTX(ctx, cudaGetLastError());
     return RT_OK;
 }
@@ -712,15 +706,13 @@ using namespace rtc;
 extern "C" rt_status rt_trace_closest(rt_context *ctx, rt_stream stream, uint64_t accel, const rt_ray *rays,
                                       rt_hit *hits, rt_hit_ext *hits_ext, uint32_t n) {
     if (!ctx || !accel || (n && (!rays || !hits))) return set_error(ctx, RT_ERR_INVALID_ARG, "rt_trace_closest: null argument");
-    return launch_batch(ctx, static_cast<cudaStream_t>(stream), accel, rays, hits, hits_ext, nullptr, n, false,
-                        nullptr);
+    return launch_batch(ctx, static_cast<cudaStream_t>(stream), accel, rays, hits, hits_ext, nullptr, n, false);
 }
 
 extern "C" rt_status rt_trace_any(rt_context *ctx, rt_stream stream, uint64_t accel, const rt_ray *rays,
                                   uint8_t *occluded, uint32_t n) {
     if (!ctx || !accel || (n && (!rays || !occluded))) return set_error(ctx, RT_ERR_INVALID_ARG, "rt_trace_any: null argument");
-    return launch_batch(ctx, static_cast<cudaStream_t>(stream), accel, rays, nullptr, nullptr, occluded, n, true,
-                        nullptr);
+    return launch_batch(ctx, static_cast<cudaStream_t>(stream), accel, rays, nullptr, nullptr, occluded, n, true);
 }
 
 // ---------------------------------------------------------------------------
@@ -884,7 +876,7 @@ int trace_host(rt_context *ctx, cudaStream_t st, uint64_t accel, const rt_ray *h
         reachable_in_place(hrays, (uint64_t)n * 32u, pageable) &&
         reachable_in_place(hout, (uint64_t)n * out_size, pageable))
         return launch_batch(ctx, st, accel, hrays, any ? nullptr : static_cast<rt_hit *>(hout), nullptr,
-                            any ? static_cast<uint8_t *>(hout) : nullptr, n, any, nullptr);
+                            any ? static_cast<uint8_t *>(hout) : nullptr, n, any);
     const HostSlots H = host_slots(scratch_bytes);
     if (H.chunk == 0) return set_error(ctx, RT_ERR_OOM, "rt_trace_*_host: scratch smaller than rt_trace_host_scratch_bytes(1)");
     if (reinterpret_cast<uintptr_t>(scratch) & 255u) return set_error(ctx, RT_ERR_INVALID_ARG, "rt_trace_*_host: scratch must be 256-byte aligned");
@@ -919,8 +911,7 @@ int trace_host(rt_context *ctx, cudaStream_t st, uint64_t accel, const rt_ray *h
         RT_CUDA_CTX(ctx, cudaEventRecord(ctx->ev_loaded[s], ctx->h2d));
         RT_CUDA_CTX(ctx, cudaStreamWaitEvent(ts, ctx->ev_loaded[s], 0));
         rc = launch_batch(ctx, ts, accel, reinterpret_cast<const rt_ray *>(rays_d),
-                          any ? nullptr : reinterpret_cast<rt_hit *>(out_d), nullptr, any ? out_d : nullptr, m, any,
-                          nullptr);
+                          any ? nullptr : reinterpret_cast<rt_hit *>(out_d), nullptr, any ? out_d : nullptr, m, any);
         if (rc) return rc;
         RT_CUDA_CTX(ctx, cudaEventRecord(ctx->ev_traced[s], ts));
         RT_CUDA_CTX(ctx, cudaStreamWaitEvent(ctx->d2h, ctx->ev_traced[s], 0));
@@ -977,8 +968,16 @@ extern "C" rt_status rt_trace_stats(rt_context *ctx, rt_stream stream, uint64_t 
     if (!ctx || !accel || !counters || (n && !rays)) return set_error(ctx, RT_ERR_INVALID_ARG, "rt_trace_stats: null argument");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     RT_CUDA_CTX(ctx, cudaMemsetAsync(counters, 0, 16, st));
-    // No hit output: the counters are the result.
-    return launch_batch(ctx, st, accel, rays, nullptr, nullptr, nullptr, n, any_hit != 0, counters);
+    if (n == 0) return RT_OK;
+    uint32_t blocks = 8u * (uint32_t)ctx->sm_count;
+    const uint32_t need = (n + kTraceThreads - 1) / kTraceThreads;
+    if (blocks > need) blocks = need;
+    const uint8_t *A = reinterpret_cast<const uint8_t *>(accel);
+    const float4 *R = reinterpret_cast<const float4 *>(rays);
+    if (any_hit) k_trace_stats<true><<<blocks, kTraceThreads, 0, st>>>(A, R, n, counters, ctx->d_err);
+    else k_trace_stats<false><<<blocks, kTraceThreads, 0, st>>>(A, R, n, counters, ctx->d_err);
+    RT_CUDA_CTX(ctx, cudaGetLastError());
+    return RT_OK;
 }
 
 extern "C" rt_status rt_trace_rays(rt_context *ctx, rt_stream stream, const rt_pipeline *p, const rt_sbt *sbt,

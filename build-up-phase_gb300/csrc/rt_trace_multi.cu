@@ -16,18 +16,18 @@ namespace {
 template <bool ANY, int THREADS, bool MIXED = false>
 void launch_ring(const BatchArgs &a, uint32_t ring, uint32_t blocks, cudaStream_t st) {
     switch (ring) {
-    case 8: k_trace_blas<ANY, false, true, THREADS, 8, MIXED><<<blocks, THREADS, 0, st>>>(a); break;
-    case 32: k_trace_blas<ANY, false, true, THREADS, 32, MIXED><<<blocks, THREADS, 0, st>>>(a); break;
-    default: k_trace_blas<ANY, false, true, THREADS, 16, MIXED><<<blocks, THREADS, 0, st>>>(a); break;
+    case 8: k_trace_blas<ANY, true, THREADS, 8, MIXED><<<blocks, THREADS, 0, st>>>(a); break;
+    case 32: k_trace_blas<ANY, true, THREADS, 32, MIXED><<<blocks, THREADS, 0, st>>>(a); break;
+    default: k_trace_blas<ANY, true, THREADS, 16, MIXED><<<blocks, THREADS, 0, st>>>(a); break;
     }
 }
 
 template <bool ANY, int THREADS, bool MIXED = false>
 const void *kernel_ring(uint32_t ring) {
     switch (ring) {
-    case 8: return (const void *)k_trace_blas<ANY, false, true, THREADS, 8, MIXED>;
-    case 32: return (const void *)k_trace_blas<ANY, false, true, THREADS, 32, MIXED>;
-    default: return (const void *)k_trace_blas<ANY, false, true, THREADS, 16, MIXED>;
+    case 8: return (const void *)k_trace_blas<ANY, true, THREADS, 8, MIXED>;
+    case 32: return (const void *)k_trace_blas<ANY, true, THREADS, 32, MIXED>;
+    default: return (const void *)k_trace_blas<ANY, true, THREADS, 16, MIXED>;
     }
 }
 

@@ -12,11 +12,12 @@
 // and keeps its traversal stack in a shared-memory ring of RING entries whose
 // bottom spills to local memory.
 //
-// Visiting order (identical in the CPU restatement, so hits and statistics
-// agree exactly): a node's leaf records first, in ascending record order,
-// then its internal children in ascending (slot ^ ray octant); remaining
-// siblings are pushed as one group.  Closest hit = smallest t, ties broken by
-// the smallest triangle index.
+// Visiting order: internal children in ascending (slot ^ ray octant), the
+// remaining siblings pushed as one group; the leaf records met on the way are
+// tested in batches (see the triangle queue below).  Closest hit = smallest t,
+// ties broken by the smallest triangle index, so the result does not depend
+// on when a record is tested and equals the CPU restatement's, which tests a
+// node's records as it visits the node.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -73,7 +74,6 @@ struct BatchArgs {
     uint32_t refill;         // refill when at least this many lanes are idle
     uint32_t *counter;
     uint32_t *err;
-    unsigned long long *stats;
     const uint32_t *n_dev;   // when set: the ray count, read on the device
     uint32_t out_rec;        // closest hit: write the leaf-record index
     // mixed launches: a second queue of any-hit rays after the closest-hit
@@ -84,25 +84,53 @@ struct BatchArgs {
     uint32_t n2;
 };
 
+// ---------------------------------------------------------------------------
+// Triangle queue
+// ---------------------------------------------------------------------------
+// A node visit leaves a lane 0.2-0.3 triangles to test on average, so testing
+// them on the spot runs the triangle test with two or three of a warp's 32
+// lanes.  Instead each lane appends the leaf records it meets to its warp's
+// queue in shared memory (record index and lane) and walks on; once there are
+// as many entries as lanes with a ray, the whole warp tests them, one entry per
+// lane with the owner's ray read by shuffles, and hands the hits back to their
+// owners.  The closest hit of a ray is the least (t, triangle) of the triangles
+// tested, whatever their order; a ray walks a few nodes more because its far
+// limit shrinks a few visits later.  A lane keeps its ray until its last entry
+// has been tested.  1M soup, 4.15M primary and incoherent rays: 28.6 entries
+// per batch, 18.4 nodes and 4.4 triangles per ray against 17.7 and 4.0 when
+// every triangle is tested on the spot, 28.1 of 32 lanes walking per node step
+// (2M box, mixed launches: 27.4).  With the box test's instruction count this
+// took the launch from 1.92 to 1.68 ms (1.86 to 1.55 G warp instructions), the
+// path tracer's 2M-triangle frame of four samples from 25.7 to 23.4 ms.  What
+// bounds it now: issue slots (78 % busy) and the L1 data path (70 %: a node is
+// five 16-byte loads per lane, nearly every one a wavefront of its own).
+constexpr uint32_t kTriQueue = 64;  // entries per warp: below 32 before an append of at most 32
+constexpr int kTriDrain = 8;   // lanes waiting for their entries alone before a partial batch is tested
+
+__device__ __forceinline__ float4 xyz_of(const uint4 &q) {
+    return make_float4(__uint_as_float(q.x), __uint_as_float(q.y), __uint_as_float(q.z), 0.f);
+}
+
 // MIXED: one launch over two queues -- the closest-hit rays (rays, n_dev;
 // results to hits) and then the any-hit rays (rays2, n_dev2; results to
 // occluded) -- each ray walked exactly as in a launch of its own kind; the
 // path tracer traces a depth's shadow rays and the next depth's extension
 // rays together, so the two share one launch tail.
 // Register budget: the closest-hit and mixed single-structure kernels fit
-// nine 128-thread blocks per SM (56 registers; 36 warps against 32 at 64
-// registers: 2,093 -> 2,111 M rays/s on the 1M soup, 6.72 -> 6.58 ms per
-// path-traced sample).  The any-hit and multi-scene kernels keep eight
-// blocks and 64 registers: any-hit shadow rays run 1,287 M rays/s there
-// against 1,202 at nine blocks, and the multi-scene kernels spill at 56.
-// The box test pairs the z planes too (isect_node<true>) where it pays: in
-// the 64-register kernels, and in the mixed kernel despite 20 bytes of spill
-// (path tracer 6.30 -> 6.23 ms per sample; the closest-hit kernel loses 2 %
-// with it).
-template <bool ANY, bool STATS, bool MULTI, int THREADS, int RING, bool MIXED = false>
+// nine 128-thread blocks per SM (56 registers; at eight blocks and 64
+// registers the 1M soup's rays take 1.71 instead of 1.68 ms, the path-traced
+// frame 23.3 instead of 22.6); the any-hit and multi-scene kernels keep eight
+// blocks and 64 registers.
+template <bool ANY, bool MULTI, int THREADS, int RING, bool MIXED = false>
 __global__ void __launch_bounds__(THREADS, ((MULTI || ANY) ? 1024 : 1152) / THREADS) k_trace_blas(const BatchArgs a) {
     static_assert((RING & (RING - 1)) == 0 && RING <= kMaxDepth, "RING is a power of two");
     __shared__ uint2 s_stack[RING][THREADS];
+    __shared__ uint32_t s_qrec[THREADS / 32][kTriQueue];
+    __shared__ uint8_t s_qlane[THREADS / 32][kTriQueue];
+    // per lane, touched once per ray or improved hit: u, v, leaf record and
+    // triangle of the best hit so far; the ray's index
+    __shared__ uint4 s_best[ANY ? 1 : THREADS];
+    __shared__ uint32_t s_ray[THREADS];
     const uint4 *nodes = nullptr, *prims = nullptr;
     // A tree walk visits each node at most once: more visits, or a node index
     // past the end, can only come from a corrupt structure.
@@ -116,149 +144,132 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY) ? 1024 : 1152) / THRE
         empty = hd->prim_count == 0;
         max_visits = hd->node_count;
     }
+    constexpr uint32_t kFull = 0xffffffffu;
     const int tid = threadIdx.x, lane = tid & 31;
+    uint32_t *qrec = s_qrec[tid >> 5];
+    uint8_t *qlane = s_qlane[tid >> 5];
 
-    bool active = false, exhausted = false;
-    uint32_t ray_idx = 0;
+    bool have_ray = false, exhausted = false, pending = false;
     Ray r;
-    float tmin = 0.f;
-    Hit h;
-    h.t = 0.f; h.u = 0.f; h.v = 0.f; h.rec = kNone; h.tri = kNone; h.inst = 0; h.found = false;
+    r.o[0] = r.o[1] = r.o[2] = 0.f;
+    r.sx = r.sy = r.sz = 0.f;
+    r.prio = r.kxyz = 0u;
+    float tmin = 0.f, tbest = 0.f;  // tbest: the ray's far limit, then its best hit
+    bool found = false;
     uint32_t node = 0;
-    bool pending = false;
-    uint2 g = make_uint2(0u, 0u);
     int sp = 0, lo = 0;
     uint2 spill[kMaxDepth];
-    unsigned long long n_nodes = 0, n_tris = 0;
     uint32_t visits = 0;
+    uint32_t head = 0, tail = 0;  // queue positions tested / appended so far (the same in every lane)
+    uint32_t last = ~0u;          // position of this lane's latest entry
     const uint32_t n1 = a.n_dev ? min(*a.n_dev, a.n) : a.n;
     const uint32_t n_rays = MIXED ? n1 + min(*a.n_dev2, a.n2) : n1;
     bool any_ray = ANY;  // this lane's ray is an any-hit ray
+    // Fewer rays than lanes: each warp takes its share of them in as few lanes
+    // as that needs, so that the rays' walks do not wait on one another.
+    const uint32_t warps = gridDim.x * (THREADS / 32);
+    const uint32_t share = n_rays / warps + 1u;
+    const uint32_t lanes = share >= 32u ? kFull : (1u << share) - 1u;
+    const int refill = (int)min(a.refill, min(share, 32u));
 
     for (;;) {
-        // ---- refill idle lanes from the global counter
-        const uint32_t idle = __ballot_sync(0xffffffffu, !active);
-        if (!exhausted && __popc(idle) >= (int)a.refill) {
-            const uint32_t cnt = __popc(idle);
-            uint32_t base = 0;
-            if (lane == 0) base = atomicAdd(a.counter, cnt);
-            base = __shfl_sync(0xffffffffu, base, 0);
-            if (base + cnt >= n_rays) exhausted = true;
-            if (!active) {
-                uint32_t idx = base + __popc(idle & ((1u << lane) - 1u));
-                if (idx < n_rays) {
-                    const float4 *ray_src = a.rays;
-                    const uint32_t *scene_src = a.ray_scene;
-                    if (MIXED) {
-                        any_ray = idx >= n1;
-                        if (any_ray) {
-                            idx -= n1;
-                            ray_src = a.rays2;
-                            scene_src = a.ray_scene2;
-                        }
+        // ---- lanes whose walk and tests are done: write the result, refill
+        const bool waiting = (int)(last - head) >= 0;
+        uint32_t done = __ballot_sync(kFull, !pending && !waiting);
+        if (done == kFull || (!exhausted && __popc(done & lanes) >= refill)) {
+            if (have_ray && !pending && !waiting) {
+                have_ray = false;
+                const uint32_t ray_idx = s_ray[tid];
+                if (ANY || (MIXED && any_ray)) {
+                    if (a.occluded) a.occluded[ray_idx] = found ? 1u : 0u;
+                } else {
+                    uint4 best = make_uint4(0u, 0u, kNone, kNone);
+                    if (found) best = s_best[tid];
+                    const float4 out = make_float4(found ? tbest : kInf, __uint_as_float(a.out_rec ? best.z : best.w),
+                                                   __uint_as_float(best.x), __uint_as_float(best.y));
+                    if (a.hits) a.hits[ray_idx] = out;
+                    if (!MULTI && a.hits_ext) {
+                        rt_hit_ext x;
+                        x.t = out.x; x.u = out.z; x.v = out.w;
+                        x.instance_id = found ? 0u : kNone;
+                        x.custom_index = 0;
+                        x.geometry_index = found ? ldg4(prims + (size_t)best.z * 3u + 1).w : 0u;
+                        x.primitive_id = found ? ldg4(prims + (size_t)best.z * 3u + 2).w : kNone;
+                        x.sbt_record = x.geometry_index;
+                        a.hits_ext[ray_idx] = x;
                     }
-                    if (MULTI) {
-                        const uint32_t s = __ldg(scene_src + idx);
-                        if (s < a.n_scenes) {
-                            const uint4 *tv = reinterpret_cast<const uint4 *>(a.scenes + s);
-                            const uint4 t0 = ldg4(tv), t1 = ldg4(tv + 1);
-                            nodes = reinterpret_cast<const uint4 *>(((uint64_t)t0.y << 32) | t0.x);
-                            prims = reinterpret_cast<const uint4 *>(((uint64_t)t0.w << 32) | t0.z);
-                            max_visits = t1.x;
-                            empty = t1.x == 0u || t1.y == 0u;
-                        } else {
-                            report_error(a.err, RT_ERR_BOUNDS, 0x77000000u | (s & 0xffffffu));
-                            empty = true;
-                        }
-                    }
-                    const float4 r0 = __ldg(ray_src + 2u * idx), r1 = __ldg(ray_src + 2u * idx + 1u);
-                    const float o[3] = {r0.x, r0.y, r0.z}, d[3] = {r1.x, r1.y, r1.z};
-                    ray_setup(r, o, d);
-                    tmin = r0.w;
-                    h.t = r1.w; h.u = 0.f; h.v = 0.f; h.rec = kNone; h.tri = kNone; h.found = false;
-                    ray_idx = idx;
-                    active = true;
-                    node = 0;          // start at the root
-                    visits = 0;
-                    pending = !empty;  // an empty structure resolves as a miss
-                    g = make_uint2(0u, 0u);
-                    sp = 0;
-                    lo = 0;
                 }
             }
-        }
-        if (!__any_sync(0xffffffffu, active)) {
-            if (exhausted) break;
-            continue;
-        }
-        // ---- traversal steps until too many lanes are idle
-        for (;;) {
-            if (active) {
-                bool finish = false;
-                if (pending && (visits >= max_visits || node >= max_visits)) {
-                    report_error(a.err, RT_ERR_BOUNDS, 0x76000000u | ray_idx);
-                    pending = false;
-                    finish = true;
-                }
-                if (pending) {
-                    pending = false;
-                    ++visits;
-                    NodeWords nd = load_node(nodes, node);
-                    uint32_t nh, ph;
-                    isect_node<ANY || MULTI || MIXED>(r, nd, tmin, h.t, nh, ph);
-                    if (STATS) n_nodes++;
-                    const uint32_t pbase = nd.w1.y;
-                    while (ph) {
-                        const uint32_t i = __ffs(ph) - 1;
-                        ph &= ph - 1u;
-                        const uint4 *rec = prims + (size_t)(pbase + i) * 3u;
-                        const uint4 q0 = ldg4(rec), q1 = ldg4(rec + 1), q2 = ldg4(rec + 2);
-                        if (STATS) n_tris++;
-                        float t, u, v;
-                        if (!isect_tri(r,
-                                       make_float4(__uint_as_float(q0.x), __uint_as_float(q0.y),
-                                                   __uint_as_float(q0.z), 0.f),
-                                       make_float4(__uint_as_float(q1.x), __uint_as_float(q1.y),
-                                                   __uint_as_float(q1.z), 0.f),
-                                       make_float4(__uint_as_float(q2.x), __uint_as_float(q2.y),
-                                                   __uint_as_float(q2.z), 0.f),
-                                       tmin, h.t, t, u, v))
-                            continue;
-                        if (ANY || (MIXED && any_ray)) {
-                            h.t = t; h.found = true;
-                            finish = true;
-                            break;
-                        }
-                        if (t < h.t || (t == h.t && q0.w < h.tri)) {
-                            h.t = t; h.u = u; h.v = v; h.rec = pbase + i; h.tri = q0.w; h.found = true;
-                        }
+            if (exhausted) break;  // every lane is done
+            const uint32_t want = done & lanes;
+            const uint32_t cnt = __popc(want);
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(a.counter, cnt);
+            base = __shfl_sync(kFull, base, 0);
+            if (base + cnt >= n_rays) exhausted = true;
+            uint32_t idx = base + __popc(want & ((1u << lane) - 1u));
+            if (((want >> lane) & 1u) && idx < n_rays) {
+                const float4 *ray_src = a.rays;
+                const uint32_t *scene_src = a.ray_scene;
+                if (MIXED) {
+                    any_ray = idx >= n1;
+                    if (any_ray) {
+                        idx -= n1;
+                        ray_src = a.rays2;
+                        scene_src = a.ray_scene2;
                     }
-                    g = make_uint2(nd.w1.x, nh | ((nd.w0.w >> 24) << 8));
                 }
-                // ---- next node: from the current group, else pop
-                while (!finish) {
-                    if (g.y & 0xffu) {
-                        const uint32_t k = __ffs(g.y & 0xffu) - 1;
-                        g.y &= ~(1u << k);
-                        const uint32_t s = k ^ r.oct;
-                        node = g.x + __popc((g.y >> 8) & ((1u << s) - 1u));
-                        pending = true;
-                        if (g.y & 0xffu) {
-                            if (sp >= kMaxDepth) {
-                                report_error(a.err, RT_ERR_BOUNDS, 0x72000000u | ray_idx);
-                                finish = true;
-                                break;
-                            }
-                            if (sp - lo == RING) {
-                                spill[lo] = s_stack[lo & (RING - 1)][tid];
-                                ++lo;
-                            }
-                            s_stack[sp & (RING - 1)][tid] = g;
-                            ++sp;
-                        }
-                        break;
+                if (MULTI) {
+                    const uint32_t s = __ldg(scene_src + idx);
+                    if (s < a.n_scenes) {
+                        const uint4 *tv = reinterpret_cast<const uint4 *>(a.scenes + s);
+                        const uint4 t0 = ldg4(tv), t1 = ldg4(tv + 1);
+                        nodes = reinterpret_cast<const uint4 *>(((uint64_t)t0.y << 32) | t0.x);
+                        prims = reinterpret_cast<const uint4 *>(((uint64_t)t0.w << 32) | t0.z);
+                        max_visits = t1.x;
+                        empty = t1.x == 0u || t1.y == 0u;
+                    } else {
+                        report_error(a.err, RT_ERR_BOUNDS, 0x77000000u | (s & 0xffffffu));
+                        empty = true;
                     }
-                    if (sp == 0) { finish = true; break; }
+                }
+                const float4 r0 = __ldg(ray_src + 2u * idx), r1 = __ldg(ray_src + 2u * idx + 1u);
+                const float o[3] = {r0.x, r0.y, r0.z}, d[3] = {r1.x, r1.y, r1.z};
+                ray_setup(r, o, d);
+                tmin = r0.w;
+                tbest = r1.w;
+                found = false;
+                s_ray[tid] = idx;
+                have_ray = true;
+                node = 0;          // start at the root
+                visits = 0;
+                pending = !empty;  // an empty structure resolves as a miss
+                sp = 0;
+                lo = 0;
+                last = head - 1u;
+            }
+            done = __ballot_sync(kFull, !pending && !((int)(last - head) >= 0));
+            if (done == kFull) continue;
+        }
+        const int busy = 32 - __popc(done);  // lanes with a walk or tests to go
+        // a partial batch once too many of them wait for their entries
+        const int walking = __popc(__ballot_sync(kFull, pending));
+        const bool drain = walking == 0 || busy - walking >= kTriDrain;
+
+        // ---- one node per lane, then the lane's next node
+        uint32_t ph = 0u, pbase = 0u;
+        if (pending) {
+            pending = false;
+            if (visits >= max_visits || node >= max_visits) {
+                report_error(a.err, RT_ERR_BOUNDS, 0x76000000u | s_ray[tid]);
+            } else {
+                ++visits;
+                const NodeWords nd = load_node(nodes, node);
+                const uint32_t hits = isect_node(r, nd, tmin, tbest);
+                ph = leaf_records(nd, hits);
+                pbase = nd.w1.y;
+                uint2 g = child_group(nd, hits);
+                if (!group_left(g) && sp > 0) {
                     --sp;
                     if (sp >= lo) {
                         g = s_stack[sp & (RING - 1)][tid];
@@ -267,43 +278,109 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY) ? 1024 : 1152) / THRE
                         lo = sp;
                     }
                 }
-                if (finish) {
-                    // ---- write the result
-                    if (ANY || (MIXED && any_ray)) {
-                        if (a.occluded) a.occluded[ray_idx] = h.found ? 1u : 0u;
-                    } else {
-                        float4 out;
-                        if (h.found) out = make_float4(h.t, __uint_as_float(a.out_rec ? h.rec : h.tri), h.u, h.v);
-                        else out = make_float4(kInf, __uint_as_float(kNone), 0.f, 0.f);
-                        if (a.hits) a.hits[ray_idx] = out;
-                        if (!MULTI && a.hits_ext) {
-                            rt_hit_ext x;
-                            x.t = out.x; x.u = out.z; x.v = out.w;
-                            x.instance_id = h.found ? 0u : kNone;
-                            x.custom_index = 0;
-                            x.geometry_index = h.found ? ldg4(prims + (size_t)h.rec * 3u + 1).w : 0u;
-                            x.primitive_id = h.found ? ldg4(prims + (size_t)h.rec * 3u + 2).w : kNone;
-                            x.sbt_record = x.geometry_index;
-                            a.hits_ext[ray_idx] = x;
+                if (group_left(g)) {
+                    node = take_child(g, r.prio);
+                    pending = true;
+                    if (group_left(g)) {
+                        if (sp >= kMaxDepth) {
+                            report_error(a.err, RT_ERR_BOUNDS, 0x72000000u | s_ray[tid]);
+                            pending = false;
+                        } else {
+                            if (sp - lo == RING) {
+                                spill[lo] = s_stack[lo & (RING - 1)][tid];
+                                ++lo;
+                            }
+                            s_stack[sp & (RING - 1)][tid] = g;
+                            ++sp;
                         }
                     }
-                    active = false;
-                    pending = false;
                 }
             }
-            const uint32_t act = __ballot_sync(0xffffffffu, active);
-            if (act == 0u) break;
-            if (!exhausted && (uint32_t)__popc(~act) >= a.refill) break;
         }
-    }
-    if (STATS) {
-        for (int o = 16; o > 0; o >>= 1) {
-            n_nodes += __shfl_xor_sync(0xffffffffu, n_nodes, o);
-            n_tris += __shfl_xor_sync(0xffffffffu, n_tris, o);
-        }
-        if (lane == 0) {
-            atomicAdd(a.stats, n_nodes);
-            atomicAdd(a.stats + 1, n_tris);
+
+        // ---- append the leaf records met, test a batch when there is one
+        for (;;) {
+            const uint32_t m = __ballot_sync(kFull, ph != 0u);
+            if (m == 0u && !drain) break;
+            if (ph) {
+                const uint32_t i = __ffs(ph) - 1;
+                ph &= ph - 1u;
+                last = tail + __popc(m & ((1u << lane) - 1u));
+                qrec[last & (kTriQueue - 1u)] = pbase + i;
+                qlane[last & (kTriQueue - 1u)] = (uint8_t)lane;
+            }
+            tail += __popc(m);
+            const int cnt = (int)(tail - head);
+            if (cnt >= busy || (m == 0u && cnt > 0)) {
+                const uint32_t k = min(cnt, 32);
+                __syncwarp();
+                const uint32_t qi = (head + (uint32_t)lane) & (kTriQueue - 1u);
+                const bool have = (uint32_t)lane < k;
+                const uint32_t src = have ? (uint32_t)qlane[qi] : (uint32_t)lane;
+                const uint32_t rec = have ? qrec[qi] : 0u;
+                __syncwarp();  // read before the next append reuses the slots
+                head += k;
+                Ray tr;
+                tr.o[0] = __shfl_sync(kFull, r.o[0], src);
+                tr.o[1] = __shfl_sync(kFull, r.o[1], src);
+                tr.o[2] = __shfl_sync(kFull, r.o[2], src);
+                tr.sx = __shfl_sync(kFull, r.sx, src);
+                tr.sy = __shfl_sync(kFull, r.sy, src);
+                tr.sz = __shfl_sync(kFull, r.sz, src);
+                tr.kxyz = __shfl_sync(kFull, r.kxyz, src);
+                const float t_lo = __shfl_sync(kFull, tmin, src), t_hi = __shfl_sync(kFull, tbest, src);
+                const uint4 *pr = prims;
+                if (MULTI)
+                    pr = reinterpret_cast<const uint4 *>(
+                        __shfl_sync(kFull, (unsigned long long)reinterpret_cast<uintptr_t>(prims), src));
+                float t = 0.f, u = 0.f, v = 0.f;
+                uint32_t tri = kNone;
+                bool hit = false;
+                if (have) {
+                    const uint4 *p = pr + (size_t)rec * 3u;
+                    const uint4 q0 = ldg4(p), q1 = ldg4(p + 1), q2 = ldg4(p + 2);
+                    tri = q0.w;
+                    hit = isect_tri(tr, xyz_of(q0), xyz_of(q1), xyz_of(q2), t_lo, t_hi, t, u, v);
+                }
+                if (ANY) {
+                    const uint32_t fm = __reduce_or_sync(kFull, hit ? 1u << src : 0u);
+                    if ((fm >> lane) & 1u) {
+                        found = true;
+                        pending = false;
+                        ph = 0u;
+                    }
+                } else {
+                    // each owner compares its hits in turn and then takes the
+                    // winner's coordinates
+                    int win = -1;
+                    uint32_t best_tri = 0u;
+                    for (uint32_t hm = __ballot_sync(kFull, hit); hm; hm &= hm - 1u) {
+                        const int l = __ffs(hm) - 1;
+                        const uint32_t s = __shfl_sync(kFull, src, l), ht = __shfl_sync(kFull, tri, l);
+                        const float tt = __shfl_sync(kFull, t, l);
+                        if ((uint32_t)lane == s && !(MIXED && any_ray && found) && tt <= tbest) {
+                            if (tt < tbest || !found || ht < (win < 0 ? s_best[tid].w : best_tri)) {
+                                tbest = tt;
+                                best_tri = ht;
+                                win = l;
+                                found = true;
+                            }
+                        }
+                    }
+                    const uint32_t from = win < 0 ? (uint32_t)lane : (uint32_t)win;
+                    const float bu = __shfl_sync(kFull, u, from), bv = __shfl_sync(kFull, v, from);
+                    const uint32_t br = __shfl_sync(kFull, rec, from);
+                    if (win >= 0) {
+                        if (MIXED && any_ray) {
+                            pending = false;
+                            ph = 0u;
+                        } else {
+                            s_best[tid] = make_uint4(__float_as_uint(bu), __float_as_uint(bv), br, best_tri);
+                        }
+                    }
+                }
+            }
+            if (m == 0u) break;
         }
     }
 }
