@@ -187,6 +187,22 @@ __global__ void k_empty_root(uint8_t *accel) {
 // prep
 // ---------------------------------------------------------------------------
 
+// Records of consecutive threads, 48 bytes each, leave through shared memory as
+// whole lines (a thread's own three 16-byte stores are 48 bytes apart from its
+// neighbour's: twelve lines per store instruction).  Called by every thread of
+// a 256-thread block; `count` records from dst on.
+constexpr uint32_t kRecThreads = 256;
+__device__ __forceinline__ void store_records(uint4 *dst, const uint4 (&rec)[3], uint4 *s_rec, uint32_t count) {
+#pragma unroll
+    for (int w = 0; w < 3; ++w) s_rec[threadIdx.x * 3u + w] = rec[w];
+    __syncthreads();
+#pragma unroll
+    for (uint32_t w = 0; w < 3u; ++w) {
+        const uint32_t e = w * kRecThreads + threadIdx.x;
+        if (e < count * 3u) dst[e] = s_rec[e];
+    }
+}
+
 // Leaf record and box of triangle p of geometry g (build-input index gi):
 // the three vertices (transformed when the geometry has a transform) in .xyz
 // and the ids in .w; NaN vertices and the empty box for a triangle that is
@@ -195,28 +211,37 @@ __global__ void k_empty_root(uint8_t *accel) {
 __device__ bool tri_record(const GeomParams &gp, uint32_t g, uint32_t p, uint32_t gi, uint4 *r, Box &b,
                            uint32_t *err, uint32_t *hdr_status) {
     const rt_geometry_triangles &G = gp.g[g];
+    // the three indices in one round of loads, the nine coordinates in the
+    // next (a check between them would put them in six)
+    uint32_t idx[3];
     float v[3][3];
     bool ok = true;
-    for (int k = 0; k < 3; ++k) {
-        uint32_t idx = G.index_type == RT_INDEX_UINT32 ? G.indices[3u * p + (uint32_t)k] : 3u * p + (uint32_t)k;
-        if (idx > G.max_vertex) {
-            ok = false;
-            report_error(err, RT_ERR_BOUNDS, gi);
-            if (hdr_status) atomicCAS(hdr_status, 0u, (uint32_t)(-RT_ERR_BOUNDS));
-            break;
+#pragma unroll
+    for (uint32_t k = 0; k < 3u; ++k) {
+        idx[k] = G.index_type == RT_INDEX_UINT32 ? __ldg(G.indices + 3u * p + k) : 3u * p + k;
+        ok = ok && idx[k] <= G.max_vertex;
+    }
+    if (ok) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const float *src = reinterpret_cast<const float *>(reinterpret_cast<const uint8_t *>(G.vertices) +
+                                                               (size_t)idx[k] * G.vertex_stride);
+#pragma unroll
+            for (int a = 0; a < 3; ++a) v[k][a] = __ldg(src + a);
         }
-        const float *src = reinterpret_cast<const float *>(reinterpret_cast<const uint8_t *>(G.vertices) +
-                                                           (size_t)idx * G.vertex_stride);
-        float pt[3] = {src[0], src[1], src[2]};
         if (G.transform) {
-            const float *m = &G.transform->m[0][0];
             float mm[12];
 #pragma unroll
-            for (int q = 0; q < 12; ++q) mm[q] = __ldg(m + q);
-            xform_point(mm, pt, v[k]);
-        } else {
-            v[k][0] = pt[0]; v[k][1] = pt[1]; v[k][2] = pt[2];
+            for (int q = 0; q < 12; ++q) mm[q] = __ldg(&G.transform->m[0][0] + q);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const float pt[3] = {v[k][0], v[k][1], v[k][2]};
+                xform_point(mm, pt, v[k]);
+            }
         }
+    } else {
+        report_error(err, RT_ERR_BOUNDS, gi);
+        if (hdr_status) atomicCAS(hdr_status, 0u, (uint32_t)(-RT_ERR_BOUNDS));
     }
     if (ok)
         for (int k = 0; k < 3; ++k)
@@ -238,11 +263,13 @@ __device__ bool tri_record(const GeomParams &gp, uint32_t g, uint32_t p, uint32_
     return ok;
 }
 
-__global__ void __launch_bounds__(256) k_prep_tris(const GeomParams gp, uint32_t n, uint4 *__restrict__ recs,
+__global__ void __launch_bounds__(kRecThreads) k_prep_tris(const GeomParams gp, uint32_t n, uint4 *__restrict__ recs,
                                                     float *__restrict__ boxes, int32_t *cbounds, uint32_t *err,
                                                     uint32_t *hdr_status) {
-    uint32_t gi = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ uint4 s_rec[kRecThreads * 3];
+    const uint32_t base = blockIdx.x * kRecThreads, gi = base + threadIdx.x;
     int32_t cmin[3] = {INT32_MAX, INT32_MAX, INT32_MAX}, cmax[3] = {INT32_MIN, INT32_MIN, INT32_MIN};
+    uint4 rec[3] = {};
     if (gi < n) {
         // geometry g with table[g] <= gi < table[g+1]
         uint32_t lo = 0, hi = gp.n_geoms;
@@ -253,7 +280,7 @@ __global__ void __launch_bounds__(256) k_prep_tris(const GeomParams gp, uint32_t
         const uint32_t g = lo;
         const uint32_t p = gi - gp.table[g];
         Box b;
-        const bool ok = tri_record(gp, g, p, gi, recs + (size_t)gi * 3u, b, err, hdr_status);
+        const bool ok = tri_record(gp, g, p, gi, rec, b, err, hdr_status);
         store_box(boxes, gi, b);
         if (ok)
             for (int a = 0; a < 3; ++a) {
@@ -262,6 +289,7 @@ __global__ void __launch_bounds__(256) k_prep_tris(const GeomParams gp, uint32_t
                 cmax[a] = o;
             }
     }
+    store_records(recs + (size_t)base * 3u, rec, s_rec, n - base < kRecThreads ? n - base : kRecThreads);
     block_minmax_atomic(cbounds, cmin, cmax);
 }
 
@@ -662,29 +690,6 @@ __device__ __forceinline__ uint4 frame_word(const QFrame &f, uint32_t imask) {
     const uint32_t w = ((uint32_t)(uint8_t)(int8_t)f.e[0]) | ((uint32_t)(uint8_t)(int8_t)f.e[1] << 8) |
                        ((uint32_t)(uint8_t)(int8_t)f.e[2] << 16) | (imask << 24);
     return make_uint4(__float_as_uint(f.p[0]), __float_as_uint(f.p[1]), __float_as_uint(f.p[2]), w);
-}
-
-// Words 0, 2, 3, 4 of a wide node from its box and its slots' boxes: the
-// child boxes as six byte planes (lo x, lo y, lo z, hi x, hi y, hi z), byte s
-// of a plane for slot s.  Used by the refit; the build's phase A writes the
-// same bytes one slot per lane.
-__device__ void encode_node(const Box &node, const Box sbox[8], const bool used[8], uint32_t imask, uint4 *o) {
-    const QFrame f = node_frame(node);
-    uint32_t q[12] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
-#pragma unroll
-    for (int s = 0; s < 8; ++s) {
-        uint32_t ql[3], qh[3];
-        quantise_child(f, used[s], sbox[s], ql, qh);
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            q[2 * a + (s >> 2)] |= ql[a] << (8 * (s & 3));
-            q[6 + 2 * a + (s >> 2)] |= qh[a] << (8 * (s & 3));
-        }
-    }
-    o[0] = frame_word(f, imask);
-    o[2] = make_uint4(q[0], q[1], q[2], q[3]);
-    o[3] = make_uint4(q[4], q[5], q[6], q[7]);
-    o[4] = make_uint4(q[8], q[9], q[10], q[11]);
 }
 
 // ---------------------------------------------------------------------------
@@ -1329,13 +1334,14 @@ int run_build(rt_context *ctx, cudaStream_t st, const BuildCall &bc, const GeomP
 // breadth-first order (every child after its parent); a node's exact box is
 // the union of its slots' boxes -- the union of its primitives' boxes, as in
 // the build, since min/max in a total order do not depend on grouping -- and
-// is quantised by the build's encode_node.  The nodes are walked bottom-up:
-// one thread starts at each node without internal children, and the last of
-// a parent's children to arrive (an atomic counter per node) goes on to the
-// parent.
+// is quantised as the build quantises it.
+//
+// Two launches: the records with their boxes, one block finding the levels of
+// the tree beside them; then the nodes, a level at a time from the bottom,
+// one thread per node and a grid barrier between levels.
 
 struct RefitLayout {
-    uint64_t flag, leaf_box, node_box, parent, arrive, total;
+    uint64_t flag, leaf_box, node_box, levels, list, total;
 };
 
 RefitLayout refit_layout(uint32_t n) {
@@ -1347,132 +1353,375 @@ RefitLayout refit_layout(uint32_t n) {
         return o;
     };
     const uint64_t cap = node_capacity_for(n);
-    L.flag = take(16);
+    L.flag = take(16);  // 256 bytes, as all are rounded up to
     L.leaf_box = take((uint64_t)n * 32u);
     L.node_box = take(cap * 32u);
-    L.parent = take(cap * 4u);
-    L.arrive = take(cap * 4u);
+    L.levels = take(cap * 4u);   // end of each level (at most one level per node)
+    L.list = take(cap * 4u);     // internal nodes by level
     L.total = off;
     return L;
 }
 
-// The structure must be the one the inputs describe.
-__global__ void k_refit_begin(const rt_accel_header *h, uint32_t kind, uint32_t n, uint32_t n_geoms, uint32_t cap,
-                              uint32_t *flag, uint32_t *err) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    const bool ok = h->magic == RT_ACCEL_MAGIC && h->kind == kind && h->prim_count == n &&
-                    (kind != RT_ACCEL_KIND_BLAS || h->geom_count == n_geoms) && h->node_capacity == cap &&
-                    h->node_count >= 1u && h->node_count <= cap && h->node_offset == RT_ACCEL_HEADER_BYTES &&
-                    h->prim_offset == RT_ACCEL_HEADER_BYTES + (uint64_t)cap * 80u;
-    *flag = ok ? 1u : 0u;
-    if (!ok) report_error(err, RT_ERR_INVALID_ARG, 0x68000000u);
+constexpr uint32_t kRefitLevels = 256;  // more levels than any build makes: a corrupt structure
+// words of the flag area: valid, number of levels, grid barrier (two words),
+// children claimed, blocks done
+constexpr uint32_t kRefitValid = 0, kRefitDepth = 1, kRefitBar = 2, kRefitKids = 4, kRefitDone = 5;
+
+// Whether the structure is the one the inputs describe.
+__device__ __forceinline__ bool refit_matches(const rt_accel_header *h, uint32_t kind, uint32_t n, uint32_t n_geoms,
+                                              uint32_t cap) {
+    return h->magic == RT_ACCEL_MAGIC && h->kind == kind && h->prim_count == n &&
+           (kind != RT_ACCEL_KIND_BLAS || h->geom_count == n_geoms) && h->node_capacity == cap && h->node_count >= 1u &&
+           h->node_count <= cap && h->node_offset == RT_ACCEL_HEADER_BYTES &&
+           h->prim_offset == RT_ACCEL_HEADER_BYTES + (uint64_t)cap * 80u;
 }
 
-__global__ void __launch_bounds__(256) k_refit_links(const uint4 *nodes, const rt_accel_header *h, uint32_t cap,
-                                                      const uint32_t *flag, uint32_t *parent, uint32_t *arrive,
-                                                      uint32_t *err) {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= cap || *flag == 0u) return;
-    const uint32_t nc = h->node_count;
-    if (k >= nc) return;
-    arrive[k] = 0u;
-    const uint32_t imask = nodes[(size_t)k * 5u].w >> 24;
-    const uint32_t cb = nodes[(size_t)k * 5u + 1u].x;
-    const uint32_t ni = (uint32_t)__popc(imask);
-    for (uint32_t j = 0; j < ni; ++j) {
-        const uint32_t c = cb + j;
-        if (c <= k || c >= nc) {  // children follow their parent in breadth-first order
-            report_error(err, RT_ERR_BOUNDS, 0x69000000u | (k & 0xffffffu));
-            return;
+// One block: the levels of the breadth-first order.  A level ends where the
+// children of the last internal node of the level above end, found by a
+// backward scan of that level.
+__device__ void refit_levels(const uint4 *nodes, uint32_t nc, uint32_t *flag, uint32_t *levels,
+                             uint32_t *err) {
+    __shared__ uint32_t s_last;
+    uint32_t lo = 0u, hi = 1u, depth = 0u;
+    for (;;) {
+        if (threadIdx.x == 0) {
+            levels[depth] = hi;
+            s_last = 0u;
         }
-        parent[c] = k;
-    }
-}
-
-__global__ void __launch_bounds__(256) k_refit_tris(const GeomParams gp, uint32_t n, uint4 *recs, float *leaf_box,
-                                                     const uint32_t *flag, uint32_t *err, uint32_t *hdr_status) {
-    const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= n || *flag == 0u) return;
-    uint4 *rec = recs + (size_t)r * 3u;
-    const uint32_t gi = rec[0].w, g = rec[1].w, p = rec[2].w;
-    Box b = box_empty();
-    if (g < gp.n_geoms && p < gp.g[g].tri_count && gi == gp.table[g] + p)
-        tri_record(gp, g, p, gi, rec, b, err, hdr_status);
-    else
-        report_error(err, RT_ERR_BOUNDS, 0x6a000000u | (r & 0xffffffu));
-    store_box(leaf_box, r, b);
-}
-
-__global__ void __launch_bounds__(256) k_refit_inst(const rt_instance *inst, uint32_t n, uint4 *recs,
-                                                     float *leaf_box, const uint32_t *flag, uint32_t *err) {
-    const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= n || *flag == 0u) return;
-    uint4 *rec = recs + (size_t)r * 5u;
-    const uint32_t i = rec[4].x;
-    Box b = box_empty();
-    if (i < n) {
-        const rt_instance I = inst[i];
-        inst_record(I, i, rec, b);
-    } else {
-        report_error(err, RT_ERR_BOUNDS, 0x6b000000u | (r & 0xffffffu));
-    }
-    store_box(leaf_box, r, b);
-}
-
-__global__ void __launch_bounds__(256) k_refit_nodes(uint4 *nodes, rt_accel_header *h, uint32_t cap, uint32_t n,
-                                                      const float *leaf_box, float *node_box, const uint32_t *parent,
-                                                      uint32_t *arrive, const uint32_t *flag, uint32_t *err) {
-    const uint32_t k0 = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k0 >= cap || *flag == 0u) return;
-    const uint32_t nc = h->node_count;
-    if (k0 >= nc || (__ldcg(nodes + (size_t)k0 * 5u).w >> 24) != 0u) return;  // start below every internal child
-    uint32_t k = k0;
-    for (int step = 0;; ++step) {
-        if (step >= 256) {  // deeper than any build makes: a corrupt structure
-            report_error(err, RT_ERR_BOUNDS, 0x6c000000u | (k & 0xffffffu));
-            return;
-        }
-        uint4 *o = nodes + (size_t)k * 5u;
-        const uint4 w0 = __ldcg(o), w1 = __ldcg(o + 1);
-        const uint32_t imask = w0.w >> 24, cb = w1.x, pb = w1.y;
-        Box sbox[8];
-        bool used[8];
-        Box node = box_empty();
-        for (int s = 0; s < 8; ++s) {
-            const uint32_t meta = ((s < 4 ? w1.z : w1.w) >> (8 * (s & 3))) & 0xffu;
-            used[s] = meta != 0u;
-            sbox[s] = box_empty();
-            if ((imask >> s) & 1u) {
-                const uint32_t c = cb + (uint32_t)__popc(imask & ((1u << s) - 1u));
-                if (c < nc) sbox[s] = load_box(node_box, c);
-                else report_error(err, RT_ERR_BOUNDS, 0x6d000000u | (k & 0xffffffu));
-            } else if (meta) {
-                const uint32_t cnt = (uint32_t)__popc(meta >> 5), first = pb + (meta & 0x1fu);
-                if (first + cnt <= n) {
-                    for (uint32_t j = 0; j < cnt; ++j) sbox[s] = box_union(sbox[s], load_box(leaf_box, first + j));
-                } else {
-                    report_error(err, RT_ERR_BOUNDS, 0x6e000000u | (k & 0xffffffu));
-                }
+        ++depth;
+        if (hi == nc) break;
+        // the last internal node of [lo, hi), as index + 1
+        uint32_t last = 0u;
+        for (uint32_t end = hi; end > lo && last == 0u; end = end - lo > blockDim.x ? end - blockDim.x : lo) {
+            __syncthreads();
+            if (threadIdx.x < end - lo) {
+                const uint32_t k = end - 1u - threadIdx.x;
+                if ((__ldcg(nodes + (size_t)k * 5u).w >> 24) != 0u) atomicMax(&s_last, k + 1u);
             }
-            if (used[s]) node = box_union(node, sbox[s]);
+            __syncthreads();
+            last = s_last;
         }
-        encode_node(node, sbox, used, imask, o);
-        store_box(node_box, k, node);
-        if (k == 0u) {
-            for (int q = 0; q < 3; ++q) { h->bounds_lo[q] = node.lo[q]; h->bounds_hi[q] = node.hi[q]; }
+        uint32_t next = 0u;
+        if (last) {
+            const uint32_t k = last - 1u;
+            next = __ldcg(nodes + (size_t)k * 5u + 1u).x +
+                   (uint32_t)__popc(__ldcg(nodes + (size_t)k * 5u).w >> 24);
+        }
+        __syncthreads();
+        if (next <= hi || next > nc || depth == kRefitLevels) {
+            if (threadIdx.x == 0) {
+                report_error(err, RT_ERR_BOUNDS, 0x69000000u | (hi & 0xffffffu));
+                flag[kRefitDepth] = 0u;
+            }
             return;
         }
-        __threadfence();  // the box is visible before the arrival is counted
-        const uint32_t p = parent[k];
-        if (p >= k) {  // the root, or a node no parent claimed
-            report_error(err, RT_ERR_BOUNDS, 0x6f000000u | (k & 0xffffffu));
-            return;
-        }
-        const uint32_t need = (uint32_t)__popc(__ldcg(nodes + (size_t)p * 5u).w >> 24);
-        if (atomicAdd(arrive + p, 1u) + 1u != need) return;
-        __threadfence();
-        k = p;
+        lo = hi;
+        hi = next;
     }
+    if (threadIdx.x == 0) flag[kRefitDepth] = depth;
+}
+
+// Leaf records and their boxes from the new inputs, one thread per record;
+// block 0 finds the levels.  Bound by memory: 62 us for 2M triangles, 250 MB of
+// DRAM traffic.
+template <bool INST>
+__global__ void __launch_bounds__(kRecThreads) k_refit_records(const GeomParams gp, const rt_instance *inst, uint32_t n,
+                                                        uint32_t cap, uint8_t *accel, float *leaf_box, uint32_t *flag,
+                                                        uint32_t *levels, uint32_t *err) {
+    rt_accel_header *h = reinterpret_cast<rt_accel_header *>(accel);
+    const bool ok = refit_matches(h, INST ? RT_ACCEL_KIND_TLAS : RT_ACCEL_KIND_BLAS, n, gp.n_geoms, cap);
+    if (blockIdx.x == 0) {
+        if (threadIdx.x == 0) {
+            flag[kRefitValid] = ok ? 1u : 0u;
+            for (uint32_t w = kRefitBar; w <= kRefitDone; ++w) flag[w] = 0u;
+            if (!ok) report_error(err, RT_ERR_INVALID_ARG, 0x68000000u);
+        }
+        if (ok)
+            refit_levels(reinterpret_cast<const uint4 *>(accel + RT_ACCEL_HEADER_BYTES), h->node_count, flag, levels,
+                         err);
+        return;
+    }
+    if (!ok) return;
+    const uint32_t base = (blockIdx.x - 1u) * blockDim.x, r = base + threadIdx.x;
+    uint4 *recs = reinterpret_cast<uint4 *>(accel + RT_ACCEL_HEADER_BYTES + (uint64_t)cap * 80u);
+    Box b = box_empty();
+    if (INST) {
+        if (r >= n) return;
+        uint4 *rec = recs + (size_t)r * 5u;
+        const uint32_t i = rec[4].x;
+        if (i < n) {
+            const rt_instance I = inst[i];
+            inst_record(I, i, rec, b);
+        } else {
+            report_error(err, RT_ERR_BOUNDS, 0x6b000000u | (r & 0xffffffu));
+        }
+        store_box(leaf_box, r, b);
+    } else {
+        // the block's records in and out as whole lines
+        __shared__ uint4 s_rec[kRecThreads * 3];
+        const uint32_t count = n - base < kRecThreads ? n - base : kRecThreads;
+        uint4 *tile = recs + (size_t)base * 3u;
+#pragma unroll
+        for (uint32_t w = 0; w < 3u; ++w) {
+            const uint32_t e = w * kRecThreads + threadIdx.x;
+            if (e < count * 3u) s_rec[e] = tile[e];
+        }
+        __syncthreads();
+        uint4 rec[3];
+#pragma unroll
+        for (int w = 0; w < 3; ++w) rec[w] = s_rec[threadIdx.x * 3u + w];
+        __syncthreads();
+        if (r < n) {
+            const uint32_t gi = rec[0].w, g = rec[1].w, p = rec[2].w;
+            if (g < gp.n_geoms && p < gp.g[g].tri_count && gi == gp.table[g] + p)
+                tri_record(gp, g, p, gi, rec, b, err, reinterpret_cast<uint32_t *>(accel) + 7);  // header status
+            else
+                report_error(err, RT_ERR_BOUNDS, 0x6a000000u | (r & 0xffffffu));
+            store_box(leaf_box, r, b);
+        }
+        store_records(tile, rec, s_rec, count);
+    }
+}
+
+// Union of boxes without NaN coordinates (triangles with one are inactive and
+// have the empty box): min and max order -0 below +0 and infinities as the
+// total order of box_union does.  Instance boxes can hold NaN.
+template <bool INST>
+__device__ __forceinline__ Box refit_union(const Box &x, const Box &y) {
+    if constexpr (INST) {
+        return box_union(x, y);
+    } else {
+        Box b;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) { b.lo[a] = fminf(x.lo[a], y.lo[a]); b.hi[a] = fmaxf(x.hi[a], y.hi[a]); }
+        return b;
+    }
+}
+
+// Internal nodes listed for level l: the spare fourth word of leaf box l, which
+// store_box left at zero (a tree has no more levels than leaf records).
+__device__ __forceinline__ uint32_t *refit_count(float *leaf_box, uint32_t l) {
+    return reinterpret_cast<uint32_t *>(leaf_box) + (size_t)l * 8u + 3u;
+}
+
+// Eight lanes per node and one slot per lane, four nodes of a warp's 32 at a
+// time.  A lane's chain is short -- its slot's box, the union by shuffles, its
+// own bytes -- where one thread for all eight slots ran through 1,400
+// instructions (5 us a level); the nodes' words were loaded a node per lane
+// and come by shuffles, and the next four nodes' boxes are fetched before the
+// current ones are used.
+struct RefitSlot {
+    uint32_t k;             // node, kNone: none
+    uint32_t imask, meta, i, cnt;
+    bool inner;
+    float4 lo, hi;          // the slot's (first) box
+};
+
+// The words of node `base + lane`, kept by its lane.
+struct RefitWords {
+    uint32_t imask, child_base, prim_base, meta_lo, meta_hi;
+};
+
+__device__ __forceinline__ RefitSlot refit_take(uint32_t &todo, uint32_t base, const RefitWords &w, uint32_t c_lo,
+                                                uint32_t c_hi, uint32_t n, const float *leaf_box,
+                                                const float *node_box, uint32_t *err) {
+    const uint32_t j = threadIdx.x & 7u, group = (threadIdx.x & 31u) >> 3;
+    uint32_t bit = 0u;
+#pragma unroll
+    for (uint32_t g = 0; g < 4u; ++g) {
+        const uint32_t low = todo & (0u - todo);
+        if (g == group) bit = low;
+        todo ^= low;
+    }
+    const uint32_t src = bit ? (uint32_t)__ffs((int)bit) - 1u : 0u;
+    RefitSlot s;
+    s.k = bit ? base + src : kNone;
+    s.imask = __shfl_sync(kFullMask, w.imask, src);
+    const uint32_t cb = __shfl_sync(kFullMask, w.child_base, src), pb = __shfl_sync(kFullMask, w.prim_base, src);
+    const uint32_t m_lo = __shfl_sync(kFullMask, w.meta_lo, src), m_hi = __shfl_sync(kFullMask, w.meta_hi, src);
+    s.meta = __byte_perm(m_lo, m_hi, j) & 0xffu;
+    s.inner = ((s.imask >> j) & 1u) != 0u;
+    s.i = s.inner ? cb + (uint32_t)__popc(s.imask & ((1u << j) - 1u)) : pb + (s.meta & 0x1fu);
+    s.cnt = s.inner ? 1u : (uint32_t)__popc(s.meta >> 5);
+    s.lo = make_float4(kInf, kInf, kInf, 0.0f);
+    s.hi = make_float4(-kInf, -kInf, -kInf, 0.0f);
+    if (bit && s.meta) {
+        if (s.i + s.cnt > (s.inner ? c_hi : n) || (s.inner && s.i < c_lo)) {
+            report_error(err, RT_ERR_BOUNDS, (s.inner ? 0x6d000000u : 0x6e000000u) | (s.k & 0xffffffu));
+            s.cnt = 0u;
+        } else {
+            const float4 *p = reinterpret_cast<const float4 *>(s.inner ? node_box : leaf_box) + (size_t)s.i * 2u;
+            s.lo = __ldcg(p);
+            s.hi = __ldcg(p + 1);
+        }
+    } else {
+        s.cnt = 0u;
+    }
+    return s;
+}
+
+// Completes the group's node; returns its internal children (lane 0 of the
+// group, else 0).
+template <bool INST>
+__device__ __forceinline__ uint32_t refit_node(const RefitSlot &s, uint4 *nodes, rt_accel_header *h,
+                                               const float *leaf_box, float *node_box) {
+    const uint32_t j = threadIdx.x & 7u;
+    Box sb;
+    sb.lo[0] = s.lo.x; sb.lo[1] = s.lo.y; sb.lo[2] = s.lo.z;
+    sb.hi[0] = s.hi.x; sb.hi[1] = s.hi.y; sb.hi[2] = s.hi.z;
+    if (s.cnt > 1u) {  // a leaf's further records, at most two
+        const Box b1 = load_box(leaf_box, s.i + 1u), b2 = load_box(leaf_box, s.i + s.cnt - 1u);
+        sb = refit_union<INST>(refit_union<INST>(sb, b1), b2);
+    }
+    Box node = sb;  // an unused slot's box is empty
+#pragma unroll
+    for (int d = 1; d < 8; d <<= 1) {
+        Box t;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            t.lo[q] = __shfl_xor_sync(kFullMask, node.lo[q], d);
+            t.hi[q] = __shfl_xor_sync(kFullMask, node.hi[q], d);
+        }
+        node = refit_union<INST>(node, t);
+    }
+    if (s.k == kNone) return 0u;
+    const QFrame f = node_frame(node);
+    uint32_t ql[3], qh[3];
+    quantise_child(f, s.meta != 0u, sb, ql, qh);
+    uint4 *o = nodes + (size_t)s.k * 5u;
+    uint8_t *bytes = reinterpret_cast<uint8_t *>(o);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        bytes[32 + 8 * q + j] = (uint8_t)ql[q];
+        bytes[56 + 8 * q + j] = (uint8_t)qh[q];
+    }
+    if (j != 0u) return 0u;
+    *o = frame_word(f, s.imask);
+    store_box(node_box, s.k, node);
+    if (s.k == 0u)
+        for (int q = 0; q < 3; ++q) { h->bounds_lo[q] = node.lo[q]; h->bounds_hi[q] = node.hi[q]; }
+    return (uint32_t)__popc(s.imask);
+}
+
+// Appends the lanes' internal nodes to their levels' lists (one atomic per
+// level a warp meets); level l's list starts at its first node's index.
+__device__ __forceinline__ void refit_append(bool want, uint32_t k, uint32_t depth, const uint32_t *s_levels,
+                                             uint32_t *list, float *leaf_box) {
+    uint32_t l = 0u;
+    if (want)
+        while (l + 1u < depth && k >= s_levels[l]) ++l;
+    for (uint32_t left = __ballot_sync(kFullMask, want); left;) {
+        const int lead = __ffs((int)left) - 1;
+        const uint32_t ll = __shfl_sync(kFullMask, l, lead);
+        const uint32_t peers = __ballot_sync(kFullMask, want && l == ll);
+        uint32_t pos = 0u;
+        if ((int)(threadIdx.x & 31u) == lead) pos = atomicAdd(refit_count(leaf_box, ll), (uint32_t)__popc(peers));
+        pos = __shfl_sync(kFullMask, pos, lead);
+        if (want && l == ll)
+            list[(ll ? s_levels[ll - 1u] : 0u) + pos + (uint32_t)__popc(peers & ((1u << (threadIdx.x & 31u)) - 1u))] = k;
+        left &= ~peers;
+    }
+}
+
+// The nodes: all without internal children first, in any order (four of five),
+// 32 per warp and step, the others listed by level; then the lists a level at
+// a time from the bottom, a grid barrier between levels.  Once the levels left
+// are small, one block goes on alone with block barriers.  2M-triangle box (11
+// levels, 643,300 nodes): 130 us -- 70 for the nodes without internal children,
+// 7-10 for each of the seven large levels (of which the barrier is about 4), 2
+// for each small one.  Before, one thread started at each childless node and
+// the last of a parent's children to arrive climbed on: 249 us, most warps
+// climbing with a lane or two; the parents' links took a launch of 13 more.
+constexpr uint32_t kRefitThreads = 512;
+constexpr uint32_t kRefitAlone = 512;  // nodes: a few steps of the block's 64 groups
+template <bool INST>
+__global__ void __launch_bounds__(kRefitThreads, INST ? 1 : 2) k_refit_nodes(uint8_t *accel, uint32_t n,
+                                                                             float *leaf_box, float *node_box,
+                                                                             uint32_t *flag, const uint32_t *levels,
+                                                                             uint32_t *list, uint32_t *err) {
+    __shared__ uint32_t s_levels[kRefitLevels];
+    const uint32_t depth = flag[kRefitDepth];
+    if (flag[kRefitValid] == 0u || depth == 0u) return;
+    for (uint32_t l = threadIdx.x; l < depth; l += blockDim.x) s_levels[l] = levels[l];
+    __syncthreads();
+    rt_accel_header *h = reinterpret_cast<rt_accel_header *>(accel);
+    uint4 *nodes = reinterpret_cast<uint4 *>(accel + RT_ACCEL_HEADER_BYTES);
+    const uint32_t nc = s_levels[depth - 1u], lane = threadIdx.x & 31u;
+    uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, warps = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t base = 32u * warp; base < nc; base += 32u * warps) {
+        const uint32_t k = base + lane;
+        RefitWords w = {1u, 0u, 0u, 0u, 0u};
+        if (k < nc) {
+            const uint4 w0 = __ldcg(nodes + (size_t)k * 5u), w1 = __ldcg(nodes + (size_t)k * 5u + 1u);
+            w = {w0.w >> 24, w1.x, w1.y, w1.z, w1.w};
+        }
+        refit_append(k < nc && w.imask != 0u, k, depth, s_levels, list, leaf_box);
+        uint32_t todo = __ballot_sync(kFullMask, w.imask == 0u);
+        if (todo == 0u) continue;
+        RefitSlot cur = refit_take(todo, base, w, 0u, 0u, n, leaf_box, node_box, err);
+        while (todo) {
+            const RefitSlot next = refit_take(todo, base, w, 0u, 0u, n, leaf_box, node_box, err);
+            refit_node<INST>(cur, nodes, h, leaf_box, node_box);
+            cur = next;
+        }
+        refit_node<INST>(cur, nodes, h, leaf_box, node_box);
+    }
+    // the levels above `top` are small enough for one block
+    uint32_t top = 0u;
+    while (top < depth && s_levels[top] - (top ? s_levels[top - 1u] : 0u) <= kRefitAlone) ++top;
+    bool alone = false;
+    uint32_t kids = 0u;
+    for (uint32_t l = depth - 1u; l-- > 0u;) {  // the last level has no internal nodes
+        if (!alone) {
+            if (!coop_sync(flag + kRefitBar, gridDim.x, err, 0x6c000000u | l)) return;
+            alone = l < top;
+            if (alone && blockIdx.x != 0u) break;
+            if (alone) {
+                warp = threadIdx.x >> 5;
+                warps = blockDim.x >> 5;
+            }
+        } else {
+            __syncthreads();
+        }
+        const uint32_t lo = l ? s_levels[l - 1u] : 0u, hi = s_levels[l];
+        const uint32_t count = min(__ldcg(refit_count(leaf_box, l)), hi - lo);
+        for (uint32_t i = 4u * warp; i < count; i += 4u * warps) {
+            // four nodes of the list, one per group; their words by the first four lanes
+            uint32_t k = kNone;
+            RefitWords w = {0u, 0u, 0u, 0u, 0u};
+            if (lane < 4u && i + lane < count) {
+                k = __ldcg(list + lo + i + lane);
+                const uint4 w0 = __ldcg(nodes + (size_t)k * 5u), w1 = __ldcg(nodes + (size_t)k * 5u + 1u);
+                w = {w0.w >> 24, w1.x, w1.y, w1.z, w1.w};
+            }
+            uint32_t todo = __ballot_sync(kFullMask, k != kNone);
+            RefitSlot s = refit_take(todo, 0u, w, hi, s_levels[l + 1u], n, leaf_box, node_box, err);
+            s.k = __shfl_sync(kFullMask, k, s.k == kNone ? 31 : (int)s.k);
+            kids += refit_node<INST>(s, nodes, h, leaf_box, node_box);
+        }
+    }
+    // the last block to finish checks that every node below the root has been
+    // claimed by a parent
+    kids = __reduce_add_sync(kFullMask, kids);
+    if (lane == 0u && kids) atomicAdd(flag + kRefitKids, kids);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(flag + kRefitDone, 1u) + 1u == gridDim.x && __ldcg(flag + kRefitKids) != nc - 1u)
+            report_error(err, RT_ERR_BOUNDS, 0x6f000000u);
+    }
+}
+
+template <bool INST>
+int refit_grid(rt_context *ctx) {
+    static thread_local int cached_dev = -1, cached = 0;
+    if (cached_dev == ctx->device) return cached;
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_refit_nodes<INST>, (int)kRefitThreads, 0) != cudaSuccess)
+        return 0;
+    cached = per_sm * ctx->sm_count;
+    cached_dev = ctx->device;
+    return cached;
 }
 
 int run_refit(rt_context *ctx, cudaStream_t st, uint32_t kind, uint32_t n, uint32_t n_geoms, const GeomParams *gp,
@@ -1489,24 +1738,29 @@ int run_refit(rt_context *ctx, cudaStream_t st, uint32_t kind, uint32_t n, uint3
     uint8_t *A = static_cast<uint8_t *>(accel);
     uint8_t *S = static_cast<uint8_t *>(scratch);
     const uint32_t cap = node_capacity_for(n);
-    rt_accel_header *hdr = reinterpret_cast<rt_accel_header *>(A);
-    uint4 *nodes = reinterpret_cast<uint4 *>(A + RT_ACCEL_HEADER_BYTES);
-    uint4 *recs = reinterpret_cast<uint4 *>(A + RT_ACCEL_HEADER_BYTES + (uint64_t)cap * 80u);
     uint32_t *flag = reinterpret_cast<uint32_t *>(S + L.flag);
     float *leaf_box = reinterpret_cast<float *>(S + L.leaf_box);
     float *node_box = reinterpret_cast<float *>(S + L.node_box);
-    uint32_t *parent = reinterpret_cast<uint32_t *>(S + L.parent);
-    uint32_t *arrive = reinterpret_cast<uint32_t *>(S + L.arrive);
-    uint32_t *hdr_status = reinterpret_cast<uint32_t *>(A) + 7;  // rt_accel_header::status
-    k_refit_begin<<<1, 32, 0, st>>>(hdr, kind, n, n_geoms, cap, flag, ctx->d_err);
-    RT_CUDA_CTX(ctx, cudaMemsetAsync(parent, 0xff, (size_t)cap * 4u, st));
-    const unsigned nbc = (cap + 255u) / 256u, nbn = (n + 255u) / 256u;
-    k_refit_links<<<nbc, 256, 0, st>>>(nodes, hdr, cap, flag, parent, arrive, ctx->d_err);
+    uint32_t *levels = reinterpret_cast<uint32_t *>(S + L.levels);
+    uint32_t *list = reinterpret_cast<uint32_t *>(S + L.list);
+    static const GeomParams empty_gp{};  // a top-level structure has no geometries
+    const unsigned nbn = (n + 255u) / 256u + 1u;
     if (kind == RT_ACCEL_KIND_BLAS)
-        k_refit_tris<<<nbn, 256, 0, st>>>(*gp, n, recs, leaf_box, flag, ctx->d_err, hdr_status);
+        k_refit_records<false><<<nbn, 256, 0, st>>>(*gp, nullptr, n, cap, A, leaf_box, flag, levels, ctx->d_err);
     else
-        k_refit_inst<<<nbn, 256, 0, st>>>(instances, n, recs, leaf_box, flag, ctx->d_err);
-    k_refit_nodes<<<nbc, 256, 0, st>>>(nodes, hdr, cap, n, leaf_box, node_box, parent, arrive, flag, ctx->d_err);
+        k_refit_records<true><<<nbn, 256, 0, st>>>(empty_gp, instances, n, cap, A, leaf_box, flag, levels, ctx->d_err);
+    RT_CUDA_CTX(ctx, cudaGetLastError());
+    const bool blas = kind == RT_ACCEL_KIND_BLAS;
+    const int resident = blas ? refit_grid<false>(ctx) : refit_grid<true>(ctx);
+    if (resident <= 0) return set_error(ctx, RT_ERR_CUDA, "cooperative occupancy query failed");
+    unsigned grid = (cap + kRefitThreads / 8u - 1u) / (kRefitThreads / 8u);  // eight lanes per node
+    if (grid > (unsigned)resident) grid = (unsigned)resident;
+    uint32_t nn = n;
+    uint32_t *err = ctx->d_err;
+    void *args[] = {&A, &nn, &leaf_box, &node_box, &flag, &levels, &list, &err};
+    RT_CUDA_CTX(ctx, cudaLaunchCooperativeKernel(blas ? (const void *)k_refit_nodes<false>
+                                                      : (const void *)k_refit_nodes<true>,
+                                                 dim3(grid), dim3(kRefitThreads), args, 0, st));
     RT_CUDA_CTX(ctx, cudaGetLastError());
     return RT_OK;
 }
