@@ -1307,9 +1307,13 @@ int run_build(rt_context *ctx, cudaStream_t st, const BuildCall &bc, const GeomP
     RT_CUDA_CTX(ctx, cudaMemsetAsync(ca.bar, 0, 2u * sizeof(uint32_t), st));
     int G = coop_grid(ctx);
     if (G <= 0) return set_error(ctx, RT_ERR_CUDA, "cooperative occupancy query failed");
-    // Small levels gain nothing from a huge grid; fewer blocks make each
-    // grid barrier cheaper.
-    unsigned want = (unsigned)((cap + kCollapseThreads * 4u - 1u) / (kCollapseThreads * 4u));
+    // A block handles 32 nodes at a time (eight lanes each), and a small tree
+    // is a chain of levels: 64 nodes of capacity per block (a level of a 12,345-
+    // triangle tree at most one step: build 246 us; 1,024 per block: 291, the
+    // levels' later steps waiting on the first's loads).  More blocks make each
+    // grid barrier dearer, but not by what a step costs.
+    constexpr unsigned kNodesPerBlock = kCollapseThreads / 4;
+    unsigned want = (unsigned)((cap + kNodesPerBlock - 1u) / kNodesPerBlock);
     if (want < 1u) want = 1u;
     if ((int)want < G) G = (int)want;
     void *args[] = {&ca};
