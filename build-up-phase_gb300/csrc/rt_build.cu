@@ -77,7 +77,7 @@ BuildLayout build_layout(uint32_t n, uint32_t rec_bytes, int passes) {
     L.node_box = take(ni * 32u);
     L.node_cost = take(ni * 4u);
     L.leafable = take(ni);
-    L.other = take(ni * 8u);  // k_tree: per internal node, the first child's reference and far end
+    L.other = take(ni * 8u);  // k_tree_climb: per internal node, the first child's reference and far end
     L.leaf_box = take((uint64_t)n * 32u);
     L.wq = take(cap * 4u);
     L.slots = take(cap * 32u);
@@ -154,6 +154,22 @@ __device__ __forceinline__ void block_minmax_atomic(int32_t *cbounds, const int3
     }
 }
 
+// Union of triangle (INST false) or instance boxes.  A triangle with a NaN
+// coordinate is inactive and has the empty box, so triangle boxes hold none and
+// min / max order -0 below +0 and infinities as the total order of box_union
+// does; instance boxes can hold NaN.
+template <bool INST>
+__device__ __forceinline__ Box union_of(const Box &x, const Box &y) {
+    if constexpr (INST) {
+        return box_union(x, y);
+    } else {
+        Box b;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) { b.lo[a] = fminf(x.lo[a], y.lo[a]); b.hi[a] = fmaxf(x.hi[a], y.hi[a]); }
+        return b;
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Header / init
 // ---------------------------------------------------------------------------
@@ -162,7 +178,8 @@ __global__ void k_init(rt_accel_header hdr, uint8_t *accel, int32_t *cbounds, ui
                        uint32_t write_table) {
     int t = threadIdx.x;
     if (t == 0) *reinterpret_cast<rt_accel_header *>(accel) = hdr;
-    if (t == 0) *root = kNone;  // the radix tree's root: none until k_tree completes it
+    // the radix tree's root (none until it is completed) and the subtrees k_tree leaves
+    if (t == 0) { root[0] = kNone; root[1] = 0u; }
     if (t < 3) { cbounds[t] = INT32_MAX; cbounds[3 + t] = INT32_MIN; }
     if (write_table) {
         uint32_t *tab = reinterpret_cast<uint32_t *>(accel + hdr.geom_offset);
@@ -431,12 +448,12 @@ __global__ void __launch_bounds__(256) k_morton(const float *__restrict__ boxes,
 // and r + 1, or the right child of the node split between l - 1 and l --
 // whichever boundary's keys share the longer prefix (never equal: the keys
 // are unique with their indices).  Internal node i is the one split between
-// keys i and i + 1.  The first child to reach a node exchanges its reference
-// and the far end of its range into the node's 64-bit word; the second child
-// gets them back, so it knows its sibling and the node's range, and
-// computes the node: box, SAH cost and the leaf decision (the refit), then
-// climbs on.  Same tree as a top-down Karras construction, in one launch and
-// without its per-node searches.
+// keys i and i + 1.  The first child to reach a node leaves its reference and
+// the far end of its range there (in shared memory, or exchanged into the
+// node's 64-bit word); the second child finds them, so it knows its sibling
+// and the node's range, and the node is computed: box, SAH cost and the leaf
+// decision (the refit).  Same tree as a top-down Karras construction, without
+// its per-node searches.
 
 // Common-prefix length of the keys on either side of boundary b | b + 1, the
 // index breaking ties between equal keys.
@@ -457,6 +474,8 @@ struct TreeArgs {
     uint64_t *other;       // per internal node: all ones, then the first child's reference and far end
     float *leaf_box;
     uint32_t *root;        // the root's reference
+    uint32_t *left;        // subtrees k_tree leaves to k_tree_climb: their references
+    uint32_t *n_left;
     uint32_t *err;
 };
 
@@ -480,39 +499,94 @@ __global__ void k_tree_root(uint32_t *root, uint32_t n, uint32_t *err) {
     *root = kLeafBit;
 }
 
-// Six blocks per SM (40 registers): more climbs in flight than the five of
-// an unbounded register count (1M soup build 0.718 -> 0.715 ms, 2M box 1.336
-// -> 1.322 ms).
-__global__ void __launch_bounds__(256, 6) k_tree(TreeArgs a) {
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t n = a.n;
-    if (j >= n) return;
-    // the leaf's box and the keys around its range, in one round of loads
-    const uint32_t id = __ldg(a.ids + j);
-    uint64_t kl = __ldg(a.keys + j), kr = kl;
-    uint64_t klm = j > 0 ? __ldg(a.keys + j - 1) : 0ull, krp = j + 1 < n ? __ldg(a.keys + j + 1) : 0ull;
-    if (id >= n) report_error(a.err, RT_ERR_BOUNDS, 0x67000000u | (j & 0xffffffu));  // not a sorted id
-    const Box lb = id < n ? load_box(a.boxes, id) : box_empty();
-    store_box(a.leaf_box, j, lb);
-    if (n < 2) return;
-    uint32_t me = kLeafBit | j, l = j, r = j;
-    Box mb = lb;
-    float mcost = RT_SAH_PRIM;
+// A block per kTreeKeys consecutive keys.  Nodes inside the block's keys are
+// completed in shared memory, in rounds: a child leaves its subtree (reference,
+// range end, box, cost) in its side's slot of the boundary it belongs to, and
+// the second to arrive lists the boundary for the next round, whose threads
+// complete the listed nodes -- packed into the first warps, where climbing on
+// in the thread that arrived second left a warp's loop running for three or
+// four of its lanes.  What is left then -- children at the block's edges and
+// those whose sibling reaches past them -- goes to a list, and a second launch
+// climbs on from there through the exchange words in global memory: a twentieth
+// of the nodes, at 1.5 us a level.  Both are latency-bound (a round in shared
+// memory is about 0.5 us).  1M soup: 70 + 42 us; 145 with one thread per leaf
+// climbing all the way through global memory (5.5 of 32 lanes busy), 146 with
+// the rest of the climb inside this kernel (its chain keeps the block's shared
+// memory); blocks of 512 keys 666 us for the whole build, 256 661, 1,024 686.
+constexpr uint32_t kTreeKeys = 256;
+
+// A subtree on its way up: reference, key range, box, cost.
+struct Climb {
+    uint32_t me, l, r;
+    Box box;
+    float cost;
+};
+
+// The node split between keys p and p + 1 over the climbing subtree c and its
+// sibling: stores it and makes it the climbing subtree.
+template <bool INST>
+__device__ __forceinline__ void complete_node(const TreeArgs &a, uint32_t p, bool left, uint32_t sib, const Box &sb,
+                                              float scost, uint32_t nl, uint32_t nr, Climb &c) {
+    const Box &bl = left ? c.box : sb, &br = left ? sb : c.box;
+    const float cl = left ? c.cost : scost, cr = left ? scost : c.cost;
+    const Box b = union_of<INST>(bl, br);
+    const float an = half_area(b);
+    float split;
+    if (an > 0.0f) {
+        const float sah = half_area(bl) * cl + half_area(br) * cr;
+        split = RT_SAH_NODE + sah / an;
+    } else {
+        split = RT_SAH_NODE + (cl + cr);
+    }
+    const uint32_t count = nr - nl + 1u;
+    const float leaf = (float)count * RT_SAH_PRIM;
+    const bool lf = count <= (uint32_t)RT_MAX_LEAF_PRIMS && leaf <= split;
+    const float cost = lf ? leaf : split;
+    store_box(a.node_box, p, b);
+    a.node_cost[p] = cost;
+    a.leafable[p] = lf ? 1 : 0;
+    a.bin[p] = make_uint4(left ? c.me : sib, left ? sib : c.me, nl, nr);
+    c.me = p;
+    c.l = nl;
+    c.r = nr;
+    c.box = b;
+    c.cost = cost;
+}
+
+// Climbs through global memory until the sibling is not there yet.
+template <bool INST>
+__device__ __forceinline__ void climb_global(const TreeArgs &a, uint32_t me) {
+    const uint32_t n = a.n, mi = me & ~kLeafBit;
+    Climb c;
+    c.me = me;
+    if (me & kLeafBit) {
+        c.l = c.r = mi;
+        c.box = load_box(a.leaf_box, mi);
+        c.cost = RT_SAH_PRIM;
+    } else {
+        const uint4 nd = __ldcg(a.bin + mi);
+        c.l = nd.z;
+        c.r = nd.w;
+        c.box = load_box(a.node_box, mi);
+        c.cost = __ldcg(a.node_cost + mi);
+    }
+    uint64_t kl = __ldg(a.keys + c.l), kr = __ldg(a.keys + c.r);
+    uint64_t klm = c.l > 0u ? __ldg(a.keys + c.l - 1u) : 0ull, krp = c.r + 1u < n ? __ldg(a.keys + c.r + 1u) : 0ull;
     // A radix tree over 2^30 keys is at most 96 levels deep (63 key bits +
     // 32 index bits); the cap only guards against inconsistent keys.
     for (int climb = 0;; ++climb) {
         if (climb >= 256) {
-            report_error(a.err, RT_ERR_BOUNDS, 0x61000000u | j);
+            report_error(a.err, RT_ERR_BOUNDS, 0x61000000u | (c.l & 0xffffffu));
             return;
         }
-        const bool left = l == 0u ? true : (r == n - 1u ? false : boundary_delta(kr, krp, r) > boundary_delta(klm, kl, l - 1u));
-        const uint32_t p = left ? r : l - 1u;
-        const uint64_t got = exch_acq_rel(a.other + p, ((uint64_t)me << 32) | (left ? l : r));
+        const bool left = c.l == 0u ? true : (c.r == n - 1u ? false : boundary_delta(kr, krp, c.r) > boundary_delta(klm, kl, c.l - 1u));
+        const uint32_t p = left ? c.r : c.l - 1u;
+        const uint64_t got = exch_acq_rel(a.other + p, ((uint64_t)c.me << 32) | (left ? c.l : c.r));
         if (got == ~0ull) return;  // first child here: the sibling computes the node
         const uint32_t sib = (uint32_t)(got >> 32), far = (uint32_t)got;
-        const uint32_t nl = left ? l : far, nr = left ? far : r;
+        const uint32_t nl = left ? c.l : far, nr = left ? far : c.r;
         if (nl > nr || nr >= n) {
-            report_error(a.err, RT_ERR_BOUNDS, 0x61000000u | j);
+            report_error(a.err, RT_ERR_BOUNDS, 0x61000000u | (c.l & 0xffffffu));
             return;
         }
         // the sibling's box and cost and the keys around the node's range,
@@ -523,38 +597,142 @@ __global__ void __launch_bounds__(256, 6) k_tree(TreeArgs a) {
         const bool sl = (sib & kLeafBit) != 0u;
         const Box sb = sl ? load_box(a.leaf_box, sib & ~kLeafBit) : load_box(a.node_box, sib);
         const float scost = sl ? RT_SAH_PRIM : __ldcg(a.node_cost + sib);
-        const Box &bl = left ? mb : sb, &br = left ? sb : mb;
-        const float cl = left ? mcost : scost, cr = left ? scost : mcost;
-        const Box b = box_union(bl, br);
-        const float an = half_area(b);
-        float split;
-        if (an > 0.0f) {
-            const float sah = half_area(bl) * cl + half_area(br) * cr;
-            split = RT_SAH_NODE + sah / an;
-        } else {
-            split = RT_SAH_NODE + (cl + cr);
-        }
-        const uint32_t count = nr - nl + 1u;
-        const float leaf = (float)count * RT_SAH_PRIM;
-        const bool lf = count <= (uint32_t)RT_MAX_LEAF_PRIMS && leaf <= split;
-        mcost = lf ? leaf : split;
-        store_box(a.node_box, p, b);
-        a.node_cost[p] = mcost;
-        a.leafable[p] = lf ? 1 : 0;
-        a.bin[p] = make_uint4(left ? me : sib, left ? sib : me, nl, nr);
-        mb = b;
-        me = p;
-        l = nl;
-        r = nr;
+        complete_node<INST>(a, p, left, sib, sb, scost, nl, nr, c);
         kl = k_nl;
         kr = k_nr;
         klm = k_nlm;
         krp = k_nrp;
-        if (l == 0u && r == n - 1u) {
+        if (c.l == 0u && c.r == n - 1u) {
             *a.root = p;
             return;
         }
     }
+}
+
+struct TreeShared {
+    // common-prefix lengths at the boundaries base - 1 | base, base | base + 1,
+    // ... (-1 before the first and after the last key of all)
+    int16_t delta[kTreeKeys + 1];
+    uint16_t list[2][kTreeKeys];  // boundaries with both children, this round's and the next's
+    uint32_t listed[3], left;
+    // boundary base + i | base + i + 1: who has arrived (bit 0 / 1: the left /
+    // right child) and the children; the last index, never a boundary inside,
+    // holds the left child at the block's right edge and the right child at
+    // its left edge
+    uint32_t seen[kTreeKeys];
+    uint32_t ref[2][kTreeKeys], far[2][kTreeKeys];
+    float box[2][6][kTreeKeys], cost[2][kTreeKeys];
+};
+
+__device__ __forceinline__ Climb tree_child(const TreeShared &s, uint32_t side, uint32_t i, uint32_t l, uint32_t r) {
+    Climb c;
+    c.me = s.ref[side][i];
+    c.l = l;
+    c.r = r;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        c.box.lo[q] = s.box[side][q][i];
+        c.box.hi[q] = s.box[side][3 + q][i];
+    }
+    c.cost = s.cost[side][i];
+    return c;
+}
+
+// Hands subtree c to the boundary it belongs to.
+__device__ __forceinline__ void tree_arrive(const TreeArgs &a, TreeShared &s, const Climb &c, uint32_t base,
+                                            uint32_t count, uint32_t round) {
+    if (c.l == 0u && c.r == a.n - 1u) {
+        *a.root = c.me;
+        return;
+    }
+    const bool left = s.delta[c.r - base + 1u] > s.delta[c.l - base];
+    const uint32_t side = left ? 0u : 1u;
+    uint32_t i = (left ? c.r : c.l - 1u) - base;
+    const bool edge = i >= count - 1u;  // (also below base)
+    if (edge) i = kTreeKeys - 1u;
+    s.ref[side][i] = c.me;
+    s.far[side][i] = left ? c.l : c.r;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        s.box[side][q][i] = c.box.lo[q];
+        s.box[side][3 + q][i] = c.box.hi[q];
+    }
+    s.cost[side][i] = c.cost;
+    __threadfence_block();
+    const uint32_t seen = atomicOr(&s.seen[i], 1u << side);
+    // keys out of order (only a sort that gave up leaves them so) can bring a
+    // side twice: that node stays without a parent
+    if ((seen >> side) & 1u) report_error(a.err, RT_ERR_BOUNDS, 0x61000000u | (c.l & 0xffffffu));
+    else if (!edge && seen) s.list[round & 1u][atomicAdd(&s.listed[round % 3u], 1u)] = (uint16_t)i;
+}
+
+template <bool INST>
+__global__ void __launch_bounds__(kTreeKeys, 1536 / kTreeKeys) k_tree(TreeArgs a) {
+    __shared__ TreeShared s;
+    const uint32_t t = threadIdx.x, base = blockIdx.x * kTreeKeys, j = base + t, n = a.n;
+    const uint32_t count = min(n - base, kTreeKeys);
+    Climb c;
+    if (t == 0) {
+        s.listed[0] = s.listed[1] = s.left = 0u;
+        s.delta[0] = base > 0u ? (int16_t)boundary_delta(__ldg(a.keys + base - 1u), __ldg(a.keys + base), base - 1u) : -1;
+    }
+    s.seen[t] = 0u;
+    if (t < count) {
+        const uint32_t id = __ldg(a.ids + j);
+        const uint64_t key = __ldg(a.keys + j), next = j + 1u < n ? __ldg(a.keys + j + 1u) : 0ull;
+        s.delta[t + 1u] = j + 1u < n ? (int16_t)boundary_delta(key, next, j) : -1;
+        if (j + 1u < n) a.other[j] = ~0ull;  // k_tree_climb's exchange word: no child yet
+        if (id >= n) report_error(a.err, RT_ERR_BOUNDS, 0x67000000u | (j & 0xffffffu));  // not a sorted id
+        c.box = id < n ? load_box(a.boxes, id) : box_empty();
+        store_box(a.leaf_box, j, c.box);
+        c.me = kLeafBit | j;
+        c.l = c.r = j;
+        c.cost = RT_SAH_PRIM;
+    }
+    if (n < 2) return;
+    __syncthreads();
+    if (t < count) tree_arrive(a, s, c, base, count, 0u);
+    __syncthreads();
+    // a boundary is listed once, so there are at most count - 1 rounds
+    for (uint32_t round = 0;; ++round) {
+        const uint32_t m = s.listed[round % 3u];
+        if (m == 0u) break;
+        if (t == 0) s.listed[(round + 2u) % 3u] = 0u;
+        if (t < m) {
+            const uint32_t i = s.list[round & 1u][t], nl = s.far[0][i], nr = s.far[1][i];
+            if (nl < base || nl > base + i || nr <= base + i || nr >= base + count) {
+                report_error(a.err, RT_ERR_BOUNDS, 0x61000000u | ((base + i) & 0xffffffu));
+            } else {
+                c = tree_child(s, 0u, i, nl, base + i);
+                const Climb o = tree_child(s, 1u, i, base + i + 1u, nr);
+                complete_node<INST>(a, base + i, true, o.me, o.box, o.cost, nl, nr, c);
+                tree_arrive(a, s, c, base, count, round + 1u);
+            }
+        }
+        __syncthreads();
+    }
+    // the children left (the last index: one at each edge)
+    const uint32_t seen = s.seen[t];
+    const bool both = seen == 3u && t == kTreeKeys - 1u;
+    const uint32_t k = both ? 2u : ((seen == 1u || seen == 2u) ? 1u : 0u);
+    uint32_t pos = 0u;
+    if (k) pos = atomicAdd(&s.left, k);
+    __syncthreads();
+    if (t == 0) s.listed[0] = atomicAdd(a.n_left, s.left);
+    __syncthreads();
+    if (k) {
+        uint32_t *out = a.left + s.listed[0] + pos;
+        out[0] = s.ref[seen == 2u ? 1 : 0][t];
+        if (both) out[1] = s.ref[1][t];
+    }
+}
+
+// The subtrees k_tree left, one thread each.
+template <bool INST>
+__global__ void __launch_bounds__(128) k_tree_climb(TreeArgs a) {
+    const uint32_t m = *a.n_left;
+    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < m; q += gridDim.x * blockDim.x)
+        climb_global<INST>(a, __ldg(a.left + q));
 }
 
 // ---------------------------------------------------------------------------
@@ -1266,7 +1444,6 @@ int run_build(rt_context *ctx, cudaStream_t st, const BuildCall &bc, const GeomP
     if (sst) return set_error(ctx, sst, "radix sort launch failed");
 
     uint4 *bin = reinterpret_cast<uint4 *>(S + L.bin);
-    if (n >= 2) RT_CUDA_CTX(ctx, cudaMemsetAsync(S + L.other, 0xff, (size_t)(n - 1) * 8u, st));
     TreeArgs ta;
     ta.n = n;
     ta.keys = keys0;
@@ -1279,8 +1456,20 @@ int run_build(rt_context *ctx, cudaStream_t st, const BuildCall &bc, const GeomP
     ta.other = reinterpret_cast<uint64_t *>(S + L.other);
     ta.leaf_box = reinterpret_cast<float *>(S + L.leaf_box);
     ta.root = root_word;
+    ta.left = reinterpret_cast<uint32_t *>(keys1);  // free: the sort has left its result in keys0/ids0
+    ta.n_left = root_word + 1;
     ta.err = ctx->d_err;
-    k_tree<<<nb, 256, 0, st>>>(ta);
+    const unsigned tree_blocks = (n + kTreeKeys - 1u) / kTreeKeys;
+    // about 20 subtrees are left per block of k_tree
+    unsigned climb_blocks = (tree_blocks + 3u) / 4u;
+    if (climb_blocks > 8u * (unsigned)ctx->sm_count) climb_blocks = 8u * (unsigned)ctx->sm_count;
+    if (bc.kind == RT_ACCEL_KIND_BLAS) {
+        k_tree<false><<<tree_blocks, kTreeKeys, 0, st>>>(ta);
+        if (tree_blocks > 1u) k_tree_climb<false><<<climb_blocks, 128, 0, st>>>(ta);
+    } else {
+        k_tree<true><<<tree_blocks, kTreeKeys, 0, st>>>(ta);
+        if (tree_blocks > 1u) k_tree_climb<true><<<climb_blocks, 128, 0, st>>>(ta);
+    }
     if (n >= 2) k_tree_root<<<1, 1, 0, st>>>(root_word, n, ctx->d_err);
     RT_CUDA_CTX(ctx, cudaGetLastError());
 
@@ -1487,21 +1676,6 @@ __global__ void __launch_bounds__(kRecThreads) k_refit_records(const GeomParams 
     }
 }
 
-// Union of boxes without NaN coordinates (triangles with one are inactive and
-// have the empty box): min and max order -0 below +0 and infinities as the
-// total order of box_union does.  Instance boxes can hold NaN.
-template <bool INST>
-__device__ __forceinline__ Box refit_union(const Box &x, const Box &y) {
-    if constexpr (INST) {
-        return box_union(x, y);
-    } else {
-        Box b;
-#pragma unroll
-        for (int a = 0; a < 3; ++a) { b.lo[a] = fminf(x.lo[a], y.lo[a]); b.hi[a] = fmaxf(x.hi[a], y.hi[a]); }
-        return b;
-    }
-}
-
 // Internal nodes listed for level l: the spare fourth word of leaf box l, which
 // store_box left at zero (a tree has no more levels than leaf records).
 __device__ __forceinline__ uint32_t *refit_count(float *leaf_box, uint32_t l) {
@@ -1575,7 +1749,7 @@ __device__ __forceinline__ uint32_t refit_node(const RefitSlot &s, uint4 *nodes,
     sb.hi[0] = s.hi.x; sb.hi[1] = s.hi.y; sb.hi[2] = s.hi.z;
     if (s.cnt > 1u) {  // a leaf's further records, at most two
         const Box b1 = load_box(leaf_box, s.i + 1u), b2 = load_box(leaf_box, s.i + s.cnt - 1u);
-        sb = refit_union<INST>(refit_union<INST>(sb, b1), b2);
+        sb = union_of<INST>(union_of<INST>(sb, b1), b2);
     }
     Box node = sb;  // an unused slot's box is empty
 #pragma unroll
@@ -1586,7 +1760,7 @@ __device__ __forceinline__ uint32_t refit_node(const RefitSlot &s, uint4 *nodes,
             t.lo[q] = __shfl_xor_sync(kFullMask, node.lo[q], d);
             t.hi[q] = __shfl_xor_sync(kFullMask, node.hi[q], d);
         }
-        node = refit_union<INST>(node, t);
+        node = union_of<INST>(node, t);
     }
     if (s.k == kNone) return 0u;
     const QFrame f = node_frame(node);
