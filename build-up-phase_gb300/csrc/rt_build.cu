@@ -33,7 +33,7 @@ namespace rtc {
 namespace {
 
 constexpr int kMaxGeoms = 256;
-constexpr int kCollapseThreads = 256;
+constexpr int kCollapseThreads = 512;
 constexpr int kMaxCoopBlocks = 4096;
 constexpr uint32_t kNone = 0xffffffffu;
 
@@ -757,7 +757,7 @@ struct CollapseArgs {
     uint32_t *blk;
     uint4 *nodes_out;
     rt_accel_header *hdr;
-    uint32_t *bar;  // grid barrier: arrival count, generation (zeroed before the launch)
+    uint32_t *bar;  // grid barrier: arrival count, generation (zeroed before the launch); block 0's state after its levels
     uint32_t *err;
 };
 
@@ -928,7 +928,8 @@ __device__ __forceinline__ int group_argmin(float key, bool ok) {
 // (bits 0-7) and each leaf slot's primitive count minus one (two bits per
 // slot from bit 8).  Returns the node's internal children and primitives
 // (every lane of the group).
-__device__ __forceinline__ void collapse_phase_a(const CollapseArgs &a, uint32_t k, bool valid, uint32_t &n_int, uint32_t &n_prim) {
+__device__ __forceinline__ void collapse_phase_a(const CollapseArgs &a, uint32_t k, bool valid, uint4 *s_info,
+                                                 uint32_t &n_int, uint32_t &n_prim) {
     const int j = (int)(threadIdx.x & 7u);
     const int gb = (int)(threadIdx.x & 24u);
     // wq and the hand-off arrays are written by other blocks of this launch
@@ -976,6 +977,56 @@ __device__ __forceinline__ void collapse_phase_a(const CollapseArgs &a, uint32_t
         }
     }
     bool act = src_open;
+    // Whole tables: when every openable node of the first two levels fits in
+    // the node and none of the third is opened, the widening opens exactly
+    // those, in descending area (a child's area is at most its parent's), and
+    // an opened node's second child goes to lane 2 + its rank: no loop.  Equal
+    // or NaN areas take the loop below.
+    {
+        const bool p1 = src_open && j < 2 && info_open(t1), p2 = src_open && j < 4 && info_open(t2);
+        const bool p3 = src_open && info_open(t3);
+        const uint32_t o1 = (__ballot_sync(kFullMask, p1) >> gb) & 3u, o2 = (__ballot_sync(kFullMask, p2) >> gb) & 15u;
+        const uint32_t o3 = (__ballot_sync(kFullMask, p3) >> gb) & 255u;
+        const int total = 2 + __popc(o1) + __popc(o2);
+        const float a1 = p1 ? t1.area : -1.0f, a2 = p2 ? t2.area : -1.0f;
+        uint32_t r1 = 0u, r2 = 0u, same = 0u;
+        float least = kInf;
+#pragma unroll
+        for (int q = 0; q < 6; ++q) {
+            const float x = q < 2 ? __shfl_sync(kFullMask, a1, gb | q) : __shfl_sync(kFullMask, a2, gb | (q - 2));
+            r1 += x > a1 ? 1u : 0u;
+            r2 += x > a2 ? 1u : 0u;
+            if (x != -1.0f) {
+                least = fminf(least, x);
+                same += (p1 && q != j && x == a1) || (p2 && q != j + 2 && x == a2) || x != x ? 1u : 0u;
+            }
+        }
+        bool below = true;  // this lane's third-level node stays closed
+        if (p3) below = total == (int)a.width && t3.area < least;
+        const uint32_t bad = (__ballot_sync(kFullMask, !below || same != 0u) >> gb) & 255u;
+        const bool whole = src_open && total <= (int)a.width && bad == 0u;
+        if (__any_sync(kFullMask, whole)) {
+            // lanes of the second- and third-level nodes
+            const int q1 = __shfl_sync(kFullMask, (int)r1, gb | ((j >> 1) & 1));
+            const int l2 = (j & 1) ? 2 + q1 : (j >> 1);
+            const int q2 = __shfl_sync(kFullMask, (int)r2, gb | (j >> 1)), m2 = __shfl_sync(kFullMask, l2, gb | (j >> 1));
+            const int l3 = (j & 1) ? 2 + q2 : m2;
+            uint4 *slot = s_info + (threadIdx.x & ~7u);
+            if (whole) {
+                if (j < 2 && !p1) slot[j] = make_uint4(t1.ref, t1.kid0, t1.kid1, t1.cnt);
+                if (j < 4 && ((o1 >> (j >> 1)) & 1u) && !p2) slot[l2 & 7] = make_uint4(t2.ref, t2.kid0, t2.kid1, t2.cnt);
+                if ((o2 >> (j >> 1)) & 1u) slot[l3 & 7] = make_uint4(t3.ref, t3.kid0, t3.kid1, t3.cnt);
+            }
+            __syncwarp();
+            if (whole) {
+                const uint4 m = slot[j];
+                mine = {m.x, m.y, m.z, m.w, 0.0f};
+                n = total;
+                act = false;
+            }
+            __syncwarp();
+        }
+    }
     for (;;) {
         act = act && n < (int)a.width;
         if (!__any_sync(kFullMask, act)) break;
@@ -1029,8 +1080,50 @@ __device__ __forceinline__ void collapse_phase_a(const CollapseArgs &a, uint32_t
     }
     uint32_t used = 0u;
     int my_slot = -1;
+    // Without NaN costs: as soon as the first least slots of the children left
+    // are all different, each child keeps its own (its least slot stays free
+    // until its turn), so the rounds end there.
+    const float reach = (fabsf(d[0]) + fabsf(d[1])) + fabsf(d[2]);
+    const bool plain = ((__ballot_sync(kFullMask, have && !(reach < kInf)) >> gb) & 255u) == 0u;
+    {
+        bool go = valid && plain;
+        float v = kInf;
+        int vs = 0;
+        bool scan = true;
+        while (__any_sync(kFullMask, go)) {
+            const bool cand = go && have && my_slot < 0;
+            if (scan) {
+                v = kInf;
+                vs = -1;
+#pragma unroll
+                for (int s = 0; s < 8; ++s)
+                    if (((used >> s) & 1u) == 0u && (vs < 0 || cost[s] < v)) {
+                        v = cost[s];
+                        vs = s;
+                    }
+            }
+            uint32_t uni = cand ? 1u << vs : 0u;
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) uni |= __shfl_xor_sync(kFullMask, uni, o);
+            const uint32_t cm = (__ballot_sync(kFullMask, cand) >> gb) & 0xffu;
+            const bool distinct = __popc(uni) == __popc(cm);
+            const int bc = group_argmin(v, cand);
+            const int bs = __shfl_sync(kFullMask, vs, gb | (bc < 0 ? 0 : bc));
+            if (go) {
+                if (distinct) {
+                    if (cand) my_slot = vs;
+                    used |= uni;
+                    go = false;
+                } else {
+                    if (j == bc) my_slot = bs;
+                    used |= 1u << bs;
+                    scan = vs == bs;
+                }
+            }
+        }
+    }
     for (int it = 0; it < 8; ++it) {
-        const bool go = valid && it < n;
+        const bool go = valid && !plain && it < n;
         if (!__any_sync(kFullMask, go)) break;
         const bool cand = go && j < n && my_slot < 0;
         const int s0 = __ffs((int)(~used & 0xffu)) - 1;
@@ -1235,24 +1328,57 @@ __device__ bool coop_sync(uint32_t *bar, uint32_t nblocks, uint32_t *err, uint32
     return s_ok != 0;
 }
 
-__global__ void __launch_bounds__(kCollapseThreads, 4) k_collapse(CollapseArgs a) {
+// Two blocks of 512 threads per SM: half the arrivals of four of 256 at each
+// grid barrier (1M soup build 624 -> 607 us), the same 32 warps.  1M soup: 338
+// us before the widening and the slot rounds ended early, blocks of 512 and
+// block 0's levels, 274 now; of that 150 are the 241,000-node level's phase A
+// (2,000 instructions per warp and four nodes, 41 % of the issue slots) and 6
+// a grid barrier.
+__global__ void __launch_bounds__(kCollapseThreads, 2) k_collapse(CollapseArgs a) {
     __shared__ uint32_t s_red[kCollapseThreads / 32];
     __shared__ uint4 s_red4[kCollapseThreads / 32];
+    __shared__ uint4 s_info[kCollapseThreads];
     const uint32_t G = gridDim.x, b = blockIdx.x, t = threadIdx.x;
     const uint32_t root_ref = a.root_dev ? __ldcg(a.root_dev) : a.root_ref;
-    if (b == 0 && t == 0) a.wq[0] = root_ref;
-    if (!coop_sync(a.bar, G, a.err, 0x64000000u)) return;
+    // The first levels, up to one step of a block, are block 0's alone: block
+    // barriers in the place of two grid barriers a level (7 us a level where a
+    // level of 512 nodes takes 18).  The others wait at the first grid barrier
+    // and take over the state it leaves.
+    bool alone = b == 0;
     uint32_t level_start = 0, level_count = 1, prim_next = 0, depth = 0;
+    if (alone) {
+        if (t == 0) a.wq[0] = root_ref;
+        __syncthreads();
+    } else {
+        if (!coop_sync(a.bar, G, a.err, 0x64000000u)) return;
+        level_start = __ldcg(a.bar + 2);
+        level_count = __ldcg(a.bar + 3);
+        prim_next = __ldcg(a.bar + 4);
+        depth = __ldcg(a.bar + 5);
+    }
     // Every block evaluates the same level sizes, so all leave together; the
     // level cap (a wide tree is never deeper than its <= 96-level binary
     // tree) only guards against corrupt inputs.
-    while (level_count > 0) {
+    for (;;) {
+        if (alone && (level_count > (uint32_t)kCollapseThreads / 8u || level_count == 0u || depth >= 256 ||
+                      level_start + level_count > a.capacity)) {
+            if (t == 0) {
+                a.bar[2] = level_start;
+                a.bar[3] = level_count;
+                a.bar[4] = prim_next;
+                a.bar[5] = depth;
+            }
+            alone = false;
+            if (!coop_sync(a.bar, G, a.err, 0x64000000u)) return;
+        }
+        if (level_count == 0u) break;
         if (depth >= 256 || level_start + level_count > a.capacity) {
             if (b == 0 && t == 0) report_error(a.err, RT_ERR_BOUNDS, 0x62000000u | depth);
             break;
         }
         ++depth;
-        const uint32_t chunk = (level_count + G - 1u) / G;
+        const uint32_t blocks = alone ? 1u : G;
+        const uint32_t chunk = (level_count + blocks - 1u) / blocks;
         const uint32_t c0 = min(b * chunk, level_count), c1 = min(c0 + chunk, level_count);
         uint32_t my_int = 0, my_prim = 0;
         // eight lanes per node (collapse_phase_a); the loop is block-uniform
@@ -1260,7 +1386,7 @@ __global__ void __launch_bounds__(kCollapseThreads, 4) k_collapse(CollapseArgs a
             const uint32_t k = kb + (t >> 3);
             const bool valid = k < c1;
             uint32_t ni, np;
-            collapse_phase_a(a, level_start + k, valid, ni, np);
+            collapse_phase_a(a, level_start + k, valid, s_info, ni, np);
             if (valid && (t & 7u) == 0u) {
                 a.counts[level_start + k] = ni | (np << 16);
                 my_int += ni;
@@ -1272,16 +1398,18 @@ __global__ void __launch_bounds__(kCollapseThreads, 4) k_collapse(CollapseArgs a
             my_int = bs.x;
             my_prim = bs.y;
         }
-        if (t == 0) { a.blk[2 * b] = my_int; a.blk[2 * b + 1] = my_prim; }
-        if (!coop_sync(a.bar, G, a.err, 0x64000000u | depth)) return;
-        uint32_t pre_i = 0, pre_p = 0, tot_i = 0, tot_p = 0;
-        for (uint32_t q = t; q < G; q += kCollapseThreads) {
-            uint32_t vi = __ldcg(a.blk + 2 * q), vp = __ldcg(a.blk + 2 * q + 1);
-            tot_i += vi;
-            tot_p += vp;
-            if (q < b) { pre_i += vi; pre_p += vp; }
-        }
-        {
+        uint32_t pre_i = 0, pre_p = 0, tot_i = my_int, tot_p = my_prim;
+        if (!alone) {
+            if (t == 0) { a.blk[2 * b] = my_int; a.blk[2 * b + 1] = my_prim; }
+            if (!coop_sync(a.bar, G, a.err, 0x64000000u | depth)) return;
+            tot_i = 0;
+            tot_p = 0;
+            for (uint32_t q = t; q < G; q += kCollapseThreads) {
+                uint32_t vi = __ldcg(a.blk + 2 * q), vp = __ldcg(a.blk + 2 * q + 1);
+                tot_i += vi;
+                tot_p += vp;
+                if (q < b) { pre_i += vi; pre_p += vp; }
+            }
             const uint4 bs = block_sum4<kCollapseThreads>(make_uint4(pre_i, pre_p, tot_i, tot_p), s_red4);
             pre_i = bs.x;
             pre_p = bs.y;
@@ -1305,7 +1433,11 @@ __global__ void __launch_bounds__(kCollapseThreads, 4) k_collapse(CollapseArgs a
         level_start = next_start;
         level_count = tot_i;
         prim_next += tot_p;
-        if (!coop_sync(a.bar, G, a.err, 0x65000000u | depth)) return;
+        if (alone) {
+            __syncthreads();
+        } else if (!coop_sync(a.bar, G, a.err, 0x65000000u | depth)) {
+            return;
+        }
     }
     if (b == 0 && t == 0) {
         Box rb = ref_box(a, root_ref);
@@ -1496,11 +1628,11 @@ int run_build(rt_context *ctx, cudaStream_t st, const BuildCall &bc, const GeomP
     RT_CUDA_CTX(ctx, cudaMemsetAsync(ca.bar, 0, 2u * sizeof(uint32_t), st));
     int G = coop_grid(ctx);
     if (G <= 0) return set_error(ctx, RT_ERR_CUDA, "cooperative occupancy query failed");
-    // A block handles 32 nodes at a time (eight lanes each), and a small tree
-    // is a chain of levels: 64 nodes of capacity per block (a level of a 12,345-
-    // triangle tree at most one step: build 246 us; 1,024 per block: 291, the
-    // levels' later steps waiting on the first's loads).  More blocks make each
-    // grid barrier dearer, but not by what a step costs.
+    // A block handles 64 nodes at a time (eight lanes each), and a small tree
+    // is a chain of levels: 128 nodes of capacity per block, so that a level of
+    // a 12,345-triangle tree is at most one step (build 235 us; 239 at 64 or
+    // 256 per block; at 1,024 the levels' later steps wait on the first's
+    // loads).
     constexpr unsigned kNodesPerBlock = kCollapseThreads / 4;
     unsigned want = (unsigned)((cap + kNodesPerBlock - 1u) / kNodesPerBlock);
     if (want < 1u) want = 1u;
