@@ -160,8 +160,6 @@ __device__ void encode_row(const rt_cache_input &in, const CacheState *S, __nv_b
         *reinterpret_cast<uint32_t *>(out + k) = pack_bf16(f[k], f[k + 1]);
 }
 
-constexpr int kQueryRows = 128;
-
 // ---------------------------------------------------------------------------
 // Training: forward + backward over 128-row tiles, gradients into S->grads
 // ---------------------------------------------------------------------------
@@ -507,28 +505,36 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_cache_fwd_bwd(CacheState *
 // Inference on the 5th-generation tensor cores (tcgen05 + TMEM)
 // ---------------------------------------------------------------------------
 //
-// One CTA = 4 warps = 128 threads, one query row per thread, 128-row tiles.
-// Operands live in shared memory in the canonical K-major layout without
-// swizzle: 8-row x 16-byte core matrices; element (r, k) of a tile with K
-// columns sits at (r/8)*16K + (k/8)*128 + (r%8)*16 + (k%8)*2 bytes, so one
-// MMA step of K = 16 is described by LBO = 128 (next core matrix along K) and
-// SBO = 16K (next 8-row group).  Thread 0 issues tcgen05.mma.kind::f16 with
-// M = 128, N = 64 (N = 16 for the output layer), K = 16 per instruction,
-// BF16 x BF16 -> FP32 accumulators in TMEM (row r = TMEM lane r), and commits
-// to an mbarrier.  The accumulators start from the layer's bias (written with
-// tcgen05.st), so the MMAs add the bias.  The epilogue of every thread reads
-// its row's 64 accumulators with tcgen05.ld (each warp its own 32-lane
-// quarter), applies ReLU and packs BF16 in one cvt.rn.relu.bf16x2.f32 per
-// pair, writes the row into the next layer's A tile and the next layer's bias
-// into the columns it has read; fence.proxy.async makes the generic-proxy
-// stores visible to the next MMA.  Every mbarrier wait is bounded: on expiry the kernel records
-// RT_ERR_TIMEOUT, waits once more (bounded) for its MMAs, frees its TMEM and
-// returns.
+// One CTA per SM with five independent groups of 4 warps = 128 threads, one
+// query row per thread, 128-row tiles; the groups share one copy of the weights
+// in shared memory, and the tensor core works on one group's layer while the
+// others encode or run their epilogues.
+//
+// Weights and encoded inputs live in shared memory in the canonical K-major
+// layout without swizzle: 8-row x 16-byte core matrices; element (r, k) of a
+// tile with K columns sits at (r/8)*16K + (k/8)*128 + (r%8)*16 + (k%8)*2 bytes,
+// so one MMA step of K = 16 is described by LBO = 128 (next core matrix along
+// K) and SBO = 16K (next 8-row group).  A group's thread 0 issues
+// tcgen05.mma.kind::f16 with M = 128, N = 64 (N = 16 for the output layer),
+// K = 16 per instruction, BF16 x BF16 -> FP32 accumulators in TMEM (row r =
+// TMEM lane r), and commits to the group's mbarrier, on which the group waits.
+//
+// A layer starts with one MMA that sets the accumulators to the bias: a tile of
+// ones times the bias split in three BF16 parts, whose sum is the FP32 bias
+// exactly, so the layer's MMAs add onto the bias.  The epilogue of every thread
+// reads its row's 64 accumulators with tcgen05.ld (each warp its own 32-lane
+// quarter), applies ReLU and packs BF16 in one cvt.rn.relu.bf16x2.f32 per pair,
+// and writes the row back to TMEM as the next layer's A operand (two BF16 per
+// 32-bit column): the activations never pass through shared memory.  Every
+// mbarrier wait is bounded: on expiry the kernel records RT_ERR_TIMEOUT, waits
+// once more (bounded) for its MMAs, frees its TMEM and returns.
 
 constexpr int kTcRows = 128;
-constexpr int kTcGroups = 4;                      // independent 128-row tile groups per CTA
+constexpr int kTcGroups = 5;                      // independent 128-row tile groups per CTA
 constexpr int kTcThreads = 128 * kTcGroups;
-constexpr uint32_t kTcTmemCols = 64u * kTcGroups;  // one 64-column accumulator per group
+constexpr uint32_t kTcTmemCols = 512;             // a power of two; 96 per group are used
+constexpr uint32_t kTcGroupCols = 96;             // 64 accumulators, 32 columns of BF16 pairs
+constexpr uint32_t kTcACol = 64;
 // tile byte sizes / offsets
 __host__ __device__ constexpr uint32_t tc_tile_bytes(int rows, int k) { return (uint32_t)(rows / 8) * 16u * k; }
 __host__ __device__ constexpr uint32_t tc_w_off(int l) {
@@ -537,17 +543,16 @@ __host__ __device__ constexpr uint32_t tc_w_off(int l) {
     return o;
 }
 constexpr uint32_t kTcWBytes = tc_w_off(6);                        // 47104: all weights, shared by the groups
-constexpr uint32_t kTcBias = kTcWBytes;                            // 336 floats
-constexpr uint32_t kTcBar = kTcBias + 336u * 4u;                   // one mbarrier per group + the TMEM address
-constexpr uint32_t kTcGroupBase = (kTcBar + 64u + 127u) & ~127u;
-// per group: the K = 96 input tile (reused as the second hidden tile once
-// layer 0 has read it) and the first hidden tile (K = 64)
-constexpr uint32_t kTcA0 = 0;
-constexpr uint32_t kTcH0 = tc_tile_bytes(kTcRows, 96);
-constexpr uint32_t kTcH1 = kTcA0;
-constexpr uint32_t kTcGroupBytes = kTcH0 + tc_tile_bytes(kTcRows, 64);  // 40960
+constexpr uint32_t kTcBias = kTcWBytes;                            // per layer, the bias as a K = 16 operand
+__host__ __device__ constexpr uint32_t tc_bias_off(int l) { return kTcBias + (uint32_t)l * tc_tile_bytes(64, 16); }
+constexpr uint32_t kTcOnes = tc_bias_off(5) + tc_tile_bytes(16, 16);  // 128 x 16 ones
+constexpr uint32_t kTcBar = kTcOnes + tc_tile_bytes(kTcRows, 16);  // one mbarrier per group + the TMEM address
+constexpr uint32_t kTcGroupBase = (kTcBar + 8u * kTcGroups + 8u + 127u) & ~127u;
+constexpr uint32_t kTcGroupBytes = tc_tile_bytes(kTcRows, 96);     // per group: the K = 96 input tile
 constexpr uint32_t kTcSmem = kTcGroupBase + kTcGroups * kTcGroupBytes;
 static_assert(kTcSmem <= 227u * 1024u, "shared memory of the inference kernel");
+static_assert(kTcSmem < (1u << 18), "descriptor addresses do not wrap");
+static_assert(kTcGroups * kTcGroupCols <= kTcTmemCols, "TMEM of the inference kernel");
 constexpr int kTcSpinLimit = 1 << 20;
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
@@ -593,32 +598,41 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity)
         if (mbar_try_wait(bar, parity)) return true;
     return false;
 }
-__device__ __forceinline__ void tc_ld16(uint32_t taddr, float (&v)[16]) {
-    uint32_t r[16];
+// A from TMEM (two BF16 per column), B from shared memory.
+__device__ __forceinline__ void tc_mma_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc) {
     asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr));
-#pragma unroll
-    for (int k = 0; k < 16; ++k) v[k] = __uint_as_float(r[k]);
+        "{\n\t.reg .pred p;\n\tsetp.eq.b32 p, 0, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(tmem_d),
+        "r"(tmem_a), "l"(db), "r"(idesc));
 }
-__device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-// 16 consecutive accumulator columns of this thread's TMEM lane from a
-// 16-byte aligned shared-memory array (four 16-byte loads)
-__device__ __forceinline__ void tc_st16_smem(uint32_t taddr, const float *src) {
-    const float4 *p = reinterpret_cast<const float4 *>(src);
-    const float4 a = p[0], b = p[1], c = p[2], d = p[3];
-    const float v[16] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y, c.z, c.w, d.x, d.y, d.z, d.w};
+// 32 consecutive columns of this thread's TMEM lane
+__device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&r)[32]) {
     asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(
-            taddr),
-        "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])), "r"(__float_as_uint(v[3])),
-        "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])), "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7])),
-        "r"(__float_as_uint(v[8])), "r"(__float_as_uint(v[9])), "r"(__float_as_uint(v[10])),
-        "r"(__float_as_uint(v[11])), "r"(__float_as_uint(v[12])), "r"(__float_as_uint(v[13])),
-        "r"(__float_as_uint(v[14])), "r"(__float_as_uint(v[15]))
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr));
+}
+__device__ __forceinline__ void tc_st32(uint32_t taddr, const uint32_t (&r)[32]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(taddr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
         : "memory");
+}
+__device__ __forceinline__ void tc_ld4(uint32_t taddr, uint32_t (&r)[4]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(taddr));
+}
+// Waits for the thread's TMEM loads; the registers pass through, so that no use
+// of them moves above the wait.
+__device__ __forceinline__ void tc_wait_ld(uint32_t (&r)[32]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]), "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]), "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31])
+                 :
+                 : "memory");
+}
+__device__ __forceinline__ void tc_wait_ld(uint32_t (&r)[4]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]) : : "memory");
 }
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // max(lo, 0) and max(hi, 0) rounded to BF16 and packed (lo in the low half):
@@ -636,13 +650,83 @@ __device__ __forceinline__ void group_sync(int group) {
     asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "r"(kTcRows) : "memory");
 }
 
+// Two-wide FP32 arithmetic (each half rounded as the scalar instruction).
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    uint64_t x, y, d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "f"(a.x), "f"(a.y));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(y) : "f"(b.x), "f"(b.y));
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(x), "l"(y));
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(d));
+    return r;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    uint64_t x, y, d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "f"(a.x), "f"(a.y));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(y) : "f"(b.x), "f"(b.y));
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(x), "l"(y));
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(d));
+    return r;
+}
+
+// encode_row's 96 features of one row into the K = 96 input tile: the same
+// operations, axes 0 and 1 two at a time, each eight features stored as they
+// are ready.
+__device__ __forceinline__ void encode_to_tile(const rt_cache_input &in, const float (&lo)[3], const float (&ext)[3],
+                                               uint8_t *tile, int r) {
+    float s[3], c[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const float pn = ext[a] > 0.0f ? (in.pos[a] - lo[a]) / ext[a] : 0.0f;
+        sincospif(pn, &s[a], &c[a]);
+    }
+    auto put = [&](int kc, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+        *reinterpret_cast<uint4 *>(tile + tc_off(r, 8 * kc, 96)) = make_uint4(x, y, z, w);
+    };
+    {
+        float2 sv = make_float2(s[0], s[1]), cv = make_float2(c[0], c[1]);
+#pragma unroll
+        for (int kc = 0; kc < 3; ++kc) {
+            uint32_t p0[4], p1[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                p0[k] = pack_bf16(sv.x, cv.x);
+                p1[k] = pack_bf16(sv.y, cv.y);
+                const float2 s2 = mul2(mul2(make_float2(2.0f, 2.0f), sv), cv);
+                const float2 c2 = mul2(add2(cv, make_float2(-sv.x, -sv.y)), add2(cv, sv));
+                sv = s2;
+                cv = c2;
+            }
+            put(kc, p0[0], p0[1], p0[2], p0[3]);
+            put(3 + kc, p1[0], p1[1], p1[2], p1[3]);
+        }
+    }
+    float s1 = s[2], c1 = c[2];
+#pragma unroll
+    for (int kc = 0; kc < 3; ++kc) {
+        uint32_t p[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            p[k] = pack_bf16(s1, c1);
+            const float s2 = 2.0f * s1 * c1, c2 = (c1 - s1) * (c1 + s1);
+            s1 = s2;
+            c1 = c2;
+        }
+        put(6 + kc, p[0], p[1], p[2], p[3]);
+    }
+    put(9, pack_bf16(in.dir[0], in.dir[1]), pack_bf16(in.dir[2], in.normal[0]), pack_bf16(in.normal[1], in.normal[2]),
+        pack_bf16(in.albedo[0], in.albedo[1]));
+    put(10, pack_bf16(in.albedo[2], 0.0f), 0u, 0u, 0u);
+    put(11, 0u, 0u, 0u, 0u);
+}
+
 __global__ void __launch_bounds__(kTcThreads, 1) k_cache_query_tc(const CacheState *S, const rt_cache_input *in,
                                                                   float4 *out, uint32_t n, const uint32_t *n_dev,
                                                                   uint32_t *err) {
     if (n_dev) n = min(n, *n_dev);
     extern __shared__ __align__(16) uint8_t smem[];
     uint8_t *sW = smem;
-    float *sB = reinterpret_cast<float *>(smem + kTcBias);
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + kTcBar);
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + kTcBar + 8u * kTcGroups);
     // per group: set by a thread whose barrier wait ran out, before the
@@ -651,22 +735,31 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_cache_query_tc(const CacheSta
     __shared__ int s_gfail[kTcGroups];
     const int tid = threadIdx.x, warp = tid >> 5;
     const int group = tid / kTcRows, gtid = tid % kTcRows;
-    uint8_t *gsm = smem + kTcGroupBase + (uint32_t)group * kTcGroupBytes;
+    uint8_t *tile_a = smem + kTcGroupBase + (uint32_t)group * kTcGroupBytes;
 
-    // ---- weights (canonical K-major) and biases into shared memory, once
-    for (int l = 0; l < kLayers; ++l) {
-        const int kin = in_dim(l), nout = l == 5 ? 16 : 64, nreal = out_dim(l);
-        const __nv_bfloat16 *gw = S->wbf + w_off(l);
-        __nv_bfloat16 *dst = reinterpret_cast<__nv_bfloat16 *>(sW + tc_w_off(l));
-        for (int e = tid; e < nout * kin; e += kTcThreads) {
-            const int o = e / kin, i = e % kin;
-            dst[tc_off(o, i, kin) / 2] = o < nreal ? gw[o * kin + i] : __float2bfloat16(0.0f);
-        }
+    // ---- weights (canonical K-major, eight inputs of an output per 16-byte
+    // chunk), the split biases and the ones, once
+    constexpr int kChunks = 64 * 12 + 4 * 64 * 8 + 16 * 8;
+    for (int e = tid; e < kChunks; e += kTcThreads) {
+        int l, o, c;
+        train_chunk(e, l, o, c);
+        uint4 w = make_uint4(0u, 0u, 0u, 0u);
+        if (o < out_dim(l)) w = __ldg(reinterpret_cast<const uint4 *>(S->wbf + w_off(l)) + o * (in_dim(l) / 8) + c);
+        *reinterpret_cast<uint4 *>(sW + tc_w_off(l) + tc_off(o, 8 * c, in_dim(l))) = w;
     }
     for (int e = tid; e < 336; e += kTcThreads) {
         const int l = e < 320 ? e / 64 : 5, o = e < 320 ? e % 64 : e - 320;
-        sB[e] = o < out_dim(l) ? S->params[b_off(l) + o] : 0.0f;
+        const float b = o < out_dim(l) ? S->params[b_off(l) + o] : 0.0f;
+        // hi + mid + lo == b: 8 significant bits each of its 24
+        const float hi = __bfloat162float(__float2bfloat16(b)), r1 = b - hi;
+        const float mid = __bfloat162float(__float2bfloat16(r1)), r2 = r1 - mid;
+        uint8_t *dst = smem + tc_bias_off(l) + tc_off(o, 0, 16);
+        *reinterpret_cast<uint4 *>(dst) = make_uint4(pack_bf16(hi, mid), pack_bf16(r2, 0.0f), 0u, 0u);
+        *reinterpret_cast<uint4 *>(dst + 128) = make_uint4(0u, 0u, 0u, 0u);
     }
+    for (int e = tid; e < kTcRows * 2; e += kTcThreads)
+        *reinterpret_cast<uint4 *>(smem + kTcOnes + 16 * e) =
+            make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
     if (tid < kTcGroups) s_gfail[tid] = 0;
     if (tid == 0) {
         for (int g = 0; g < kTcGroups; ++g)
@@ -686,39 +779,37 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_cache_query_tc(const CacheSta
     tc_fence_after();
     // this group's accumulator columns; warp w of the group reads TMEM lanes
     // [32 (w % 4), 32 (w % 4) + 32)
-    const uint32_t tmem = *tmem_slot + 64u * (uint32_t)group;
+    const uint32_t tmem = *tmem_slot + kTcGroupCols * (uint32_t)group;
     const uint32_t bar_a = smem_u32(bars + group);
     const uint32_t w_base = smem_u32(sW);
+    // operand descriptors (the address field counts 16 bytes; a step of K = 16
+    // is 256): ones, biases, input tile, weights of layer 0 and from layer 1 on
+    const uint64_t d_ones = tc_desc(w_base + kTcOnes, 128u, 256u), d_bias = tc_desc(w_base + kTcBias, 128u, 256u);
+    const uint64_t d_in = tc_desc(smem_u32(tile_a), 128u, 16u * 96u), d_w0 = tc_desc(w_base, 128u, 16u * 96u);
+    const uint64_t d_w1 = tc_desc(w_base + tc_w_off(1), 128u, 16u * 64u);
     uint32_t phase = 0;
     volatile int *gfail = s_gfail + group;
     const uint32_t tiles = (n + kTcRows - 1) / kTcRows;
     const uint32_t lane_base = (uint32_t)(32 * (warp & 3)) << 16;
+    float lo[3], ext[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        lo[a] = S->lo[a];
+        ext[a] = S->hi[a] - S->lo[a];
+    }
 
-    // The groups run independently (own tiles, buffers, barrier, phase): the
-    // tensor core works on one group's layer while the others encode or run
-    // their epilogues.
+    // The groups run independently (own tiles, buffers, barrier, phase); tiles
+    // go to the SMs before they go to the groups of one.
     // this thread's input row of the group's next tile, loaded one tile ahead
     const uint32_t tile_stride = gridDim.x * kTcGroups;
-    uint32_t tile = blockIdx.x * kTcGroups + (uint32_t)group;
-    rt_cache_input cur;
+    uint32_t tile = blockIdx.x + gridDim.x * (uint32_t)group;
+    rt_cache_input cur = {};
     if (tile < tiles && tile * kTcRows + (uint32_t)gtid < n) cur = in[tile * kTcRows + (uint32_t)gtid];
     for (; tile < tiles; tile += tile_stride) {
-        // ---- encode this thread's row into the K = 96 input tile
+        // ---- encode this thread's row into the K = 96 input tile (a row past
+        // the end encodes whatever the thread holds: its output is dropped)
         const uint32_t row = tile * kTcRows + (uint32_t)gtid;
-        {
-            __align__(16) __nv_bfloat16 feat[96];
-            if (row < n) {
-                encode_row(cur, S, feat);
-            } else {
-                for (int k = 0; k < 96; ++k) feat[k] = __float2bfloat16(0.0f);
-            }
-            for (int kc = 0; kc < 12; ++kc)
-                *reinterpret_cast<uint4 *>(gsm + kTcA0 + tc_off(gtid, 8 * kc, 96)) =
-                    *reinterpret_cast<const uint4 *>(feat + 8 * kc);
-        }
-        // layer 0's bias into this row's accumulators: the MMAs add onto it
-        for (int c16 = 0; c16 < 4; ++c16) tc_st16_smem(tmem + lane_base + 16u * c16, sB + 16 * c16);
-        tc_wait_st();
+        encode_to_tile(cur, lo, ext, tile_a, gtid);
         {
             const uint32_t nrow = (tile + tile_stride) * kTcRows + (uint32_t)gtid;
             if (tile + tile_stride < tiles && nrow < n) cur = in[nrow];  // in flight during the layers
@@ -727,71 +818,65 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_cache_query_tc(const CacheSta
         tc_fence_before();
         group_sync(group);
         tc_fence_after();
+        if (*gfail) break;  // read after the barrier: the same for the whole group
+        bool failed = false;
 #pragma unroll 1
         for (int l = 0; l < kLayers; ++l) {
-            const int kin = in_dim(l);
-            const uint32_t a_base = smem_u32(gsm + (l == 0 ? kTcA0 : ((l & 1) ? kTcH0 : kTcH1)));
-            const uint32_t b_base = w_base + tc_w_off(l);
-            // the issuing thread alone waits for the MMAs; the rest of the
-            // group sleeps in the group barrier instead of polling
             if (gtid == 0) {
-                const uint32_t idesc = tc_idesc(kTcRows, l == 5 ? 16 : 64);
-                for (int ks = 0; ks < kin / 16; ++ks) {
-                    const uint64_t da = tc_desc(a_base + 256u * ks, 128u, 16u * kin);
-                    const uint64_t db = tc_desc(b_base + 256u * ks, 128u, 16u * kin);
-                    tc_mma(tmem, da, db, idesc, 1u);  // onto the bias
+                const uint32_t idesc = l == 5 ? tc_idesc(kTcRows, 16) : tc_idesc(kTcRows, 64);
+                // accumulators = bias
+                tc_mma(tmem, d_ones, d_bias + (uint32_t)l * (tc_tile_bytes(64, 16) >> 4), idesc, 0u);
+                if (l == 0) {
+#pragma unroll
+                    for (uint32_t ks = 0; ks < 6u; ++ks) tc_mma(tmem, d_in + 16u * ks, d_w0 + 16u * ks, idesc, 1u);
+                } else {
+                    const uint64_t db = d_w1 + (uint32_t)(l - 1) * (tc_tile_bytes(64, 64) >> 4);
+#pragma unroll
+                    for (uint32_t ks = 0; ks < 4u; ++ks) tc_mma_ta(tmem, tmem + kTcACol + 8u * ks, db + 16u * ks, idesc);
                 }
                 tc_commit(bar_a);
-                if (!mbar_wait_bounded(bar_a, phase)) {
-                    report_error(err, RT_ERR_TIMEOUT, 0x90000000u | (uint32_t)l);
-                    mbar_wait_bounded(bar_a, phase);  // once more: no MMA may outlive the TMEM
-                    *gfail = 1;
-                }
-                tc_fence_before();
+            }
+            if (!mbar_wait_bounded(bar_a, phase)) {
+                report_error(err, RT_ERR_TIMEOUT, 0x90000000u | (uint32_t)l);
+                mbar_wait_bounded(bar_a, phase);  // once more: no MMA may outlive the TMEM
+                *gfail = 1;
             }
             phase ^= 1u;
-            group_sync(group);
+            __syncwarp();
             tc_fence_after();
-            if (*gfail) break;  // read after the barrier: the same for the whole group
             if (l < 5) {
-                // hidden layer: ReLU -> BF16 row of the next A tile; the
-                // next layer's bias replaces each column group once read
-                uint8_t *next = gsm + ((l & 1) ? kTcH1 : kTcH0);
-                const float *nbias = sB + 64 * (l + 1);
+                // hidden layer: ReLU -> BF16 row, the next layer's A
+                uint32_t v0[32], v1[32], p[32];
+                tc_ld32(tmem + lane_base, v0);
+                tc_ld32(tmem + lane_base + 32u, v1);
+                tc_wait_ld(v0);
+                tc_wait_ld(v1);
 #pragma unroll
-                for (int c32 = 0; c32 < 2; ++c32) {
-                    // two 16-column loads in flight per wait
-                    float v[2][16];
-                    tc_ld16(tmem + lane_base + 32u * c32, v[0]);
-                    tc_ld16(tmem + lane_base + 32u * c32 + 16u, v[1]);
-                    tc_wait_ld();
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const int c16 = 2 * c32 + h;
-                        if (l < 4 || c16 == 0) tc_st16_smem(tmem + lane_base + 16u * c16, nbias + 16 * c16);
-                        uint32_t packed[8];
-#pragma unroll
-                        for (int k = 0; k < 8; ++k) packed[k] = relu_pack_bf16(v[h][2 * k], v[h][2 * k + 1]);
-                        *reinterpret_cast<uint4 *>(next + tc_off(gtid, 16 * c16, 64)) =
-                            make_uint4(packed[0], packed[1], packed[2], packed[3]);
-                        *reinterpret_cast<uint4 *>(next + tc_off(gtid, 16 * c16 + 8, 64)) =
-                            make_uint4(packed[4], packed[5], packed[6], packed[7]);
-                    }
+                for (int k = 0; k < 16; ++k) {
+                    p[k] = relu_pack_bf16(__uint_as_float(v0[2 * k]), __uint_as_float(v0[2 * k + 1]));
+                    p[16 + k] = relu_pack_bf16(__uint_as_float(v1[2 * k]), __uint_as_float(v1[2 * k + 1]));
                 }
+                tc_st32(tmem + lane_base + kTcACol, p);
                 tc_wait_st();
             } else {
-                float v[16];
-                tc_ld16(tmem + lane_base, v);
-                tc_wait_ld();
-                if (row < n) out[row] = make_float4(v[0], v[1], v[2], 0.0f);
+                uint32_t v[4];
+                tc_ld4(tmem + lane_base, v);
+                tc_wait_ld(v);
+                if (row < n)
+                    out[row] = make_float4(__uint_as_float(v[0]), __uint_as_float(v[1]), __uint_as_float(v[2]), 0.0f);
             }
-            fence_async_smem();
-            tc_fence_before();
-            group_sync(group);
-            tc_fence_after();
-            if (*gfail) break;
+            if (l < 5) {
+                tc_fence_before();
+                group_sync(group);
+                tc_fence_after();
+                failed = *gfail != 0;
+                if (failed) break;
+            }
         }
-        if (*gfail) break;
+        if (failed) break;
+        // the next tile's encoding may overwrite the input tile (layer 0 has
+        // read it), and the barrier after it orders this tile's last TMEM
+        // reads before the next MMAs
     }
     // ---- teardown: every MMA has been waited for (a group that gave up
     // waited once more); free the TMEM
@@ -938,9 +1023,9 @@ extern "C" rt_status rt_cache_query(rt_context *ctx, rt_stream stream, const voi
     if (n == 0) return RT_OK;
     int rc = set_smem(ctx);
     if (rc) return rc;
-    const uint32_t groups = (n + kQueryRows * kTcGroups - 1) / (kQueryRows * kTcGroups);
+    const uint32_t tiles = (n + kTcRows - 1) / kTcRows;
     uint32_t grid = (uint32_t)ctx->sm_count;
-    if (grid > groups) grid = groups;
+    if (grid > tiles) grid = tiles;
     k_cache_query_tc<<<grid, kTcThreads, kTcSmem, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const CacheState *>(cache), in, reinterpret_cast<float4 *>(out), n, nullptr, ctx->d_err);
     RT_CUDA_CTX(ctx, cudaGetLastError());
@@ -1088,9 +1173,9 @@ int cache_query_dev(rt_context *ctx, cudaStream_t st, const void *cache, const r
     if (max_n == 0) return RT_OK;
     int rc = set_smem(ctx);
     if (rc) return rc;
-    const uint32_t groups = (max_n + kQueryRows * kTcGroups - 1) / (kQueryRows * kTcGroups);
+    const uint32_t tiles = (max_n + kTcRows - 1) / kTcRows;
     uint32_t grid = (uint32_t)ctx->sm_count;
-    if (grid > groups) grid = groups;
+    if (grid > tiles) grid = tiles;
     k_cache_query_tc<<<grid, kTcThreads, kTcSmem, st>>>(static_cast<const CacheState *>(cache), in,
                                                  reinterpret_cast<float4 *>(out), max_n, n_dev, ctx->d_err);
     RT_CUDA_CTX(ctx, cudaGetLastError());
