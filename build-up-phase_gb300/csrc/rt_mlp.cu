@@ -178,9 +178,11 @@ __device__ void encode_row(const rt_cache_input &in, const CacheState *S, __nv_b
 // kernel before it to complete (its writes visible) before it reads or
 // writes anything, so a launch's scheduling overlaps the previous kernel's
 // tail.  Launched without the attribute both instructions do nothing.
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_enter() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    pdl_launch();
+    pdl_wait();
 }
 
 constexpr int kTrainRows = 128;
@@ -277,10 +279,10 @@ __device__ __forceinline__ void warp_dense_wt(const uint32_t (&a)[KS][4], const 
     }
 }
 
-// dW[o][i] += sum_r delta[r][o] * A[r][i] over the tile's 128 rows for the
+// dW[o][i] += sum_r delta[r][o] * A[r][i] over the tile's ROWS rows for the
 // outputs [o0, o0 + 16) and NT n-tiles of inputs from i0, on the tensor
 // cores; rows o >= OUT (padding) are dropped.
-template <int IN, int OUT, int NT>
+template <int IN, int OUT, int NT, int ROWS>
 __device__ __forceinline__ void warp_grad_w(const __nv_bfloat16 *sD, const __nv_bfloat16 *sA, int as, int o0, int i0,
                                             float *gW, float *gb, int lane) {
     const int row = lane & 7, mat = lane >> 3, g = lane >> 2, q = lane & 3;
@@ -288,7 +290,7 @@ __device__ __forceinline__ void warp_grad_w(const __nv_bfloat16 *sD, const __nv_
 #pragma unroll
     for (int j = 0; j < NT; ++j) c[j][0] = c[j][1] = c[j][2] = c[j][3] = 0.0f;
 #pragma unroll 2
-    for (int ks = 0; ks < kTrainRows / 16; ++ks) {
+    for (int ks = 0; ks < ROWS / 16; ++ks) {
         const int r = 16 * ks;
         // A = delta^T (m = output, k = row): matrices (rows r..r+7 | r+8..r+15) x (o0.. | o0+8..)
         uint32_t a[4];
@@ -333,23 +335,24 @@ __device__ __forceinline__ void warp_grad_w(const __nv_bfloat16 *sD, const __nv_
 // warps whose input range reaches it take one more n-tile and the MMAs leave
 // the bias gradient sum_r delta[r][o] there: no separate row loop (it held two
 // warps for ~2 us per layer while the block waited at its barrier).
+template <int ROWS>
 __device__ __forceinline__ void grads_of_layer(int L, const __nv_bfloat16 *sD, const __nv_bfloat16 *ain, int as,
                                                float *grads, int warp, int lane) {
     if (L == 0) {
         if (warp >> 2)
-            warp_grad_w<96, 64, 8>(sD, ain, as, 16 * (warp & 3), 48, grads + w_off(0), grads + b_off(0), lane);
+            warp_grad_w<96, 64, 8, ROWS>(sD, ain, as, 16 * (warp & 3), 48, grads + w_off(0), grads + b_off(0), lane);
         else
-            warp_grad_w<96, 64, 6>(sD, ain, as, 16 * (warp & 3), 0, grads + w_off(0), grads + b_off(0), lane);
+            warp_grad_w<96, 64, 6, ROWS>(sD, ain, as, 16 * (warp & 3), 0, grads + w_off(0), grads + b_off(0), lane);
     } else if (L == 5) {
         if (warp == 7)
-            warp_grad_w<64, 8, 2>(sD, ain, as, 0, 56, grads + w_off(5), grads + b_off(5), lane);
+            warp_grad_w<64, 8, 2, ROWS>(sD, ain, as, 0, 56, grads + w_off(5), grads + b_off(5), lane);
         else
-            warp_grad_w<64, 8, 1>(sD, ain, as, 0, 8 * warp, grads + w_off(5), grads + b_off(5), lane);
+            warp_grad_w<64, 8, 1, ROWS>(sD, ain, as, 0, 8 * warp, grads + w_off(5), grads + b_off(5), lane);
     } else {
         if (warp >> 2)
-            warp_grad_w<64, 64, 6>(sD, ain, as, 16 * (warp & 3), 32, grads + w_off(L), grads + b_off(L), lane);
+            warp_grad_w<64, 64, 6, ROWS>(sD, ain, as, 16 * (warp & 3), 32, grads + w_off(L), grads + b_off(L), lane);
         else
-            warp_grad_w<64, 64, 4>(sD, ain, as, 16 * (warp & 3), 0, grads + w_off(L), grads + b_off(L), lane);
+            warp_grad_w<64, 64, 4, ROWS>(sD, ain, as, 16 * (warp & 3), 0, grads + w_off(L), grads + b_off(L), lane);
     }
 }
 
@@ -359,7 +362,8 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_cache_fwd_bwd(CacheState *
                                                                     const float4 *targets, uint32_t n,
                                                                     float inv_count, const uint32_t *n_dev,
                                                                     uint32_t row0, uint32_t bump_step) {
-    pdl_enter();
+    pdl_wait();
+    pdl_launch();
     if (bump_step && blockIdx.x == 0 && threadIdx.x == 0) S->step += 1u;
     if (n_dev) {
         // rows [row0, row0 + n) of a set whose size is produced on the device
@@ -457,7 +461,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_cache_fwd_bwd(CacheState *
             __syncthreads();  // delta_L and every activation complete
             const __nv_bfloat16 *ain = L == 0 ? sIn : sAct + (L - 1) * kTrainRows * kActStride;
             const int as = L == 0 ? kInStride : kActStride;
-            grads_of_layer(L, sD, ain, as, S->grads, warp, lane);
+            grads_of_layer<kTrainRows>(L, sD, ain, as, S->grads, warp, lane);
             if (L == 0) break;
             // delta_{L-1} = (delta_L W_L) * relu'(act_{L-1})
             float dc[8][4];
@@ -499,6 +503,214 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_cache_fwd_bwd(CacheState *
     // block loss -> state (mean over samples and channels)
     for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
     if (lane == 0) atomicAdd(&S->loss, loss * inv_count);
+}
+
+// ---------------------------------------------------------------------------
+// Small batches: tiles of 32 or 64 rows
+// ---------------------------------------------------------------------------
+//
+// A batch is one chain of layer steps per tile, and a batch of 4,096 rows is 32
+// tiles of 128: most SMs idle, and each warp runs 32 MMAs per layer step and as
+// many for its weight gradients.  With smaller tiles a layer step is split over
+// the eight warps by rows and columns (16 x 16 outputs each with 32 rows, 16 x
+// 32 with 64), the activations passing through shared memory, so the chain is
+// shorter and more SMs work; the price is a tile's 23,368 gradient reductions,
+// which more tiles do more often.  The deltas alternate between two buffers, so
+// a backward step has one barrier.  Every output sums in the order of the
+// 128-row kernel.
+//
+// 65,536 samples, us at tiles of 128 / 64 / 32 rows: batches of 1,024 1,208 /
+// 952 / 810; 4,096 310 / 245 / 276 (45 of them the reductions); 8,192 161 / 140
+// / 154; 16,384 89 / 122 / 145.  (The sums of four blocks added up in a cluster
+// first: 1,042 and 280 at 1,024 and 4,096 with 32 rows.)
+
+constexpr size_t small_smem(int rows) {
+    return (size_t)kTwElems * 2 + (size_t)kBiasFloats * 4 + (size_t)rows * kInStride * 2 +
+           (size_t)5 * rows * kActStride * 2 + (size_t)2 * rows * kDStride * 2;
+}
+static_assert(small_smem(64) <= 227u * 1024u, "shared memory of the small-batch kernel");
+
+// encode_row's features of a tile's rows, four or eight lanes per row: lanes 0-2
+// an axis each, lane 3 the rest.
+template <int ROWS>
+__device__ __forceinline__ void encode_small(const rt_cache_input *in, uint32_t row0, uint32_t n, const CacheState *S,
+                                             __nv_bfloat16 *sIn) {
+    constexpr uint32_t kLanes = kTrainThreads / ROWS;
+    const uint32_t r = threadIdx.x / kLanes, part = threadIdx.x % kLanes, row = row0 + r;
+    if (part > 3u) return;
+    uint32_t *dst = reinterpret_cast<uint32_t *>(sIn + r * kInStride + 24u * part);
+    if (row >= n) {
+#pragma unroll
+        for (int k = 0; k < 12; ++k) dst[k] = 0u;
+        return;
+    }
+    if (part < 3u) {
+        const float lo = S->lo[part], ext = S->hi[part] - lo;
+        const float pn = ext > 0.0f ? (in[row].pos[part] - lo) / ext : 0.0f;
+        float s, c;
+        sincospif(pn, &s, &c);
+#pragma unroll
+        for (int k = 0; k < 12; ++k) {
+            dst[k] = pack_bf16(s, c);
+            const float s2 = 2.0f * s * c, c2 = (c - s) * (c + s);
+            s = s2;
+            c = c2;
+        }
+    } else {
+        const rt_cache_input x = in[row];
+        dst[0] = pack_bf16(x.dir[0], x.dir[1]);
+        dst[1] = pack_bf16(x.dir[2], x.normal[0]);
+        dst[2] = pack_bf16(x.normal[1], x.normal[2]);
+        dst[3] = pack_bf16(x.albedo[0], x.albedo[1]);
+        dst[4] = pack_bf16(x.albedo[2], 0.0f);
+#pragma unroll
+        for (int k = 5; k < 12; ++k) dst[k] = 0u;
+    }
+}
+
+// after_adam: the launch before is this training call's own Adam step, so the
+// inputs were there before it and are encoded while it still runs.
+template <int ROWS>
+__global__ void __launch_bounds__(kTrainThreads, 1) k_cache_fwd_bwd_small(CacheState *S, const rt_cache_input *in,
+                                                                          const float4 *targets, uint32_t n,
+                                                                          float inv_count, const uint32_t *n_dev,
+                                                                          uint32_t row0, uint32_t bump_step,
+                                                                          uint32_t after_adam) {
+    constexpr int kSmallSlabs = ROWS / 16;  // 16-row slabs; also a warp's 8-column tiles
+    constexpr int kSmallNt = kSmallSlabs;
+    extern __shared__ __align__(16) uint8_t smem[];
+    __nv_bfloat16 *sW = reinterpret_cast<__nv_bfloat16 *>(smem);
+    float *sB = reinterpret_cast<float *>(sW + kTwElems);
+    __nv_bfloat16 *sIn = reinterpret_cast<__nv_bfloat16 *>(sB + kBiasFloats);
+    __nv_bfloat16 *sAct = sIn + ROWS * kInStride;
+    __nv_bfloat16 *sDelta = sAct + 5 * ROWS * kActStride;
+    {
+        // the ones columns of the bias gradients (row padding, never written otherwise)
+        const uint4 ones = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
+        for (int e = threadIdx.x; e < 6 * ROWS; e += kTrainThreads) {
+            const int t = e / ROWS, r = e % ROWS;
+            if (t == 0) *reinterpret_cast<uint4 *>(sIn + r * kInStride + 96) = ones;
+            else *reinterpret_cast<uint4 *>(sAct + (t - 1) * ROWS * kActStride + r * kActStride + 64) = ones;
+        }
+    }
+    if (!after_adam) pdl_wait();
+    if (n_dev) {
+        // rows [row0, row0 + n) of a set whose size is produced on the device
+        const uint32_t total = *n_dev;
+        n = total > row0 ? min(n, total - row0) : 0u;
+        in += row0;
+        targets += row0;
+        inv_count = 1.0f / (3.0f * (float)n);
+    }
+    const uint32_t tiles = (n + ROWS - 1) / ROWS;
+    if (blockIdx.x < tiles) encode_small<ROWS>(in, blockIdx.x * ROWS, n, S, sIn);
+    if (after_adam) pdl_wait();
+    pdl_launch();
+    if (bump_step && blockIdx.x == 0 && threadIdx.x == 0) S->step += 1u;
+    if (blockIdx.x >= tiles) return;
+    load_weights_train(S, sW, sB);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int g = lane >> 2, q = lane & 3;
+    const int r0 = 16 * (warp % kSmallSlabs), col0 = 8 * kSmallNt * (warp / kSmallSlabs);  // this warp's rows and columns
+    float loss = 0.0f;
+    for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        if (tile != blockIdx.x) {
+            __syncthreads();
+            encode_small<ROWS>(in, tile * ROWS, n, S, sIn);
+        }
+        __syncthreads();
+        // ---- forward, keeping post-activations for the backward pass
+        auto store2 = [&](__nv_bfloat16 *m, int stride, const float (&c)[kSmallNt][4], bool relu) {
+#pragma unroll
+            for (int j = 0; j < kSmallNt; ++j) {
+                const float x0 = relu ? fmaxf(c[j][0], 0.0f) : c[j][0], x1 = relu ? fmaxf(c[j][1], 0.0f) : c[j][1];
+                const float x2 = relu ? fmaxf(c[j][2], 0.0f) : c[j][2], x3 = relu ? fmaxf(c[j][3], 0.0f) : c[j][3];
+                *reinterpret_cast<uint32_t *>(m + (r0 + g) * stride + col0 + 8 * j + 2 * q) = pack_bf16(x0, x1);
+                *reinterpret_cast<uint32_t *>(m + (r0 + g + 8) * stride + col0 + 8 * j + 2 * q) = pack_bf16(x2, x3);
+            }
+        };
+        {
+            uint32_t a0[6][4];
+            load_a<6>(sIn, kInStride, r0, lane, a0);
+            float c[kSmallNt][4];
+            warp_dense<6, kSmallNt>(a0, sW + tw_off(0) + col0 * w_stride(0), w_stride(0), sB + col0, c, lane);
+            store2(sAct, kActStride, c, true);
+        }
+#pragma unroll 1
+        for (int l = 1; l <= 4; ++l) {
+            __syncthreads();
+            uint32_t a[4][4];
+            load_a<4>(sAct + (l - 1) * ROWS * kActStride, kActStride, r0, lane, a);
+            float c[kSmallNt][4];
+            warp_dense<4, kSmallNt>(a, sW + tw_off(l) + col0 * w_stride(l), w_stride(l), sB + 64 * l + col0, c, lane);
+            store2(sAct + l * ROWS * kActStride, kActStride, c, true);
+        }
+        __syncthreads();
+        if (warp < kSmallSlabs) {
+            uint32_t a[4][4];
+            load_a<4>(sAct + 4 * ROWS * kActStride, kActStride, r0, lane, a);
+            float y[1][4];
+            warp_dense<4, 1>(a, sW + tw_off(5), w_stride(5), sB + 320, y, lane);
+            // ---- loss gradient at the outputs (cols 0..2 of each row);
+            // delta_5 as BF16 (cols 0..15, 3..15 zero)
+            float dy[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int rr = r0 + g + (e >= 2 ? 8 : 0), col = 2 * q + (e & 1);
+                const uint32_t row = tile * ROWS + rr;
+                dy[e] = 0.0f;
+                if (col < 3 && row < n) {
+                    const float4 tg = targets[row];
+                    const float yt = col == 0 ? tg.x : (col == 1 ? tg.y : tg.z);
+                    const float diff = y[0][e] - yt, den = y[0][e] * y[0][e] + 0.01f;
+                    dy[e] = 2.0f * diff / den * inv_count;
+                    loss += diff * diff / den;
+                }
+            }
+            *reinterpret_cast<uint32_t *>(sDelta + (r0 + g) * kDStride + 2 * q) = pack_bf16(dy[0], dy[1]);
+            *reinterpret_cast<uint32_t *>(sDelta + (r0 + g + 8) * kDStride + 2 * q) = pack_bf16(dy[2], dy[3]);
+            *reinterpret_cast<uint32_t *>(sDelta + (r0 + g) * kDStride + 8 + 2 * q) = 0u;
+            *reinterpret_cast<uint32_t *>(sDelta + (r0 + g + 8) * kDStride + 8 + 2 * q) = 0u;
+        }
+        // ---- backward, layers 5 .. 0
+#pragma unroll 1
+        for (int L = 5; L >= 0; --L) {
+            __syncthreads();  // delta_L complete; the other buffer is free
+            const __nv_bfloat16 *dcur = sDelta + ((L + 1) & 1) * ROWS * kDStride;
+            __nv_bfloat16 *dnext = sDelta + (L & 1) * ROWS * kDStride;
+            const __nv_bfloat16 *ain = L == 0 ? sIn : sAct + (L - 1) * ROWS * kActStride;
+            const int as = L == 0 ? kInStride : kActStride;
+            if (L > 0) {
+                // delta_{L-1} = (delta_L W_L) * relu'(act_{L-1}), first: the next step waits for it
+                float dc[kSmallNt][4];
+                if (L == 5) {
+                    uint32_t a1[1][4];
+                    load_a<1>(dcur, kDStride, r0, lane, a1);
+                    warp_dense_wt<1, kSmallNt>(a1, sW + tw_off(5) + col0, w_stride(5), dc, lane);
+                } else {
+                    uint32_t ad[4][4];
+                    load_a<4>(dcur, kDStride, r0, lane, ad);
+                    warp_dense_wt<4, kSmallNt>(ad, sW + tw_off(L) + col0, w_stride(L), dc, lane);
+                }
+#pragma unroll
+                for (int j = 0; j < kSmallNt; ++j) {
+                    const __nv_bfloat162 m0 =
+                        *reinterpret_cast<const __nv_bfloat162 *>(ain + (r0 + g) * kActStride + col0 + 8 * j + 2 * q);
+                    const __nv_bfloat162 m1 = *reinterpret_cast<const __nv_bfloat162 *>(
+                        ain + (r0 + g + 8) * kActStride + col0 + 8 * j + 2 * q);
+                    if (!(__bfloat162float(m0.x) > 0.0f)) dc[j][0] = 0.0f;
+                    if (!(__bfloat162float(m0.y) > 0.0f)) dc[j][1] = 0.0f;
+                    if (!(__bfloat162float(m1.x) > 0.0f)) dc[j][2] = 0.0f;
+                    if (!(__bfloat162float(m1.y) > 0.0f)) dc[j][3] = 0.0f;
+                }
+                store2(dnext, kDStride, dc, false);
+            }
+            grads_of_layer<ROWS>(L, dcur, ain, as, S->grads, warp, lane);
+        }
+    }
+    // block loss -> state (mean over samples and channels)
+    for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
+    if (lane == 0 && warp < kSmallSlabs) atomicAdd(&S->loss, loss * inv_count);
 }
 
 // ---------------------------------------------------------------------------
@@ -892,8 +1104,17 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_cache_query_tc(const CacheSta
 // the k_cache_fwd_bwd launch before).  Thread 0 also hands the batch's mean
 // loss to loss_out and clears it for the next batch.
 __global__ void k_cache_adam(CacheState *S, float *loss_out) {
-    pdl_enter();
+    pdl_launch();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    // written by earlier Adam steps only, which were complete when the launch
+    // before this one (forward and backward) let this one start
+    float m0 = 0.0f, v0 = 0.0f, p0 = 0.0f;
+    if (i < kParams) {
+        m0 = __ldcg(S->m + i);
+        v0 = __ldcg(S->v + i);
+        p0 = __ldcg(S->params + i);
+    }
+    pdl_wait();
     if (i == 0) {
         if (loss_out) *loss_out = S->loss;
         S->loss = 0.0f;
@@ -901,13 +1122,13 @@ __global__ void k_cache_adam(CacheState *S, float *loss_out) {
     if (i >= kParams) return;
     const uint32_t t = S->step;
     const float g = S->grads[i];
-    const float m = S->beta1 * S->m[i] + (1.0f - S->beta1) * g;
-    const float v = S->beta2 * S->v[i] + (1.0f - S->beta2) * g * g;
+    const float m = S->beta1 * m0 + (1.0f - S->beta1) * g;
+    const float v = S->beta2 * v0 + (1.0f - S->beta2) * g * g;
     S->m[i] = m;
     S->v[i] = v;
     const float mh = m / (1.0f - powf(S->beta1, (float)t));
     const float vh = v / (1.0f - powf(S->beta2, (float)t));
-    const float p = S->params[i] - S->lr * mh / (sqrtf(vh) + S->eps);
+    const float p = p0 - S->lr * mh / (sqrtf(vh) + S->eps);
     S->params[i] = p;
     S->wbf[i] = __float2bfloat16(p);
     S->grads[i] = 0.0f;
@@ -938,18 +1159,34 @@ cudaError_t launch_pdl(void (*kernel)(KArgs...), unsigned grid, unsigned threads
 int set_smem(rt_context *ctx) {
     RT_CUDA_CTX(ctx, cudaFuncSetAttribute(k_cache_query_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem));
     RT_CUDA_CTX(ctx, cudaFuncSetAttribute(k_cache_fwd_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrainSmem));
+    RT_CUDA_CTX(ctx, cudaFuncSetAttribute(k_cache_fwd_bwd_small<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)small_smem(32)));
+    RT_CUDA_CTX(ctx, cudaFuncSetAttribute(k_cache_fwd_bwd_small<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)small_smem(64)));
     return RT_OK;
 }
 
+// One batch of at most n rows (n_dev: rows [row0, row0 + n) of *n_dev).
 int launch_fwd_bwd(rt_context *ctx, cudaStream_t st, CacheState *S, const rt_cache_input *in, const float *tg,
-                   uint32_t n, uint32_t bump_step) {
-    const uint32_t tiles = (n + kTrainRows - 1) / kTrainRows;
-    uint32_t grid = (uint32_t)ctx->sm_count;
-    if (grid > tiles) grid = tiles;
-    if (grid == 0) return RT_OK;
-    RT_CUDA_CTX(ctx, launch_pdl(k_cache_fwd_bwd, grid, kTrainThreads, kTrainSmem, st, S, in,
-                                reinterpret_cast<const float4 *>(tg), n, 1.0f / (3.0f * (float)n),
-                                static_cast<const uint32_t *>(nullptr), 0u, bump_step));
+                   uint32_t n, const uint32_t *n_dev, uint32_t row0, uint32_t bump_step, uint32_t after_adam) {
+    if (n == 0) return RT_OK;
+    const float inv = n_dev ? 0.0f : 1.0f / (3.0f * (float)n);
+    const float4 *t4 = reinterpret_cast<const float4 *>(tg);
+    const uint32_t sms = (uint32_t)ctx->sm_count;
+    // the shortest chain while its reductions are few, one wave of 64-row tiles
+    // while there is one (measured above the kernel)
+    const uint32_t tiles32 = (n + 31u) / 32u, tiles64 = (n + 63u) / 64u;
+    if (tiles32 <= 64u) {
+        RT_CUDA_CTX(ctx, launch_pdl(k_cache_fwd_bwd_small<32>, tiles32, kTrainThreads, small_smem(32), st, S, in, t4, n,
+                                    inv, n_dev, row0, bump_step, after_adam));
+    } else if (tiles64 <= sms) {
+        RT_CUDA_CTX(ctx, launch_pdl(k_cache_fwd_bwd_small<64>, tiles64, kTrainThreads, small_smem(64), st, S, in, t4, n,
+                                    inv, n_dev, row0, bump_step, after_adam));
+    } else {
+        const uint32_t tiles = (n + kTrainRows - 1) / kTrainRows;
+        RT_CUDA_CTX(ctx, launch_pdl(k_cache_fwd_bwd, tiles < sms ? tiles : sms, kTrainThreads, kTrainSmem, st, S, in,
+                                    t4, n, inv, n_dev, row0, bump_step));
+    }
     return RT_OK;
 }
 
@@ -1043,7 +1280,7 @@ extern "C" rt_status rt_cache_train(rt_context *ctx, rt_stream stream, void *cac
     CacheState *S = static_cast<CacheState *>(cache);
     for (uint32_t b = 0; b < n; b += batch) {
         const uint32_t m = (n - b) < batch ? (n - b) : batch;
-        rc = launch_fwd_bwd(ctx, st, S, in + b, targets + 4u * (size_t)b, m, 1u);
+        rc = launch_fwd_bwd(ctx, st, S, in + b, targets + 4u * (size_t)b, m, nullptr, 0u, 1u, b ? 1u : 0u);
         if (rc) return rc;
         RT_CUDA_CTX(ctx, launch_pdl(k_cache_adam, (kParams + 255) / 256, 256, 0, st, S, loss_out));
     }
@@ -1060,7 +1297,7 @@ extern "C" rt_status rt_cache_gradient(rt_context *ctx, rt_stream stream, void *
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     CacheState *S = static_cast<CacheState *>(cache);
     RT_CUDA_CTX(ctx, cudaMemsetAsync(S->grads, 0, sizeof(float) * kParams, st));
-    rc = launch_fwd_bwd(ctx, st, S, in, targets, n, 0u);
+    rc = launch_fwd_bwd(ctx, st, S, in, targets, n, nullptr, 0u, 0u, 0u);
     if (rc) return rc;
     RT_CUDA_CTX(ctx, cudaMemcpyAsync(grad_out, S->grads, sizeof(float) * kParams, cudaMemcpyDeviceToDevice, st));
     RT_CUDA_CTX(ctx, cudaMemsetAsync(S->grads, 0, sizeof(float) * kParams, st));
@@ -1192,11 +1429,8 @@ int cache_train_dev(rt_context *ctx, cudaStream_t st, void *cache, const rt_cach
     CacheState *S = static_cast<CacheState *>(cache);
     for (uint32_t b = 0; b < max_n; b += batch) {
         const uint32_t m = (max_n - b) < batch ? (max_n - b) : batch;
-        const uint32_t tiles = (m + kTrainRows - 1) / kTrainRows;
-        uint32_t grid = (uint32_t)ctx->sm_count;
-        if (grid > tiles) grid = tiles;
-        RT_CUDA_CTX(ctx, launch_pdl(k_cache_fwd_bwd, grid, kTrainThreads, kTrainSmem, st, S, in,
-                                    reinterpret_cast<const float4 *>(targets), m, 0.0f, n_dev, b, 1u));
+        rc = launch_fwd_bwd(ctx, st, S, in, targets, m, n_dev, b, 1u, b ? 1u : 0u);
+        if (rc) return rc;
         RT_CUDA_CTX(ctx, launch_pdl(k_cache_adam, (kParams + 255) / 256, 256, 0, st, S,
                                     static_cast<float *>(nullptr)));
     }
