@@ -38,6 +38,7 @@ constexpr int kRing = 8;
 constexpr uint32_t kAnyBlocksPerSm = 1024u / kTraceThreads;  // resident blocks the any-hit kernel is bounded for
 constexpr int kMaxDepth = 64;       // total stack entries per ray
 constexpr uint32_t kNone = 0xffffffffu;
+constexpr uint32_t kMinusZero = 0x80000000u;  // the bits of -0; in a record index (below 2^30) the mark of a hit at t = -0
 
 struct Hit {
     float t, u, v;
@@ -125,10 +126,12 @@ template <bool ANY, bool MULTI, int THREADS, int RING, bool MIXED = false>
 __global__ void __launch_bounds__(THREADS, ((MULTI || ANY) ? 1024 : 1152) / THREADS) k_trace_blas(const BatchArgs a) {
     static_assert((RING & (RING - 1)) == 0 && RING <= kMaxDepth, "RING is a power of two");
     __shared__ uint2 s_stack[RING][THREADS];
-    __shared__ uint32_t s_qrec[THREADS / 32][kTriQueue];
-    __shared__ uint8_t s_qlane[THREADS / 32][kTriQueue];
-    // per lane, touched once per ray or improved hit: u, v, leaf record and
-    // triangle of the best hit so far; the ray's index
+    __shared__ uint2 s_queue[THREADS / 32][kTriQueue];  // leaf record, lane
+    // per lane: the triangle test's part of the ray (written once per ray, read
+    // by whichever lane tests); the best hit so far -- t as an ordered integer;
+    // u, v, leaf record and triangle (kNone: no hit) --; the ray's index
+    __shared__ float4 s_shear[THREADS];
+    __shared__ int32_t s_t[ANY ? 1 : THREADS];
     __shared__ uint4 s_best[ANY ? 1 : THREADS];
     __shared__ uint32_t s_ray[THREADS];
     const uint4 *nodes = nullptr, *prims = nullptr;
@@ -146,14 +149,13 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY) ? 1024 : 1152) / THRE
     }
     constexpr uint32_t kFull = 0xffffffffu;
     const int tid = threadIdx.x, lane = tid & 31;
-    uint32_t *qrec = s_qrec[tid >> 5];
-    uint8_t *qlane = s_qlane[tid >> 5];
+    uint2 *queue = s_queue[tid >> 5];
+    const int warp0 = tid & ~31;  // lane 0's thread
 
     bool have_ray = false, exhausted = false, pending = false;
     Ray r;
     r.o[0] = r.o[1] = r.o[2] = 0.f;
-    r.sx = r.sy = r.sz = 0.f;
-    r.prio = r.kxyz = 0u;
+    r.prio = 0u;
     float tmin = 0.f, tbest = 0.f;  // tbest: the ray's far limit, then its best hit
     bool found = false;
     uint32_t node = 0;
@@ -162,6 +164,7 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY) ? 1024 : 1152) / THRE
     uint32_t visits = 0;
     uint32_t head = 0, tail = 0;  // queue positions tested / appended so far (the same in every lane)
     uint32_t last = ~0u;          // position of this lane's latest entry
+    uint32_t error = 0u;          // detail word of an error this lane's ray met
     const uint32_t n1 = a.n_dev ? min(*a.n_dev, a.n) : a.n;
     const uint32_t n_rays = MIXED ? n1 + min(*a.n_dev2, a.n2) : n1;
     bool any_ray = ANY;  // this lane's ray is an any-hit ray
@@ -180,12 +183,19 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY) ? 1024 : 1152) / THRE
             if (have_ray && !pending && !waiting) {
                 have_ray = false;
                 const uint32_t ray_idx = s_ray[tid];
+                if (error) {
+                    report_error(a.err, RT_ERR_BOUNDS, error | ray_idx);
+                    error = 0u;
+                }
                 if (ANY || (MIXED && any_ray)) {
                     if (a.occluded) a.occluded[ray_idx] = found ? 1u : 0u;
                 } else {
-                    uint4 best = make_uint4(0u, 0u, kNone, kNone);
-                    if (found) best = s_best[tid];
-                    const float4 out = make_float4(found ? tbest : kInf, __uint_as_float(a.out_rec ? best.z : best.w),
+                    uint4 best = s_best[tid];
+                    found = best.w != kNone;
+                    const float t = (best.z & kMinusZero) ? -0.0f : tbest;
+                    best.z &= ~kMinusZero;
+                    if (!found) best = make_uint4(0u, 0u, kNone, kNone);
+                    const float4 out = make_float4(found ? t : kInf, __uint_as_float(a.out_rec ? best.z : best.w),
                                                    __uint_as_float(best.x), __uint_as_float(best.y));
                     if (a.hits) a.hits[ray_idx] = out;
                     if (!MULTI && a.hits_ext) {
@@ -240,6 +250,11 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY) ? 1024 : 1152) / THRE
                 tbest = r1.w;
                 found = false;
                 s_ray[tid] = idx;
+                s_shear[tid] = make_float4(r.sx, r.sy, r.sz, __uint_as_float(r.kxyz));
+                if (!ANY) {
+                    s_t[tid] = ford(tbest);
+                    s_best[tid].w = kNone;
+                }
                 have_ray = true;
                 node = 0;          // start at the root
                 visits = 0;
@@ -257,77 +272,85 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY) ? 1024 : 1152) / THRE
         const bool drain = walking == 0 || busy - walking >= kTriDrain;
 
         // ---- one node per lane, then the lane's next node
-        uint32_t ph = 0u, pbase = 0u;
-        if (pending) {
+        // leaf slots met (bits), the record reached in the first of them, and
+        // the node's slot bytes and record base
+        uint32_t leaves = 0u, step = 0u, meta_lo = 0u, meta_hi = 0u, pbase = 0u;
+        // (errors are noted and reported with the result: no calls in here, and
+        // the rare cases -- a spilled stack entry -- are the only branches)
+        if (pending && (visits >= max_visits || node >= max_visits)) {
             pending = false;
-            if (visits >= max_visits || node >= max_visits) {
-                report_error(a.err, RT_ERR_BOUNDS, 0x76000000u | s_ray[tid]);
-            } else {
-                ++visits;
-                const NodeWords nd = load_node(nodes, node);
-                const uint32_t hits = isect_node(r, nd, tmin, tbest);
-                ph = leaf_records(nd, hits);
-                pbase = nd.w1.y;
-                uint2 g = child_group(nd, hits);
-                if (!group_left(g) && sp > 0) {
-                    --sp;
-                    if (sp >= lo) {
-                        g = s_stack[sp & (RING - 1)][tid];
-                    } else {
-                        g = spill[sp];
-                        lo = sp;
-                    }
-                }
-                if (group_left(g)) {
-                    node = take_child(g, r.prio);
-                    pending = true;
-                    if (group_left(g)) {
-                        if (sp >= kMaxDepth) {
-                            report_error(a.err, RT_ERR_BOUNDS, 0x72000000u | s_ray[tid]);
-                            pending = false;
-                        } else {
-                            if (sp - lo == RING) {
-                                spill[lo] = s_stack[lo & (RING - 1)][tid];
-                                ++lo;
-                            }
-                            s_stack[sp & (RING - 1)][tid] = g;
-                            ++sp;
-                        }
-                    }
-                }
+            error = 0x76000000u;
+        }
+        if (pending) {
+            ++visits;
+            const NodeWords nd = load_node(nodes, node);
+            const uint32_t hits = isect_node(r, nd, tmin, tbest);
+            leaves = hits & ~(nd.w0.w >> 24);
+            meta_lo = nd.w1.z;
+            meta_hi = nd.w1.w;
+            pbase = nd.w1.y;
+            uint2 g = child_group(nd, hits);
+            const bool pop = !group_left(g) && sp > 0;
+            if (pop) {
+                --sp;
+                g = s_stack[sp & (RING - 1)][tid];
+            }
+            if (pop && sp < lo) {
+                g = spill[sp];
+                lo = sp;
+            }
+            pending = group_left(g);
+            node = take_child(g, r.prio);  // (of no group: unused)
+            const bool push = pending && group_left(g);
+            if (push && sp - lo == RING) {
+                spill[lo] = s_stack[lo & (RING - 1)][tid];
+                ++lo;
+            }
+            if (push) {
+                s_stack[sp & (RING - 1)][tid] = g;
+                ++sp;
+            }
+            if (sp > kMaxDepth) {
+                pending = false;
+                error = 0x72000000u;
             }
         }
 
         // ---- append the leaf records met, test a batch when there is one
-        for (;;) {
-            const uint32_t m = __ballot_sync(kFull, ph != 0u);
-            if (m == 0u && !drain) break;
-            if (ph) {
-                const uint32_t i = __ffs(ph) - 1;
-                ph &= ph - 1u;
+        uint32_t m = __ballot_sync(kFull, leaves != 0u);
+        while (m != 0u || (drain && tail != head)) {
+            // a leaf's meta byte: its record count in unary (bits 5-7; none for
+            // an unused slot), then its first record's offset
+            if (leaves) {
+                const uint32_t meta = __byte_perm(meta_lo, meta_hi, (uint32_t)__ffs((int)leaves) - 1u) & 0xffu;
                 last = tail + __popc(m & ((1u << lane) - 1u));
-                qrec[last & (kTriQueue - 1u)] = pbase + i;
-                qlane[last & (kTriQueue - 1u)] = (uint8_t)lane;
+                queue[last & (kTriQueue - 1u)] =
+                    make_uint2((meta & 0x20u) ? pbase + (meta & 0x1fu) + step : kNone, (uint32_t)lane);
+                const bool again = ((meta >> 6 >> step) & 1u) != 0u;
+                step = again ? step + 1u : 0u;
+                leaves = again ? leaves : leaves & (leaves - 1u);
             }
             tail += __popc(m);
+            m = __ballot_sync(kFull, leaves != 0u);
             const int cnt = (int)(tail - head);
-            if (cnt >= busy || (m == 0u && cnt > 0)) {
+            if (cnt >= busy || (m == 0u && drain)) {
                 const uint32_t k = min(cnt, 32);
                 __syncwarp();
-                const uint32_t qi = (head + (uint32_t)lane) & (kTriQueue - 1u);
-                const bool have = (uint32_t)lane < k;
-                const uint32_t src = have ? (uint32_t)qlane[qi] : (uint32_t)lane;
-                const uint32_t rec = have ? qrec[qi] : 0u;
+                uint2 e = make_uint2(kNone, (uint32_t)lane);
+                if ((uint32_t)lane < k) e = queue[(head + (uint32_t)lane) & (kTriQueue - 1u)];
+                const uint32_t rec = e.x, src = e.y;
+                const bool have = rec != kNone;
                 __syncwarp();  // read before the next append reuses the slots
                 head += k;
                 Ray tr;
                 tr.o[0] = __shfl_sync(kFull, r.o[0], src);
                 tr.o[1] = __shfl_sync(kFull, r.o[1], src);
                 tr.o[2] = __shfl_sync(kFull, r.o[2], src);
-                tr.sx = __shfl_sync(kFull, r.sx, src);
-                tr.sy = __shfl_sync(kFull, r.sy, src);
-                tr.sz = __shfl_sync(kFull, r.sz, src);
-                tr.kxyz = __shfl_sync(kFull, r.kxyz, src);
+                const float4 shear = s_shear[warp0 + src];
+                tr.sx = shear.x;
+                tr.sy = shear.y;
+                tr.sz = shear.z;
+                tr.kxyz = __float_as_uint(shear.w);
                 const float t_lo = __shfl_sync(kFull, tmin, src), t_hi = __shfl_sync(kFull, tbest, src);
                 const uint4 *pr = prims;
                 if (MULTI)
@@ -347,38 +370,37 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY) ? 1024 : 1152) / THRE
                     if ((fm >> lane) & 1u) {
                         found = true;
                         pending = false;
-                        ph = 0u;
+                        leaves = 0u;
                     }
                 } else {
-                    // each owner compares its hits in turn and then takes the
-                    // winner's coordinates
-                    int win = -1;
-                    uint32_t best_tri = 0u;
-                    for (uint32_t hm = __ballot_sync(kFull, hit); hm; hm &= hm - 1u) {
-                        const int l = __ffs(hm) - 1;
-                        const uint32_t s = __shfl_sync(kFull, src, l), ht = __shfl_sync(kFull, tri, l);
-                        const float tt = __shfl_sync(kFull, t, l);
-                        if ((uint32_t)lane == s && !(MIXED && any_ray && found) && tt <= tbest) {
-                            if (tt < tbest || !found || ht < (win < 0 ? s_best[tid].w : best_tri)) {
-                                tbest = tt;
-                                best_tri = ht;
-                                win = l;
-                                found = true;
-                            }
-                        }
+                    // the owner's best: least t, then, among the lanes that
+                    // reached it, least triangle (an improved t clears the
+                    // triangle of the old one)
+                    const int32_t key = ford(t + 0.0f);  // -0 and +0 tie
+                    int32_t *bt = s_t + warp0 + src;
+                    uint4 *best = s_best + warp0 + src;
+                    if (hit && atomicMin(bt, key) > key) best->w = kNone;
+                    __syncwarp();
+                    hit = hit && *bt == key;
+                    if (hit) atomicMin(&best->w, tri);
+                    __syncwarp();
+                    if (hit && best->w == tri) {
+                        best->x = __float_as_uint(u);
+                        best->y = __float_as_uint(v);
+                        best->z = rec | (__float_as_uint(t) == kMinusZero ? kMinusZero : 0u);
                     }
-                    const uint32_t from = win < 0 ? (uint32_t)lane : (uint32_t)win;
-                    const float bu = __shfl_sync(kFull, u, from), bv = __shfl_sync(kFull, v, from);
-                    const uint32_t br = __shfl_sync(kFull, rec, from);
-                    if (win >= 0) {
-                        if (MIXED && any_ray) {
+                    __syncwarp();
+                    if (MIXED && any_ray) {
+                        found = s_best[tid].w != kNone;
+                        if (found) {
                             pending = false;
-                            ph = 0u;
-                        } else {
-                            s_best[tid] = make_uint4(__float_as_uint(bu), __float_as_uint(bv), br, best_tri);
+                            leaves = 0u;
                         }
+                    } else {
+                        tbest = ford_inv(s_t[tid]);
                     }
                 }
+                if (ANY || MIXED) m = __ballot_sync(kFull, leaves != 0u);  // a ray that is done appends no more
             }
             if (m == 0u) break;
         }
