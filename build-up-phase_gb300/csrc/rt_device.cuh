@@ -199,32 +199,6 @@ __device__ __forceinline__ NodeWords load_node(const uint4 *nodes, uint32_t idx)
     return n;
 }
 
-// The same five words as two 32-byte loads and one of 16: a node is 16-byte
-// aligned, so its first or its last word stands alone.  Fewer wavefronts in the
-// L1 data path for a branch that a warp mostly walks on both sides (see
-// k_trace_blas).  Volatile: the loads stay together, ahead of the arithmetic;
-// let the compiler move them and the gain is lost.
-__device__ __forceinline__ void ldg32(const uint4 *p, uint4 &a, uint4 &b) {
-    asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
-                 : "l"(p));
-}
-
-__device__ __forceinline__ NodeWords load_node_wide(const uint4 *nodes, uint32_t idx) {
-    const uint4 *p = nodes + (size_t)idx * 5u;
-    NodeWords n;
-    if (reinterpret_cast<uintptr_t>(p) & 16u) {
-        n.w0 = __ldg(p + 0);
-        ldg32(p + 1, n.w1, n.w2);
-        ldg32(p + 3, n.w3, n.w4);
-    } else {
-        ldg32(p + 0, n.w0, n.w1);
-        ldg32(p + 2, n.w2, n.w3);
-        n.w4 = __ldg(p + 4);
-    }
-    return n;
-}
-
 __device__ __forceinline__ uint32_t byte_of(uint32_t w, int b) { return (w >> (8 * b)) & 0xffu; }
 
 // Byte b of w as an exact float: PRMT assembles 0x4B0000qq (= 2^23 + q) and

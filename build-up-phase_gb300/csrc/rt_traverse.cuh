@@ -147,11 +147,6 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY) ? 1024 : 1152) / THRE
         empty = hd->prim_count == 0;
         max_visits = hd->node_count;
     }
-    // 32-byte node loads: the path tracer's queues (incoherent rays of one
-    // scene, L1-bound) gain, 2M box 20.97 -> 20.40 ms per four samples; the
-    // ray queries (1M soup 1.57 -> 1.62 ms) and the batch (2.18 -> 2.27 ms),
-    // whose lanes share more of their nodes, lose.
-    constexpr bool kWideNodes = MIXED && !MULTI;
     constexpr uint32_t kFull = 0xffffffffu;
     const int tid = threadIdx.x, lane = tid & 31;
     uint2 *queue = s_queue[tid >> 5];
@@ -288,7 +283,7 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY) ? 1024 : 1152) / THRE
         }
         if (pending) {
             ++visits;
-            const NodeWords nd = kWideNodes ? load_node_wide(nodes, node) : load_node(nodes, node);
+            const NodeWords nd = load_node(nodes, node);
             const uint32_t hits = isect_node(r, nd, tmin, tbest);
             leaves = hits & ~(nd.w0.w >> 24);
             meta_lo = nd.w1.z;
