@@ -19,7 +19,7 @@
 // Visiting order: a node's leaf records first, in ascending record order, then
 // its internal children in ascending (slot ^ ray octant); remaining siblings
 // are pushed as one group (identical in the CPU restatement, whose statistics
-// k_trace_stats equals; k_trace_blas tests records in batches).  Closest hit =
+// k_trace_stats equals; the persistent kernels test records in batches).  Closest hit =
 // smallest t, ties broken by the smallest (instance, triangle) key.
 #include <cmath>
 #include <cuda.h>
@@ -226,25 +226,33 @@ __device__ bool trace_ray(const uint8_t *accel, const float o[3], const float d[
 }
 
 
-// Two-level structures (instances), persistent like k_trace_blas: warps
-// refill idle lanes from the work counter, stacks live in a shared-memory
-// ring whose bottom spills to local memory.  At an instance a lane saves the
-// TLAS node's remaining work on its stack -- the node's internal children,
-// its instances not yet walked, then a return marker -- and walks the
-// instance's BLAS with the object-space ray; popping the marker restores the
-// world ray.  The visiting order is trace_ray's: a TLAS node's instances in
-// ascending record order, each BLAS in full, then the node's internal
-// children; closest hit = smallest t, ties broken by the smallest
-// (instance id, triangle) key.  Launched beside k_trace_blas; each kernel
-// returns at once when the structure is not its kind.
+// Two-level structures (instances), persistent like k_trace_blas, with its
+// triangle queue: warps refill idle lanes from the work counter, stacks live
+// in a shared-memory ring whose bottom spills to local memory.  At a TLAS node
+// a lane saves the internal children on its stack and stops for the node's
+// instances; to enter one it saves the instances left and a return entry and
+// walks the instance's BLAS with the object-space ray.  When that walk is over
+// it takes the world ray back from shared memory and goes on in the TLAS.
+// Closest hit = smallest t, ties broken by the smallest (instance, triangle)
+// key, whatever the order.  Launched beside k_trace_blas; each kernel returns
+// at once when the structure is not its kind.
+//
+// A lane enters an instance every few nodes, and the entry (80 bytes of
+// record, a transformed ray, its divisions) costs more than a node, so lanes
+// stop for it and are served together, with those that need a new ray, once a
+// quarter of the lanes with a ray (or the refill threshold) have stopped:
+// entered on the spot, the entry and the triangle tests ran with a few lanes
+// each (10.5 active threads per instruction).  807K rays in 64 instances of
+// three meshes: 1,008 -> 822 us (without the rays set aside, kNearHits: 800; then
+// a fixed 4 / 8 / 16 stopped lanes 863 / 871 / 971, a third or an eighth of the
+// lanes 811 / 821).  What bounds it now: issue slots, half of them in steps of
+// warps whose last rays (of up to hundreds of nodes) are under way.  A lane leaves an instance without
+// waiting for its queued triangles: their part of the object-space ray stays in
+// shared memory until the lane enters the next one, before which they are
+// tested.
 constexpr uint32_t kInstGroup = 0x40000000u;   // stack entry: instances of a TLAS node still to walk
-constexpr uint32_t kReturnTop = 0x80000000u;   // stack entry: back to the TLAS
 constexpr int kInstDepth = 128;                // stack entries per ray (both levels)
-constexpr uint32_t kInstBlocksPerSm = 6;  // 80 registers (7 blocks: 72 and 72 bytes of spill, 2 % slower)
-
-__device__ __forceinline__ bool inst_key_less(float t, uint32_t inst, uint32_t tri, const Hit &h) {
-    return t < h.t || (t == h.t && (!h.found || inst < h.inst || (inst == h.inst && tri < h.tri)));
-}
+constexpr uint32_t kInstBlocksPerSm = 6;       // 80 registers (7 blocks: 72, within 1 %)
 
 template <bool ANY>
 __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(const BatchArgs a) {
@@ -255,24 +263,48 @@ __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(
     const uint32_t t_count = hd->node_count;
     const bool t_empty = hd->prim_count == 0;
     __shared__ uint2 s_stack[kRing][kTraceThreads];
+    __shared__ uint2 s_queue[kTraceThreads / 32][kTriQueue];  // leaf record, lane
+    // per lane: the world ray (origin, visiting order; inverse direction, the
+    // ray's index); the triangle test's part of the object-space ray of the
+    // instance entered last (origin, tmin; shear); the best hit so far -- t as
+    // an ordered integer; instance and triangle (~0: no hit); u, v, leaf record
+    // and the instance's record
+    __shared__ float4 s_world[2][kTraceThreads];
+    __shared__ float4 s_object[2][kTraceThreads];
+    __shared__ int32_t s_t[ANY ? 1 : kTraceThreads];
+    __shared__ unsigned long long s_key[ANY ? 1 : kTraceThreads];
+    __shared__ uint4 s_best[ANY ? 1 : kTraceThreads];
+    __shared__ uint32_t s_near[kTraceThreads / 32];  // lanes (bits) whose ray is to be set aside, see kNearHits
+    __shared__ uint32_t s_aside[ANY ? 1 : kTraceThreads];  // per lane: the last ray set aside
+    constexpr uint32_t kFull = 0xffffffffu;
     const int tid = threadIdx.x, lane = tid & 31;
+    uint2 *queue = s_queue[tid >> 5];
+    const int warp0 = tid & ~31;  // lane 0's thread
+    if (!ANY) {
+        s_aside[tid] = kNone;
+        s_near[tid >> 5] = 0u;
+    }
+    __syncwarp();
 
-    bool active = false, exhausted = false;
-    uint32_t ray_idx = 0;
-    float wo[3] = {0.f, 0.f, 0.f}, wd[3] = {0.f, 0.f, 0.f};  // the world ray
+    bool have_ray = false, exhausted = false, pending = false, in_blas = false, found = false;
     Ray r;  // the current level's ray
-    float tmin = 0.f;
-    Hit h;
-    h.t = 0.f; h.u = 0.f; h.v = 0.f; h.rec = kNone; h.tri = kNone; h.inst = 0; h.found = false;
-    uint32_t h_irec = kNone;  // TLAS record of the best hit's instance
-    uint32_t node = 0;
-    bool pending = false, in_blas = false;
-    const uint4 *bnodes = nullptr, *bprims = nullptr;
-    uint32_t b_count = 0, inst_id = 0, inst_rec = 0, visits_t = 0, visits_b = 0;
-    uint2 g = make_uint2(0u, 0u), ig = make_uint2(0u, 0u);
-    int sp = 0, lo = 0;
+    r.o[0] = r.o[1] = r.o[2] = 0.f;
+    r.prio = 0u;
+    float tmin = 0.f, tbest = 0.f;  // tbest: the ray's far limit, then its best hit
+    const uint4 *nodes = tnodes, *prims = nullptr;  // the current level's nodes; the instance's leaf records
+    uint32_t node = 0, visits = 0, count = 0;       // a walk visits each node of a level at most once
+    uint32_t inst_id = 0, inst_rec = 0;
+    uint2 ig = make_uint2(0u, 0u);  // instances of a TLAS node to enter: the lane is stopped
+    int sp = 0, lo = 0, sp_blas = 0;
     uint2 spill[kInstDepth];
+    uint32_t head = 0, tail = 0;  // queue positions tested / appended so far (the same in every lane)
+    uint32_t last = ~0u;          // position of this lane's latest entry
+    uint32_t error = 0u;          // detail word of an error this lane's ray met
     const uint32_t n_rays = a.n;
+    // fewer rays than lanes: see k_trace_blas
+    const uint32_t share = n_rays / (gridDim.x * (kTraceThreads / 32)) + 1u;
+    const uint32_t lanes = share >= 32u ? kFull : (1u << share) - 1u;
+    const int refill = (int)min(a.refill, min(share, 32u));
 
     auto push = [&](uint2 e) {
         if (sp - lo == kRing) {
@@ -282,200 +314,340 @@ __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(
         s_stack[sp & (kRing - 1)][tid] = e;
         ++sp;
     };
+    auto pop = [&]() {
+        --sp;
+        uint2 e = s_stack[sp & (kRing - 1)][tid];
+        if (sp < lo) {
+            e = spill[sp];
+            lo = sp;
+        }
+        return e;
+    };
+    auto fail = [&](uint32_t detail) {  // the walk ends here
+        pending = false;
+        ig.y = 0u;
+        error = detail;
+    };
+
+    auto world_ray = [&]() {  // back to the TLAS
+        in_blas = false;
+        nodes = tnodes;
+        count = t_count;
+        const float4 w0 = s_world[0][tid], w1 = s_world[1][tid];
+        r.o[0] = w0.x; r.o[1] = w0.y; r.o[2] = w0.z;
+        r.prio = __float_as_uint(w0.w);
+        r.invd[0] = w1.x; r.invd[1] = w1.y; r.invd[2] = w1.z;
+    };
+
+    auto result_place = [&](uint32_t ray_idx) {
+        return a.hits       ? reinterpret_cast<uint32_t *>(a.hits + ray_idx)
+               : a.hits_ext ? reinterpret_cast<uint32_t *>(a.hits_ext + ray_idx)
+                            : nullptr;
+    };
+    auto write_hit = [&](uint32_t ray_idx, bool hit, float t, float u, float v, uint32_t inst, uint32_t tri,
+                         const HitIds &ids) {
+        const float4 out = hit ? make_float4(t, __uint_as_float(tri), u, v)
+                               : make_float4(kInf, __uint_as_float(kNone), 0.f, 0.f);
+        if (a.hits) a.hits[ray_idx] = out;
+        if (a.hits_ext) {
+            rt_hit_ext x;
+            x.t = out.x; x.u = out.z; x.v = out.w;
+            x.instance_id = hit ? inst : kNone;
+            x.custom_index = hit ? ids.custom : 0u;
+            x.geometry_index = hit ? ids.geom : 0u;
+            x.primitive_id = hit ? ids.prim : kNone;
+            x.sbt_record = hit ? ids.sbt_off + ids.geom : 0u;
+            a.hits_ext[ray_idx] = x;
+        }
+    };
 
     for (;;) {
-        // ---- refill idle lanes from the global counter
-        const uint32_t idle = __ballot_sync(0xffffffffu, !active);
-        if (!exhausted && __popc(idle) >= (int)a.refill) {
-            const uint32_t cnt = __popc(idle);
-            uint32_t base = 0;
-            if (lane == 0) base = atomicAdd(a.counter, cnt);
-            base = __shfl_sync(0xffffffffu, base, 0);
-            if (base + cnt >= n_rays) exhausted = true;
-            if (!active) {
-                const uint32_t idx = base + __popc(idle & ((1u << lane) - 1u));
-                if (idx < n_rays) {
+        // ---- stopped lanes whose queued triangles are tested: result and new
+        // ray, or the next instance
+        const bool waiting = (int)(last - head) >= 0;
+        const uint32_t ready =
+            __ballot_sync(kFull, !pending && !waiting && (have_ray || (!exhausted && ((lanes >> lane) & 1u))));
+        uint32_t walking = __ballot_sync(kFull, pending);
+        // stopped lanes to wait for: they stand idle until served
+        const int serve = max(1 + __popc(__ballot_sync(kFull, have_ray)) / 4, exhausted ? 0 : refill);
+        if (__popc(ready) >= serve || (walking == 0u && tail == head)) {
+            if (ready == 0u) break;  // every lane is done
+            const bool mine = (ready >> lane) & 1u;
+            const bool enter = mine && ig.y != 0u;
+            if (mine && have_ray && !enter) {
+                have_ray = false;
+                const uint32_t ray_idx = __float_as_uint(s_world[1][tid].w);
+                if (error) {
+                    report_error(a.err, RT_ERR_BOUNDS, error);
+                    error = 0u;
+                }
+                if (ANY) {
+                    if (a.occluded) a.occluded[ray_idx] = found ? 1u : 0u;
+                } else {
+                    const uint4 best = s_best[tid];
+                    const unsigned long long key = s_key[tid];
+                    const bool hit = key != ~0ull;
+                    if (hit && ((s_near[tid >> 5] >> lane) & 1u)) {
+                        atomicAnd(&s_near[tid >> 5], ~(1u << lane));
+                        uint32_t *place = result_place(ray_idx);
+                        if (place) {
+                            *place = s_aside[tid];
+                            s_aside[tid] = ray_idx;
+                        }
+                    } else {
+                        const uint32_t rec = best.z & ~kMinusZero;
+                        HitIds ids;
+                        ids.custom = ids.sbt_off = ids.geom = ids.prim = 0u;
+                        if (hit && a.hits_ext) {
+                            const InstRec ir = load_inst(tprims, best.w);
+                            const uint8_t *blas = reinterpret_cast<const uint8_t *>(ir.accel_ref);
+                            const rt_accel_header *bh = reinterpret_cast<const rt_accel_header *>(blas);
+                            const uint4 *bp = reinterpret_cast<const uint4 *>(blas + bh->prim_offset);
+                            ids.custom = ir.cim & 0xffffffu;
+                            ids.sbt_off = ir.sof & 0xffffffu;
+                            ids.geom = ldg4(bp + (size_t)rec * 3u + 1).w;
+                            ids.prim = ldg4(bp + (size_t)rec * 3u + 2).w;
+                        }
+                        write_hit(ray_idx, hit, (best.z & kMinusZero) ? -0.0f : tbest, __uint_as_float(best.x),
+                                  __uint_as_float(best.y), (uint32_t)(key >> 32), (uint32_t)key, ids);
+                    }
+                }
+            }
+            float o[3], d[3];
+            bool fresh = false, entered = false;
+            const uint32_t want = __ballot_sync(kFull, mine && !have_ray) & lanes;
+            if (want != 0u && !exhausted) {
+                const uint32_t cnt = __popc(want);
+                uint32_t first = 0;
+                if (lane == 0) first = atomicAdd(a.counter, cnt);
+                first = __shfl_sync(kFull, first, 0);
+                if (first + cnt >= n_rays) exhausted = true;
+                const uint32_t idx = first + __popc(want & ((1u << lane) - 1u));
+                if (((want >> lane) & 1u) && idx < n_rays) {
                     const float4 r0 = __ldg(a.rays + 2u * idx), r1 = __ldg(a.rays + 2u * idx + 1u);
-                    wo[0] = r0.x; wo[1] = r0.y; wo[2] = r0.z;
-                    wd[0] = r1.x; wd[1] = r1.y; wd[2] = r1.z;
-                    ray_setup(r, wo, wd);
+                    o[0] = r0.x; o[1] = r0.y; o[2] = r0.z;
+                    d[0] = r1.x; d[1] = r1.y; d[2] = r1.z;
+                    s_world[1][tid].w = __uint_as_float(idx);
                     tmin = r0.w;
-                    h.t = r1.w; h.u = 0.f; h.v = 0.f; h.rec = kNone; h.tri = kNone; h.inst = 0; h.found = false;
-                    h_irec = kNone;
-                    ray_idx = idx;
-                    active = true;
+                    tbest = r1.w;
+                    found = false;
+                    if (!ANY) {
+                        s_t[tid] = ford(tbest + 0.0f);  // -0 and +0 tie
+                        s_key[tid] = ~0ull;
+                    }
+                    have_ray = true;
                     in_blas = false;
+                    nodes = tnodes;
                     node = 0;
+                    visits = 0;
+                    count = t_count;
                     pending = !t_empty;
-                    visits_t = 0;
-                    g = make_uint2(0u, 0u);
-                    ig = make_uint2(0u, 0u);
                     sp = 0;
                     lo = 0;
+                    last = head - 1u;
+                    fresh = true;
                 }
             }
-        }
-        if (!__any_sync(0xffffffffu, active)) {
-            if (exhausted) break;
-            continue;
-        }
-        // ---- traversal steps until too many lanes are idle
-        for (;;) {
-            if (active) {
-                bool finish = false;
-                if (pending) {
-                    pending = false;
-                    const uint32_t count = in_blas ? b_count : t_count;
-                    const uint32_t visits = in_blas ? visits_b : visits_t;
-                    if (visits >= count || node >= count) {
-                        report_error(a.err, RT_ERR_BOUNDS, (in_blas ? 0x74000000u : 0x75000000u) | (node & 0xffffffu));
-                        finish = true;
-                    } else {
-                        if (in_blas) ++visits_b;
-                        else ++visits_t;
-                        NodeWords nd = load_node(in_blas ? bnodes : tnodes, node);
-                        const uint32_t hits = isect_node(r, nd, tmin, h.t);
-                        uint32_t ph = leaf_records(nd, hits);
-                        g = child_group(nd, hits);
-                        if (!in_blas) {
-                            ig = make_uint2(nd.w1.y, ph);  // the node's instances, walked first
+            if (enter) {
+                const uint32_t rec = ig.x + (uint32_t)__ffs((int)ig.y) - 1u;
+                ig.y &= ig.y - 1u;
+                const InstRec ir = load_inst(tprims, rec);
+                const uint8_t *blas = reinterpret_cast<const uint8_t *>(ir.accel_ref);
+                const rt_accel_header *bh = reinterpret_cast<const rt_accel_header *>(blas);
+                if (((ir.cim >> 24) & 0xffu) == 0u || bh->prim_count == 0u) {
+                    // masked out (cull mask 0xFF) or empty: on to the next
+                    // instance, else to what the stack holds
+                    if (ig.y == 0u && sp > 0) {
+                        uint2 g = pop();
+                        if (g.y & kInstGroup) {
+                            ig = make_uint2(g.x, g.y & ~kInstGroup);
                         } else {
-                            const uint32_t pbase = nd.w1.y;
-                            while (ph) {
-                                const uint32_t i = __ffs(ph) - 1;
-                                ph &= ph - 1u;
-                                const uint4 *rec = bprims + (size_t)(pbase + i) * 3u;
-                                const uint4 q0 = ldg4(rec), q1 = ldg4(rec + 1), q2 = ldg4(rec + 2);
-                                float t, u, v;
-                                if (!isect_tri(r,
-                                               make_float4(__uint_as_float(q0.x), __uint_as_float(q0.y),
-                                                           __uint_as_float(q0.z), 0.f),
-                                               make_float4(__uint_as_float(q1.x), __uint_as_float(q1.y),
-                                                           __uint_as_float(q1.z), 0.f),
-                                               make_float4(__uint_as_float(q2.x), __uint_as_float(q2.y),
-                                                           __uint_as_float(q2.z), 0.f),
-                                               tmin, h.t, t, u, v))
-                                    continue;
-                                if (ANY || inst_key_less(t, inst_id, q0.w, h)) {
-                                    h.t = t; h.u = u; h.v = v; h.rec = pbase + i; h.tri = q0.w; h.inst = inst_id;
-                                    h_irec = inst_rec;
-                                    h.found = true;
-                                }
-                                if (ANY) {
-                                    finish = true;
-                                    break;
-                                }
-                            }
+                            node = take_child(g, r.prio);
+                            if (group_left(g)) push(g);
+                            pending = true;
                         }
                     }
-                }
-                // ---- next: an instance of the current TLAS node, else a node
-                while (!finish) {
-                    if (!in_blas && ig.y) {
-                        const uint32_t i = __ffs(ig.y) - 1;
-                        ig.y &= ig.y - 1u;
-                        const uint32_t rec = ig.x + i;
-                        const InstRec ir = load_inst(tprims, rec);
-                        if (((ir.cim >> 24) & 0xffu) == 0u) continue;  // masked out (cull mask 0xFF)
-                        const uint8_t *blas = reinterpret_cast<const uint8_t *>(ir.accel_ref);
-                        const rt_accel_header *bh = reinterpret_cast<const rt_accel_header *>(blas);
-                        if (bh->prim_count == 0) continue;
-                        if (sp + 3 > kInstDepth) {
-                            report_error(a.err, RT_ERR_BOUNDS, 0x71000000u);
-                            finish = true;
-                            break;
-                        }
-                        // save the TLAS node's remaining work under a return marker
-                        if (group_left(g)) push(g);
-                        if (ig.y) push(make_uint2(ig.x, ig.y | kInstGroup));
-                        push(make_uint2(0u, kReturnTop));
-                        g = make_uint2(0u, 0u);
-                        ig = make_uint2(0u, 0u);
-                        float o2[3], d2[3];
-                        xform_point(ir.w2o, wo, o2);
-                        xform_vector(ir.w2o, wd, d2);
-                        ray_setup(r, o2, d2);
-                        in_blas = true;
-                        bnodes = reinterpret_cast<const uint4 *>(blas + bh->node_offset);
-                        bprims = reinterpret_cast<const uint4 *>(blas + bh->prim_offset);
-                        b_count = bh->node_count;
-                        visits_b = 0;
-                        inst_id = ir.id;
-                        inst_rec = rec;
-                        node = 0;
-                        pending = true;
-                        break;
-                    }
-                    if (group_left(g)) {
-                        node = take_child(g, r.prio);
-                        pending = true;
-                        if (group_left(g)) {
-                            if (sp >= kInstDepth) {
-                                report_error(a.err, RT_ERR_BOUNDS, in_blas ? 0x70000000u : 0x71000000u);
-                                finish = true;
-                                break;
-                            }
-                            push(g);
-                        }
-                        break;
-                    }
-                    if (sp == 0) { finish = true; break; }
-                    --sp;
-                    uint2 e;
-                    if (sp >= lo) {
-                        e = s_stack[sp & (kRing - 1)][tid];
-                    } else {
-                        e = spill[sp];
-                        lo = sp;
-                    }
-                    if (e.y & kReturnTop) {
-                        // the TLAS work saved under the marker (if any) needs
-                        // the world ray back; with none left the walk is done
-                        if (sp == 0) { finish = true; break; }
-                        ray_setup(r, wo, wd);
-                        in_blas = false;
-                    } else if (e.y & kInstGroup) {
-                        ig = make_uint2(e.x, e.y & ~kInstGroup);
-                    } else {
-                        g = e;
-                    }
-                }
-                if (finish) {
-                    // ---- write the result
-                    if (ANY) {
-                        if (a.occluded) a.occluded[ray_idx] = h.found ? 1u : 0u;
-                    } else {
-                        const float4 out = h.found ? make_float4(h.t, __uint_as_float(h.tri), h.u, h.v)
-                                                   : make_float4(kInf, __uint_as_float(kNone), 0.f, 0.f);
-                        if (a.hits) a.hits[ray_idx] = out;
-                        if (a.hits_ext) {
-                            rt_hit_ext x;
-                            x.t = out.x; x.u = out.z; x.v = out.w;
-                            x.instance_id = h.found ? h.inst : kNone;
-                            x.custom_index = 0u;
-                            x.geometry_index = 0u;
-                            x.primitive_id = kNone;
-                            x.sbt_record = 0u;
-                            if (h.found) {
-                                const InstRec ir = load_inst(tprims, h_irec);
-                                const uint8_t *blas = reinterpret_cast<const uint8_t *>(ir.accel_ref);
-                                const rt_accel_header *bh = reinterpret_cast<const rt_accel_header *>(blas);
-                                const uint4 *bp = reinterpret_cast<const uint4 *>(blas + bh->prim_offset);
-                                x.custom_index = ir.cim & 0xffffffu;
-                                x.geometry_index = ldg4(bp + (size_t)h.rec * 3u + 1).w;
-                                x.primitive_id = ldg4(bp + (size_t)h.rec * 3u + 2).w;
-                                x.sbt_record = (ir.sof & 0xffffffu) + x.geometry_index;
-                            }
-                            a.hits_ext[ray_idx] = x;
-                        }
-                    }
-                    active = false;
-                    pending = false;
+                } else if (sp + 2 > kInstDepth) {
+                    fail(0x71000000u);
+                } else {
+                    if (ig.y) push(make_uint2(ig.x, ig.y | kInstGroup));
+                    ig.y = 0u;
+                    push(make_uint2(visits, 0u));  // the TLAS walk's, while the BLAS walk counts its own
+                    sp_blas = sp;
+                    const float4 w0 = s_world[0][tid];
+                    const float4 r1 = __ldg(a.rays + 2u * __float_as_uint(s_world[1][tid].w) + 1u);
+                    const float wo[3] = {w0.x, w0.y, w0.z}, wd[3] = {r1.x, r1.y, r1.z};
+                    xform_point(ir.w2o, wo, o);
+                    xform_vector(ir.w2o, wd, d);
+                    in_blas = true;
+                    nodes = reinterpret_cast<const uint4 *>(blas + bh->node_offset);
+                    prims = reinterpret_cast<const uint4 *>(blas + bh->prim_offset);
+                    node = 0;
+                    visits = 0;
+                    count = bh->node_count;
+                    inst_id = ir.id;
+                    inst_rec = rec;
+                    pending = true;
+                    entered = true;
                 }
             }
-            const uint32_t act = __ballot_sync(0xffffffffu, active);
-            if (act == 0u) break;
-            if (!exhausted && (uint32_t)__popc(~act) >= a.refill) break;
+            if (fresh || entered) {
+                ray_setup(r, o, d);
+                if (fresh) {
+                    s_world[0][tid] = make_float4(o[0], o[1], o[2], __uint_as_float(r.prio));
+                    s_world[1][tid].x = r.invd[0];
+                    s_world[1][tid].y = r.invd[1];
+                    s_world[1][tid].z = r.invd[2];
+                } else {
+                    s_object[0][tid] = make_float4(o[0], o[1], o[2], tmin);
+                    s_object[1][tid] = make_float4(r.sx, r.sy, r.sz, __uint_as_float(r.kxyz));
+                }
+            }
+            walking = __ballot_sync(kFull, pending);
+            if (walking == 0u) continue;
+        }
+        const uint32_t held = __ballot_sync(kFull, !pending && (int)(last - head) >= 0);
+        const int busy = __popc(walking | held);  // lanes whose triangles may be queued
+        // a partial batch once stopped lanes wait for it
+        const bool drain = walking == 0u || __popc(held) + __popc(ready & ~walking) >= serve;
+
+        // ---- one node per lane, then the lane's next node (see k_trace_blas)
+        uint32_t leaves = 0u, step = 0u, meta_lo = 0u, meta_hi = 0u, pbase = 0u;
+        if (pending && (visits >= count || node >= count))
+            fail((in_blas ? 0x74000000u : 0x75000000u) | (node & 0xffffffu));
+        if (pending) {
+            ++visits;
+            const NodeWords nd = load_node(nodes, node);
+            const uint32_t hits = isect_node(r, nd, tmin, tbest);
+            meta_lo = nd.w1.z;
+            meta_hi = nd.w1.w;
+            pbase = nd.w1.y;
+            uint2 g = child_group(nd, hits);
+            leaves = hits & ~(nd.w0.w >> 24);
+            if (!in_blas) {
+                if (leaves) {
+                    ig = make_uint2(pbase, leaf_records(nd, hits));
+                    leaves = 0u;
+                }
+                if (ig.y && group_left(g)) {
+                    push(g);
+                    g.y = 0u;
+                }
+            }
+            const bool next = ig.y == 0u && !group_left(g);
+            if (next && in_blas && sp == sp_blas) {
+                visits = pop().x;
+                world_ray();
+            }
+            if (next && sp > 0) {
+                g = pop();
+                if (g.y & kInstGroup) {
+                    ig = make_uint2(g.x, g.y & ~kInstGroup);
+                    g.y = 0u;
+                }
+            }
+            pending = group_left(g);
+            node = take_child(g, r.prio);  // (of no group: unused)
+            if (pending && group_left(g)) push(g);
+            if (sp > kInstDepth) fail(in_blas ? 0x70000000u : 0x71000000u);
+        }
+
+        // ---- append the leaf records met, test a batch when there is one
+        uint32_t m = __ballot_sync(kFull, leaves != 0u);
+        while (m != 0u || (drain && tail != head)) {
+            if (leaves) {
+                const uint32_t meta = __byte_perm(meta_lo, meta_hi, (uint32_t)__ffs((int)leaves) - 1u) & 0xffu;
+                last = tail + __popc(m & ((1u << lane) - 1u));
+                queue[last & (kTriQueue - 1u)] =
+                    make_uint2((meta & 0x20u) ? pbase + (meta & 0x1fu) + step : kNone, (uint32_t)lane);
+                const bool again = ((meta >> 6 >> step) & 1u) != 0u;
+                step = again ? step + 1u : 0u;
+                leaves = again ? leaves : leaves & (leaves - 1u);
+            }
+            tail += __popc(m);
+            m = __ballot_sync(kFull, leaves != 0u);
+            const int cnt = (int)(tail - head);
+            if (cnt >= busy || (m == 0u && drain)) {
+                const uint32_t k = min(cnt, 32);
+                __syncwarp();
+                uint2 e = make_uint2(kNone, (uint32_t)lane);
+                if ((uint32_t)lane < k) e = queue[(head + (uint32_t)lane) & (kTriQueue - 1u)];
+                const uint32_t rec = e.x, src = e.y;
+                __syncwarp();  // read before the next append reuses the slots
+                head += k;
+                const float4 ob = s_object[0][warp0 + src], shear = s_object[1][warp0 + src];
+                Ray tr;
+                tr.o[0] = ob.x; tr.o[1] = ob.y; tr.o[2] = ob.z;
+                tr.sx = shear.x;
+                tr.sy = shear.y;
+                tr.sz = shear.z;
+                tr.kxyz = __float_as_uint(shear.w);
+                const float t_hi = __shfl_sync(kFull, tbest, src);
+                const uint4 *pr = reinterpret_cast<const uint4 *>(
+                    __shfl_sync(kFull, (unsigned long long)reinterpret_cast<uintptr_t>(prims), src));
+                const uint32_t inst = ANY ? 0u : __shfl_sync(kFull, inst_id, src);
+                const uint32_t irec = ANY ? 0u : __shfl_sync(kFull, inst_rec, src);
+                float t = 0.f, u = 0.f, v = 0.f;
+                uint32_t tri = kNone;
+                bool hit = false;
+                if (rec != kNone) {
+                    const uint4 *p = pr + (size_t)rec * 3u;
+                    const uint4 q0 = ldg4(p), q1 = ldg4(p + 1), q2 = ldg4(p + 2);
+                    tri = q0.w;
+                    hit = isect_tri(tr, xyz_of(q0), xyz_of(q1), xyz_of(q2), ob.w, t_hi, t, u, v);
+                }
+                if (ANY) {
+                    const uint32_t fm = __reduce_or_sync(kFull, hit ? 1u << src : 0u);
+                    if ((fm >> lane) & 1u) {
+                        found = true;
+                        pending = false;
+                        ig.y = 0u;
+                        leaves = 0u;
+                    }
+                    m = __ballot_sync(kFull, leaves != 0u);  // a ray that is done appends no more
+                } else {
+                    // the owner's best: least t, then, among the lanes that
+                    // reached it, least (instance, triangle) (an improved t
+                    // clears the key of the old one)
+                    const int32_t tk = ford(t + 0.0f);  // -0 and +0 tie
+                    const unsigned long long key = (unsigned long long)inst << 32 | tri;
+                    int32_t *bt = s_t + warp0 + src;
+                    unsigned long long *bk = s_key + warp0 + src;
+                    const bool any_hit = hit;
+                    if (hit && atomicMin(bt, tk) > tk) *bk = ~0ull;
+                    __syncwarp();
+                    hit = hit && *bt == tk;
+                    if (hit) atomicMin(bk, key);
+                    __syncwarp();
+                    hit = hit && *bk == key;
+                    if (hit)
+                        s_best[warp0 + src] =
+                            make_uint4(__float_as_uint(u), __float_as_uint(v),
+                                       rec | (__float_as_uint(t) == kMinusZero ? kMinusZero : 0u), irec);
+                    __syncwarp();
+                    if (any_hit) {
+                        // (the best hit is in this instance or ties with one in it)
+                        const float tb = ford_inv(*bt);
+                        if (fabsf((hit ? t_hi : t) - tb) <= kNearHits * fabsf(tb)) atomicOr(&s_near[tid >> 5], 1u << src);
+                    }
+                    tbest = ford_inv(s_t[tid]);
+                }
+            }
+            if (m == 0u) break;
+        }
+    }
+
+    // ---- the rays set aside
+    if (!ANY) {
+        for (uint32_t i = s_aside[tid]; i != kNone;) {
+            const uint32_t next = *result_place(i);
+            const float4 r0 = __ldg(a.rays + 2u * i), r1 = __ldg(a.rays + 2u * i + 1u);
+            const float o[3] = {r0.x, r0.y, r0.z}, d[3] = {r1.x, r1.y, r1.z};
+            Hit h;
+            HitIds ids;
+            trace_ray<false>(a.accel, o, d, r0.w, r1.w, 0xffu, h, ids, a.err, nullptr);
+            write_hit(i, h.found, h.t, h.u, h.v, h.inst, h.tri, ids);
+            i = next;
         }
     }
 }

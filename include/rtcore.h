@@ -401,7 +401,9 @@ typedef struct rt_trace_tuning {
     uint32_t block_threads;   /* threads per block of the traversal kernel */
     uint32_t blocks_per_sm;   /* persistent blocks per SM                  */
     uint32_t batch_rays;      /* a warp refills its idle lanes (one atomic
-                                 fetch) once at least this many are idle    */
+                                 fetch) once at least this many are idle
+                                 (two-level structures: or waiting for an
+                                 instance, and a quarter of its lanes)      */
     uint32_t reserved;
 } rt_trace_tuning;
 rt_status rt_set_trace_tuning(rt_context *ctx, const rt_trace_tuning *t);
