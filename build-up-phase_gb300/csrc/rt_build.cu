@@ -174,9 +174,12 @@ __device__ __forceinline__ Box union_of(const Box &x, const Box &y) {
 // Header / init
 // ---------------------------------------------------------------------------
 
-__global__ void k_init(rt_accel_header hdr, uint8_t *accel, int32_t *cbounds, uint32_t *root, GeomParams gp,
-                       uint32_t write_table) {
+__global__ void k_init(rt_accel_header hdr, uint8_t *accel, int32_t *cbounds, uint32_t *root, uint32_t *bar,
+                       uint32_t *counters, uint32_t counter_words, GeomParams gp, uint32_t write_table) {
+    pdl_launch();
     int t = threadIdx.x;
+    for (uint32_t i = (uint32_t)t; i < counter_words; i += blockDim.x) counters[i] = 0u;  // the sort's
+    if (t < 2) bar[t] = 0u;  // k_collapse's grid barrier
     if (t == 0) *reinterpret_cast<rt_accel_header *>(accel) = hdr;
     // the radix tree's root (none until it is completed) and the subtrees k_tree leaves
     if (t == 0) { root[0] = kNone; root[1] = 0u; }
@@ -284,6 +287,7 @@ __global__ void __launch_bounds__(kRecThreads) k_prep_tris(const GeomParams gp, 
                                                     float *__restrict__ boxes, int32_t *cbounds, uint32_t *err,
                                                     uint32_t *hdr_status) {
     __shared__ uint4 s_rec[kRecThreads * 3];
+    pdl_enter();
     const uint32_t base = blockIdx.x * kRecThreads, gi = base + threadIdx.x;
     int32_t cmin[3] = {INT32_MAX, INT32_MAX, INT32_MAX}, cmax[3] = {INT32_MIN, INT32_MIN, INT32_MIN};
     uint4 rec[3] = {};
@@ -363,6 +367,7 @@ __device__ void inst_record(const rt_instance &I, uint32_t i, uint4 *r, Box &b) 
 __global__ void __launch_bounds__(256) k_prep_inst(const rt_instance *__restrict__ inst, uint32_t n,
                                                     uint4 *__restrict__ recs, float *__restrict__ boxes,
                                                     int32_t *cbounds) {
+    pdl_enter();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     int32_t cmin[3] = {INT32_MAX, INT32_MAX, INT32_MAX}, cmax[3] = {INT32_MIN, INT32_MIN, INT32_MIN};
     if (i < n) {
@@ -387,16 +392,23 @@ __global__ void __launch_bounds__(256) k_prep_inst(const rt_instance *__restrict
 __global__ void __launch_bounds__(256) k_morton(const float *__restrict__ boxes, uint32_t n,
                                                  const int32_t *__restrict__ cbounds, int bpa,
                                                  uint64_t *__restrict__ keys, uint32_t *__restrict__ ids,
-                                                 uint32_t *__restrict__ hist, int passes) {
+                                                 uint32_t *__restrict__ hist, int passes,
+                                                 uint32_t *__restrict__ status, uint64_t status_words) {
+    pdl_launch();
+    // the sort's tile status, zero before its first pass
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < status_words;
+         i += (uint64_t)gridDim.x * blockDim.x)
+        status[i] = 0u;
     __shared__ uint32_t sh[8 * 256];
     for (int i = threadIdx.x; i < 8 * 256; i += blockDim.x) sh[i] = 0u;
     __syncthreads();
+    pdl_wait();
     float lo[3], scale[3];
     const float maxq = (float)((1u << bpa) - 1u), cells = (float)(1u << bpa);
-    const bool any = cbounds[0] != INT32_MAX;
+    const bool any = __ldcg(cbounds) != INT32_MAX;
     float cext = 0.0f;  // longest axis of the centroid bounds
     for (int a = 0; a < 3; ++a) {
-        float l = any ? ford_inv(cbounds[a]) : 0.0f, h = any ? ford_inv(cbounds[3 + a]) : 0.0f;
+        float l = any ? ford_inv(__ldcg(cbounds + a)) : 0.0f, h = any ? ford_inv(__ldcg(cbounds + 3 + a)) : 0.0f;
         float ext = h - l;
         lo[a] = l;
         scale[a] = ext > 0.0f ? cells / ext : 0.0f;
@@ -486,17 +498,6 @@ __device__ __forceinline__ uint64_t exch_acq_rel(uint64_t *p, uint64_t v) {
     uint64_t old;
     asm volatile("atom.acq_rel.gpu.global.exch.b64 %0, [%1], %2;" : "=l"(old) : "l"(p), "l"(v) : "memory");
     return old;
-}
-
-// The root k_tree completed: a completed root is reached only through nodes
-// completed in this build, every reference in range.  If keys left out of
-// order by a sort that gave up kept it from completing one, leaf 0 stands in
-// and RT_ERR_BOUNDS is recorded, so the collapse reads nothing out of range.
-__global__ void k_tree_root(uint32_t *root, uint32_t n, uint32_t *err) {
-    const uint32_t r = *root, i = r & ~kLeafBit;
-    if ((r & kLeafBit) ? i < n : i + 1u < n) return;
-    report_error(err, RT_ERR_BOUNDS, 0x66000000u | (i & 0xffffffu));
-    *root = kLeafBit;
 }
 
 // A block per kTreeKeys consecutive keys.  Nodes inside the block's keys are
@@ -671,15 +672,16 @@ __global__ void __launch_bounds__(kTreeKeys, 1536 / kTreeKeys) k_tree(TreeArgs a
     __shared__ TreeShared s;
     const uint32_t t = threadIdx.x, base = blockIdx.x * kTreeKeys, j = base + t, n = a.n;
     const uint32_t count = min(n - base, kTreeKeys);
+    pdl_enter();
     Climb c;
     if (t == 0) {
         s.listed[0] = s.listed[1] = s.left = 0u;
-        s.delta[0] = base > 0u ? (int16_t)boundary_delta(__ldg(a.keys + base - 1u), __ldg(a.keys + base), base - 1u) : -1;
+        s.delta[0] = base > 0u ? (int16_t)boundary_delta(__ldcg(a.keys + base - 1u), __ldcg(a.keys + base), base - 1u) : -1;
     }
     s.seen[t] = 0u;
     if (t < count) {
-        const uint32_t id = __ldg(a.ids + j);
-        const uint64_t key = __ldg(a.keys + j), next = j + 1u < n ? __ldg(a.keys + j + 1u) : 0ull;
+        const uint32_t id = __ldcg(a.ids + j);
+        const uint64_t key = __ldcg(a.keys + j), next = j + 1u < n ? __ldcg(a.keys + j + 1u) : 0ull;
         s.delta[t + 1u] = j + 1u < n ? (int16_t)boundary_delta(key, next, j) : -1;
         if (j + 1u < n) a.other[j] = ~0ull;  // k_tree_climb's exchange word: no child yet
         if (id >= n) report_error(a.err, RT_ERR_BOUNDS, 0x67000000u | (j & 0xffffffu));  // not a sorted id
@@ -730,9 +732,10 @@ __global__ void __launch_bounds__(kTreeKeys, 1536 / kTreeKeys) k_tree(TreeArgs a
 // The subtrees k_tree left, one thread each.
 template <bool INST>
 __global__ void __launch_bounds__(128) k_tree_climb(TreeArgs a) {
-    const uint32_t m = *a.n_left;
+    pdl_enter();
+    const uint32_t m = __ldcg(a.n_left);
     for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < m; q += gridDim.x * blockDim.x)
-        climb_global<INST>(a, __ldg(a.left + q));
+        climb_global<INST>(a, __ldcg(a.left + q));
 }
 
 // ---------------------------------------------------------------------------
@@ -1339,7 +1342,19 @@ __global__ void __launch_bounds__(kCollapseThreads, 2) k_collapse(CollapseArgs a
     __shared__ uint4 s_red4[kCollapseThreads / 32];
     __shared__ uint4 s_info[kCollapseThreads];
     const uint32_t G = gridDim.x, b = blockIdx.x, t = threadIdx.x;
-    const uint32_t root_ref = a.root_dev ? __ldcg(a.root_dev) : a.root_ref;
+    // The root k_tree completed: a completed root is reached only through nodes
+    // completed in this build, every reference in range.  If keys left out of
+    // order by a sort that gave up kept it from completing one, leaf 0 stands in
+    // and RT_ERR_BOUNDS is recorded, so nothing is read out of range.
+    uint32_t root_ref = a.root_ref;
+    if (a.root_dev) {
+        root_ref = __ldcg(a.root_dev);
+        const uint32_t i = root_ref & ~kLeafBit;
+        if (!((root_ref & kLeafBit) ? i < a.n : i + 1u < a.n)) {
+            if (blockIdx.x == 0 && threadIdx.x == 0) report_error(a.err, RT_ERR_BOUNDS, 0x66000000u | (i & 0xffffffu));
+            root_ref = kLeafBit;
+        }
+    }
     // The first levels, up to one step of a block, are block 0's alone: block
     // barriers in the place of two grid barriers a level (7 us a level where a
     // level of 512 nodes takes 18).  The others wait at the first grid barrier
@@ -1479,6 +1494,12 @@ __global__ void __launch_bounds__(256) k_gather_records(const uint4 *__restrict_
 // ---------------------------------------------------------------------------
 // Host driver shared by BLAS and TLAS
 // ---------------------------------------------------------------------------
+//
+// A small build is a chain of short launches, so they overlap (pdl_enter) up to
+// the collapse, and what has to start at zero -- the sort's counters and tile
+// status, the collapse's barrier -- is cleared by the kernels before: with the
+// small sort tiles the 12,345-triangle build went from 232 to 156 us, the 1M soup
+// (whose sort keeps its tiles) from 600 to 563.
 
 int coop_grid(rt_context *ctx) {
     static int cached_dev = -1, cached = 0;
@@ -1540,7 +1561,11 @@ int run_build(rt_context *ctx, cudaStream_t st, const BuildCall &bc, const GeomP
     int32_t *cb = reinterpret_cast<int32_t *>(S + L.misc);
     static GeomParams empty_gp;  // zero-initialised; used by TLAS builds
     uint32_t *root_word = reinterpret_cast<uint32_t *>(S + L.misc + 64u);
-    k_init<<<1, 256, 0, st>>>(h, A, cb, root_word, gp ? *gp : empty_gp, gp ? 1u : 0u);
+    uint32_t *bar = reinterpret_cast<uint32_t *>(S + L.misc + 128u);
+    // (the tree's arrays, from L.bin to L.misc, are free during the sort)
+    const SortCounters sc = sort_counters(n, passes, S + L.sort, S + L.bin);
+    k_init<<<1, 256, 0, st>>>(h, A, cb, root_word, bar, sc.counters, sc.counter_words, gp ? *gp : empty_gp,
+                              gp ? 1u : 0u);
     RT_CUDA_CTX(ctx, cudaGetLastError());
     uint32_t *hdr_status = reinterpret_cast<uint32_t *>(A) + 7;  // rt_accel_header::status
     if (n == 0) {
@@ -1552,9 +1577,9 @@ int run_build(rt_context *ctx, cudaStream_t st, const BuildCall &bc, const GeomP
     float *boxes = reinterpret_cast<float *>(S + L.boxes);
     const unsigned nb = (n + 255u) / 256u;
     if (bc.kind == RT_ACCEL_KIND_BLAS) {
-        k_prep_tris<<<nb, 256, 0, st>>>(*gp, n, recs, boxes, cb, ctx->d_err, hdr_status);
+        RT_CUDA_CTX(ctx, launch_pdl(k_prep_tris, nb, 256, 0, st, *gp, n, recs, boxes, cb, ctx->d_err, hdr_status));
     } else {
-        k_prep_inst<<<nb, 256, 0, st>>>(instances, n, recs, boxes, cb);
+        RT_CUDA_CTX(ctx, launch_pdl(k_prep_inst, nb, 256, 0, st, instances, n, recs, boxes, cb));
     }
     RT_CUDA_CTX(ctx, cudaGetLastError());
 
@@ -1562,17 +1587,14 @@ int run_build(rt_context *ctx, cudaStream_t st, const BuildCall &bc, const GeomP
     uint64_t *keys1 = reinterpret_cast<uint64_t *>(S + L.keys1);
     uint32_t *ids0 = reinterpret_cast<uint32_t *>(S + L.ids0);
     uint32_t *ids1 = reinterpret_cast<uint32_t *>(S + L.ids1);
-    void *sort_s = S + L.sort;
-    uint32_t *hist = sort_hist_ptr(sort_s);
-    RT_CUDA_CTX(ctx, cudaMemsetAsync(hist, 0, 8u * 256u * 4u, st));
     {
         unsigned g = nb;
         unsigned cap_g = (unsigned)ctx->sm_count * 8u;
         if (g > cap_g) g = cap_g;
-        k_morton<<<g, 256, 0, st>>>(boxes, n, cb, bpa, keys0, ids0, hist, passes);
-        RT_CUDA_CTX(ctx, cudaGetLastError());
+        RT_CUDA_CTX(ctx, launch_pdl(k_morton, g, 256, 0, st, boxes, n, cb, bpa, keys0, ids0, sc.counters, passes, sc.status,
+                                    sc.status_words));
     }
-    int sst = sort_pairs(ctx, st, keys0, ids0, keys1, ids1, n, 8 * passes, sort_s, true, ctx->d_err);
+    int sst = sort_pairs(ctx, st, keys0, ids0, keys1, ids1, n, 8 * passes, S + L.sort, &sc, ctx->d_err);
     if (sst) return set_error(ctx, sst, "radix sort launch failed");
 
     uint4 *bin = reinterpret_cast<uint4 *>(S + L.bin);
@@ -1595,15 +1617,10 @@ int run_build(rt_context *ctx, cudaStream_t st, const BuildCall &bc, const GeomP
     // about 20 subtrees are left per block of k_tree
     unsigned climb_blocks = (tree_blocks + 3u) / 4u;
     if (climb_blocks > 8u * (unsigned)ctx->sm_count) climb_blocks = 8u * (unsigned)ctx->sm_count;
-    if (bc.kind == RT_ACCEL_KIND_BLAS) {
-        k_tree<false><<<tree_blocks, kTreeKeys, 0, st>>>(ta);
-        if (tree_blocks > 1u) k_tree_climb<false><<<climb_blocks, 128, 0, st>>>(ta);
-    } else {
-        k_tree<true><<<tree_blocks, kTreeKeys, 0, st>>>(ta);
-        if (tree_blocks > 1u) k_tree_climb<true><<<climb_blocks, 128, 0, st>>>(ta);
-    }
-    if (n >= 2) k_tree_root<<<1, 1, 0, st>>>(root_word, n, ctx->d_err);
-    RT_CUDA_CTX(ctx, cudaGetLastError());
+    const bool blas = bc.kind == RT_ACCEL_KIND_BLAS;
+    RT_CUDA_CTX(ctx, launch_pdl(blas ? k_tree<false> : k_tree<true>, tree_blocks, kTreeKeys, 0, st, ta));
+    if (tree_blocks > 1u)
+        RT_CUDA_CTX(ctx, launch_pdl(blas ? k_tree_climb<false> : k_tree_climb<true>, climb_blocks, 128, 0, st, ta));
 
     CollapseArgs ca;
     ca.n = n;
@@ -1623,14 +1640,13 @@ int run_build(rt_context *ctx, cudaStream_t st, const BuildCall &bc, const GeomP
     ca.blk = reinterpret_cast<uint32_t *>(S + L.blk);
     ca.nodes_out = reinterpret_cast<uint4 *>(A + h.node_offset);
     ca.hdr = reinterpret_cast<rt_accel_header *>(A);
-    ca.bar = reinterpret_cast<uint32_t *>(S + L.misc + 128u);
+    ca.bar = bar;
     ca.err = ctx->d_err;
-    RT_CUDA_CTX(ctx, cudaMemsetAsync(ca.bar, 0, 2u * sizeof(uint32_t), st));
     int G = coop_grid(ctx);
     if (G <= 0) return set_error(ctx, RT_ERR_CUDA, "cooperative occupancy query failed");
     // A block handles 64 nodes at a time (eight lanes each), and a small tree
     // is a chain of levels: 128 nodes of capacity per block, so that a level of
-    // a 12,345-triangle tree is at most one step (build 235 us; 239 at 64 or
+    // a 12,345-triangle tree is at most one step (build 235 us then; 239 at 64 or
     // 256 per block; at 1,024 the levels' later steps wait on the first's
     // loads).
     constexpr unsigned kNodesPerBlock = kCollapseThreads / 4;

@@ -332,6 +332,20 @@ __device__ __forceinline__ uint32_t take_child(uint2 &g, uint32_t prio) {
     return g.x + __popc((g.y >> 8) & (bit - 1u));
 }
 
+// Programmatic dependent launch between kernels of a chain: each lets the next
+// one launch as soon as all of its own blocks run, then waits for the kernel
+// before it to complete (its writes visible) before it reads or writes anything
+// that kernel does, so a launch's scheduling overlaps the previous kernel's
+// tail.  Every thread waits, so a kernel completes after all before it.  What
+// the kernel before writes is not read through the read-only path.  Launched
+// without the attribute both instructions do nothing.
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_enter() {
+    pdl_launch();
+    pdl_wait();
+}
+
 // Device-side error reporting: the first error code wins.
 __device__ __forceinline__ void report_error(uint32_t *err, int code, uint32_t detail) {
     if (err) {

@@ -103,6 +103,23 @@ int launch_queue_trace_multi_mixed(rt_context *ctx, cudaStream_t st, const void 
 // Loads the two traversal kernels of a shape (before a graph capture).
 int prepare_queue_trace_multi(rt_context *ctx, const TraceShape &shape);
 
+// Launch with programmatic stream serialization (see pdl_enter).
+template <typename... KArgs, typename... Args>
+cudaError_t launch_pdl(void (*kernel)(KArgs...), unsigned grid, unsigned threads, size_t smem, cudaStream_t st,
+                       Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
 // MLP cache launchers whose row counts live on the device (rt_mlp.cu).
 int cache_query_dev(rt_context *ctx, cudaStream_t st, const void *cache, const rt_cache_input *in, float *out,
                     const uint32_t *n_dev, uint32_t max_n);
@@ -111,10 +128,18 @@ int cache_train_dev(rt_context *ctx, cudaStream_t st, void *cache, const rt_cach
 
 // Sort (rt_sort.cu)
 uint64_t sort_scratch_bytes(uint32_t n, int passes);
+// What a sort with fused key generation needs zeroed beforehand: counters
+// (the digits' first, which the caller then counts) and tile status.
+struct SortCounters {
+    uint32_t *counters, *status;
+    uint32_t counter_words;
+    uint64_t status_words;
+    bool small;  // the small tiles
+};
+SortCounters sort_counters(uint32_t n, int passes, void *scratch, void *area);
 int sort_pairs(const rt_context *ctx, cudaStream_t stream, uint64_t *keys0, uint32_t *vals0, uint64_t *keys1,
-               uint32_t *vals1, uint32_t n, int key_bits, void *scratch, bool hist_done, uint32_t *err,
+               uint32_t *vals1, uint32_t n, int key_bits, void *scratch, const SortCounters *ready, uint32_t *err,
                uint32_t withhold = 0u);
-uint32_t *sort_hist_ptr(void *scratch);
 
 // Forgets the cached device address of the allocation-free build's static
 // scratch array on `device` (rt_build.cu); rt_context_create calls it so that

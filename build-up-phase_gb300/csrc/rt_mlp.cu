@@ -172,19 +172,6 @@ __device__ void encode_row(const rt_cache_input &in, const CacheState *S, __nv_b
 // per weight and tile), then delta_{L-1} = (delta_L W_L) * relu'(A_{L-1})
 // with W_L read transposed by ldmatrix.trans from its forward layout.
 
-// Programmatic dependent launch between the training kernels (forward +
-// backward, Adam, the next batch's forward + backward): each kernel lets the
-// next one launch as soon as all of its own blocks run, then waits for the
-// kernel before it to complete (its writes visible) before it reads or
-// writes anything, so a launch's scheduling overlaps the previous kernel's
-// tail.  Launched without the attribute both instructions do nothing.
-__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_enter() {
-    pdl_launch();
-    pdl_wait();
-}
-
 constexpr int kTrainRows = 128;
 constexpr int kTrainThreads = 256;
 __host__ __device__ constexpr int tw_rows(int l) { return l == 5 ? 16 : 64; }  // weight rows kept in shared memory
@@ -1137,23 +1124,6 @@ __global__ void k_cache_adam(CacheState *S, float *loss_out) {
 __global__ void k_cache_refresh_bf16(CacheState *S) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < kParams) S->wbf[i] = __float2bfloat16(S->params[i]);
-}
-
-// Launch with programmatic stream serialization (see pdl_enter).
-template <typename... KArgs, typename... Args>
-cudaError_t launch_pdl(void (*kernel)(KArgs...), unsigned grid, unsigned threads, size_t smem, cudaStream_t st,
-                       Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
 int set_smem(rt_context *ctx) {

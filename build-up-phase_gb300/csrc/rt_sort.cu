@@ -31,7 +31,13 @@ constexpr int kSortWarps = kSortThreads / 32;
 // waves, 1M-key soup build 0.807 ms; 16: 123 tiles, 0.792 ms then and equal
 // to 14 now on the soup; 14: 2M box 1.317 -> 1.306 ms)
 constexpr int kSortItems = 14;
-constexpr int kSortTile = kSortThreads * kSortItems;
+// Few keys: a tile is a serial chain (load, rank, look back, scatter), and
+// 12,345 keys were two tiles of it.  Build of 12,345 / 100K / 300K / 500K
+// triangles: 3 keys per thread 160 / 223 / 307 / 391 us, 4 165 / 226 / 298 / 387,
+// 8 183 / 238 / 306 / 395, 14 201 / 262 / 328 / 402 (156 / 224 / 314 / 394 at 3
+// with the launches overlapped); 700K keys are a draw, 1M 602 against 565.
+constexpr int kSortItemsSmall = 3;
+constexpr uint32_t kSortSmall = 1u << 19;  // keys up to which the small tiles are taken
 constexpr int kRankGroup = 8;  // keys ranked together (their votes, atomics and shuffles back to back)
 constexpr int kRadix = 256;
 // Statuses read per look-back round trip.  Tiles of one wave publish their
@@ -42,8 +48,13 @@ constexpr uint32_t kFlagAgg = 1u << 30;
 constexpr uint32_t kFlagIncl = 2u << 30;
 constexpr uint32_t kValueMask = (1u << 30) - 1u;
 
-constexpr size_t kSortSmemBytes =
-    (size_t)kSortTile * 8u + (size_t)kSortTile * 4u + (size_t)kSortWarps * kRadix * 4u;
+constexpr size_t sort_smem_bytes(int items) {
+    return (size_t)kSortThreads * items * 12u + (size_t)kSortWarps * kRadix * 4u;
+}
+constexpr uint64_t sort_tiles(uint32_t n, int items) {
+    const uint64_t tile = (uint64_t)kSortThreads * items;
+    return n > 0u ? (n + tile - 1u) / tile : 1u;
+}
 
 // Digit mask of pass p when sorting on the low key_bits bits.
 __host__ __device__ __forceinline__ uint32_t digit_mask(int key_bits, int p) {
@@ -93,6 +104,10 @@ __device__ __forceinline__ uint32_t block_scan256(uint32_t v, uint32_t *s_warp, 
     return excl;
 }
 
+// Launched while the kernel before may still be running (see pdl_enter); a later
+// pass (shift > 0) has its tile and the digits' prefix, which do not depend on
+// the pass before, at hand when the wait ends.
+template <int ITEMS>
 __global__ void __launch_bounds__(kSortThreads) k_onesweep(const uint64_t *__restrict__ kin,
                                                             const uint32_t *__restrict__ vin,
                                                             uint64_t *__restrict__ kout,
@@ -101,32 +116,38 @@ __global__ void __launch_bounds__(kSortThreads) k_onesweep(const uint64_t *__res
                                                             uint32_t *__restrict__ status,
                                                             uint32_t *__restrict__ tile_counter, uint32_t *err,
                                                             uint32_t spin_limit, uint32_t withhold) {
+    constexpr int kTile = kSortThreads * ITEMS;
     extern __shared__ __align__(16) uint8_t smem[];
     uint64_t *s_keys = reinterpret_cast<uint64_t *>(smem);
-    uint32_t *s_vals = reinterpret_cast<uint32_t *>(s_keys + kSortTile);
-    uint32_t *s_whist = s_vals + kSortTile;  // [warp][digit]
+    uint32_t *s_vals = reinterpret_cast<uint32_t *>(s_keys + kTile);
+    uint32_t *s_whist = s_vals + kTile;  // [warp][digit]
     __shared__ uint32_t s_digit_excl[kRadix];
     __shared__ uint32_t s_global[kRadix];
     __shared__ uint32_t s_warp[kRadix / 32 + 1];
     __shared__ uint32_t s_tile;
 
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    // (the first pass waits before it lets the second launch: what the second
+    // reads ahead of its own wait is complete then)
+    if (shift == 0) pdl_wait();
+    pdl_launch();
     if (t == 0) s_tile = atomicAdd(tile_counter, 1u);
     for (int i = t; i < kSortWarps * kRadix; i += kSortThreads) s_whist[i] = 0u;
-    __syncthreads();
+    const uint32_t gex = block_scan256(t < kRadix ? hist[t] : 0u, s_warp, nullptr);
     const uint32_t tile = s_tile;
-    const uint32_t base = tile * (uint32_t)kSortTile;
+    const uint32_t base = tile * (uint32_t)kTile;
+    if (shift > 0) pdl_wait();
 
-    uint64_t k[kSortItems];
-    uint32_t v[kSortItems];
-    uint32_t rank[kSortItems];
-    const uint32_t wbase = base + (uint32_t)w * 32u * kSortItems;
+    uint64_t k[ITEMS];
+    uint32_t v[ITEMS];
+    uint32_t rank[ITEMS];
+    const uint32_t wbase = base + (uint32_t)w * 32u * ITEMS;
 #pragma unroll
-    for (int j = 0; j < kSortItems; ++j) {
+    for (int j = 0; j < ITEMS; ++j) {
         uint32_t idx = wbase + (uint32_t)j * 32u + (uint32_t)lane;
         bool valid = idx < n;
-        k[j] = valid ? kin[idx] : 0ull;
-        v[j] = valid ? vin[idx] : 0u;
+        k[j] = valid ? __ldcg(kin + idx) : 0ull;
+        v[j] = valid ? __ldcg(vin + idx) : 0u;
     }
     const uint32_t lt = (1u << lane) - 1u;
     // Peers of each key (the valid lanes holding the same digit) from eight
@@ -137,12 +158,12 @@ __global__ void __launch_bounds__(kSortThreads) k_onesweep(const uint64_t *__res
     // (applied in issue order, which keeps the ranks in input order), then
     // the shuffles of the old counts, so no key waits on the one before it.
 #pragma unroll
-    for (int j0 = 0; j0 < kSortItems; j0 += kRankGroup) {
+    for (int j0 = 0; j0 < ITEMS; j0 += kRankGroup) {
         uint32_t pm[kRankGroup], old[kRankGroup];
 #pragma unroll
         for (int jj = 0; jj < kRankGroup; ++jj) {
             const int j = j0 + jj;
-            if (j >= kSortItems) break;  // a last, shorter group
+            if (j >= ITEMS) break;  // a last, shorter group
             const uint32_t d = (uint32_t)(k[j] >> shift) & dmask;
             uint32_t peers = __ballot_sync(0xffffffffu, wbase + (uint32_t)j * 32u + (uint32_t)lane < n);
 #pragma unroll
@@ -155,7 +176,7 @@ __global__ void __launch_bounds__(kSortThreads) k_onesweep(const uint64_t *__res
 #pragma unroll
         for (int jj = 0; jj < kRankGroup; ++jj) {
             const int j = j0 + jj;
-            if (j >= kSortItems) break;
+            if (j >= ITEMS) break;
             const uint32_t d = (uint32_t)(k[j] >> shift) & dmask;
             old[jj] = 0u;
             if ((int)(__ffs(pm[jj]) - 1) == lane)
@@ -164,7 +185,7 @@ __global__ void __launch_bounds__(kSortThreads) k_onesweep(const uint64_t *__res
 #pragma unroll
         for (int jj = 0; jj < kRankGroup; ++jj) {
             const int j = j0 + jj;
-            if (j >= kSortItems) break;
+            if (j >= ITEMS) break;
             const int leader = pm[jj] ? __ffs(pm[jj]) - 1 : lane;
             rank[j] = __shfl_sync(0xffffffffu, old[jj], leader) + (uint32_t)__popc(pm[jj] & lt);
         }
@@ -183,7 +204,6 @@ __global__ void __launch_bounds__(kSortThreads) k_onesweep(const uint64_t *__res
         total = s;
     }
     uint32_t dex = block_scan256(total, s_warp, nullptr);
-    uint32_t gex = block_scan256(t < kRadix ? hist[t] : 0u, s_warp, nullptr);
     if (t < kRadix) {
         s_digit_excl[t] = dex;
         volatile uint32_t *st = status;
@@ -229,7 +249,7 @@ __global__ void __launch_bounds__(kSortThreads) k_onesweep(const uint64_t *__res
     __syncthreads();
 
 #pragma unroll
-    for (int j = 0; j < kSortItems; ++j) {
+    for (int j = 0; j < ITEMS; ++j) {
         uint32_t idx = wbase + (uint32_t)j * 32u + (uint32_t)lane;
         if (idx < n) {
             uint32_t d = (uint32_t)(k[j] >> shift) & dmask;
@@ -239,7 +259,7 @@ __global__ void __launch_bounds__(kSortThreads) k_onesweep(const uint64_t *__res
         }
     }
     __syncthreads();
-    const uint32_t tile_n = (n - base) < (uint32_t)kSortTile ? (n - base) : (uint32_t)kSortTile;
+    const uint32_t tile_n = (n - base) < (uint32_t)kTile ? (n - base) : (uint32_t)kTile;
     for (uint32_t i = (uint32_t)t; i < tile_n; i += kSortThreads) {
         uint64_t key = s_keys[i];
         uint32_t d = (uint32_t)(key >> shift) & dmask;
@@ -253,63 +273,86 @@ __global__ void __launch_bounds__(kSortThreads) k_onesweep(const uint64_t *__res
     }
 }
 
+template <int ITEMS>
+int launch_passes(const rt_context *ctx, cudaStream_t stream, uint64_t *const keys[2], uint32_t *const vals[2],
+                  uint32_t n, int key_bits, const uint32_t *hist, uint32_t *status, uint32_t *counters, uint32_t *err,
+                  uint32_t withhold) {
+    const int passes = (key_bits + 7) / 8;
+    const uint64_t tiles = sort_tiles(n, ITEMS);
+    RT_CUDA_TRY(cudaFuncSetAttribute(k_onesweep<ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)sort_smem_bytes(ITEMS)));
+    for (int p = 0; p < passes; ++p) {
+        RT_CUDA_TRY(launch_pdl(k_onesweep<ITEMS>, (unsigned)tiles, kSortThreads, sort_smem_bytes(ITEMS), stream,
+                               keys[p & 1], vals[p & 1], keys[~p & 1], vals[~p & 1], n, 8 * p, digit_mask(key_bits, p),
+                               hist + p * kRadix, status + (size_t)p * tiles * kRadix, counters + p, err,
+                               ctx->sort_spin_limit, withhold));
+    }
+    return RT_OK;
+}
+
+// Counters of each pass's digits, then the passes' tile counters.
+constexpr uint64_t kCounterBytes = 8u * kRadix * 4u + 256u;
+
 }  // namespace
 
 uint64_t sort_scratch_bytes(uint32_t n, int passes) {
-    uint64_t tiles = ((uint64_t)n + kSortTile - 1) / kSortTile;
-    if (tiles == 0) tiles = 1;
+    const uint64_t tiles = sort_tiles(n, kSortItems);
     // histograms (8 x 256) + tile counters (8) + status (passes x tiles x 256)
-    return align_up(8u * kRadix * 4u, 256) + align_up(8u * 4u, 256) +
-           align_up((uint64_t)passes * tiles * kRadix * 4u, 256);
+    return kCounterBytes + align_up((uint64_t)passes * tiles * kRadix * 4u, 256);
 }
 
-// Sorts (keys0, vals0) on the low 8*passes key bits, using (keys1, vals1) as
-// the ping-pong buffer.  After an even number of passes the result is back in
-// keys0/vals0.  `keys_hist_done`: the caller already accumulated the digit
-// histograms into the scratch (fused with key generation).
+// `area`: where the status of more small tiles than the scratch is sized for
+// goes, at most 6 bytes per key and 8 KB (for at least 1,537 keys).
+SortCounters sort_counters(uint32_t n, int passes, void *scratch, void *area) {
+    SortCounters c;
+    c.small = n <= kSortSmall;
+    const uint64_t tiles = sort_tiles(n, c.small ? kSortItemsSmall : kSortItems);
+    c.counters = static_cast<uint32_t *>(scratch);
+    c.counter_words = (uint32_t)(kCounterBytes / 4u);
+    c.status = tiles > sort_tiles(n, kSortItems) ? static_cast<uint32_t *>(area) : c.counters + c.counter_words;
+    c.status_words = (uint64_t)passes * tiles * kRadix;
+    return c;
+}
+
+// Sorts (keys0, vals0) on the low key_bits key bits, using (keys1, vals1) as
+// the ping-pong buffer; the result is back in keys0/vals0.  `ready`: the caller
+// has zeroed its counters and status and then counted the digits (fused with
+// key generation); otherwise they are in the scratch.
 int sort_pairs(const rt_context *ctx, cudaStream_t stream, uint64_t *keys0, uint32_t *vals0, uint64_t *keys1,
-               uint32_t *vals1, uint32_t n, int key_bits, void *scratch, bool hist_done, uint32_t *err,
+               uint32_t *vals1, uint32_t n, int key_bits, void *scratch, const SortCounters *ready, uint32_t *err,
                uint32_t withhold) {
     if (n == 0) return RT_OK;
     const int passes = (key_bits + 7) / 8;
     if (n > kValueMask) return RT_ERR_UNSUPPORTED;
-    uint8_t *s = static_cast<uint8_t *>(scratch);
-    uint32_t *hist = reinterpret_cast<uint32_t *>(s);
-    uint32_t *counters = reinterpret_cast<uint32_t *>(s + align_up(8u * kRadix * 4u, 256));
-    uint32_t *status = reinterpret_cast<uint32_t *>(s + align_up(8u * kRadix * 4u, 256) + align_up(8u * 4u, 256));
-    uint64_t tiles = ((uint64_t)n + kSortTile - 1) / kSortTile;
-    // counters and status must start at zero; the histogram too unless the
-    // caller filled it.
-    if (!hist_done) {
-        RT_CUDA_TRY(cudaMemsetAsync(hist, 0, 8u * kRadix * 4u, stream));
+    SortCounters c;
+    if (ready) {
+        c = *ready;
+    } else {
+        c.small = false;
+        c.counters = static_cast<uint32_t *>(scratch);
+        c.status = c.counters + kCounterBytes / 4u;
+        RT_CUDA_TRY(cudaMemsetAsync(scratch, 0, kCounterBytes + (size_t)passes * sort_tiles(n, kSortItems) * kRadix * 4u,
+                                    stream));
         int blocks = (int)((n + 255u) / 256u);
         int cap = ctx->sm_count * 8;
         if (blocks > cap) blocks = cap;
-        k_sort_hist<<<blocks, 256, 0, stream>>>(keys0, n, key_bits, hist);
+        k_sort_hist<<<blocks, 256, 0, stream>>>(keys0, n, key_bits, c.counters);
         RT_CUDA_TRY(cudaGetLastError());
     }
-    RT_CUDA_TRY(cudaMemsetAsync(counters, 0, 8u * 4u, stream));
-    RT_CUDA_TRY(cudaMemsetAsync(status, 0, (size_t)passes * tiles * kRadix * 4u, stream));
-    RT_CUDA_TRY(cudaFuncSetAttribute(k_onesweep, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)kSortSmemBytes));
-    for (int p = 0; p < passes; ++p) {
-        const uint64_t *ki = (p & 1) ? keys1 : keys0;
-        const uint32_t *vi = (p & 1) ? vals1 : vals0;
-        uint64_t *ko = (p & 1) ? keys0 : keys1;
-        uint32_t *vo = (p & 1) ? vals0 : vals1;
-        k_onesweep<<<(unsigned)tiles, kSortThreads, kSortSmemBytes, stream>>>(
-            ki, vi, ko, vo, n, 8 * p, digit_mask(key_bits, p), hist + p * kRadix, status + (size_t)p * tiles * kRadix, counters + p, err,
-            ctx->sort_spin_limit, withhold);
-        RT_CUDA_TRY(cudaGetLastError());
-    }
+    uint64_t *const keys[2] = {keys0, keys1};
+    uint32_t *const vals[2] = {vals0, vals1};
+    uint32_t *tile_counters = c.counters + 8 * kRadix;
+    const int st = c.small ? launch_passes<kSortItemsSmall>(ctx, stream, keys, vals, n, key_bits, c.counters, c.status,
+                                                            tile_counters, err, withhold)
+                           : launch_passes<kSortItems>(ctx, stream, keys, vals, n, key_bits, c.counters, c.status,
+                                                       tile_counters, err, withhold);
+    if (st) return st;
     if (passes & 1) {
         RT_CUDA_TRY(cudaMemcpyAsync(keys0, keys1, (size_t)n * 8u, cudaMemcpyDeviceToDevice, stream));
         RT_CUDA_TRY(cudaMemcpyAsync(vals0, vals1, (size_t)n * 4u, cudaMemcpyDeviceToDevice, stream));
     }
     return RT_OK;
 }
-
-uint32_t *sort_hist_ptr(void *scratch) { return static_cast<uint32_t *>(scratch); }
 
 }  // namespace rtc
 
@@ -347,7 +390,7 @@ extern "C" rt_status rt_sort_pairs(rt_context *ctx, rt_stream stream, uint64_t *
     uint64_t *k1 = reinterpret_cast<uint64_t *>(s);
     uint32_t *v1 = reinterpret_cast<uint32_t *>(s + (size_t)n * 8u);
     void *sort_s = s + rtc::align_up((uint64_t)n * 12u, 256);
-    int st = rtc::sort_pairs(ctx, static_cast<cudaStream_t>(stream), keys, vals, k1, v1, n, (int)key_bits, sort_s, false,
+    int st = rtc::sort_pairs(ctx, static_cast<cudaStream_t>(stream), keys, vals, k1, v1, n, (int)key_bits, sort_s, nullptr,
                              ctx->d_err, ctx->sort_withhold);
     if (st) return rtc::set_error(ctx, st, "rt_sort_pairs: launch failed");
     return RT_OK;
