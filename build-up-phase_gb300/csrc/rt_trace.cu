@@ -243,7 +243,7 @@ __device__ bool trace_ray(const uint8_t *accel, const float o[3], const float d[
 // quarter of the lanes with a ray (or the refill threshold) have stopped:
 // entered on the spot, the entry and the triangle tests ran with a few lanes
 // each (10.5 active threads per instruction).  807K rays in 64 instances of
-// three meshes: 1,008 -> 822 us (without the rays set aside, kNearHits: 800; then
+// three meshes: 1,008 -> 815 us (without the rays set aside, kNearHits: 800; then
 // a fixed 4 / 8 / 16 stopped lanes 863 / 871 / 971, a third or an eighth of the
 // lanes 811 / 821).  What bounds it now: issue slots, half of them in steps of
 // warps whose last rays (of up to hundreds of nodes) are under way.  A lane leaves an instance without
@@ -254,6 +254,27 @@ constexpr uint32_t kInstGroup = 0x40000000u;   // stack entry: instances of a TL
 constexpr int kInstDepth = 128;                // stack entries per ray (both levels)
 constexpr uint32_t kInstBlocksPerSm = 6;       // 80 registers (7 blocks: 72, within 1 %)
 
+// is_flat in the instance's space or the world's: a hit's record and instance
+// record.
+__device__ __forceinline__ bool is_flat_inst(const uint4 *tprims, const uint4 &best) {
+    const InstRec ir = load_inst(tprims, best.w);
+    const uint8_t *blas = reinterpret_cast<const uint8_t *>(ir.accel_ref);
+    const rt_accel_header *bh = reinterpret_cast<const rt_accel_header *>(blas);
+    const uint4 *p = reinterpret_cast<const uint4 *>(blas + bh->prim_offset) + (size_t)(best.z & ~kMinusZero) * 3u;
+    if (is_flat(p)) return true;
+    // the world normal: the transposed world-to-object matrix times the object's
+    const float4 q0 = xyz_of(ldg4(p)), q1 = xyz_of(ldg4(p + 1)), q2 = xyz_of(ldg4(p + 2));
+    const float ax = q1.x - q0.x, ay = q1.y - q0.y, az = q1.z - q0.z;
+    const float bx = q2.x - q0.x, by = q2.y - q0.y, bz = q2.z - q0.z;
+    const float nx = ay * bz - az * by, ny = az * bx - ax * bz, nz = ax * by - ay * bx;
+    float w[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) w[a] = fabsf((ir.w2o[a] * nx + ir.w2o[4 + a] * ny) + ir.w2o[8 + a] * nz);
+    const float most = fmax3(w[0], w[1], w[2]);
+    const float rest = (w[0] + w[1]) + w[2] - most;
+    return !(rest > kFlat * most);
+}
+
 template <bool ANY>
 __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(const BatchArgs a) {
     const rt_accel_header *hd = reinterpret_cast<const rt_accel_header *>(a.accel);
@@ -263,7 +284,7 @@ __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(
     const uint32_t t_count = hd->node_count;
     const bool t_empty = hd->prim_count == 0;
     __shared__ uint2 s_stack[kRing][kTraceThreads];
-    __shared__ uint2 s_queue[kTraceThreads / 32][kTriQueue];  // leaf record, lane
+    __shared__ uint2 s_queue[kTraceThreads / 32][kTriQueue];  // leaf record, lane | step << 5
     // per lane: the world ray (origin, visiting order; inverse direction, the
     // ray's index); the triangle test's part of the object-space ray of the
     // instance entered last (origin, tmin; shear); the best hit so far -- t as
@@ -276,6 +297,7 @@ __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(
     __shared__ uint4 s_best[ANY ? 1 : kTraceThreads];
     __shared__ uint32_t s_near[kTraceThreads / 32];  // lanes (bits) whose ray is to be set aside, see kNearHits
     __shared__ uint32_t s_aside[ANY ? 1 : kTraceThreads];  // per lane: the last ray set aside
+    __shared__ uint32_t s_step[ANY ? 1 : kTraceThreads];   // the step (node visit) of the best hit so far
     constexpr uint32_t kFull = 0xffffffffu;
     const int tid = threadIdx.x, lane = tid & 31;
     uint2 *queue = s_queue[tid >> 5];
@@ -299,6 +321,7 @@ __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(
     uint2 spill[kInstDepth];
     uint32_t head = 0, tail = 0;  // queue positions tested / appended so far (the same in every lane)
     uint32_t last = ~0u;          // position of this lane's latest entry
+    uint32_t step = 0u;           // node visits of the warp so far
     uint32_t error = 0u;          // detail word of an error this lane's ray met
     const uint32_t n_rays = a.n;
     // fewer rays than lanes: see k_trace_blas
@@ -512,7 +535,8 @@ __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(
         const bool drain = walking == 0u || __popc(held) + __popc(ready & ~walking) >= serve;
 
         // ---- one node per lane, then the lane's next node (see k_trace_blas)
-        uint32_t leaves = 0u, step = 0u, meta_lo = 0u, meta_hi = 0u, pbase = 0u;
+        ++step;
+        uint32_t leaves = 0u, nth = 0u, meta_lo = 0u, meta_hi = 0u, pbase = 0u;
         if (pending && (visits >= count || node >= count))
             fail((in_blas ? 0x74000000u : 0x75000000u) | (node & 0xffffffu));
         if (pending) {
@@ -559,9 +583,9 @@ __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(
                 const uint32_t meta = __byte_perm(meta_lo, meta_hi, (uint32_t)__ffs((int)leaves) - 1u) & 0xffu;
                 last = tail + __popc(m & ((1u << lane) - 1u));
                 queue[last & (kTriQueue - 1u)] =
-                    make_uint2((meta & 0x20u) ? pbase + (meta & 0x1fu) + step : kNone, (uint32_t)lane);
-                const bool again = ((meta >> 6 >> step) & 1u) != 0u;
-                step = again ? step + 1u : 0u;
+                    make_uint2((meta & 0x20u) ? pbase + (meta & 0x1fu) + nth : kNone, step << 5 | (uint32_t)lane);
+                const bool again = ((meta >> 6 >> nth) & 1u) != 0u;
+                nth = again ? nth + 1u : 0u;
                 leaves = again ? leaves : leaves & (leaves - 1u);
             }
             tail += __popc(m);
@@ -572,7 +596,7 @@ __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(
                 __syncwarp();
                 uint2 e = make_uint2(kNone, (uint32_t)lane);
                 if ((uint32_t)lane < k) e = queue[(head + (uint32_t)lane) & (kTriQueue - 1u)];
-                const uint32_t rec = e.x, src = e.y;
+                const uint32_t rec = e.x, src = e.y & 31u;
                 __syncwarp();  // read before the next append reuses the slots
                 head += k;
                 const float4 ob = s_object[0][warp0 + src], shear = s_object[1][warp0 + src];
@@ -620,15 +644,21 @@ __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(
                     if (hit) atomicMin(bk, key);
                     __syncwarp();
                     hit = hit && *bk == key;
-                    if (hit)
+                    uint32_t other = 0u;  // the other hit's step
+                    if (hit) {
+                        other = s_step[warp0 + src];
+                        s_step[warp0 + src] = e.y >> 5;
                         s_best[warp0 + src] =
                             make_uint4(__float_as_uint(u), __float_as_uint(v),
                                        rec | (__float_as_uint(t) == kMinusZero ? kMinusZero : 0u), irec);
+                    }
                     __syncwarp();
                     if (any_hit) {
-                        // (the best hit is in this instance or ties with one in it)
+                        // see k_trace_blas; the best hit may be an earlier instance's
                         const float tb = ford_inv(*bt);
-                        if (fabsf((hit ? t_hi : t) - tb) <= kNearHits * fabsf(tb)) atomicOr(&s_near[tid >> 5], 1u << src);
+                        if (fabsf((hit ? t_hi : t) - tb) <= kNearHits * fabsf(tb) &&
+                            s_step[warp0 + src] != (hit ? other : e.y >> 5) && is_flat_inst(tprims, s_best[warp0 + src]))
+                            atomicOr(&s_near[tid >> 5], 1u << src);
                     }
                     tbest = ford_inv(s_t[tid]);
                 }
@@ -859,6 +889,7 @@ int launch_queue_trace_mixed(rt_context *ctx, cudaStream_t st, const uint8_t *ac
     a.out_rec = 1;
     a.counter = counter;
     uint32_t per_sm = ctx->tuning.blocks_per_sm ? ctx->tuning.blocks_per_sm : 8u;
+    if (per_sm > kAnyBlocksPerSm) per_sm = kAnyBlocksPerSm;
     uint32_t blocks = per_sm * (uint32_t)ctx->sm_count;
     const uint32_t need = (uint32_t)(((uint64_t)max_n * 2u + kTraceThreads - 1) / kTraceThreads);
     if (blocks > need) blocks = need;

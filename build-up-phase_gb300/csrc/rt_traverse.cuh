@@ -35,7 +35,7 @@ constexpr int kTraceThreads = 128;  // block size of the single-structure kernel
 // 16 entries did (1M soup: 2,150 -> 2,159 M rays/s; path tracer 6.33 -> 6.29
 // ms per sample); deeper entries spill to local memory.
 constexpr int kRing = 8;
-constexpr uint32_t kAnyBlocksPerSm = 1024u / kTraceThreads;  // resident blocks the any-hit kernel is bounded for
+constexpr uint32_t kAnyBlocksPerSm = 1024u / kTraceThreads;  // resident blocks the any-hit and mixed kernels are bounded for
 constexpr int kMaxDepth = 64;       // total stack entries per ray
 constexpr uint32_t kNone = 0xffffffffu;
 constexpr uint32_t kMinusZero = 0x80000000u;  // the bits of -0; in a record index (below 2^30) the mark of a hit at t = -0
@@ -112,12 +112,15 @@ struct BatchArgs {
 // than the triangle, would have cut off: rounding, seen where the two hits are
 // coincident or nearly so and the triangle lies in an axis plane, so that its
 // boxes have no thickness to spare.  A ray whose best hit is such a triangle,
-// with another hit within kNearHits of its distance, is set aside -- its result's
+// with another node's hit within kNearHits of its distance, is set aside -- its result's
 // place links the lane's rays of that kind -- and walked in order once the lane
 // is done with the others.  (12 coincident copies of 60 axis-parallel triangles,
-// 1M rays: 0 to 3 rays differed from the restatement.  The check costs the
-// mixed launches 1 %; walking such a ray again within the loop cost the soup's
-// rays 13 %, in a function called on the spot 40 %: registers on every path.)
+// 1M rays: 0 to 3 rays differed from the restatement.  The check is within 1 %
+// of the soup's and the 2M box's time; walking such a ray again within the loop
+// cost the soup's rays 13 %, in a function called on the spot 40 %: registers on
+// every path.  A box whose every triangle is there twice, 1M rays: 298 us, 210
+// with them once, 690 with hits of one node taken for two and a loop per ray;
+// 342 when every record is tested on the spot.)
 constexpr float kNearHits = 0x1p-12f;
 constexpr float kFlat = 0x1p-8f;  // extent along an axis over the largest extent
 constexpr uint32_t kTriQueue = 64;  // entries per warp: below 32 before an append of at most 32
@@ -136,61 +139,20 @@ __device__ __forceinline__ bool is_flat(const uint4 *p) {
     return fmin3(ex, ey, ez) <= kFlat * fmax3(ex, ey, ez);
 }
 
-// The closest hit of a ray (origin and tmin, direction and tmax), every record
-// tested as its node is visited.
-__device__ __forceinline__ Hit walk_in_order(const uint4 *nodes, const uint4 *prims, uint32_t count,
-                                             const float4 &r0, const float4 &r1) {
-    const float o[3] = {r0.x, r0.y, r0.z}, d[3] = {r1.x, r1.y, r1.z};
-    Ray r;
-    ray_setup(r, o, d);
-    Hit h;
-    h.t = r1.w; h.u = 0.f; h.v = 0.f; h.rec = kNone; h.tri = kNone; h.inst = 0u; h.found = false;
-    uint2 stack[kMaxDepth];
-    int sp = 0;
-    uint32_t node = 0;
-    // (what the first walk reported of a corrupt structure is not reported again)
-    for (uint32_t visits = 0; visits < count && node < count; ++visits) {
-        const NodeWords nd = load_node(nodes, node);
-        const uint32_t hits = isect_node(r, nd, r0.w, h.t);
-        for (uint32_t recs = leaf_records(nd, hits); recs; recs &= recs - 1u) {
-            const uint32_t rec = nd.w1.y + (uint32_t)__ffs((int)recs) - 1u;
-            const uint4 *p = prims + (size_t)rec * 3u;
-            const uint4 q0 = ldg4(p), q1 = ldg4(p + 1), q2 = ldg4(p + 2);
-            float t, u, v;
-            if (!isect_tri(r, xyz_of(q0), xyz_of(q1), xyz_of(q2), r0.w, h.t, t, u, v)) continue;
-            if (t < h.t || (t == h.t && q0.w < h.tri)) {
-                h.t = t; h.u = u; h.v = v; h.rec = rec; h.tri = q0.w; h.found = true;
-            }
-        }
-        uint2 g = child_group(nd, hits);
-        if (!group_left(g)) {
-            if (sp == 0) break;
-            g = stack[--sp];
-        }
-        node = take_child(g, r.prio);
-        if (group_left(g)) {
-            if (sp == kMaxDepth) break;
-            stack[sp++] = g;
-        }
-    }
-    return h;
-}
-
 // MIXED: one launch over two queues -- the closest-hit rays (rays, n_dev;
 // results to hits) and then the any-hit rays (rays2, n_dev2; results to
 // occluded) -- each ray walked exactly as in a launch of its own kind; the
 // path tracer traces a depth's shadow rays and the next depth's extension
 // rays together, so the two share one launch tail.
-// Register budget: the closest-hit and mixed single-structure kernels fit
-// nine 128-thread blocks per SM (56 registers; at eight blocks and 64
-// registers the 1M soup's rays take 1.71 instead of 1.68 ms, the path-traced
-// frame 23.3 instead of 22.6); the any-hit and multi-scene kernels keep eight
-// blocks and 64 registers.
+// Register budget: the closest-hit single-structure kernel fits nine 128-thread
+// blocks per SM (56 registers; at eight blocks and 64 registers the 1M soup's
+// rays take 1.71 instead of 1.68 ms); the others keep eight blocks and 64
+// registers (mixed, nine blocks: 2M box 21.26 ms per four samples, eight 20.85).
 template <bool ANY, bool MULTI, int THREADS, int RING, bool MIXED = false>
-__global__ void __launch_bounds__(THREADS, ((MULTI || ANY) ? 1024 : 1152) / THREADS) k_trace_blas(const BatchArgs a) {
+__global__ void __launch_bounds__(THREADS, ((MULTI || ANY || MIXED) ? 1024 : 1152) / THREADS) k_trace_blas(const BatchArgs a) {
     static_assert((RING & (RING - 1)) == 0 && RING <= kMaxDepth, "RING is a power of two");
     __shared__ uint2 s_stack[RING][THREADS];
-    __shared__ uint2 s_queue[THREADS / 32][kTriQueue];  // leaf record, lane
+    __shared__ uint2 s_queue[THREADS / 32][kTriQueue];  // leaf record, lane | visits << 5
     // per lane: the triangle test's part of the ray (written once per ray, read
     // by whichever lane tests); the best hit so far -- t as an ordered integer;
     // u, v, leaf record and triangle (kNone: no hit) --; the ray's index
@@ -200,6 +162,7 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY) ? 1024 : 1152) / THRE
     __shared__ uint32_t s_ray[THREADS];
     __shared__ uint32_t s_near[THREADS / 32];  // lanes (bits) whose ray is to be set aside, see kNearHits
     __shared__ uint32_t s_aside[ANY ? 1 : THREADS];  // per lane: the last ray set aside
+    __shared__ uint32_t s_visit[ANY ? 1 : THREADS];  // the node visit of the best hit so far
     const uint4 *nodes = nullptr, *prims = nullptr;
     // A tree walk visits each node at most once: more visits, or a node index
     // past the end, can only come from a corrupt structure.
@@ -365,7 +328,7 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY) ? 1024 : 1152) / THRE
         // ---- one node per lane, then the lane's next node
         // leaf slots met (bits), the record reached in the first of them, and
         // the node's slot bytes and record base
-        uint32_t leaves = 0u, step = 0u, meta_lo = 0u, meta_hi = 0u, pbase = 0u;
+        uint32_t leaves = 0u, nth = 0u, meta_lo = 0u, meta_hi = 0u, pbase = 0u;
         // (errors are noted and reported with the result: no calls in here, and
         // the rare cases -- a spilled stack entry -- are the only branches)
         if (pending && (visits >= max_visits || node >= max_visits)) {
@@ -416,9 +379,9 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY) ? 1024 : 1152) / THRE
                 const uint32_t meta = __byte_perm(meta_lo, meta_hi, (uint32_t)__ffs((int)leaves) - 1u) & 0xffu;
                 last = tail + __popc(m & ((1u << lane) - 1u));
                 queue[last & (kTriQueue - 1u)] =
-                    make_uint2((meta & 0x20u) ? pbase + (meta & 0x1fu) + step : kNone, (uint32_t)lane);
-                const bool again = ((meta >> 6 >> step) & 1u) != 0u;
-                step = again ? step + 1u : 0u;
+                    make_uint2((meta & 0x20u) ? pbase + (meta & 0x1fu) + nth : kNone, visits << 5 | (uint32_t)lane);
+                const bool again = ((meta >> 6 >> nth) & 1u) != 0u;
+                nth = again ? nth + 1u : 0u;
                 leaves = again ? leaves : leaves & (leaves - 1u);
             }
             tail += __popc(m);
@@ -429,7 +392,7 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY) ? 1024 : 1152) / THRE
                 __syncwarp();
                 uint2 e = make_uint2(kNone, (uint32_t)lane);
                 if ((uint32_t)lane < k) e = queue[(head + (uint32_t)lane) & (kTriQueue - 1u)];
-                const uint32_t rec = e.x, src = e.y;
+                const uint32_t rec = e.x, src = e.y & 31u;
                 const bool have = rec != kNone;
                 __syncwarp();  // read before the next append reuses the slots
                 head += k;
@@ -477,16 +440,21 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY) ? 1024 : 1152) / THRE
                     if (hit) atomicMin(&best->w, tri);
                     __syncwarp();
                     hit = hit && best->w == tri;
+                    uint32_t other = 0u;  // the other hit's visit
                     if (hit) {
+                        other = s_visit[warp0 + src];
+                        s_visit[warp0 + src] = e.y >> 5;
                         best->x = __float_as_uint(u);
                         best->y = __float_as_uint(v);
                         best->z = rec | (__float_as_uint(t) == kMinusZero ? kMinusZero : 0u);
                     }
                     __syncwarp();
                     if (any_hit) {
-                        // this hit against the best one, the best against the one before
+                        // this hit against the best one, the best against the
+                        // one before; records of one node are tested together
                         const float tb = ford_inv(*bt);
                         if (fabsf((hit ? t_hi : t) - tb) <= kNearHits * fabsf(tb) &&
+                            s_visit[warp0 + src] != (hit ? other : e.y >> 5) &&
                             is_flat(pr + (size_t)(best->z & ~kMinusZero) * 3u))
                             atomicOr(&s_near[tid >> 5], 1u << src);
                     }
@@ -506,14 +474,59 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY) ? 1024 : 1152) / THRE
         }
     }
 
-    // ---- the rays set aside
+    // ---- the rays set aside, each lane its own, every record tested as its
+    // node is visited (one loop over rays and nodes: the lanes' walks differ)
     if (!ANY) {
-        for (uint32_t i = s_aside[tid]; i != kNone;) {
-            const uint32_t next = *result_place(i);
-            if (MULTI) scene_of(__ldg(a.ray_scene + i));
-            const Hit h = walk_in_order(nodes, prims, max_visits, __ldg(a.rays + 2u * i), __ldg(a.rays + 2u * i + 1u));
-            write_hit(i, h.found, h.t, h.u, h.v, h.rec, h.tri);
-            i = next;
+        uint32_t idx = kNone, next = s_aside[tid], at = 0u, seen = 0u;
+        int depth = 0;
+        bool walking = false;
+        Hit h;
+        h.t = 0.f; h.u = 0.f; h.v = 0.f; h.rec = kNone; h.tri = kNone;
+        Ray w;
+        w.prio = 0u;
+        float t_lo = 0.f;
+        uint2 stack[kMaxDepth];
+        for (;;) {
+            if (!walking) {
+                if (idx != kNone) write_hit(idx, h.tri != kNone, h.t, h.u, h.v, h.rec, h.tri);
+                idx = next;
+                if (idx == kNone) break;
+                next = *result_place(idx);
+                if (MULTI) scene_of(__ldg(a.ray_scene + idx));
+                const float4 r0 = __ldg(a.rays + 2u * idx), r1 = __ldg(a.rays + 2u * idx + 1u);
+                const float o[3] = {r0.x, r0.y, r0.z}, d[3] = {r1.x, r1.y, r1.z};
+                ray_setup(w, o, d);
+                t_lo = r0.w;
+                h.t = r1.w;
+                h.tri = kNone;
+                at = 0u;
+                seen = 0u;
+                depth = 0;
+            }
+            // (what the first walk reported of a corrupt structure is not reported again)
+            walking = seen < max_visits && at < max_visits;
+            if (!walking) continue;
+            ++seen;
+            const NodeWords nd = load_node(nodes, at);
+            const uint32_t hits = isect_node(w, nd, t_lo, h.t);
+            for (uint32_t recs = leaf_records(nd, hits); recs; recs &= recs - 1u) {
+                const uint32_t rec = nd.w1.y + (uint32_t)__ffs((int)recs) - 1u;
+                const uint4 *p = prims + (size_t)rec * 3u;
+                const uint4 q0 = ldg4(p), q1 = ldg4(p + 1), q2 = ldg4(p + 2);
+                float t, u, v;
+                if (!isect_tri(w, xyz_of(q0), xyz_of(q1), xyz_of(q2), t_lo, h.t, t, u, v)) continue;
+                if (t < h.t || q0.w < h.tri) {  // (t <= h.t)
+                    h.t = t; h.u = u; h.v = v; h.rec = rec; h.tri = q0.w;
+                }
+            }
+            uint2 g = child_group(nd, hits);
+            if (!group_left(g) && depth > 0) g = stack[--depth];
+            walking = group_left(g);
+            at = take_child(g, w.prio);  // (of no group: unused)
+            if (walking && group_left(g)) {
+                if (depth < kMaxDepth) stack[depth++] = g;
+                else walking = false;
+            }
         }
     }
 }

@@ -393,9 +393,9 @@ rt_status rt_trace_stats(rt_context *ctx, rt_stream stream, uint64_t accel,
 /* ------------------------------------------------------------------------ */
 
 /* Launch shape of the traversal kernel.  blocks_per_sm applies to every
- * single-structure traversal (ray-query calls and rt_path_trace; any-hit
- * launches use at most 8); batch_rays to the ray-query calls only -- the path
- * tracer's queue traversals refill at 8 idle lanes, the batch uses its own
+ * single-structure traversal (ray-query calls and rt_path_trace; any-hit and
+ * mixed launches use at most 8); batch_rays to the ray-query calls only -- the
+ * path tracer's queue traversals refill at 8 idle lanes, the batch uses its own
  * autotuned shape.  Defaults: 128, 9, 4. */
 typedef struct rt_trace_tuning {
     uint32_t block_threads;   /* threads per block of the traversal kernel */
