@@ -123,7 +123,8 @@ __device__ __forceinline__ float sel3(uint32_t k, float x, float y, float z) {
     return k == 0 ? x : (k == 1 ? y : z);
 }
 
-__device__ __forceinline__ void ray_setup(Ray &r, const float o[3], const float d[3]) {
+// The box test's part of a ray: all a walk needs until it meets a triangle.
+__device__ __forceinline__ void ray_setup_box(Ray &r, const float o[3], const float d[3]) {
     uint32_t oct = 0;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
@@ -134,6 +135,11 @@ __device__ __forceinline__ void ray_setup(Ray &r, const float o[3], const float 
         oct |= (r.invd[a] < 0.0f ? 1u : 0u) << a;
     }
     r.prio = child_priority(oct);
+}
+
+// The triangle test's part, of a ray set up for the box test.
+__device__ __forceinline__ void ray_setup_shear(Ray &r) {
+    const float *d = r.d;
     float ax = fabsf(d[0]), ay = fabsf(d[1]), az = fabsf(d[2]);
     uint32_t kz = ax >= ay ? (ax >= az ? 0u : 2u) : (ay >= az ? 1u : 2u);
     uint32_t kx = kz == 2u ? 0u : kz + 1u;
@@ -146,6 +152,11 @@ __device__ __forceinline__ void ray_setup(Ray &r, const float o[3], const float 
     // the largest component's reciprocal, computed above unless the whole
     // direction is below RT_DIR_EPS
     r.sz = fabsf(dkz) < RT_DIR_EPS ? 1.0f / dkz : sel3(kz, r.invd[0], r.invd[1], r.invd[2]);
+}
+
+__device__ __forceinline__ void ray_setup(Ray &r, const float o[3], const float d[3]) {
+    ray_setup_box(r, o, d);
+    ray_setup_shear(r);
 }
 
 // Returns true and (t, u, v) when the triangle is hit with t in [tmin, tmax].

@@ -51,7 +51,7 @@ struct LocalStack {
 };
 
 template <bool ANY>
-__device__ bool traverse_blas_simple(const uint8_t *accel, const Ray &r, float tmin, Hit &h, uint64_t &hkey,
+__device__ bool traverse_blas_simple(const uint8_t *accel, Ray &r, float tmin, Hit &h, uint64_t &hkey,
                                      uint32_t inst, uint32_t *err, unsigned long long *stats) {
     const rt_accel_header *hd = reinterpret_cast<const rt_accel_header *>(accel);
     if (hd->prim_count == 0) return false;
@@ -60,6 +60,7 @@ __device__ bool traverse_blas_simple(const uint8_t *accel, const Ray &r, float t
     LocalStack st;
     st.sp = 0;
     uint32_t node = 0;
+    bool sheared = false;  // r is set up for boxes, for triangles once it meets one
     // A tree walk visits each node at most once; more visits (or a node
     // index past the end) can only come from a corrupt structure.
     const uint32_t max_visits = hd->node_count;
@@ -79,6 +80,8 @@ __device__ bool traverse_blas_simple(const uint8_t *accel, const Ray &r, float t
             const uint4 *rec = prims + (size_t)(pbase + i) * 3u;
             uint4 a = ldg4(rec), b = ldg4(rec + 1), c = ldg4(rec + 2);
             if (stats) stats[1]++;
+            if (!sheared) ray_setup_shear(r);
+            sheared = true;
             float t, u, v;
             if (!isect_tri(r, make_float4(__uint_as_float(a.x), __uint_as_float(a.y), __uint_as_float(a.z), 0.f),
                            make_float4(__uint_as_float(b.x), __uint_as_float(b.y), __uint_as_float(b.z), 0.f),
@@ -148,7 +151,7 @@ __device__ bool trace_ray(const uint8_t *accel, const float o[3], const float d[
     ids.custom = 0; ids.sbt_off = 0; ids.geom = 0; ids.prim = 0;
     uint64_t hkey = ~0ull;
     Ray r;
-    ray_setup(r, o, d);
+    ray_setup_box(r, o, d);
     const uint8_t *hit_blas = accel;
     if (hd->kind == RT_ACCEL_KIND_BLAS) {
         bool any = traverse_blas_simple<ANY>(accel, r, tmin, h, hkey, 0u, err, stats);
@@ -185,7 +188,7 @@ __device__ bool trace_ray(const uint8_t *accel, const float o[3], const float d[
             xform_point(ir.w2o, o, o2);
             xform_vector(ir.w2o, d, d2);
             Ray r2;
-            ray_setup(r2, o2, d2);
+            ray_setup_box(r2, o2, d2);
             const uint8_t *blas = reinterpret_cast<const uint8_t *>(ir.accel_ref);
             bool hit = traverse_blas_simple<ANY>(blas, r2, tmin, h, hkey, ir.id, err, stats);
             // instances occur once in a TLAS: a best hit carrying this id
@@ -721,7 +724,6 @@ struct PipelineArgs {
     const float *sbt;
     uint32_t sbt_count, sbt_stride;
     float4 *out;
-    rt_ray *rays_out;  // when set: write the primary rays instead of tracing
     uint32_t *err;
 };
 
@@ -736,32 +738,22 @@ __device__ __forceinline__ void raygen(const PipelineArgs &a, uint32_t x, uint32
     dir[2] = (p * 0.0f + q * 0.0f) + -1.0f;
 }
 
-// Six blocks per SM (80 registers): the walk is latency-bound (1200x800
-// pixels of the two-instance sample: 22.5 us; 24.3 at five blocks, 23.1 at
-// eight, 26.2 with the compiler's choice of 126 registers).
+// Six blocks per SM (80 registers).  Two thirds of the issue slots are busy: 590
+// instructions per warp with the triangle test's ray setup (divisions) done for
+// every level and instance, before a triangle is met, and both kinds of walk in
+// one kernel.  1200x800 pixels of the two-instance sample: 22.5 -> 20.5 us (5 or
+// 7 blocks per SM the same, 4 22.5).
+template <bool ANY>
 __global__ void __launch_bounds__(128, 6) k_pipeline(const PipelineArgs a) {
     const uint32_t x = blockIdx.x * 16u + (threadIdx.x & 15u);
     const uint32_t y = blockIdx.y * 8u + (threadIdx.x >> 4);
     if (x >= a.width || y >= a.height) return;
     float dir[3];
     raygen(a, x, y, dir);
-    const size_t pix = (size_t)y * a.width + x;
-    if (a.rays_out) {
-        rt_ray rr;
-        rr.org[0] = a.cam[0]; rr.org[1] = a.cam[1]; rr.org[2] = a.cam[2];
-        rr.dir[0] = dir[0]; rr.dir[1] = dir[1]; rr.dir[2] = dir[2];
-        rr.tmin = a.tmin;
-        rr.tmax = a.tmax;
-        a.rays_out[pix] = rr;
-        return;
-    }
     Hit h;
     HitIds ids;
     float c[3];
-    if (a.ray_flags & RT_RAY_FLAG_TERMINATE_ON_FIRST_HIT)
-        trace_ray<true>(a.accel, a.cam, dir, a.tmin, a.tmax, a.cull_mask & 0xffu, h, ids, a.err, nullptr);
-    else
-        trace_ray<false>(a.accel, a.cam, dir, a.tmin, a.tmax, a.cull_mask & 0xffu, h, ids, a.err, nullptr);
+    trace_ray<ANY>(a.accel, a.cam, dir, a.tmin, a.tmax, a.cull_mask & 0xffu, h, ids, a.err, nullptr);
     if (!h.found) {
         c[0] = a.miss[0]; c[1] = a.miss[1]; c[2] = a.miss[2];
     } else if (a.ray_flags & RT_RAY_FLAG_SKIP_CLOSEST_HIT) {
@@ -782,7 +774,20 @@ __global__ void __launch_bounds__(128, 6) k_pipeline(const PipelineArgs a) {
             report_error(a.err, RT_ERR_BOUNDS, 0x73000000u | rec);
         }
     }
-    a.out[pix] = make_float4(c[0], c[1], c[2], 0.0f);
+    a.out[(size_t)y * a.width + x] = make_float4(c[0], c[1], c[2], 0.0f);
+}
+
+// The raygen's rays alone.
+__global__ void __launch_bounds__(128) k_primary_rays(const PipelineArgs a, rt_ray *rays) {
+    const uint32_t x = blockIdx.x * 16u + (threadIdx.x & 15u);
+    const uint32_t y = blockIdx.y * 8u + (threadIdx.x >> 4);
+    if (x >= a.width || y >= a.height) return;
+    rt_ray rr;
+    raygen(a, x, y, rr.dir);
+    rr.org[0] = a.cam[0]; rr.org[1] = a.cam[1]; rr.org[2] = a.cam[2];
+    rr.tmin = a.tmin;
+    rr.tmax = a.tmax;
+    rays[(size_t)y * a.width + x] = rr;
 }
 
 // ---------------------------------------------------------------------------
@@ -1211,10 +1216,10 @@ extern "C" rt_status rt_trace_rays(rt_context *ctx, rt_stream stream, const rt_p
     a.sbt_count = sbt && sbt->hit_colors ? sbt->hit_record_count : 0u;
     a.sbt_stride = sbt ? (sbt->hit_record_stride < 3u ? 3u : sbt->hit_record_stride) : 3u;
     a.out = reinterpret_cast<float4 *>(out);
-    a.rays_out = nullptr;
     a.err = ctx->d_err;
     dim3 grid((width + 15u) / 16u, (height + 7u) / 8u);
-    k_pipeline<<<grid, 128, 0, static_cast<cudaStream_t>(stream)>>>(a);
+    const auto kernel = (p->ray_flags & RT_RAY_FLAG_TERMINATE_ON_FIRST_HIT) ? k_pipeline<true> : k_pipeline<false>;
+    kernel<<<grid, 128, 0, static_cast<cudaStream_t>(stream)>>>(a);
     RT_CUDA_CTX(ctx, cudaGetLastError());
     return RT_OK;
 }
@@ -1231,10 +1236,9 @@ extern "C" rt_status rt_generate_primary_rays(rt_context *ctx, rt_stream stream,
     a.height = height;
     a.tmin = tmin;
     a.tmax = tmax;
-    a.rays_out = rays;
     a.err = ctx->d_err;
     dim3 grid((width + 15u) / 16u, (height + 7u) / 8u);
-    k_pipeline<<<grid, 128, 0, static_cast<cudaStream_t>(stream)>>>(a);
+    k_primary_rays<<<grid, 128, 0, static_cast<cudaStream_t>(stream)>>>(a, rays);
     RT_CUDA_CTX(ctx, cudaGetLastError());
     return RT_OK;
 }
