@@ -170,6 +170,7 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY || MIXED) ? 1024 : 115
     bool empty = true;
     if (!MULTI) {
         const rt_accel_header *hd = reinterpret_cast<const rt_accel_header *>(a.accel);
+        if (!MIXED && !a.n_dev) pdl_launch();  // a ray query's k_trace_inst
         if (hd->kind != RT_ACCEL_KIND_BLAS) return;  // k_trace_inst handles it
         nodes = reinterpret_cast<const uint4 *>(a.accel + hd->node_offset);
         prims = reinterpret_cast<const uint4 *>(a.accel + hd->prim_offset);
