@@ -83,7 +83,7 @@ int launch_queue_trace_mixed(rt_context *ctx, cudaStream_t st, const uint8_t *ac
 struct TraceShape {
     uint32_t threads;        // 128 or 256
     uint32_t blocks_per_sm;
-    uint32_t ring;           // 8, 16 or 32 shared-memory stack entries per ray
+    uint32_t ring;           // 8, 16 or 32 entries of shared memory per ray (rt_trace_multi.cu)
     uint32_t refill;         // 1..32
 };
 

@@ -727,6 +727,11 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_cache_fwd_bwd_small(CacheS
 // 32-bit column): the activations never pass through shared memory.  Every
 // mbarrier wait is bounded: on expiry the kernel records RT_ERR_TIMEOUT, waits
 // once more (bounded) for its MMAs, frees its TMEM and returns.
+//
+// 2,073,600 queries: 141 us, tensor pipe 62 % busy (an MMA of N = 64 fills half
+// of it), the rest the encoding and the epilogues.  248 us with four groups, the
+// biases stored to TMEM for every row and layer and the activations written to
+// shared memory in the MMA's layout.
 
 constexpr int kTcRows = 128;
 constexpr int kTcGroups = 5;                      // independent 128-row tile groups per CTA

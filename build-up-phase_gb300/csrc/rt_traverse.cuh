@@ -100,11 +100,12 @@ struct BatchArgs {
 // has been tested.  1M soup, 4.15M primary and incoherent rays: 28.6 entries
 // per batch, 18.4 nodes and 4.4 triangles per ray against 17.7 and 4.0 when
 // every triangle is tested on the spot, 28.1 of 32 lanes walking per node step
-// (2M box, mixed launches: 27.4).  With the box test's instruction count this
-// took the launch from 1.92 to 1.68 ms (1.86 to 1.55 G warp instructions), the
-// path tracer's 2M-triangle frame of four samples from 25.7 to 23.4 ms.  What
-// bounds it now: issue slots (78 % busy) and the L1 data path (70 %: a node is
-// five 16-byte loads per lane, nearly every one a wavefront of its own).
+// (2M box, mixed launches: 27.4).  With the box test's instruction count, the
+// 64-bit queue entry and the hits' shared-memory minima this took the launch from
+// 1.92 to 1.56 ms, the path tracer's 2M-triangle frame of four samples from 25.7
+// to 20.9.  What bounds it now: issue slots (79 % busy) and the L1 data path
+// (78 %: a node is five 16-byte loads per lane, nearly every one a wavefront of
+// its own).
 //
 // In the order of the CPU restatement a record is tested, and the far limit
 // shrunk, before the next node's boxes.  A walk that goes on meanwhile can only
@@ -146,7 +147,7 @@ __device__ __forceinline__ bool is_flat(const uint4 *p) {
 // rays together, so the two share one launch tail.
 // Register budget: the closest-hit single-structure kernel fits nine 128-thread
 // blocks per SM (56 registers; at eight blocks and 64 registers the 1M soup's
-// rays take 1.71 instead of 1.68 ms); the others keep eight blocks and 64
+// rays took 1.71 instead of 1.68 ms); the others keep eight blocks and 64
 // registers (mixed, nine blocks: 2M box 21.26 ms per four samples, eight 20.85).
 template <bool ANY, bool MULTI, int THREADS, int RING, bool MIXED = false>
 __global__ void __launch_bounds__(THREADS, ((MULTI || ANY || MIXED) ? 1024 : 1152) / THREADS) k_trace_blas(const BatchArgs a) {

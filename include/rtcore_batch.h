@@ -50,9 +50,11 @@ typedef struct rt_batch_params {
 typedef struct rt_batch_tuning {
     uint32_t trace_threads;        /* traversal block size: 128 or 256       */
     uint32_t trace_blocks_per_sm;  /* persistent traversal blocks per SM     */
-    uint32_t stack_ring;           /* shared-memory stack entries per ray:
-                                      8, 16 or 32 (deeper entries spill to
-                                      local memory)                          */
+    uint32_t stack_ring;           /* shared memory per ray, in entries: 8,
+                                      16 or 32.  The triangle queue has the
+                                      room of eight: 8 and 16 keep eight
+                                      stack entries there, 32 sixteen (deeper
+                                      ones spill to local memory)            */
     uint32_t refill;               /* a traversal warp refills when at least
                                       this many of its lanes are idle (1-32) */
     uint32_t shade_threads;        /* block size of the shading kernels:
