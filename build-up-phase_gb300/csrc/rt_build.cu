@@ -493,10 +493,13 @@ struct TreeArgs {
 
 // Exchange with release (this thread's box and cost stores are visible to
 // the thread that reads the value) and acquire (the first child's stores are
-// visible to this thread's later loads) at device scope.
+// visible to this thread's later loads), at device scope or, where all climbers
+// are of one block, the block's.
+template <bool BLOCK>
 __device__ __forceinline__ uint64_t exch_acq_rel(uint64_t *p, uint64_t v) {
     uint64_t old;
-    asm volatile("atom.acq_rel.gpu.global.exch.b64 %0, [%1], %2;" : "=l"(old) : "l"(p), "l"(v) : "memory");
+    if (BLOCK) asm volatile("atom.acq_rel.cta.global.exch.b64 %0, [%1], %2;" : "=l"(old) : "l"(p), "l"(v) : "memory");
+    else asm volatile("atom.acq_rel.gpu.global.exch.b64 %0, [%1], %2;" : "=l"(old) : "l"(p), "l"(v) : "memory");
     return old;
 }
 
@@ -555,7 +558,7 @@ __device__ __forceinline__ void complete_node(const TreeArgs &a, uint32_t p, boo
 }
 
 // Climbs through global memory until the sibling is not there yet.
-template <bool INST>
+template <bool INST, bool BLOCK>
 __device__ __forceinline__ void climb_global(const TreeArgs &a, uint32_t me) {
     const uint32_t n = a.n, mi = me & ~kLeafBit;
     Climb c;
@@ -582,7 +585,7 @@ __device__ __forceinline__ void climb_global(const TreeArgs &a, uint32_t me) {
         }
         const bool left = c.l == 0u ? true : (c.r == n - 1u ? false : boundary_delta(kr, krp, c.r) > boundary_delta(klm, kl, c.l - 1u));
         const uint32_t p = left ? c.r : c.l - 1u;
-        const uint64_t got = exch_acq_rel(a.other + p, ((uint64_t)c.me << 32) | (left ? c.l : c.r));
+        const uint64_t got = exch_acq_rel<BLOCK>(a.other + p, ((uint64_t)c.me << 32) | (left ? c.l : c.r));
         if (got == ~0ull) return;  // first child here: the sibling computes the node
         const uint32_t sib = (uint32_t)(got >> 32), far = (uint32_t)got;
         const uint32_t nl = left ? c.l : far, nr = left ? far : c.r;
@@ -730,12 +733,12 @@ __global__ void __launch_bounds__(kTreeKeys, 1536 / kTreeKeys) k_tree(TreeArgs a
 }
 
 // The subtrees k_tree left, one thread each.
-template <bool INST>
-__global__ void __launch_bounds__(128) k_tree_climb(TreeArgs a) {
+template <bool INST, bool BLOCK>
+__global__ void __launch_bounds__(BLOCK ? 1024 : 128) k_tree_climb(TreeArgs a) {
     pdl_enter();
     const uint32_t m = __ldcg(a.n_left);
     for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < m; q += gridDim.x * blockDim.x)
-        climb_global<INST>(a, __ldcg(a.left + q));
+        climb_global<INST, BLOCK>(a, __ldcg(a.left + q));
 }
 
 // ---------------------------------------------------------------------------
@@ -1614,13 +1617,19 @@ int run_build(rt_context *ctx, cudaStream_t st, const BuildCall &bc, const GeomP
     ta.n_left = root_word + 1;
     ta.err = ctx->d_err;
     const unsigned tree_blocks = (n + kTreeKeys - 1u) / kTreeKeys;
-    // about 20 subtrees are left per block of k_tree
+    // About 20 subtrees are left per block of k_tree; up to 2,000 of them climb in
+    // one block, whose exchanges need no device-wide fence (build of 12,345 /
+    // 25,000 triangles 154 / 171 -> 148 / 166 us, 40,000 179 -> 193: not there).
+    constexpr unsigned kOneBlockClimb = 100;
     unsigned climb_blocks = (tree_blocks + 3u) / 4u;
     if (climb_blocks > 8u * (unsigned)ctx->sm_count) climb_blocks = 8u * (unsigned)ctx->sm_count;
     const bool blas = bc.kind == RT_ACCEL_KIND_BLAS;
     RT_CUDA_CTX(ctx, launch_pdl(blas ? k_tree<false> : k_tree<true>, tree_blocks, kTreeKeys, 0, st, ta));
     if (tree_blocks > 1u)
-        RT_CUDA_CTX(ctx, launch_pdl(blas ? k_tree_climb<false> : k_tree_climb<true>, climb_blocks, 128, 0, st, ta));
+        RT_CUDA_CTX(ctx, tree_blocks <= kOneBlockClimb
+                             ? launch_pdl(blas ? k_tree_climb<false, true> : k_tree_climb<true, true>, 1u, 1024, 0, st, ta)
+                             : launch_pdl(blas ? k_tree_climb<false, false> : k_tree_climb<true, false>, climb_blocks, 128,
+                                          0, st, ta));
 
     CollapseArgs ca;
     ca.n = n;

@@ -45,3 +45,14 @@ def test_instance_tree_blocks_match_oracle(ctx, orc, n):
 
     compare_accels(GpuTlas(ctx, instances(gb.addr)).bytes(), orc.build_tlas(instances(ptr_of(ob)))[0], 80,
                    ignore_ref=True)
+
+
+@pytest.mark.parametrize("kind", ["soup", "equal", "line"])
+@pytest.mark.parametrize("n", [25_600, 25_601])
+def test_climb_in_one_block_or_many_matches_oracle(ctx, orc, kind, n):
+    """100 blocks of keys: the largest tree whose rest one block climbs."""
+    v, i = _triangles(kind, n)
+    g = GpuBlas(ctx, [(v, i, None)])
+    o, rc = orc.build_blas([(v, i, None)])
+    assert rc == 0
+    compare_accels(g.bytes(), o, 48)
