@@ -1880,8 +1880,9 @@ __device__ __forceinline__ RefitSlot refit_take(uint32_t &todo, uint32_t base, c
     s.cnt = s.inner ? 1u : (uint32_t)__popc(s.meta >> 5);
     s.lo = make_float4(kInf, kInf, kInf, 0.0f);
     s.hi = make_float4(-kInf, -kInf, -kInf, 0.0f);
-    if (bit && s.meta) {
-        if (s.i + s.cnt > (s.inner ? c_hi : n) || (s.inner && s.i < c_lo)) {
+    if (bit && s.meta && s.cnt) {
+        const uint32_t end = s.inner ? c_hi : n;  // (compared without a sum, which a corrupt base could wrap)
+        if (s.i >= end || s.cnt > end - s.i || (s.inner && s.i < c_lo)) {
             report_error(err, RT_ERR_BOUNDS, (s.inner ? 0x6d000000u : 0x6e000000u) | (s.k & 0xffffffu));
             s.cnt = 0u;
         } else {
