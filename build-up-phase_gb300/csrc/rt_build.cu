@@ -1983,6 +1983,7 @@ __global__ void __launch_bounds__(kRefitThreads, INST ? 1 : 2) k_refit_nodes(uin
     rt_accel_header *h = reinterpret_cast<rt_accel_header *>(accel);
     uint4 *nodes = reinterpret_cast<uint4 *>(accel + RT_ACCEL_HEADER_BYTES);
     const uint32_t nc = s_levels[depth - 1u], lane = threadIdx.x & 31u;
+    const uint32_t last_level = depth > 1u ? s_levels[depth - 2u] : 0u;  // no node from here on has children
     uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, warps = (gridDim.x * blockDim.x) >> 5;
     for (uint32_t base = 32u * warp; base < nc; base += 32u * warps) {
         const uint32_t k = base + lane;
@@ -1991,7 +1992,9 @@ __global__ void __launch_bounds__(kRefitThreads, INST ? 1 : 2) k_refit_nodes(uin
             const uint4 w0 = __ldcg(nodes + (size_t)k * 5u), w1 = __ldcg(nodes + (size_t)k * 5u + 1u);
             w = {w0.w >> 24, w1.x, w1.y, w1.z, w1.w};
         }
-        refit_append(k < nc && w.imask != 0u, k, depth, s_levels, list, leaf_box);
+        const bool inner = k < nc && w.imask != 0u;
+        if (inner && k >= last_level) report_error(err, RT_ERR_BOUNDS, 0x69000000u | (k & 0xffffffu));
+        refit_append(inner, k, depth, s_levels, list, leaf_box);
         uint32_t todo = __ballot_sync(kFullMask, w.imask == 0u);
         if (todo == 0u) continue;
         RefitSlot cur = refit_take(todo, base, w, 0u, 0u, n, leaf_box, node_box, err);

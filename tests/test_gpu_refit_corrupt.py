@@ -53,3 +53,20 @@ def test_damaged_references_are_reported(ctx, damage):
     built = g2.bytes().copy()
     g2.refit(ctx, [(v, i, None)])
     assert g2.bytes().tobytes() == built.tobytes()
+
+
+@pytest.mark.parametrize("n", [1, 3000])
+def test_children_below_the_last_level_are_reported(ctx, n):
+    import rtcore
+    import rtcore.scenes as S
+    v, i = S.soup(13, n)
+    g = GpuBlas(ctx, [(v, i, None)])
+    buf = g.bytes().copy()
+    h = header(buf)
+    lo, hi = int(h["node_offset"]), int(h["node_offset"]) + 80 * int(h["node_count"])
+    nodes = buf[lo:hi].view(NODE_DTYPE)
+    nodes["imask"][-1] |= 1  # the last node's first slot as an internal child
+    g.accel[:len(buf)].copy_(dev(buf))
+    with pytest.raises(rtcore.RtError) as e:
+        g.refit(ctx, [(v, i, None)])
+    assert e.value.code == rtcore.RT_ERR_BOUNDS
