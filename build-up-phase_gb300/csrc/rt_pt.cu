@@ -641,7 +641,8 @@ __global__ void k_bt_setup(const BtScene *bt, uint32_t n_scenes, TravScene *view
     v.prims = nullptr;
     v.node_count = 0u;
     v.prim_count = 0u;
-    v.pad[0] = v.pad[1] = 0u;
+    v.slack = 0.0f;
+    v.pad = 0u;
     const bool used = sc.width != 0u && sc.height != 0u;  // no path refers to a scene without pixels
     if (used && sc.accel) {
         const rt_accel_header *hd = reinterpret_cast<const rt_accel_header *>(sc.accel);
@@ -650,6 +651,7 @@ __global__ void k_bt_setup(const BtScene *bt, uint32_t n_scenes, TravScene *view
             v.prims = reinterpret_cast<const uint4 *>(sc.accel + hd->prim_offset);
             v.node_count = hd->prim_count ? hd->node_count : 0u;
             v.prim_count = hd->prim_count;
+            v.slack = box_slack(hd);
         } else {
             // the path tracer shades bottom-level structures only
             report_error(err, RT_ERR_UNSUPPORTED, 0x78000000u | s);

@@ -237,8 +237,8 @@ __device__ bool trace_ray(const uint8_t *accel, const float o[3], const float d[
 // walks the instance's BLAS with the object-space ray.  When that walk is over
 // it takes the world ray back from shared memory and goes on in the TLAS.
 // Closest hit = smallest t, ties broken by the smallest (instance, triangle)
-// key, whatever the order.  Launched beside k_trace_blas; each kernel returns
-// at once when the structure is not its kind.
+// key.  Launched beside k_trace_blas; each kernel returns at once when the
+// structure is not its kind.
 //
 // A lane enters an instance every few nodes, and the entry (80 bytes of
 // record, a transformed ray, its divisions) costs more than a node, so lanes
@@ -246,37 +246,19 @@ __device__ bool trace_ray(const uint8_t *accel, const float o[3], const float d[
 // quarter of the lanes with a ray (or the refill threshold) have stopped:
 // entered on the spot, the entry and the triangle tests ran with a few lanes
 // each (10.5 active threads per instruction).  807K rays in 64 instances of
-// three meshes: 1,008 -> 815 us (without the rays set aside, kNearHits: 800; then
-// a fixed 4 / 8 / 16 stopped lanes 863 / 871 / 971, a third or an eighth of the
-// lanes 811 / 821).  What bounds it now: issue slots, half of them in steps of
-// warps whose last rays (of up to hundreds of nodes) are under way.  A lane leaves an instance without
-// waiting for its queued triangles: their part of the object-space ray stays in
-// shared memory until the lane enters the next one, before which they are
-// tested.
+// three meshes: 1,008 -> 810 us (then a fixed 4 / 8 / 16 stopped lanes 863 / 871 /
+// 971, a third or an eighth of the lanes 811 / 821).  What bounds it now: issue
+// slots, half of them in steps of warps whose last rays (of up to hundreds of
+// nodes) are under way.
+//
+// The answer is that of a walk in order (see boxes_may_exceed): a lane goes on
+// in the TLAS, and enters the next instance, with every triangle it has met
+// tested, so the TLAS nodes' boxes and an instance's first meet the same far
+// limit as there, and only hits within one instance can have come too late for
+// its boxes.
 constexpr uint32_t kInstGroup = 0x40000000u;   // stack entry: instances of a TLAS node still to walk
 constexpr int kInstDepth = 128;                // stack entries per ray (both levels)
 constexpr uint32_t kInstBlocksPerSm = 6;       // 80 registers (7 blocks: 72, within 1 %)
-
-// is_flat in the instance's space or the world's: a hit's record and instance
-// record.
-__device__ __forceinline__ bool is_flat_inst(const uint4 *tprims, const uint4 &best) {
-    const InstRec ir = load_inst(tprims, best.w);
-    const uint8_t *blas = reinterpret_cast<const uint8_t *>(ir.accel_ref);
-    const rt_accel_header *bh = reinterpret_cast<const rt_accel_header *>(blas);
-    const uint4 *p = reinterpret_cast<const uint4 *>(blas + bh->prim_offset) + (size_t)(best.z & ~kMinusZero) * 3u;
-    if (is_flat(p)) return true;
-    // the world normal: the transposed world-to-object matrix times the object's
-    const float4 q0 = xyz_of(ldg4(p)), q1 = xyz_of(ldg4(p + 1)), q2 = xyz_of(ldg4(p + 2));
-    const float ax = q1.x - q0.x, ay = q1.y - q0.y, az = q1.z - q0.z;
-    const float bx = q2.x - q0.x, by = q2.y - q0.y, bz = q2.z - q0.z;
-    const float nx = ay * bz - az * by, ny = az * bx - ax * bz, nz = ax * by - ay * bx;
-    float w[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) w[a] = fabsf((ir.w2o[a] * nx + ir.w2o[4 + a] * ny) + ir.w2o[8 + a] * nz);
-    const float most = fmax3(w[0], w[1], w[2]);
-    const float rest = (w[0] + w[1]) + w[2] - most;
-    return !(rest > kFlat * most);
-}
 
 template <bool ANY>
 __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(const BatchArgs a) {
@@ -299,18 +281,16 @@ __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(
     __shared__ int32_t s_t[ANY ? 1 : kTraceThreads];
     __shared__ unsigned long long s_key[ANY ? 1 : kTraceThreads];
     __shared__ uint4 s_best[ANY ? 1 : kTraceThreads];
-    __shared__ uint32_t s_near[kTraceThreads / 32];  // lanes (bits) whose ray is to be set aside, see kNearHits
-    __shared__ uint32_t s_aside[ANY ? 1 : kTraceThreads];  // per lane: the last ray set aside
-    __shared__ uint32_t s_step[ANY ? 1 : kTraceThreads];   // the step (node visit) of the best hit so far
+    __shared__ uint32_t s_step[ANY ? 1 : kTraceThreads];  // the step (node visit) of the best hit in this instance (0: none)
+    __shared__ int32_t s_prev[ANY ? 1 : kTraceThreads];   // the nearest hit of an earlier step in it, as an ordered integer
     constexpr uint32_t kFull = 0xffffffffu;
     const int tid = threadIdx.x, lane = tid & 31;
     uint2 *queue = s_queue[tid >> 5];
     const int warp0 = tid & ~31;  // lane 0's thread
-    if (!ANY) {
-        s_aside[tid] = kNone;
-        s_near[tid >> 5] = 0u;
-    }
-    __syncwarp();
+    // (one more entry than the stack's: the last ray set aside)
+    uint2 spill[kInstDepth + 1];
+    uint32_t &aside = spill[kInstDepth].x;
+    aside = kNone;
 
     bool have_ray = false, exhausted = false, pending = false, in_blas = false, found = false;
     Ray r;  // the current level's ray
@@ -322,7 +302,6 @@ __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(
     uint32_t inst_id = 0, inst_rec = 0;
     uint2 ig = make_uint2(0u, 0u);  // instances of a TLAS node to enter: the lane is stopped
     int sp = 0, lo = 0, sp_blas = 0;
-    uint2 spill[kInstDepth];
     uint32_t head = 0, tail = 0;  // queue positions tested / appended so far (the same in every lane)
     uint32_t last = ~0u;          // position of this lane's latest entry
     uint32_t step = 0u;           // node visits of the warp so far
@@ -394,7 +373,10 @@ __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(
         const bool waiting = (int)(last - head) >= 0;
         const uint32_t ready =
             __ballot_sync(kFull, !pending && !waiting && (have_ray || (!exhausted && ((lanes >> lane) & 1u))));
-        uint32_t walking = __ballot_sync(kFull, pending);
+        // (the far limit a TLAS node's boxes meet is that of every triangle met
+        // before, so that what a walk in order tests there is the same)
+        bool can_step = pending && (ANY || in_blas || !waiting);
+        uint32_t walking = __ballot_sync(kFull, can_step);
         // stopped lanes to wait for: they stand idle until served
         const int serve = max(1 + __popc(__ballot_sync(kFull, have_ray)) / 4, exhausted ? 0 : refill);
         if (__popc(ready) >= serve || (walking == 0u && tail == head)) {
@@ -414,12 +396,11 @@ __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(
                     const uint4 best = s_best[tid];
                     const unsigned long long key = s_key[tid];
                     const bool hit = key != ~0ull;
-                    if (hit && ((s_near[tid >> 5] >> lane) & 1u)) {
-                        atomicAnd(&s_near[tid >> 5], ~(1u << lane));
+                    if (hit && (best.z & kLate)) {
                         uint32_t *place = result_place(ray_idx);
                         if (place) {
-                            *place = s_aside[tid];
-                            s_aside[tid] = ray_idx;
+                            *place = aside;
+                            aside = ray_idx;
                         }
                     } else {
                         const uint32_t rec = best.z & ~kMinusZero;
@@ -440,7 +421,7 @@ __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(
                     }
                 }
             }
-            float o[3], d[3];
+            float o[3], d[3], slack = 0.0f;
             bool fresh = false, entered = false;
             const uint32_t want = __ballot_sync(kFull, mine && !have_ray) & lanes;
             if (want != 0u && !exhausted) {
@@ -514,6 +495,10 @@ __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(
                     count = bh->node_count;
                     inst_id = ir.id;
                     inst_rec = rec;
+                    if (!ANY) {
+                        s_step[tid] = 0u;
+                        slack = box_slack(bh);
+                    }
                     pending = true;
                     entered = true;
                 }
@@ -527,13 +512,15 @@ __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(
                     s_world[1][tid].z = r.invd[2];
                 } else {
                     s_object[0][tid] = make_float4(o[0], o[1], o[2], tmin);
-                    s_object[1][tid] = make_float4(r.sx, r.sy, r.sz, __uint_as_float(r.kxyz));
+                    s_object[1][tid] =
+                        make_float4(r.sx, r.sy, r.sz, __uint_as_float(ANY ? r.kxyz : pack_slack(r, o, slack)));
                 }
             }
-            walking = __ballot_sync(kFull, pending);
+            can_step = pending && (ANY || in_blas || !((int)(last - head) >= 0));
+            walking = __ballot_sync(kFull, can_step);
             if (walking == 0u) continue;
         }
-        const uint32_t held = __ballot_sync(kFull, !pending && (int)(last - head) >= 0);
+        const uint32_t held = __ballot_sync(kFull, !can_step && (int)(last - head) >= 0);
         const int busy = __popc(walking | held);  // lanes whose triangles may be queued
         // a partial batch once stopped lanes wait for it
         const bool drain = walking == 0u || __popc(held) + __popc(ready & ~walking) >= serve;
@@ -541,9 +528,11 @@ __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(
         // ---- one node per lane, then the lane's next node (see k_trace_blas)
         ++step;
         uint32_t leaves = 0u, nth = 0u, meta_lo = 0u, meta_hi = 0u, pbase = 0u;
-        if (pending && (visits >= count || node >= count))
+        if (can_step && (visits >= count || node >= count)) {
+            can_step = false;
             fail((in_blas ? 0x74000000u : 0x75000000u) | (node & 0xffffffu));
-        if (pending) {
+        }
+        if (can_step) {
             ++visits;
             const NodeWords nd = load_node(nodes, node);
             const uint32_t hits = isect_node(r, nd, tmin, tbest);
@@ -641,29 +630,31 @@ __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(
                     const unsigned long long key = (unsigned long long)inst << 32 | tri;
                     int32_t *bt = s_t + warp0 + src;
                     unsigned long long *bk = s_key + warp0 + src;
-                    const bool any_hit = hit;
+                    const uint32_t own = e.y >> 5;
+                    const bool hit_too = hit;
                     if (hit && atomicMin(bt, tk) > tk) *bk = ~0ull;
                     __syncwarp();
                     hit = hit && *bt == tk;
                     if (hit) atomicMin(bk, key);
                     __syncwarp();
                     hit = hit && *bk == key;
-                    uint32_t other = 0u;  // the other hit's step
                     if (hit) {
-                        other = s_step[warp0 + src];
-                        s_step[warp0 + src] = e.y >> 5;
+                        const uint32_t before = s_step[warp0 + src];
+                        s_step[warp0 + src] = own;
+                        if (before != own) s_prev[warp0 + src] = before ? ford(t_hi + 0.0f) : kNoLimit;
                         s_best[warp0 + src] =
                             make_uint4(__float_as_uint(u), __float_as_uint(v),
                                        rec | (__float_as_uint(t) == kMinusZero ? kMinusZero : 0u), irec);
                     }
                     __syncwarp();
-                    if (any_hit) {
-                        // see k_trace_blas; the best hit may be an earlier instance's
-                        const float tb = ford_inv(*bt);
-                        if (fabsf((hit ? t_hi : t) - tb) <= kNearHits * fabsf(tb) &&
-                            s_step[warp0 + src] != (hit ? other : e.y >> 5) && is_flat_inst(tprims, s_best[warp0 + src]))
-                            atomicOr(&s_near[tid >> 5], 1u << src);
+                    if (hit_too && !hit && own < s_step[warp0 + src]) atomicMin(s_prev + warp0 + src, tk);
+                    __syncwarp();
+                    if (hit) {  // see boxes_may_exceed
+                        const int32_t prev = s_prev[warp0 + src];
+                        if (prev != kNoLimit && boxes_may_exceed(tr, pr + (size_t)rec * 3u, ford_inv(prev)))
+                            s_best[warp0 + src].z |= kLate;
                     }
+                    __syncwarp();
                     tbest = ford_inv(s_t[tid]);
                 }
             }
@@ -673,7 +664,7 @@ __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(
 
     // ---- the rays set aside
     if (!ANY) {
-        for (uint32_t i = s_aside[tid]; i != kNone;) {
+        for (uint32_t i = aside; i != kNone;) {
             const uint32_t next = *result_place(i);
             const float4 r0 = __ldg(a.rays + 2u * i), r1 = __ldg(a.rays + 2u * i + 1u);
             const float o[3] = {r0.x, r0.y, r0.z}, d[3] = {r1.x, r1.y, r1.z};

@@ -15,9 +15,9 @@
 // Visiting order: internal children in ascending (slot ^ ray octant), the
 // remaining siblings pushed as one group; the leaf records met on the way are
 // tested in batches (see the triangle queue below).  Closest hit = smallest t,
-// ties broken by the smallest triangle index, so the result does not depend
-// on when a record is tested and equals the CPU restatement's, which tests a
-// node's records as it visits the node.
+// ties broken by the smallest triangle index, among the triangles that a walk
+// testing each node's records as it visits the node would test: the CPU
+// restatement's hit, bit for bit, whatever is tested together.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -39,6 +39,8 @@ constexpr uint32_t kAnyBlocksPerSm = 1024u / kTraceThreads;  // resident blocks 
 constexpr int kMaxDepth = 64;       // total stack entries per ray
 constexpr uint32_t kNone = 0xffffffffu;
 constexpr uint32_t kMinusZero = 0x80000000u;  // the bits of -0; in a record index (below 2^30) the mark of a hit at t = -0
+constexpr uint32_t kLate = 0x40000000u;       // in a record index: a hit in whose place an in-order walk may find another
+constexpr int32_t kNoLimit = 0x7fffffff;      // as an ordered integer: beyond every distance
 
 struct Hit {
     float t, u, v;
@@ -58,7 +60,8 @@ struct TravScene {
     const uint4 *prims;
     uint32_t node_count;
     uint32_t prim_count;
-    uint32_t pad[2];
+    float slack;  // box_slack of the structure
+    uint32_t pad;
 };
 static_assert(sizeof(TravScene) == 32, "TravScene is read as two 16-byte words");
 
@@ -94,36 +97,37 @@ struct BatchArgs {
 // queue in shared memory (record index and lane) and walks on; once there are
 // as many entries as lanes with a ray, the whole warp tests them, one entry per
 // lane with the owner's ray read by shuffles, and hands the hits back to their
-// owners.  The closest hit of a ray is the least (t, triangle) of the triangles
-// tested, whatever their order; a ray walks a few nodes more because its far
-// limit shrinks a few visits later.  A lane keeps its ray until its last entry
+// owners.  A ray walks a few nodes more because its far limit shrinks a few
+// visits later.  A lane keeps its ray until its last entry
 // has been tested.  1M soup, 4.15M primary and incoherent rays: 28.6 entries
 // per batch, 18.4 nodes and 4.4 triangles per ray against 17.7 and 4.0 when
 // every triangle is tested on the spot, 28.1 of 32 lanes walking per node step
 // (2M box, mixed launches: 27.4).  With the box test's instruction count, the
 // 64-bit queue entry and the hits' shared-memory minima this took the launch from
-// 1.92 to 1.56 ms, the path tracer's 2M-triangle frame of four samples from 25.7
-// to 20.9.  What bounds it now: issue slots (79 % busy) and the L1 data path
+// 1.92 to 1.58 ms, the path tracer's 2M-triangle frame of four samples from 25.7
+// to 20.6.  What bounds it now: issue slots (79 % busy) and the L1 data path
 // (78 %: a node is five 16-byte loads per lane, nearly every one a wavefront of
 // its own).
 //
 // In the order of the CPU restatement a record is tested, and the far limit
-// shrunk, before the next node's boxes.  A walk that goes on meanwhile can only
-// end differently if it accepts a triangle whose boxes an earlier hit, no nearer
-// than the triangle, would have cut off: rounding, seen where the two hits are
-// coincident or nearly so and the triangle lies in an axis plane, so that its
-// boxes have no thickness to spare.  A ray whose best hit is such a triangle,
-// with another node's hit within kNearHits of its distance, is set aside -- its result's
-// place links the lane's rays of that kind -- and walked in order once the lane
-// is done with the others.  (12 coincident copies of 60 axis-parallel triangles,
-// 1M rays: 0 to 3 rays differed from the restatement.  The check is within 1 %
-// of the soup's and the 2M box's time; walking such a ray again within the loop
-// cost the soup's rays 13 %, in a function called on the spot 40 %: registers on
-// every path.  A box whose every triangle is there twice, 1M rays: 298 us, 210
-// with them once, 690 with hits of one node taken for two and a loop per ray;
-// 342 when every record is tested on the spot.)
-constexpr float kNearHits = 0x1p-12f;
-constexpr float kFlat = 0x1p-8f;  // extent along an axis over the largest extent
+// shrunk, before the next node's boxes.  A walk that goes on meanwhile visits
+// more, and can only end differently by a triangle X that it tests and the other
+// walk does not: one of the boxes above X lets the ray in beyond an earlier
+// hit's distance, rounding included, while X's own distance is no greater -- X
+// lies on the face of its box where the ray enters, or the ray starts there.
+// boxes_may_exceed bounds from X's vertices where those boxes let the ray in.  A
+// ray whose best hit has that bound beyond the nearest earlier hit of another
+// node (records of one node are tested together in either walk) is set aside --
+// its result's place links the lane's rays of that kind -- and walked in order
+// once the lane is done with the others.  For any other ray the hit is the other
+// walk's: its far limits are hits no nearer than X, so every box above X lets
+// the ray in there too, X is tested, and nothing it tests is better.
+// (12 coincident copies of 60 axis-parallel triangles, 1M rays: 0 to 3 rays
+// differ without this, 2 to 4 of rays that start on the triangles with a window
+// of 2^-12 of t in the place of the bound.  It costs the soup's rays 2 %, 1.55 ->
+// 1.58 ms, the 2M box's frame 0.5 %; in the 56-register kernel 8 % with the ray
+// held through the merge instead of read again.)
+constexpr float kBoxSlack = 0x1p-20f;
 constexpr uint32_t kTriQueue = 64;  // entries per warp: below 32 before an append of at most 32
 constexpr int kTriDrain = 8;   // lanes waiting for their entries alone before a partial batch is tested
 
@@ -131,13 +135,47 @@ __device__ __forceinline__ float4 xyz_of(const uint4 &q) {
     return make_float4(__uint_as_float(q.x), __uint_as_float(q.y), __uint_as_float(q.z), 0.f);
 }
 
-// Whether a leaf record's triangle is all but parallel to an axis plane.
-__device__ __forceinline__ bool is_flat(const uint4 *p) {
-    const float4 q0 = xyz_of(ldg4(p)), q1 = xyz_of(ldg4(p + 1)), q2 = xyz_of(ldg4(p + 2));
-    const float ex = fmax3(q0.x, q1.x, q2.x) - fmin3(q0.x, q1.x, q2.x);
-    const float ey = fmax3(q0.y, q1.y, q2.y) - fmin3(q0.y, q1.y, q2.y);
-    const float ez = fmax3(q0.z, q1.z, q2.z) - fmin3(q0.z, q1.z, q2.z);
-    return fmin3(ex, ey, ez) <= kFlat * fmax3(ex, ey, ez);
+// kBoxSlack times the greatest coordinate of a structure's bounds; infinite where
+// a node's quantisation steps (at most 2^RT_QEXP_MAX) may not reach its bounds.
+__device__ __forceinline__ float box_slack(const rt_accel_header *h) {
+    const float4 lo = *reinterpret_cast<const float4 *>(h->bounds_lo), hi = *reinterpret_cast<const float4 *>(h->bounds_hi);
+    const float m = fmaxf(fmax3(fabsf(lo.x), fabsf(lo.y), fabsf(lo.z)), fmax3(fabsf(hi.x), fabsf(hi.y), fabsf(hi.z)));
+    return m < 0x1p100f ? kBoxSlack * m : kInf;
+}
+
+// A ray's slack and axis order in one word (the slack rounded up, a multiple of 64).
+__device__ __forceinline__ uint32_t pack_slack(const Ray &r, const float o[3], float scene_slack) {
+    const float slack = __fmaf_rn(fmax3(fabsf(o[0]), fabsf(o[1]), fabsf(o[2])), kBoxSlack, scene_slack);
+    return ((__float_as_uint(slack) & ~63u) + 64u) | r.kxyz;
+}
+
+// Whether a box around the triangle of leaf record p, in a node anywhere above
+// it, could let the ray in beyond `limit` (a hit's distance); r: origin, shear
+// and pack_slack's word.
+//
+// Along axis a such a box's near plane lies no further along the ray than the
+// triangle's nearest vertex, and isect_node's distance to it is off by less than
+// 6 * 2^-24 D |1 / d_a|, D the greatest distance along an axis between the
+// origin and anything in the scene: two roundings of (frame origin - ray origin)
+// / d_a, one of the fma, the step exact.  Compared are (nearest vertex - origin
+// + slack) / d_z and limit d_a / d_z, d_z the shear's axis, whose own roundings
+// stay below 5 * 2^-24 D; the slack is 16 * 2^-24 D.  Products too small to carry
+// that accuracy, and limits next to zero, count as exceeded.
+__device__ __forceinline__ bool boxes_may_exceed(const Ray &r, const uint4 *p, float limit) {
+    const float slack = __uint_as_float(r.kxyz & ~63u);
+    const uint32_t kx = r.kxyz & 3u, kz = (r.kxyz >> 4) & 3u;
+    bool exceeds = !(limit >= 0x1p-40f);
+#pragma unroll
+    for (uint32_t a = 0; a < 3u; ++a) {
+        const float s = a == kz ? 1.0f : (a == kx ? r.sx : r.sy);
+        const bool neg = ((__float_as_uint(s) ^ __float_as_uint(r.sz)) >> 31) != 0u;
+        const float *v = reinterpret_cast<const float *>(p) + a;
+        const float v0 = __ldg(v), v1 = __ldg(v + 4), v2 = __ldg(v + 8);
+        const float ahead = (neg ? r.o[a] - fmax3(v0, v1, v2) : fmin3(v0, v1, v2) - r.o[a]) + slack;
+        const bool within = fabsf(s) >= 0x1p-60f && ahead * fabsf(r.sz) < limit * fabsf(s);
+        exceeds = exceeds || !(ahead <= 0.0f || within);
+    }
+    return exceeds;
 }
 
 // MIXED: one launch over two queues -- the closest-hit rays (rays, n_dev;
@@ -156,14 +194,13 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY || MIXED) ? 1024 : 115
     __shared__ uint2 s_queue[THREADS / 32][kTriQueue];  // leaf record, lane | visits << 5
     // per lane: the triangle test's part of the ray (written once per ray, read
     // by whichever lane tests); the best hit so far -- t as an ordered integer;
-    // u, v, leaf record and triangle (kNone: no hit) --; the ray's index
+    // u, v, leaf record and triangle (kNone: no hit)
     __shared__ float4 s_shear[THREADS];
     __shared__ int32_t s_t[ANY ? 1 : THREADS];
     __shared__ uint4 s_best[ANY ? 1 : THREADS];
-    __shared__ uint32_t s_ray[THREADS];
-    __shared__ uint32_t s_near[THREADS / 32];  // lanes (bits) whose ray is to be set aside, see kNearHits
-    __shared__ uint32_t s_aside[ANY ? 1 : THREADS];  // per lane: the last ray set aside
-    __shared__ uint32_t s_visit[ANY ? 1 : THREADS];  // the node visit of the best hit so far
+    __shared__ uint32_t s_visit[ANY ? 1 : THREADS];  // the node visit of the best hit so far (0: no hit)
+    __shared__ int32_t s_prev[ANY ? 1 : THREADS];    // the nearest hit of an earlier visit, as an ordered integer
+    __shared__ float s_slack[THREADS / 32];          // box_slack of the structure
     const uint4 *nodes = nullptr, *prims = nullptr;
     // A tree walk visits each node at most once: more visits, or a node index
     // past the end, can only come from a corrupt structure.
@@ -179,14 +216,17 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY || MIXED) ? 1024 : 115
         max_visits = hd->node_count;
     }
     constexpr uint32_t kFull = 0xffffffffu;
+    constexpr bool kFewRegisters = !MULTI && !ANY && !MIXED;
     const int tid = threadIdx.x, lane = tid & 31;
     uint2 *queue = s_queue[tid >> 5];
     const int warp0 = tid & ~31;  // lane 0's thread
 
-    if (!ANY) {
-        s_aside[tid] = kNone;
-        s_near[tid >> 5] = 0u;
-    }
+    // (one more entry than the stack's: the last ray set aside, this lane's ray)
+    uint2 spill[kMaxDepth + 1];
+    uint32_t &aside = spill[kMaxDepth].x, &ray_index = spill[kMaxDepth].y;
+    aside = kNone;
+    if (!ANY && !MULTI && lane == 0)
+        s_slack[tid >> 5] = empty ? 0.0f : box_slack(reinterpret_cast<const rt_accel_header *>(a.accel));
     __syncwarp();
 
     bool have_ray = false, exhausted = false, pending = false;
@@ -197,7 +237,6 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY || MIXED) ? 1024 : 115
     bool found = false;
     uint32_t node = 0;
     int sp = 0, lo = 0;
-    uint2 spill[kMaxDepth];
     uint32_t visits = 0;
     uint32_t head = 0, tail = 0;  // queue positions tested / appended so far (the same in every lane)
     uint32_t last = ~0u;          // position of this lane's latest entry
@@ -232,13 +271,14 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY || MIXED) ? 1024 : 115
             a.hits_ext[ray_idx] = x;
         }
     };
-    auto scene_of = [&](uint32_t s) {
+    auto scene_of = [&](uint32_t s) {  // returns the structure's slack
         const uint4 *tv = reinterpret_cast<const uint4 *>(a.scenes + s);
         const uint4 t0 = ldg4(tv), t1 = ldg4(tv + 1);
         nodes = reinterpret_cast<const uint4 *>(((uint64_t)t0.y << 32) | t0.x);
         prims = reinterpret_cast<const uint4 *>(((uint64_t)t0.w << 32) | t0.z);
         max_visits = t1.x;
         empty = t1.x == 0u || t1.y == 0u;
+        return __uint_as_float(t1.z);
     };
 
     for (;;) {
@@ -248,9 +288,7 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY || MIXED) ? 1024 : 115
         if (done == kFull || (!exhausted && __popc(done & lanes) >= refill)) {
             if (have_ray && !pending && !waiting) {
                 have_ray = false;
-                const uint32_t ray_idx = s_ray[tid];
-                const bool set_aside = !ANY && ((s_near[tid >> 5] >> lane) & 1u);
-                if (set_aside) atomicAnd(&s_near[tid >> 5], ~(1u << lane));
+                const uint32_t ray_idx = ray_index;
                 if (error) {
                     report_error(a.err, RT_ERR_BOUNDS, error | ray_idx);
                     error = 0u;
@@ -259,11 +297,11 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY || MIXED) ? 1024 : 115
                     if (a.occluded) a.occluded[ray_idx] = found ? 1u : 0u;
                 } else {
                     const uint4 best = s_best[tid];
-                    if (set_aside && best.w != kNone) {
+                    if (best.w != kNone && (best.z & kLate)) {
                         uint32_t *place = result_place(ray_idx);
                         if (place) {
-                            *place = s_aside[tid];
-                            s_aside[tid] = ray_idx;
+                            *place = aside;
+                            aside = ray_idx;
                         }
                     } else {
                         write_hit(ray_idx, best.w != kNone, (best.z & kMinusZero) ? -0.0f : tbest,
@@ -290,10 +328,11 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY || MIXED) ? 1024 : 115
                         scene_src = a.ray_scene2;
                     }
                 }
+                float scene_slack = ANY || MULTI ? 0.0f : s_slack[tid >> 5];
                 if (MULTI) {
                     const uint32_t s = __ldg(scene_src + idx);
                     if (s < a.n_scenes) {
-                        scene_of(s);
+                        scene_slack = scene_of(s);
                     } else {
                         report_error(a.err, RT_ERR_BOUNDS, 0x77000000u | (s & 0xffffffu));
                         empty = true;
@@ -305,11 +344,12 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY || MIXED) ? 1024 : 115
                 tmin = r0.w;
                 tbest = r1.w;
                 found = false;
-                s_ray[tid] = idx;
-                s_shear[tid] = make_float4(r.sx, r.sy, r.sz, __uint_as_float(r.kxyz));
+                ray_index = idx;
+                s_shear[tid] = make_float4(r.sx, r.sy, r.sz, __uint_as_float(ANY ? r.kxyz : pack_slack(r, o, scene_slack)));
                 if (!ANY) {
                     s_t[tid] = ford(tbest + 0.0f);  // -0 and +0 tie
                     s_best[tid].w = kNone;
+                    s_visit[tid] = 0u;
                 }
                 have_ray = true;
                 node = 0;          // start at the root
@@ -435,31 +475,44 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY || MIXED) ? 1024 : 115
                     const int32_t key = ford(t + 0.0f);  // -0 and +0 tie
                     int32_t *bt = s_t + warp0 + src;
                     uint4 *best = s_best + warp0 + src;
-                    const bool any_hit = hit;
+                    const uint32_t visit = e.y >> 5;
+                    const bool hit_too = hit;
                     if (hit && atomicMin(bt, key) > key) best->w = kNone;
                     __syncwarp();
                     hit = hit && *bt == key;
                     if (hit) atomicMin(&best->w, tri);
                     __syncwarp();
                     hit = hit && best->w == tri;
-                    uint32_t other = 0u;  // the other hit's visit
                     if (hit) {
-                        other = s_visit[warp0 + src];
-                        s_visit[warp0 + src] = e.y >> 5;
+                        const uint32_t before = s_visit[warp0 + src];
+                        s_visit[warp0 + src] = visit;
+                        if (before != visit) s_prev[warp0 + src] = before ? ford(t_hi + 0.0f) : kNoLimit;
                         best->x = __float_as_uint(u);
                         best->y = __float_as_uint(v);
                         best->z = rec | (__float_as_uint(t) == kMinusZero ? kMinusZero : 0u);
                     }
                     __syncwarp();
-                    if (any_hit) {
-                        // this hit against the best one, the best against the
-                        // one before; records of one node are tested together
-                        const float tb = ford_inv(*bt);
-                        if (fabsf((hit ? t_hi : t) - tb) <= kNearHits * fabsf(tb) &&
-                            s_visit[warp0 + src] != (hit ? other : e.y >> 5) &&
-                            is_flat(pr + (size_t)(best->z & ~kMinusZero) * 3u))
-                            atomicOr(&s_near[tid >> 5], 1u << src);
+                    if (hit_too && !hit && visit < s_visit[warp0 + src]) atomicMin(s_prev + warp0 + src, key);
+                    __syncwarp();
+                    const int32_t prev = hit ? s_prev[warp0 + src] : kNoLimit;
+                    if (kFewRegisters) {  // the ray read again, not held through the above
+                        if (__any_sync(kFull, prev != kNoLimit)) {
+                            Ray again;
+                            again.o[0] = __shfl_sync(kFull, r.o[0], src);
+                            again.o[1] = __shfl_sync(kFull, r.o[1], src);
+                            again.o[2] = __shfl_sync(kFull, r.o[2], src);
+                            const float4 sh = s_shear[warp0 + src];
+                            again.sx = sh.x;
+                            again.sy = sh.y;
+                            again.sz = sh.z;
+                            again.kxyz = __float_as_uint(sh.w);
+                            if (prev != kNoLimit && boxes_may_exceed(again, pr + (size_t)rec * 3u, ford_inv(prev)))
+                                best->z |= kLate;
+                        }
+                    } else if (prev != kNoLimit && boxes_may_exceed(tr, pr + (size_t)rec * 3u, ford_inv(prev))) {
+                        best->z |= kLate;
                     }
+                    __syncwarp();
                     if (MIXED && any_ray) {
                         found = s_best[tid].w != kNone;
                         if (found) {
@@ -479,7 +532,7 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY || MIXED) ? 1024 : 115
     // ---- the rays set aside, each lane its own, every record tested as its
     // node is visited (one loop over rays and nodes: the lanes' walks differ)
     if (!ANY) {
-        uint32_t idx = kNone, next = s_aside[tid], at = 0u, seen = 0u;
+        uint32_t idx = kNone, next = aside, at = 0u, seen = 0u;
         int depth = 0;
         bool walking = false;
         Hit h;
@@ -487,7 +540,7 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY || MIXED) ? 1024 : 115
         Ray w;
         w.prio = 0u;
         float t_lo = 0.f;
-        uint2 stack[kMaxDepth];
+        uint2(&stack)[kMaxDepth + 1] = spill;
         for (;;) {
             if (!walking) {
                 if (idx != kNone) write_hit(idx, h.tri != kNone, h.t, h.u, h.v, h.rec, h.tri);
