@@ -954,9 +954,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_cache_query_tc(const CacheSta
     for (int e = tid; e < 336; e += kTcThreads) {
         const int l = e < 320 ? e / 64 : 5, o = e < 320 ? e % 64 : e - 320;
         const float b = o < out_dim(l) ? S->params[b_off(l) + o] : 0.0f;
-        // hi + mid + lo == b: 8 significant bits each of its 24
-        const float hi = __bfloat162float(__float2bfloat16(b)), r1 = b - hi;
-        const float mid = __bfloat162float(__float2bfloat16(r1)), r2 = r1 - mid;
+        // hi + mid + lo == b: 8 significant bits each of its 24 (rounded to zero
+        // where hi would round to infinity); of an infinity or NaN hi alone
+        const bool finite = fabsf(b) < kInf;
+        float hi = __bfloat162float(__float2bfloat16(b));
+        const bool high = finite && !(fabsf(hi) < kInf);
+        if (high) hi = __bfloat162float(__float2bfloat16_rz(b));
+        const float r1 = finite ? b - hi : 0.0f;
+        const float mid = __bfloat162float(high ? __float2bfloat16_rz(r1) : __float2bfloat16(r1)), r2 = r1 - mid;
         uint8_t *dst = smem + tc_bias_off(l) + tc_off(o, 0, 16);
         *reinterpret_cast<uint4 *>(dst) = make_uint4(pack_bf16(hi, mid), pack_bf16(r2, 0.0f), 0u, 0u);
         *reinterpret_cast<uint4 *>(dst + 128) = make_uint4(0u, 0u, 0u, 0u);
