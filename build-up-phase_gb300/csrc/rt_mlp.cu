@@ -955,20 +955,27 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_cache_query_tc(const CacheSta
         const int l = e < 320 ? e / 64 : 5, o = e < 320 ? e % 64 : e - 320;
         const float b = o < out_dim(l) ? S->params[b_off(l) + o] : 0.0f;
         // hi + mid + lo == b: 8 significant bits each of its 24 (rounded to zero
-        // where hi would round to infinity); of an infinity or NaN hi alone
-        const bool finite = fabsf(b) < kInf;
-        float hi = __bfloat162float(__float2bfloat16(b));
+        // where hi would round to infinity); of an infinity or NaN hi alone.  A
+        // small bias goes in times 2^64, against the 2^-64 in columns 3-5 of the
+        // ones: its lower parts would be below BF16's range.
+        const bool finite = fabsf(b) < kInf, small = fabsf(b) < 0x1p-60f;
+        const float v = small ? b * 0x1p64f : b;
+        float hi = __bfloat162float(__float2bfloat16(v));
         const bool high = finite && !(fabsf(hi) < kInf);
-        if (high) hi = __bfloat162float(__float2bfloat16_rz(b));
-        const float r1 = finite ? b - hi : 0.0f;
+        if (high) hi = __bfloat162float(__float2bfloat16_rz(v));
+        const float r1 = finite ? v - hi : 0.0f;
         const float mid = __bfloat162float(high ? __float2bfloat16_rz(r1) : __float2bfloat16(r1)), r2 = r1 - mid;
         uint8_t *dst = smem + tc_bias_off(l) + tc_off(o, 0, 16);
-        *reinterpret_cast<uint4 *>(dst) = make_uint4(pack_bf16(hi, mid), pack_bf16(r2, 0.0f), 0u, 0u);
+        *reinterpret_cast<uint4 *>(dst) = small ? make_uint4(0u, pack_bf16(0.0f, hi), pack_bf16(mid, r2), 0u)
+                                                : make_uint4(pack_bf16(hi, mid), pack_bf16(r2, 0.0f), 0u, 0u);
         *reinterpret_cast<uint4 *>(dst + 128) = make_uint4(0u, 0u, 0u, 0u);
     }
-    for (int e = tid; e < kTcRows * 2; e += kTcThreads)
+    for (int e = tid; e < kTcRows * 2; e += kTcThreads) {
+        constexpr uint32_t one = 0x3f80u, tiny = 0x1f80u;  // 1 and 2^-64; 8 rows' first eight columns, then the others
+        const bool first = ((e >> 3) & 1) == 0;
         *reinterpret_cast<uint4 *>(smem + kTcOnes + 16 * e) =
-            make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
+            first ? make_uint4(one | one << 16, one | tiny << 16, tiny | tiny << 16, 0u) : make_uint4(0u, 0u, 0u, 0u);
+    }
     if (tid < kTcGroups) s_gfail[tid] = 0;
     if (tid == 0) {
         for (int g = 0; g < kTcGroups; ++g)

@@ -1,6 +1,6 @@
 """Biases at the ends of FP32's range in cache inference, whose kernel adds a
-bias as three BF16 parts: infinities, values that BF16 rounds to infinity, and
-the largest finite ones, at the outputs and in a hidden layer."""
+bias as three BF16 parts: infinities, values that BF16 rounds to infinity, the
+largest finite ones and the smallest, at the outputs and in a hidden layer."""
 from __future__ import annotations
 
 import numpy as np
@@ -46,3 +46,19 @@ def test_hidden_unit_switched_off_by_its_bias(ctx, cache):  # noqa: F811
     yo = mlp.forward(params, x, (-1, -1, -1), (1, 1, 1))[:, :3]
     assert np.isfinite(y).all()
     assert np.abs(y - yo).max() < FWD_TOL * np.abs(yo).max()
+
+
+@pytest.mark.parametrize("exponent", [-149, -140, -127, -125, -110, -66, -62, -60, -58, -20, 0, 100])
+def test_bias_alone_is_the_output(ctx, cache, exponent):  # noqa: F811
+    """Output weights of 0: the outputs are the biases, to the last bit."""
+    from oracle import mlp
+    x = random_inputs(130, 5)
+    params = get_params(ctx, cache)
+    wo, bo = mlp.W_OFF[5]
+    params[wo:bo] = 0
+    rng = np.random.default_rng(exponent + 200)
+    for _ in range(8):
+        b = (rng.uniform(1, 2, 3) * 2.0 ** exponent * rng.choice([-1, 1], 3)).astype(np.float32)
+        params[bo:bo + 3] = b
+        y = _query(ctx, cache, params, x)
+        assert (y == b).all(), (b, y[0])
