@@ -574,8 +574,8 @@ __device__ __forceinline__ void climb_global(const TreeArgs &a, uint32_t me) {
         c.box = load_box(a.node_box, mi);
         c.cost = __ldcg(a.node_cost + mi);
     }
-    uint64_t kl = __ldg(a.keys + c.l), kr = __ldg(a.keys + c.r);
-    uint64_t klm = c.l > 0u ? __ldg(a.keys + c.l - 1u) : 0ull, krp = c.r + 1u < n ? __ldg(a.keys + c.r + 1u) : 0ull;
+    uint64_t kl = __ldcg(a.keys + c.l), kr = __ldcg(a.keys + c.r);
+    uint64_t klm = c.l > 0u ? __ldcg(a.keys + c.l - 1u) : 0ull, krp = c.r + 1u < n ? __ldcg(a.keys + c.r + 1u) : 0ull;
     // A radix tree over 2^30 keys is at most 96 levels deep (63 key bits +
     // 32 index bits); the cap only guards against inconsistent keys.
     for (int climb = 0;; ++climb) {
@@ -595,9 +595,9 @@ __device__ __forceinline__ void climb_global(const TreeArgs &a, uint32_t me) {
         }
         // the sibling's box and cost and the keys around the node's range,
         // in one round of loads
-        const uint64_t k_nl = left ? kl : __ldg(a.keys + nl), k_nr = left ? __ldg(a.keys + nr) : kr;
-        const uint64_t k_nlm = nl > 0u ? __ldg(a.keys + nl - 1u) : 0ull;
-        const uint64_t k_nrp = nr + 1u < n ? __ldg(a.keys + nr + 1u) : 0ull;
+        const uint64_t k_nl = left ? kl : __ldcg(a.keys + nl), k_nr = left ? __ldcg(a.keys + nr) : kr;
+        const uint64_t k_nlm = nl > 0u ? __ldcg(a.keys + nl - 1u) : 0ull;
+        const uint64_t k_nrp = nr + 1u < n ? __ldcg(a.keys + nr + 1u) : 0ull;
         const bool sl = (sib & kLeafBit) != 0u;
         const Box sb = sl ? load_box(a.leaf_box, sib & ~kLeafBit) : load_box(a.node_box, sib);
         const float scost = sl ? RT_SAH_PRIM : __ldcg(a.node_cost + sib);

@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(kSortThreads) k_onesweep(const uint64_t *__res
     pdl_launch();
     if (t == 0) s_tile = atomicAdd(tile_counter, 1u);
     for (int i = t; i < kSortWarps * kRadix; i += kSortThreads) s_whist[i] = 0u;
-    const uint32_t gex = block_scan256(t < kRadix ? hist[t] : 0u, s_warp, nullptr);
+    const uint32_t gex = block_scan256(t < kRadix ? __ldcg(hist + t) : 0u, s_warp, nullptr);
     const uint32_t tile = s_tile;
     const uint32_t base = tile * (uint32_t)kTile;
     if (shift > 0) pdl_wait();
