@@ -526,9 +526,10 @@ extern "C" rt_status rt_batch_autotune(rt_context *ctx, const rt_batch_scene *sc
         }
         return RT_OK;
     };
-    // each list holds the values other than the default
+    // each list holds the values other than the default (a ring of 8 is the kernel
+    // of 16, see rt_trace_multi.cu)
     const uint32_t refills[] = {2u, 8u, 16u};
-    const uint32_t rings[] = {8u, 32u};
+    const uint32_t rings[] = {32u};
     const uint32_t shades[] = {128u, 512u};
     for (uint32_t v : refills)
         if (v != cur.refill) {
