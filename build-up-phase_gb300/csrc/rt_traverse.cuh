@@ -201,6 +201,9 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY || MIXED) ? 1024 : 115
     __shared__ uint32_t s_visit[ANY ? 1 : THREADS];  // the node visit of the best hit so far (0: no hit)
     __shared__ int32_t s_prev[ANY ? 1 : THREADS];    // the nearest hit of an earlier visit, as an ordered integer
     __shared__ float s_slack[THREADS / 32];          // box_slack of the structure
+    static_assert(sizeof(s_stack) + sizeof(s_queue) + sizeof(s_shear) + sizeof(s_t) + sizeof(s_best) + sizeof(s_visit) +
+                          sizeof(s_prev) + sizeof(s_slack) <= 48u * 1024u,
+                  "static shared memory");
     const uint4 *nodes = nullptr, *prims = nullptr;
     // A tree walk visits each node at most once: more visits, or a node index
     // past the end, can only come from a corrupt structure.
