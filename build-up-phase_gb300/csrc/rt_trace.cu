@@ -257,6 +257,53 @@ constexpr uint32_t kInstGroup = 0x40000000u;   // stack entry: instances of a TL
 constexpr int kInstDepth = 128;                // stack entries per ray (both levels)
 constexpr uint32_t kInstBlocksPerSm = 6;       // 80 registers (7 blocks: 72, within 1 %)
 
+// Whether the boxes of an instance's BLAS let the ray in up to `limit` all the
+// way down to leaf record `rec`; if so h and ids are that record's hit.
+__device__ bool confirm_hit(const uint4 *tprims, const float o[3], const float d[3], float tmin, float tmax, uint32_t rec,
+                            uint32_t inst_rec, float limit, Hit &h, HitIds &ids) {
+    const InstRec ir = load_inst(tprims, inst_rec);
+    const uint8_t *blas = reinterpret_cast<const uint8_t *>(ir.accel_ref);
+    const rt_accel_header *bh = reinterpret_cast<const rt_accel_header *>(blas);
+    const uint4 *nodes = reinterpret_cast<const uint4 *>(blas + bh->node_offset);
+    const uint4 *p = reinterpret_cast<const uint4 *>(blas + bh->prim_offset) + (size_t)rec * 3u;
+    const uint32_t count = bh->node_count;
+    float o2[3], d2[3];
+    xform_point(ir.w2o, o, o2);
+    xform_vector(ir.w2o, d, d2);
+    Ray r;
+    ray_setup(r, o2, d2);
+    const uint4 q0 = ldg4(p), q1 = ldg4(p + 1), q2 = ldg4(p + 2);
+    if (!isect_tri(r, xyz_of(q0), xyz_of(q1), xyz_of(q2), tmin, tmax, h.t, h.u, h.v)) return false;
+    const float t_lo = fmaxf(tmin, h.t - fabsf(h.t) * 0x1p-16f);
+    uint2 stack[kMaxDepth];
+    int depth = 0;
+    uint32_t node = 0u;
+    for (uint32_t visits = 0; visits < count && node < count; ++visits) {
+        const NodeWords nd = load_node(nodes, node);
+        const uint32_t hits = isect_node(r, nd, t_lo, limit), bit = rec - nd.w1.y;
+        if (bit < 24u && ((leaf_records(nd, hits) >> bit) & 1u)) {
+            h.rec = rec;
+            h.tri = q0.w;
+            h.inst = ir.id;
+            h.found = true;
+            ids.custom = ir.cim & 0xffffffu;
+            ids.sbt_off = ir.sof & 0xffffffu;
+            ids.geom = q1.w;
+            ids.prim = q2.w;
+            return true;
+        }
+        uint2 g = child_group(nd, hits);
+        if (!group_left(g) && depth > 0) g = stack[--depth];
+        if (!group_left(g)) return false;
+        node = take_child(g, r.prio);
+        if (group_left(g)) {
+            if (depth == kMaxDepth) return false;
+            stack[depth++] = g;
+        }
+    }
+    return false;
+}
+
 template <bool ANY>
 __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(const BatchArgs a) {
     pdl_wait();
@@ -342,11 +389,6 @@ __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(
         r.invd[0] = w1.x; r.invd[1] = w1.y; r.invd[2] = w1.z;
     };
 
-    auto result_place = [&](uint32_t ray_idx) {
-        return a.hits       ? reinterpret_cast<uint32_t *>(a.hits + ray_idx)
-               : a.hits_ext ? reinterpret_cast<uint32_t *>(a.hits_ext + ray_idx)
-                            : nullptr;
-    };
     auto write_hit = [&](uint32_t ray_idx, bool hit, float t, float u, float v, uint32_t inst, uint32_t tri,
                          const HitIds &ids) {
         const float4 out = hit ? make_float4(t, __uint_as_float(tri), u, v)
@@ -394,11 +436,9 @@ __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(
                     const unsigned long long key = s_key[tid];
                     const bool hit = key != ~0ull;
                     if (hit && (best.z & kLate)) {
-                        uint32_t *place = result_place(ray_idx);
-                        if (place) {
-                            *place = aside;
-                            aside = ray_idx;
-                        }
+                        a.hits[ray_idx] = make_float4(__uint_as_float(aside), __uint_as_float(best.z & ~(kMinusZero | kLate)),
+                                                      __uint_as_float(best.w), ford_inv(s_prev[tid]));
+                        aside = ray_idx;
                     } else {
                         const uint32_t rec = best.z & ~kMinusZero;
                         HitIds ids;
@@ -659,17 +699,20 @@ __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(
         }
     }
 
-    // ---- the rays set aside
+    // ---- the rays set aside: see k_trace_blas; the hit is confirmed within its
+    // instance
     if (!ANY) {
-        for (uint32_t i = aside; i != kNone;) {
-            const uint32_t next = *result_place(i);
+        uint32_t next = kNone;
+        for (uint32_t i = aside; i != kNone; i = next) {
+            const float4 kept = a.hits[i];
+            next = __float_as_uint(kept.x);
             const float4 r0 = __ldg(a.rays + 2u * i), r1 = __ldg(a.rays + 2u * i + 1u);
             const float o[3] = {r0.x, r0.y, r0.z}, d[3] = {r1.x, r1.y, r1.z};
             Hit h;
             HitIds ids;
-            trace_ray<false>(a.accel, o, d, r0.w, r1.w, 0xffu, h, ids, a.err);
+            if (!confirm_hit(tprims, o, d, r0.w, r1.w, __float_as_uint(kept.y), __float_as_uint(kept.z), kept.w, h, ids))
+                trace_ray<false>(a.accel, o, d, r0.w, r1.w, 0xffu, h, ids, a.err);
             write_hit(i, h.found, h.t, h.u, h.v, h.inst, h.tri, ids);
-            i = next;
         }
     }
 }

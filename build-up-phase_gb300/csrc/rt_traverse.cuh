@@ -104,8 +104,8 @@ struct BatchArgs {
 // every triangle is tested on the spot, 28.1 of 32 lanes walking per node step
 // (2M box, mixed launches: 27.4).  With the box test's instruction count, the
 // 64-bit queue entry and the hits' shared-memory minima this took the launch from
-// 1.92 to 1.58 ms, the path tracer's 2M-triangle frame of four samples from 25.7
-// to 20.6.  What bounds it now: issue slots (79 % busy) and the L1 data path
+// 1.92 to 1.55 ms, the path tracer's 2M-triangle frame of four samples from 25.7
+// to 20.7.  What bounds it now: issue slots (79 % busy) and the L1 data path
 // (78 %: a node is five 16-byte loads per lane, nearly every one a wavefront of
 // its own).
 //
@@ -118,15 +118,16 @@ struct BatchArgs {
 // boxes_may_exceed bounds from X's vertices where those boxes let the ray in.  A
 // ray whose best hit has that bound beyond the nearest earlier hit of another
 // node (records of one node are tested together in either walk) is set aside --
-// its result's place links the lane's rays of that kind -- and walked in order
-// once the lane is done with the others.  For any other ray the hit is the other
+// its result's place links the lane's rays of that kind -- and its hit confirmed,
+// or the ray walked in order, once the lane is done with the others.  For any other ray the hit is the other
 // walk's: its far limits are hits no nearer than X, so every box above X lets
 // the ray in there too, X is tested, and nothing it tests is better.
 // (12 coincident copies of 60 axis-parallel triangles, 1M rays: 0 to 3 rays
 // differ without this, 2 to 4 of rays that start on the triangles with a window
-// of 2^-12 of t in the place of the bound.  It costs the soup's rays 2 %, 1.55 ->
-// 1.58 ms, the 2M box's frame 0.5 %; in the 56-register kernel 8 % with the ray
-// held through the merge instead of read again.)
+// of 2^-12 of t in the place of the bound.  The soup's rays take 1.55 ms with or
+// without it, the 2M box's frame 20.67 for 20.43; in the 56-register kernel 8 %
+// more with the ray held through the merge instead of read again, in the mixed
+// kernel 2 % more with it read again.)
 constexpr float kBoxSlack = 0x1p-20f;
 constexpr uint32_t kTriQueue = 64;  // entries per warp: below 32 before an append of at most 32
 constexpr int kTriDrain = 8;   // lanes waiting for their entries alone before a partial batch is tested
@@ -254,11 +255,6 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY || MIXED) ? 1024 : 115
     const uint32_t lanes = share >= 32u ? kFull : (1u << share) - 1u;
     const int refill = (int)min(a.refill, min(share, 32u));
 
-    auto result_place = [&](uint32_t ray_idx) {
-        return MIXED || a.hits ? reinterpret_cast<uint32_t *>(a.hits + ray_idx)
-               : a.hits_ext    ? reinterpret_cast<uint32_t *>(a.hits_ext + ray_idx)
-                               : nullptr;
-    };
     auto write_hit = [&](uint32_t ray_idx, bool hit, float t, float u, float v, uint32_t rec, uint32_t tri) {
         const float4 out = hit ? make_float4(t, __uint_as_float(a.out_rec ? rec : tri), u, v)
                                : make_float4(kInf, __uint_as_float(kNone), 0.f, 0.f);
@@ -301,11 +297,9 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY || MIXED) ? 1024 : 115
                 } else {
                     const uint4 best = s_best[tid];
                     if (best.w != kNone && (best.z & kLate)) {
-                        uint32_t *place = result_place(ray_idx);
-                        if (place) {
-                            *place = aside;
-                            aside = ray_idx;
-                        }
+                        a.hits[ray_idx] = make_float4(__uint_as_float(aside), __uint_as_float(best.z & ~(kMinusZero | kLate)),
+                                                      ford_inv(s_prev[tid]), tbest);
+                        aside = ray_idx;
                     } else {
                         write_hit(ray_idx, best.w != kNone, (best.z & kMinusZero) ? -0.0f : tbest,
                                   __uint_as_float(best.x), __uint_as_float(best.y), best.z & ~kMinusZero, best.w);
@@ -532,10 +526,17 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY || MIXED) ? 1024 : 115
         }
     }
 
-    // ---- the rays set aside, each lane its own, every record tested as its
-    // node is visited (one loop over rays and nodes: the lanes' walks differ)
+    // ---- the rays set aside, each lane its own (one loop over rays and nodes: the
+    // lanes' walks differ).  First whether the boxes above the hit found let the
+    // ray in up to the nearest earlier hit: if so a walk in order tests it too.
+    // Few boxes hold a given point, so that takes a tenth of a whole walk (23,000
+    // of the walls' 1M rays, walked at the end of their warps: the launch took 1,150
+    // us by whole walks alone, 1,037 so, 1,083 with every record tested on the
+    // spot).  Only where its record is not reached that way the whole walk in order, every
+    // record tested as its node is visited.
     if (!ANY) {
         uint32_t idx = kNone, next = aside, at = 0u, seen = 0u;
+        uint32_t found_rec = kNone;  // the hit's record, kNone in the whole walk
         int depth = 0;
         bool walking = false;
         Hit h;
@@ -546,16 +547,24 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY || MIXED) ? 1024 : 115
         uint2(&stack)[kMaxDepth + 1] = spill;
         for (;;) {
             if (!walking) {
-                if (idx != kNone) write_hit(idx, h.tri != kNone, h.t, h.u, h.v, h.rec, h.tri);
-                idx = next;
-                if (idx == kNone) break;
-                next = *result_place(idx);
-                if (MULTI) scene_of(__ldg(a.ray_scene + idx));
-                const float4 r0 = __ldg(a.rays + 2u * idx), r1 = __ldg(a.rays + 2u * idx + 1u);
-                const float o[3] = {r0.x, r0.y, r0.z}, d[3] = {r1.x, r1.y, r1.z};
-                ray_setup(w, o, d);
-                t_lo = r0.w;
-                h.t = r1.w;
+                if (idx != kNone && found_rec != kNone) {
+                    found_rec = kNone;
+                    t_lo = __ldg(a.rays + 2u * idx).w;
+                    h.t = __ldg(a.rays + 2u * idx + 1u).w;
+                } else {
+                    if (idx != kNone) write_hit(idx, h.tri != kNone, h.t, h.u, h.v, h.rec, h.tri);
+                    idx = next;
+                    if (idx == kNone) break;
+                    const float4 kept = a.hits[idx];
+                    next = __float_as_uint(kept.x);
+                    found_rec = __float_as_uint(kept.y);
+                    if (MULTI) scene_of(__ldg(a.ray_scene + idx));
+                    const float4 r0 = __ldg(a.rays + 2u * idx), r1 = __ldg(a.rays + 2u * idx + 1u);
+                    const float o[3] = {r0.x, r0.y, r0.z}, d[3] = {r1.x, r1.y, r1.z};
+                    ray_setup(w, o, d);
+                    h.t = kept.z;
+                    t_lo = fmaxf(r0.w, kept.w - fabsf(kept.w) * 0x1p-16f);
+                }
                 h.tri = kNone;
                 at = 0u;
                 seen = 0u;
@@ -567,7 +576,17 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY || MIXED) ? 1024 : 115
             ++seen;
             const NodeWords nd = load_node(nodes, at);
             const uint32_t hits = isect_node(w, nd, t_lo, h.t);
-            for (uint32_t recs = leaf_records(nd, hits); recs; recs &= recs - 1u) {
+            uint32_t recs = leaf_records(nd, hits);
+            if (found_rec != kNone) {
+                const uint32_t at_bit = found_rec - nd.w1.y;
+                recs = at_bit < 24u ? recs & (1u << at_bit) : 0u;
+                if (recs) {
+                    t_lo = __ldg(a.rays + 2u * idx).w;
+                    h.t = __ldg(a.rays + 2u * idx + 1u).w;
+                }
+            }
+            const bool reached = found_rec != kNone && recs != 0u;
+            for (; recs; recs &= recs - 1u) {
                 const uint32_t rec = nd.w1.y + (uint32_t)__ffs((int)recs) - 1u;
                 const uint4 *p = prims + (size_t)rec * 3u;
                 const uint4 q0 = ldg4(p), q1 = ldg4(p + 1), q2 = ldg4(p + 2);
@@ -576,6 +595,11 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY || MIXED) ? 1024 : 115
                 if (t < h.t || q0.w < h.tri) {  // (t <= h.t)
                     h.t = t; h.u = u; h.v = v; h.rec = rec; h.tri = q0.w;
                 }
+            }
+            if (reached) {
+                found_rec = kNone;
+                walking = false;
+                continue;
             }
             uint2 g = child_group(nd, hits);
             if (!group_left(g) && depth > 0) g = stack[--depth];
