@@ -992,7 +992,6 @@ __device__ __forceinline__ void collapse_phase_a(const CollapseArgs &a, uint32_t
         const bool p1 = src_open && j < 2 && info_open(t1), p2 = src_open && j < 4 && info_open(t2);
         const bool p3 = src_open && info_open(t3);
         const uint32_t o1 = (__ballot_sync(kFullMask, p1) >> gb) & 3u, o2 = (__ballot_sync(kFullMask, p2) >> gb) & 15u;
-        const uint32_t o3 = (__ballot_sync(kFullMask, p3) >> gb) & 255u;
         const int total = 2 + __popc(o1) + __popc(o2);
         const float a1 = p1 ? t1.area : -1.0f, a2 = p2 ? t2.area : -1.0f;
         uint32_t r1 = 0u, r2 = 0u, same = 0u;
@@ -1241,20 +1240,7 @@ __device__ void collapse_phase_b(const CollapseArgs &a, uint32_t k, uint32_t chi
     a.nodes_out[(size_t)k * 5u + 1u] = make_uint4(child_base, prim_base, meta_lo, meta_hi);
 }
 
-template <int N>
-__device__ __forceinline__ uint32_t block_sum(uint32_t v, uint32_t *s_red) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    uint32_t s = 0;
-    for (int i = 0; i < N / 32; ++i) s += s_red[i];
-    __syncthreads();
-    return s;
-}
-
-// Block-wide sums of four values at once (one shared-memory round instead
-// of four).
+// Block-wide sums of four values at once (one shared-memory round).
 template <int N>
 __device__ __forceinline__ uint4 block_sum4(uint4 v, uint4 *s_red4) {
 #pragma unroll

@@ -210,14 +210,6 @@ __device__ __forceinline__ NodeWords load_node(const uint4 *nodes, uint32_t idx)
     return n;
 }
 
-__device__ __forceinline__ uint32_t byte_of(uint32_t w, int b) { return (w >> (8 * b)) & 0xffu; }
-
-// Byte b of w as an exact float: PRMT assembles 0x4B0000qq (= 2^23 + q) and
-// one FADD removes 2^23.  Same value as (float)q without the conversion pipe.
-__device__ __forceinline__ float qbyte(uint32_t w, int b) {
-    return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7540u | (uint32_t)b)) - 8388608.0f;
-}
-
 // Three-input min/max (sm_100+ PTX); exact, so equal to two-input chains.
 __device__ __forceinline__ float fmin3(float a, float b, float c) {
     float d;

@@ -855,7 +855,7 @@ int path_trace_impl(rt_context *ctx, rt_stream stream, const rt_pt_scene *scene,
         // 1,205.  Not the traversals, whose blocks would crowd where the launch
         // before leaves room first: 200x120 pixels 666 -> 712 us.  So what they
         // read and write is complete when any other kernel starts.)
-        int rc0 = launch_queue_trace(ctx, st, accel, rays[0], S + L.hits, nullptr, &cnt[0], nw, &tcnt[0], false);
+        int rc0 = launch_queue_trace(ctx, st, accel, rays[0], S + L.hits, &cnt[0], nw, &tcnt[0]);
         if (rc0) return rc0;
         for (uint32_t d = 0; d < p->max_depth; ++d) {
             const uint32_t q = d & 1u;
@@ -1163,8 +1163,8 @@ int batch_enqueue(rt_batch_plan *pl, cudaStream_t st, uint32_t *kernels) {
             a.wave_base = base;
             // depth 0's extension rays alone; afterwards each launch traces a
             // depth's shadow rays together with the next depth's extension rays
-            int rc0 = launch_queue_trace_multi(ctx, st, views, n_sc, rsid[0], rays[0], S + L.hits, nullptr, &cnt[0], n,
-                                               &tcnt[0], false, shape);
+            int rc0 = launch_queue_trace_multi(ctx, st, views, n_sc, rsid[0], rays[0], S + L.hits, &cnt[0], n,
+                                               &tcnt[0], shape);
             if (rc0) return rc0;
             ++k;
             for (uint32_t d = 0; d < pl->p.max_depth; ++d) {

@@ -17,9 +17,9 @@
 namespace rtc {
 namespace {
 
-template <bool ANY, int THREADS, bool MIXED = false>
+template <int THREADS, bool MIXED>
 auto kernel_of(uint32_t ring) {
-    return ring == 32u ? k_trace_blas<ANY, true, THREADS, 16, MIXED> : k_trace_blas<ANY, true, THREADS, 8, MIXED>;
+    return ring == 32u ? k_trace_blas<false, true, THREADS, 16, MIXED> : k_trace_blas<false, true, THREADS, 8, MIXED>;
 }
 
 bool valid_shape(const TraceShape &shape) {
@@ -33,18 +33,16 @@ bool valid_shape(const TraceShape &shape) {
 int prepare_queue_trace_multi(rt_context *ctx, const TraceShape &shape) {
     if (!valid_shape(shape)) return set_error(ctx, RT_ERR_INVALID_ARG, "multi-scene traversal: unsupported launch shape");
     const bool wide = shape.threads == 256u;
-    const auto closest = wide ? kernel_of<false, 256>(shape.ring) : kernel_of<false, 128>(shape.ring);
-    const auto any = wide ? kernel_of<true, 256>(shape.ring) : kernel_of<true, 128>(shape.ring);
-    const auto mixed = wide ? kernel_of<false, 256, true>(shape.ring) : kernel_of<false, 128, true>(shape.ring);
+    const auto closest = wide ? kernel_of<256, false>(shape.ring) : kernel_of<128, false>(shape.ring);
+    const auto mixed = wide ? kernel_of<256, true>(shape.ring) : kernel_of<128, true>(shape.ring);
     cudaFuncAttributes fa;
-    for (const auto f : {closest, any, mixed}) RT_CUDA_CTX(ctx, cudaFuncGetAttributes(&fa, (const void *)f));
+    for (const auto f : {closest, mixed}) RT_CUDA_CTX(ctx, cudaFuncGetAttributes(&fa, (const void *)f));
     return RT_OK;
 }
 
 int launch_queue_trace_multi(rt_context *ctx, cudaStream_t st, const void *views, uint32_t n_scenes,
-                             const uint32_t *ray_scene, const void *rays, void *hits, uint8_t *occluded,
-                             const uint32_t *n_dev, uint32_t max_n, uint32_t *counter, bool any,
-                             const TraceShape &shape) {
+                             const uint32_t *ray_scene, const void *rays, void *hits, const uint32_t *n_dev,
+                             uint32_t max_n, uint32_t *counter, const TraceShape &shape) {
     if (max_n == 0) return RT_OK;
     if (!valid_shape(shape))
         return set_error(ctx, RT_ERR_INVALID_ARG, "multi-scene traversal: unsupported launch shape");
@@ -54,7 +52,6 @@ int launch_queue_trace_multi(rt_context *ctx, cudaStream_t st, const void *views
     a.n_scenes = n_scenes;
     a.rays = static_cast<const float4 *>(rays);
     a.hits = static_cast<float4 *>(hits);
-    a.occluded = occluded;
     a.n = max_n;
     a.refill = shape.refill;
     a.counter = counter;
@@ -64,9 +61,7 @@ int launch_queue_trace_multi(rt_context *ctx, cudaStream_t st, const void *views
     uint32_t blocks = shape.blocks_per_sm * (uint32_t)ctx->sm_count;
     const uint32_t need = (max_n + shape.threads - 1u) / shape.threads;
     if (blocks > need) blocks = need;
-    const bool wide = shape.threads == 256u;
-    const auto kernel = any ? (wide ? kernel_of<true, 256>(shape.ring) : kernel_of<true, 128>(shape.ring))
-                            : (wide ? kernel_of<false, 256>(shape.ring) : kernel_of<false, 128>(shape.ring));
+    const auto kernel = shape.threads == 256u ? kernel_of<256, false>(shape.ring) : kernel_of<128, false>(shape.ring);
     kernel<<<blocks, shape.threads, 0, st>>>(a);
     RT_CUDA_CTX(ctx, cudaGetLastError());
     return RT_OK;
@@ -103,8 +98,7 @@ int launch_queue_trace_multi_mixed(rt_context *ctx, cudaStream_t st, const void 
     uint32_t blocks = shape.blocks_per_sm * (uint32_t)ctx->sm_count;
     const uint32_t need = (uint32_t)(((uint64_t)max_n * 2u + shape.threads - 1u) / shape.threads);
     if (blocks > need) blocks = need;
-    const auto kernel =
-        shape.threads == 256u ? kernel_of<false, 256, true>(shape.ring) : kernel_of<false, 128, true>(shape.ring);
+    const auto kernel = shape.threads == 256u ? kernel_of<256, true>(shape.ring) : kernel_of<128, true>(shape.ring);
     kernel<<<blocks, shape.threads, 0, st>>>(a);
     RT_CUDA_CTX(ctx, cudaGetLastError());
     return RT_OK;

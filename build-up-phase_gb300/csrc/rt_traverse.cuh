@@ -98,9 +98,8 @@ struct BatchArgs {
 // as many entries as lanes with a ray, the whole warp tests them, one entry per
 // lane with the owner's ray read by shuffles, and hands the hits back to their
 // owners.  A ray walks a few nodes more because its far limit shrinks a few
-// visits later.  A lane keeps its ray until its last entry
-// has been tested.  1M soup, 4.15M primary and incoherent rays: 28.6 entries
-// per batch, 18.4 nodes and 4.4 triangles per ray against 17.7 and 4.0 when
+// visits later.  A lane keeps its ray until its last entry has been tested.  1M
+// soup, 4.15M primary and incoherent rays: 28.6 entries per batch, 18.4 nodes and 4.4 triangles per ray against 17.7 and 4.0 when
 // every triangle is tested on the spot, 28.1 of 32 lanes walking per node step
 // (2M box, mixed launches: 27.4).  With the box test's instruction count, the
 // 64-bit queue entry and the hits' shared-memory minima this took the launch from
@@ -119,9 +118,10 @@ struct BatchArgs {
 // ray whose best hit has that bound beyond the nearest earlier hit of another
 // node (records of one node are tested together in either walk) is set aside --
 // its result's place links the lane's rays of that kind -- and its hit confirmed,
-// or the ray walked in order, once the lane is done with the others.  For any other ray the hit is the other
-// walk's: its far limits are hits no nearer than X, so every box above X lets
-// the ray in there too, X is tested, and nothing it tests is better.
+// or the ray walked in order, once the lane is done with the others.  For any
+// other ray the hit is the other walk's: its far limits are hits no nearer than
+// X, so every box above X lets the ray in there too, X is tested, and nothing it
+// tests is better.
 // (12 coincident copies of 60 axis-parallel triangles, 1M rays: 0 to 3 rays
 // differ without this, 2 to 4 of rays that start on the triangles with a window
 // of 2^-12 of t in the place of the bound.  The soup's rays take 1.55 ms with or
@@ -249,7 +249,9 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY || MIXED) ? 1024 : 115
     const uint32_t n_rays = MIXED ? n1 + min(*a.n_dev2, a.n2) : n1;
     bool any_ray = ANY;  // this lane's ray is an any-hit ray
     // Fewer rays than lanes: each warp takes its share of them in as few lanes
-    // as that needs, so that the rays' walks do not wait on one another.
+    // as that needs, so that the rays' walks do not wait on one another.  So with
+    // the path tracer's queues, whose grid is that of the longest; a query's grid
+    // has a warp per 32 rays, which leaves up to about a thousand to spread.
     const uint32_t warps = gridDim.x * (THREADS / 32);
     const uint32_t share = n_rays / warps + 1u;
     const uint32_t lanes = share >= 32u ? kFull : (1u << share) - 1u;
