@@ -147,6 +147,7 @@ __device__ bool trace_ray(const uint8_t *accel, const float o[3], const float d[
     const rt_accel_header *hd = reinterpret_cast<const rt_accel_header *>(accel);
     h.t = tmax; h.u = 0.f; h.v = 0.f; h.rec = kNone; h.tri = kNone; h.inst = 0; h.found = false;
     ids.custom = 0; ids.sbt_off = 0; ids.geom = 0; ids.prim = 0;
+    if (!(tmin <= tmax)) return false;  // an empty interval, a NaN limit
     uint64_t hkey = ~0ull;
     Ray r;
     ray_setup_box(r, o, d);
@@ -488,6 +489,10 @@ __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(
                     visits = 0;
                     count = t_count;
                     pending = !t_empty;
+                    if (!(tmin <= tbest)) {  // a miss, a NaN limit too
+                        tmin = kInf;
+                        tbest = -kInf;
+                    }
                     sp = 0;
                     lo = 0;
                     last = head - 1u;
@@ -721,19 +726,42 @@ __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(
 // Traversal statistics (rt_trace_stats): node visits and triangle tests of a
 // walk in the order of the CPU restatement, which tests a node's triangles as it
 // visits the node (the kernels above test some more).  Persistent warps and the
-// stack of the kernels above, both structure kinds in one: a BLAS is walked like
-// the only instance of a TLAS.  2M rays of the 1M soup: 1,572 us (one thread per
-// ray 3,436), 800K in 64 instances 1,200; six blocks of 80 registers per SM 1,914
-// and 1,240, seven 1,761 and 1,195 (before the short way to the next node; eight
-// 1,677 and 1,180, nine 1,877 and 1,289).
-constexpr uint32_t kStatsBlocksPerSm = 8;
-template <bool ANY>
-__global__ void __launch_bounds__(kTraceThreads, kStatsBlocksPerSm)
+// stack of the kernels above, a kernel per structure kind.  2M rays of the 1M
+// soup: closest hits 1,558 us, any hit 1,273 at nine blocks per SM, 1,562 and
+// 1,300 at eight (one thread per ray 3,436 and 2,650; both kinds in one kernel
+// 1,616 and 1,343); 800K rays in 64 instances: 1,238 and 1,157 at eight, 1,261
+// and 1,175 at nine.
+constexpr uint32_t stats_blocks_per_sm(bool top) { return top ? 8u : 9u; }
+
+// isect_node under a NaN limit, as the CPU restatement compares: a child is hit
+// where tnear <= tfar, so not where either is NaN.
+__device__ uint32_t isect_node_nan(const Ray &r, const NodeWords &n, float tmin, float tcur) {
+    const float p[3] = {__uint_as_float(n.w0.x), __uint_as_float(n.w0.y), __uint_as_float(n.w0.z)};
+    const uint32_t lo[6] = {n.w2.x, n.w2.y, n.w2.z, n.w2.w, n.w3.x, n.w3.y};
+    const uint32_t hi[6] = {n.w3.z, n.w3.w, n.w4.x, n.w4.y, n.w4.z, n.w4.w};
+    uint32_t hits = 0u;
+    for (int s = 0; s < 8; ++s) {
+        float tn = tmin, tf = tcur;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const float sc = pow2f((int)(int8_t)(n.w0.w >> (8 * a))) * r.invd[a], adj = (p[a] - r.o[a]) * r.invd[a];
+            const uint32_t wl = s < 4 ? lo[2 * a] : lo[2 * a + 1], wh = s < 4 ? hi[2 * a] : hi[2 * a + 1];
+            const float ql = (float)((wl >> (8 * (s & 3))) & 0xffu), qh = (float)((wh >> (8 * (s & 3))) & 0xffu);
+            const bool neg = r.invd[a] < 0.0f;
+            tn = fmaxf(tn, __fmaf_rn(neg ? qh : ql, sc, adj));
+            tf = fminf(tf, __fmaf_rn(neg ? ql : qh, sc, adj));
+        }
+        if (tn <= tf * kTfarScale) hits |= 1u << s;
+    }
+    return hits;
+}
+
+template <bool ANY, bool TOP>
+__global__ void __launch_bounds__(kTraceThreads, stats_blocks_per_sm(TOP))
 k_trace_stats(const uint8_t *accel, const float4 *rays, uint32_t n, uint32_t refill, uint32_t *counter,
               unsigned long long *counters, uint32_t *err) {
     const rt_accel_header *hd = reinterpret_cast<const rt_accel_header *>(accel);
-    const bool top = hd->kind == RT_ACCEL_KIND_TLAS;
-    if (!top && hd->kind != RT_ACCEL_KIND_BLAS) return;
+    if (hd->kind != (TOP ? RT_ACCEL_KIND_TLAS : RT_ACCEL_KIND_BLAS)) return;
     const uint4 *tnodes = reinterpret_cast<const uint4 *>(accel + hd->node_offset);
     const uint4 *tprims = reinterpret_cast<const uint4 *>(accel + hd->prim_offset);
     const uint32_t t_count = hd->node_count;
@@ -797,7 +825,7 @@ k_trace_stats(const uint8_t *accel, const float4 *rays, uint32_t n, uint32_t ref
                 tmin = limits.x;
                 tbest = limits.y;
                 walking = true;
-                in_blas = !top;
+                in_blas = !TOP;
                 nodes = tnodes;
                 prims = tprims;
                 count = t_count;
@@ -815,9 +843,10 @@ k_trace_stats(const uint8_t *accel, const float4 *rays, uint32_t n, uint32_t ref
         ++visits;
         ++n_nodes;
         const NodeWords nd = load_node(nodes, node);
-        const uint32_t hits = isect_node(r, nd, tmin, tbest);
+        const bool limits = tmin == tmin && tbest == tbest;
+        const uint32_t hits = limits ? isect_node(r, nd, tmin, tbest) : isect_node_nan(r, nd, tmin, tbest);
         uint2 g = child_group(nd, hits), ig = make_uint2(nd.w1.y, leaf_records(nd, hits));
-        if (in_blas) {
+        if (!TOP || in_blas) {
             for (; ig.y; ig.y &= ig.y - 1u) {
                 const uint4 *p = prims + (size_t)(ig.x + (uint32_t)__ffs((int)ig.y) - 1u) * 3u;
                 const uint4 q0 = ldg4(p), q1 = ldg4(p + 1), q2 = ldg4(p + 2);
@@ -834,7 +863,7 @@ k_trace_stats(const uint8_t *accel, const float4 *rays, uint32_t n, uint32_t ref
         }
         // the next node: mostly a child, in a bare BLAS else the stack's top (past
         // the loop below 1,677 -> 1,572 us)
-        if (walking && !top && !group_left(g) && sp > 0) g = pop();
+        if (walking && !TOP && !group_left(g) && sp > 0) g = pop();
         if (walking && ig.y == 0u && group_left(g)) {
             node = take_child(g, r.prio);
             if (group_left(g)) {
@@ -845,7 +874,7 @@ k_trace_stats(const uint8_t *accel, const float4 *rays, uint32_t n, uint32_t ref
         }
         // else an instance of this node, a child, the stack
         while (walking) {
-            if (ig.y) {
+            if (TOP && ig.y) {
                 const uint32_t rec = ig.x + (uint32_t)__ffs((int)ig.y) - 1u;
                 ig.y &= ig.y - 1u;
                 const InstRec ir = load_inst(tprims, rec);
@@ -885,7 +914,7 @@ k_trace_stats(const uint8_t *accel, const float4 *rays, uint32_t n, uint32_t ref
                 break;
             }
             const uint2 e = pop();
-            if (e.y & kReturn) {
+            if (TOP && (e.y & kReturn)) {
                 if (sp == 0) {
                     walking = false;
                     break;
@@ -897,7 +926,7 @@ k_trace_stats(const uint8_t *accel, const float4 *rays, uint32_t n, uint32_t ref
                 in_blas = false;
                 nodes = tnodes;
                 count = t_count;
-            } else if (e.y & kInstGroup) {
+            } else if (TOP && (e.y & kInstGroup)) {
                 ig = make_uint2(e.x, e.y & ~kInstGroup);
             } else {
                 g = e;
@@ -1378,13 +1407,16 @@ extern "C" rt_status rt_trace_stats(rt_context *ctx, rt_stream stream, uint64_t 
     uint32_t *counter = acquire_counter(ctx, st);
     if (!counter) return set_error(ctx, RT_ERR_CUDA, "work counter reset failed");
     const uint32_t refill = ctx->tuning.batch_rays ? (ctx->tuning.batch_rays < 32u ? ctx->tuning.batch_rays : 32u) : 4u;
-    uint32_t blocks = kStatsBlocksPerSm * (uint32_t)ctx->sm_count;
-    const uint32_t need = (n + kTraceThreads - 1) / kTraceThreads;
-    if (blocks > need) blocks = need;
+    const uint32_t need = (n + kTraceThreads - 1) / kTraceThreads, sms = (uint32_t)ctx->sm_count;
     const uint8_t *A = reinterpret_cast<const uint8_t *>(accel);
     const float4 *R = reinterpret_cast<const float4 *>(rays);
-    if (any_hit) k_trace_stats<true><<<blocks, kTraceThreads, 0, st>>>(A, R, n, refill, counter, counters, ctx->d_err);
-    else k_trace_stats<false><<<blocks, kTraceThreads, 0, st>>>(A, R, n, refill, counter, counters, ctx->d_err);
+    // one of the two returns at once, as in launch_batch
+    for (const bool top : {false, true}) {
+        const auto kernel = top ? (any_hit ? k_trace_stats<true, true> : k_trace_stats<false, true>)
+                                : (any_hit ? k_trace_stats<true, false> : k_trace_stats<false, false>);
+        const uint32_t most = stats_blocks_per_sm(top) * sms;
+        kernel<<<need < most ? need : most, kTraceThreads, 0, st>>>(A, R, n, refill, counter, counters, ctx->d_err);
+    }
     RT_CUDA_CTX(ctx, cudaGetLastError());
     return RT_OK;
 }
