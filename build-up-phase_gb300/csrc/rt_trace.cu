@@ -326,8 +326,10 @@ __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(
     __shared__ int32_t s_t[ANY ? 1 : kTraceThreads];
     __shared__ unsigned long long s_key[ANY ? 1 : kTraceThreads];
     __shared__ uint4 s_best[ANY ? 1 : kTraceThreads];
-    __shared__ uint32_t s_step[ANY ? 1 : kTraceThreads];  // the step (node visit) of the best hit in this instance (0: none)
-    __shared__ int32_t s_prev[ANY ? 1 : kTraceThreads];   // the nearest hit of an earlier step in it, as an ordered integer
+    // within the instance: the step (node visit) of the best hit (0: none), the
+    // nearest hit of an earlier step, as an ordered integer
+    __shared__ uint32_t s_step[ANY ? 1 : kTraceThreads];
+    __shared__ int32_t s_prev[ANY ? 1 : kTraceThreads];
     constexpr uint32_t kFull = 0xffffffffu;
     const int tid = threadIdx.x, lane = tid & 31;
     uint2 *queue = s_queue[tid >> 5];
@@ -438,7 +440,8 @@ __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(
                     const unsigned long long key = s_key[tid];
                     const bool hit = key != ~0ull;
                     if (hit && (best.z & kLate)) {
-                        a.hits[ray_idx] = make_float4(__uint_as_float(aside), __uint_as_float(best.z & ~(kMinusZero | kLate)),
+                        const uint32_t rec = best.z & ~(kMinusZero | kLate);
+                        a.hits[ray_idx] = make_float4(__uint_as_float(aside), __uint_as_float(rec),
                                                       __uint_as_float(best.w), ford_inv(s_prev[tid]));
                         aside = ray_idx;
                     } else {
@@ -675,29 +678,31 @@ __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(
                     unsigned long long *bk = s_key + warp0 + src;
                     const uint32_t own = e.y >> 5;
                     const bool hit_too = hit;
-                    if (hit && atomicMin(bt, tk) > tk) *bk = ~0ull;
-                    __syncwarp();
-                    hit = hit && *bt == tk;
-                    if (hit) atomicMin(bk, key);
-                    __syncwarp();
-                    hit = hit && *bk == key;
-                    if (hit) {
-                        const uint32_t before = s_step[warp0 + src];
-                        s_step[warp0 + src] = own;
-                        if (before != own) s_prev[warp0 + src] = before ? ford(t_hi + 0.0f) : kNoLimit;
-                        s_best[warp0 + src] =
-                            make_uint4(__float_as_uint(u), __float_as_uint(v),
-                                       rec | (__float_as_uint(t) == kMinusZero ? kMinusZero : 0u), irec);
+                    if (__any_sync(kFull, hit)) {
+                        if (hit && atomicMin(bt, tk) > tk) *bk = ~0ull;
+                        __syncwarp();
+                        hit = hit && *bt == tk;
+                        if (hit) atomicMin(bk, key);
+                        __syncwarp();
+                        hit = hit && *bk == key;
+                        if (hit) {
+                            const uint32_t before = s_step[warp0 + src];
+                            s_step[warp0 + src] = own;
+                            if (before != own) s_prev[warp0 + src] = before ? ford(t_hi + 0.0f) : kNoLimit;
+                            s_best[warp0 + src] =
+                                make_uint4(__float_as_uint(u), __float_as_uint(v),
+                                           rec | (__float_as_uint(t) == kMinusZero ? kMinusZero : 0u), irec);
+                        }
+                        __syncwarp();
+                        if (hit_too && !hit && own < s_step[warp0 + src]) atomicMin(s_prev + warp0 + src, tk);
+                        __syncwarp();
+                        if (hit) {  // see boxes_may_exceed
+                            const int32_t prev = s_prev[warp0 + src];
+                            if (prev != kNoLimit && boxes_may_exceed(tr, pr + (size_t)rec * 3u, ford_inv(prev)))
+                                s_best[warp0 + src].z |= kLate;
+                        }
+                        __syncwarp();
                     }
-                    __syncwarp();
-                    if (hit_too && !hit && own < s_step[warp0 + src]) atomicMin(s_prev + warp0 + src, tk);
-                    __syncwarp();
-                    if (hit) {  // see boxes_may_exceed
-                        const int32_t prev = s_prev[warp0 + src];
-                        if (prev != kNoLimit && boxes_may_exceed(tr, pr + (size_t)rec * 3u, ford_inv(prev)))
-                            s_best[warp0 + src].z |= kLate;
-                    }
-                    __syncwarp();
                     tbest = ford_inv(s_t[tid]);
                 }
             }

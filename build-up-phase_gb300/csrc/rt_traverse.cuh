@@ -99,12 +99,12 @@ struct BatchArgs {
 // lane with the owner's ray read by shuffles, and hands the hits back to their
 // owners.  A ray walks a few nodes more because its far limit shrinks a few
 // visits later.  A lane keeps its ray until its last entry has been tested.  1M
-// soup, 4.15M primary and incoherent rays: 28.6 entries per batch, 18.4 nodes and 4.4 triangles per ray against 17.7 and 4.0 when
-// every triangle is tested on the spot, 28.1 of 32 lanes walking per node step
-// (2M box, mixed launches: 27.4).  With the box test's instruction count, the
+// soup, 4.15M primary and incoherent rays: 28.6 entries per batch, 18.4 nodes and
+// 4.4 triangles per ray against 17.7 and 4.0 when every triangle is tested on the
+// spot, 28.1 of 32 lanes walking per node step (2M box, mixed launches: 27.4).  With the box test's instruction count, the
 // 64-bit queue entry and the hits' shared-memory minima this took the launch from
 // 1.92 to 1.55 ms, the path tracer's 2M-triangle frame of four samples from 25.7
-// to 20.7.  What bounds it now: issue slots (79 % busy) and the L1 data path
+// to 20.4.  What bounds it now: issue slots (79 % busy) and the L1 data path
 // (78 %: a node is five 16-byte loads per lane, nearly every one a wavefront of
 // its own).
 //
@@ -124,10 +124,10 @@ struct BatchArgs {
 // tests is better.
 // (12 coincident copies of 60 axis-parallel triangles, 1M rays: 0 to 3 rays
 // differ without this, 2 to 4 of rays that start on the triangles with a window
-// of 2^-12 of t in the place of the bound.  The soup's rays take 1.55 ms with or
-// without it, the 2M box's frame 20.67 for 20.43; in the 56-register kernel 8 %
-// more with the ray held through the merge instead of read again, in the mixed
-// kernel 2 % more with it read again.)
+// of 2^-12 of t in the place of the bound.  The soup's rays take 1.55 ms with
+// either, the 2M box's frame 20.37 for 20.43; in the 56-register kernel 8 % more
+// with the ray held through the merge instead of read again, in the mixed kernel
+// 2 % more with it read again.)
 constexpr float kBoxSlack = 0x1p-20f;
 constexpr uint32_t kTriQueue = 64;  // entries per warp: below 32 before an append of at most 32
 constexpr int kTriDrain = 8;   // lanes waiting for their entries alone before a partial batch is tested
@@ -139,20 +139,27 @@ __device__ __forceinline__ float4 xyz_of(const uint4 &q) {
 // kBoxSlack times the greatest coordinate of a structure's bounds; infinite where
 // a node's quantisation steps (at most 2^RT_QEXP_MAX) may not reach its bounds.
 __device__ __forceinline__ float box_slack(const rt_accel_header *h) {
-    const float4 lo = *reinterpret_cast<const float4 *>(h->bounds_lo), hi = *reinterpret_cast<const float4 *>(h->bounds_hi);
+    const float4 lo = *reinterpret_cast<const float4 *>(h->bounds_lo);
+    const float4 hi = *reinterpret_cast<const float4 *>(h->bounds_hi);
     const float m = fmaxf(fmax3(fabsf(lo.x), fabsf(lo.y), fabsf(lo.z)), fmax3(fabsf(hi.x), fabsf(hi.y), fabsf(hi.z)));
     return m < 0x1p100f ? kBoxSlack * m : kInf;
 }
 
-// A ray's slack and axis order in one word (the slack rounded up, a multiple of 64).
+// kBoxSlack times at least the greatest distance along an axis between a ray's
+// origin and anything in the scene.
+__device__ __forceinline__ float ray_slack(const float o[3], float scene_slack) {
+    return __fmaf_rn(fmax3(fabsf(o[0]), fabsf(o[1]), fabsf(o[2])), kBoxSlack, scene_slack);
+}
+
+// A ray's slack and axis order in one word (the slack rounded up, a multiple of
+// 64), for the kernels whose lanes walk different structures.
 __device__ __forceinline__ uint32_t pack_slack(const Ray &r, const float o[3], float scene_slack) {
-    const float slack = __fmaf_rn(fmax3(fabsf(o[0]), fabsf(o[1]), fabsf(o[2])), kBoxSlack, scene_slack);
-    return ((__float_as_uint(slack) & ~63u) + 64u) | r.kxyz;
+    return ((__float_as_uint(ray_slack(o, scene_slack)) & ~63u) + 64u) | r.kxyz;
 }
 
 // Whether a box around the triangle of leaf record p, in a node anywhere above
-// it, could let the ray in beyond `limit` (a hit's distance); r: origin, shear
-// and pack_slack's word.
+// it, could let the ray in beyond `limit` (a hit's distance); r: origin and
+// shear, slack: ray_slack's.
 //
 // Along axis a such a box's near plane lies no further along the ray than the
 // triangle's nearest vertex, and isect_node's distance to it is off by less than
@@ -162,8 +169,7 @@ __device__ __forceinline__ uint32_t pack_slack(const Ray &r, const float o[3], f
 // + slack) / d_z and limit d_a / d_z, d_z the shear's axis, whose own roundings
 // stay below 5 * 2^-24 D; the slack is 16 * 2^-24 D.  Products too small to carry
 // that accuracy, and limits next to zero, count as exceeded.
-__device__ __forceinline__ bool boxes_may_exceed(const Ray &r, const uint4 *p, float limit) {
-    const float slack = __uint_as_float(r.kxyz & ~63u);
+__device__ __forceinline__ bool boxes_may_exceed(const Ray &r, float slack, const uint4 *p, float limit) {
     const uint32_t kx = r.kxyz & 3u, kz = (r.kxyz >> 4) & 3u;
     bool exceeds = !(limit >= 0x1p-40f);
 #pragma unroll
@@ -177,6 +183,11 @@ __device__ __forceinline__ bool boxes_may_exceed(const Ray &r, const uint4 *p, f
         exceeds = exceeds || !(ahead <= 0.0f || within);
     }
     return exceeds;
+}
+
+// With pack_slack's word in the ray.
+__device__ __forceinline__ bool boxes_may_exceed(const Ray &r, const uint4 *p, float limit) {
+    return boxes_may_exceed(r, __uint_as_float(r.kxyz & ~63u), p, limit);
 }
 
 // MIXED: one launch over two queues -- the closest-hit rays (rays, n_dev;
@@ -201,17 +212,16 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY || MIXED) ? 1024 : 115
     __shared__ uint4 s_best[ANY ? 1 : THREADS];
     __shared__ uint32_t s_visit[ANY ? 1 : THREADS];  // the node visit of the best hit so far (0: no hit)
     __shared__ int32_t s_prev[ANY ? 1 : THREADS];    // the nearest hit of an earlier visit, as an ordered integer
-    __shared__ float s_slack[THREADS / 32];          // box_slack of the structure
     static_assert(sizeof(s_stack) + sizeof(s_queue) + sizeof(s_shear) + sizeof(s_t) + sizeof(s_best) + sizeof(s_visit) +
-                          sizeof(s_prev) + sizeof(s_slack) <= 48u * 1024u,
+                          sizeof(s_prev) <= 48u * 1024u,
                   "static shared memory");
     const uint4 *nodes = nullptr, *prims = nullptr;
     // A tree walk visits each node at most once: more visits, or a node index
     // past the end, can only come from a corrupt structure.
     uint32_t max_visits = 0;
     bool empty = true;
+    const rt_accel_header *hd = reinterpret_cast<const rt_accel_header *>(a.accel);
     if (!MULTI) {
-        const rt_accel_header *hd = reinterpret_cast<const rt_accel_header *>(a.accel);
         if (!MIXED && !a.n_dev) pdl_launch();  // a ray query's k_trace_inst
         if (hd->kind != RT_ACCEL_KIND_BLAS) return;  // k_trace_inst handles it
         nodes = reinterpret_cast<const uint4 *>(a.accel + hd->node_offset);
@@ -229,10 +239,8 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY || MIXED) ? 1024 : 115
     uint2 spill[kMaxDepth + 1];
     uint32_t &aside = spill[kMaxDepth].x, &ray_index = spill[kMaxDepth].y;
     aside = kNone;
-    if (!ANY && !MULTI && lane == 0)
-        s_slack[tid >> 5] = empty ? 0.0f : box_slack(reinterpret_cast<const rt_accel_header *>(a.accel));
-    __syncwarp();
 
+    if (MULTI) __syncwarp();  // (registers: six scenes 2.98 ms without, 2.91 with it)
     bool have_ray = false, exhausted = false, pending = false;
     Ray r;
     r.o[0] = r.o[1] = r.o[2] = 0.f;
@@ -299,8 +307,9 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY || MIXED) ? 1024 : 115
                 } else {
                     const uint4 best = s_best[tid];
                     if (best.w != kNone && (best.z & kLate)) {
-                        a.hits[ray_idx] = make_float4(__uint_as_float(aside), __uint_as_float(best.z & ~(kMinusZero | kLate)),
-                                                      ford_inv(s_prev[tid]), tbest);
+                        const uint32_t rec = best.z & ~(kMinusZero | kLate);
+                        a.hits[ray_idx] =
+                            make_float4(__uint_as_float(aside), __uint_as_float(rec), ford_inv(s_prev[tid]), tbest);
                         aside = ray_idx;
                     } else {
                         write_hit(ray_idx, best.w != kNone, (best.z & kMinusZero) ? -0.0f : tbest,
@@ -327,7 +336,7 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY || MIXED) ? 1024 : 115
                         scene_src = a.ray_scene2;
                     }
                 }
-                float scene_slack = ANY || MULTI ? 0.0f : s_slack[tid >> 5];
+                float scene_slack = 0.0f;
                 if (MULTI) {
                     const uint32_t s = __ldg(scene_src + idx);
                     if (s < a.n_scenes) {
@@ -344,7 +353,8 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY || MIXED) ? 1024 : 115
                 tbest = r1.w;
                 found = false;
                 ray_index = idx;
-                s_shear[tid] = make_float4(r.sx, r.sy, r.sz, __uint_as_float(ANY ? r.kxyz : pack_slack(r, o, scene_slack)));
+                const uint32_t order = MULTI ? pack_slack(r, o, scene_slack) : r.kxyz;
+                s_shear[tid] = make_float4(r.sx, r.sy, r.sz, __uint_as_float(order));
                 if (!ANY) {
                     s_t[tid] = ford(tbest + 0.0f);  // -0 and +0 tie
                     s_best[tid].w = kNone;
@@ -484,42 +494,49 @@ __global__ void __launch_bounds__(THREADS, ((MULTI || ANY || MIXED) ? 1024 : 115
                     uint4 *best = s_best + warp0 + src;
                     const uint32_t visit = e.y >> 5;
                     const bool hit_too = hit;
-                    if (hit && atomicMin(bt, key) > key) best->w = kNone;
-                    __syncwarp();
-                    hit = hit && *bt == key;
-                    if (hit) atomicMin(&best->w, tri);
-                    __syncwarp();
-                    hit = hit && best->w == tri;
-                    if (hit) {
-                        const uint32_t before = s_visit[warp0 + src];
-                        s_visit[warp0 + src] = visit;
-                        if (before != visit) s_prev[warp0 + src] = before ? ford(t_hi + 0.0f) : kNoLimit;
-                        best->x = __float_as_uint(u);
-                        best->y = __float_as_uint(v);
-                        best->z = rec | (__float_as_uint(t) == kMinusZero ? kMinusZero : 0u);
-                    }
-                    __syncwarp();
-                    if (hit_too && !hit && visit < s_visit[warp0 + src]) atomicMin(s_prev + warp0 + src, key);
-                    __syncwarp();
-                    const int32_t prev = hit ? s_prev[warp0 + src] : kNoLimit;
-                    if (kFewRegisters) {  // the ray read again, not held through the above
-                        if (__any_sync(kFull, prev != kNoLimit)) {
-                            Ray again;
-                            again.o[0] = __shfl_sync(kFull, r.o[0], src);
-                            again.o[1] = __shfl_sync(kFull, r.o[1], src);
-                            again.o[2] = __shfl_sync(kFull, r.o[2], src);
-                            const float4 sh = s_shear[warp0 + src];
-                            again.sx = sh.x;
-                            again.sy = sh.y;
-                            again.sz = sh.z;
-                            again.kxyz = __float_as_uint(sh.w);
-                            if (prev != kNoLimit && boxes_may_exceed(again, pr + (size_t)rec * 3u, ford_inv(prev)))
+                    if (__any_sync(kFull, hit)) {
+                        if (hit && atomicMin(bt, key) > key) best->w = kNone;
+                        __syncwarp();
+                        hit = hit && *bt == key;
+                        if (hit) atomicMin(&best->w, tri);
+                        __syncwarp();
+                        hit = hit && best->w == tri;
+                        if (hit) {
+                            const uint32_t before = s_visit[warp0 + src];
+                            s_visit[warp0 + src] = visit;
+                            if (before != visit) s_prev[warp0 + src] = before ? ford(t_hi + 0.0f) : kNoLimit;
+                            best->x = __float_as_uint(u);
+                            best->y = __float_as_uint(v);
+                            best->z = rec | (__float_as_uint(t) == kMinusZero ? kMinusZero : 0u);
+                        }
+                        __syncwarp();
+                        if (hit_too && !hit && visit < s_visit[warp0 + src]) atomicMin(s_prev + warp0 + src, key);
+                        __syncwarp();
+                        const int32_t prev = hit ? s_prev[warp0 + src] : kNoLimit;
+                        if (kFewRegisters) {  // the ray read again, not held through the above
+                            if (__any_sync(kFull, prev != kNoLimit)) {
+                                Ray again;
+                                again.o[0] = __shfl_sync(kFull, r.o[0], src);
+                                again.o[1] = __shfl_sync(kFull, r.o[1], src);
+                                again.o[2] = __shfl_sync(kFull, r.o[2], src);
+                                const float4 sh = s_shear[warp0 + src];
+                                again.sx = sh.x;
+                                again.sy = sh.y;
+                                again.sz = sh.z;
+                                again.kxyz = __float_as_uint(sh.w);
+                                if (prev != kNoLimit && boxes_may_exceed(again, ray_slack(again.o, box_slack(hd)),
+                                                                         pr + (size_t)rec * 3u, ford_inv(prev)))
+                                    best->z |= kLate;
+                            }
+                        } else if (prev != kNoLimit) {
+                            const uint4 *p = pr + (size_t)rec * 3u;
+                            const float limit = ford_inv(prev);
+                            if (MULTI ? boxes_may_exceed(tr, p, limit)
+                                      : boxes_may_exceed(tr, ray_slack(tr.o, box_slack(hd)), p, limit))
                                 best->z |= kLate;
                         }
-                    } else if (prev != kNoLimit && boxes_may_exceed(tr, pr + (size_t)rec * 3u, ford_inv(prev))) {
-                        best->z |= kLate;
+                        __syncwarp();
                     }
-                    __syncwarp();
                     if (MIXED && any_ray) {
                         found = s_best[tid].w != kNone;
                         if (found) {
