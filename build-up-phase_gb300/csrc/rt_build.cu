@@ -1674,7 +1674,7 @@ int run_build(rt_context *ctx, cudaStream_t st, const BuildCall &bc, const GeomP
 //
 // Two launches: the records with their boxes, one block finding the levels of
 // the tree beside them; then the nodes, a level at a time from the bottom,
-// one thread per node and a grid barrier between levels.
+// eight lanes per node and a grid barrier between levels.
 
 struct RefitLayout {
     uint64_t flag, leaf_box, node_box, levels, list, total;
@@ -1758,7 +1758,7 @@ __device__ void refit_levels(const uint4 *nodes, uint32_t nc, uint32_t *flag, ui
 }
 
 // Leaf records and their boxes from the new inputs, one thread per record;
-// block 0 finds the levels.  Bound by memory: 62 us for 2M triangles, 250 MB of
+// block 0 finds the levels.  Bound by memory: 60 us for 2M triangles, 250 MB of
 // DRAM traffic.
 template <bool INST>
 __global__ void __launch_bounds__(kRecThreads) k_refit_records(const GeomParams gp, const rt_instance *inst, uint32_t n,
@@ -1949,7 +1949,7 @@ __device__ __forceinline__ void refit_append(bool want, uint32_t k, uint32_t dep
 // 32 per warp and step, the others listed by level; then the lists a level at
 // a time from the bottom, a grid barrier between levels.  Once the levels left
 // are small, one block goes on alone with block barriers.  2M-triangle box (11
-// levels, 643,300 nodes): 130 us -- 70 for the nodes without internal children,
+// levels, 643,300 nodes): 138 us -- 70 for the nodes without internal children,
 // 7-10 for each of the seven large levels (of which the barrier is about 4), 2
 // for each small one.  Before, one thread started at each childless node and
 // the last of a parent's children to arrive climbed on: 249 us, most warps

@@ -720,7 +720,8 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_cache_fwd_bwd_small(CacheS
 //
 // A layer starts with one MMA that sets the accumulators to the bias: a tile of
 // ones times the bias split in three BF16 parts, whose sum is the FP32 bias
-// exactly, so the layer's MMAs add onto the bias.  The epilogue of every thread
+// exactly (a tiny one scaled up against a column of 2^-64), so the layer's MMAs
+// add onto the bias.  The epilogue of every thread
 // reads its row's 64 accumulators with tcgen05.ld (each warp its own 32-lane
 // quarter), applies ReLU and packs BF16 in one cvt.rn.relu.bf16x2.f32 per pair,
 // and writes the row back to TMEM as the next layer's A operand (two BF16 per
@@ -728,8 +729,9 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_cache_fwd_bwd_small(CacheS
 // mbarrier wait is bounded: on expiry the kernel records RT_ERR_TIMEOUT, waits
 // once more (bounded) for its MMAs, frees its TMEM and returns.
 //
-// 2,073,600 queries: 141 us, tensor pipe 62 % busy (an MMA of N = 64 fills half
-// of it), the rest the encoding and the epilogues.  248 us with four groups, the
+// 2,073,600 queries: 141 us, tensor pipe busy 62 % of the cycles at 36 % of its
+// rate (an MMA of N = 64 fills about half of it), the rest the encoding and the
+// epilogues.  248 us with four groups, the
 // biases stored to TMEM for every row and layer and the activations written to
 // shared memory in the MMA's layout.
 

@@ -1074,11 +1074,10 @@ int launch_batch(rt_context *ctx, cudaStream_t st, uint64_t accel, const rt_ray 
 }  // namespace
 
 // Refill threshold of the path tracer's queue traversals: a warp refills once
-// eight of its lanes are idle (2M box, 4 spp per call: 6.91 / 6.56 / 6.45 /
-// 6.43 ms per sample at 2 / 4 / 6 / 8; the ray-query calls keep the context's
-// batch_rays, whose default 4 is best for the soup's primary + incoherent
-// rays; re-checked with the packed box test and the 8-entry ring: 6.26 /
-// 6.23 / 6.33 ms at 6 / 8 / 12).  The batch's autotuner chose 8 as well.
+// eight of its lanes are idle (2M box, four samples: 21.07 / 20.97 / 21.20 /
+// 21.47 ms at 6 / 8 / 10 / 12).  The batch's autotuner chose 8 as well.  The
+// ray-query calls keep the context's batch_rays (default 4; 6 is 1 % faster on
+// the soup's primary + incoherent rays).
 constexpr uint32_t kQueueRefill = 8u;
 
 // Queue-driven BLAS traversal for the wavefront path tracer: the ray count is
@@ -1305,10 +1304,12 @@ int trace_host(rt_context *ctx, cudaStream_t st, uint64_t accel, const rt_ray *h
     // Grace-Blackwell system also pageable memory, through the host page
     // tables): one launch reads the rays and writes the results where they
     // are, over NVLink-C2C.  A ray is read once (32 bytes) and a result
-    // written once, so no staging copy, chunk or ring is needed (4.15M rays
-    // of the 1M soup: 2.14 ms pinned or pageable, against 2.47 ms staged from
-    // pinned, 3.91 ms staged from pageable and 2.07 ms with rays and hits in
-    // HBM).
+    // written once -- but for a ray set aside, whose result's place is written,
+    // read and written again and which is read again, and half of a ray at each
+    // instance it enters --, so no staging copy, chunk or ring is needed (4.15M
+    // rays of the 1M soup: 1.77 ms pinned, against 2.23 ms staged from pinned
+    // and 1.56 ms with rays and hits in HBM; 800K rays in 64 instances 1.13 to
+    // 1.20 ms, staged 1.35, in HBM 1.03).
     RT_CUDA_CTX(ctx, cudaSetDevice(ctx->device));
     const bool pageable = pageable_in_place(ctx);
     if (ctx->host_transfer == RT_HOST_TRANSFER_AUTO && (reinterpret_cast<uintptr_t>(hrays) & 15u) == 0 &&

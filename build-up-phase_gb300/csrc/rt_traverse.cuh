@@ -30,10 +30,11 @@ namespace rtc {
 namespace {
 
 constexpr int kTraceThreads = 128;  // block size of the single-structure kernels
-// Shared-memory stack entries per ray of the single-structure kernels: 8 KB
-// per block, so nine blocks leave more of the SM's L1 to node fetches than
-// 16 entries did (1M soup: 2,150 -> 2,159 M rays/s; path tracer 6.33 -> 6.29
-// ms per sample); deeper entries spill to local memory.
+// Shared-memory stack entries per ray of the single-structure kernels; deeper
+// ones spill to local memory.  With the triangle queue and the rays' hits a
+// block takes 15.5 KB, of which this is 8: 16 entries leave node fetches too
+// little of the SM's L1 (64 scenes at 16 samples: 4.99 s, 4.36 at 8), and 4
+// spill too often (1M soup 1,568 us, 1,558 at 8; 64 instances 820 and 809).
 constexpr int kRing = 8;
 constexpr uint32_t kAnyBlocksPerSm = 1024u / kTraceThreads;  // resident blocks the any-hit and mixed kernels are bounded for
 constexpr int kMaxDepth = 64;       // total stack entries per ray
@@ -197,7 +198,7 @@ __device__ __forceinline__ bool boxes_may_exceed(const Ray &r, const uint4 *p, f
 // rays together, so the two share one launch tail.
 // Register budget: the closest-hit single-structure kernel fits nine 128-thread
 // blocks per SM (56 registers; at eight blocks and 64 registers the 1M soup's
-// rays took 1.71 instead of 1.68 ms); the others keep eight blocks and 64
+// rays took 1.74 instead of 1.58 ms); the others keep eight blocks and 64
 // registers (mixed, nine blocks: 2M box 21.26 ms per four samples, eight 20.85).
 template <bool ANY, bool MULTI, int THREADS, int RING, bool MIXED = false>
 __global__ void __launch_bounds__(THREADS, ((MULTI || ANY || MIXED) ? 1024 : 1152) / THREADS) k_trace_blas(const BatchArgs a) {
