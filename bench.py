@@ -71,14 +71,14 @@ BYTES_TRI = 36      # FP32 vertex triplet
 # its refit, 80 / 8 for the BVH8 node share of one leaf-equivalent
 BYTES_BUILD_PER_TRI = 48 + 12 + 24 * 8 + 2 * 24 + 80 // 8
 # DRAM bytes (read + write) of one step's traversal launch measured by ncu
-# (cold caches): 452.0 MB read + 68.6 MB written
-TRAFFIC_BYTES_PER_STEP = 520_700_000
+# (cold caches): 462.1 MB read + 69.6 MB written
+TRAFFIC_BYTES_PER_STEP = 531_700_000
 # From the same ncu capture of the step's launch: L2 sectors (32 B) moved,
 # warp instructions issued and the SIMT efficiency (active threads per warp
 # instruction / 32)
-L2_SECTORS_PER_STEP = 270_000_000
-WARP_INST_PER_STEP = 1_471_500_000
-SIMT_EFFICIENCY = 22.9 / 32
+L2_SECTORS_PER_STEP = 276_200_000
+WARP_INST_PER_STEP = 1_477_200_000
+SIMT_EFFICIENCY = 23.1 / 32
 TRAFFIC_SOURCE = "constant from one ncu capture of the step's launch (cold caches), not measured in this run"
 SMS, SMSP_PER_SM = 152, 4   # GB300: 152 SMs, four schedulers (one warp instruction per cycle each)
 L2_NOTE = ("GPU arm: L2 flushed between steps (256 MB write, outside the step events); "
