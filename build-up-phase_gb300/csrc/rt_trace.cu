@@ -181,7 +181,7 @@ __device__ bool trace_ray(const uint8_t *accel, const float o[3], const float d[
             uint32_t i = __ffs(ph) - 1;
             ph &= ph - 1u;
             InstRec ir = load_inst(prims, pbase + i);
-            if (((ir.cim >> 24) & cull_mask) == 0u) continue;
+            if (((ir.cim >> 24) & cull_mask) == 0u || ir.accel_ref == 0u) continue;
             float o2[3], d2[3];
             xform_point(ir.w2o, o, o2);
             xform_vector(ir.w2o, d, d2);
@@ -508,8 +508,9 @@ __global__ void __launch_bounds__(kTraceThreads, kInstBlocksPerSm) k_trace_inst(
                 const InstRec ir = load_inst(tprims, rec);
                 const uint8_t *blas = reinterpret_cast<const uint8_t *>(ir.accel_ref);
                 const rt_accel_header *bh = reinterpret_cast<const rt_accel_header *>(blas);
-                if (((ir.cim >> 24) & 0xffu) == 0u || bh->prim_count == 0u) {
-                    // masked out (cull mask 0xFF) or empty: on to the next
+                if (((ir.cim >> 24) & 0xffu) == 0u || !blas || bh->prim_count == 0u) {
+                    // masked out (cull mask 0xFF), without a structure (its box
+                    // is empty, but a ray of NaNs enters any) or empty: on to the next
                     // instance, else to what the stack holds
                     if (ig.y == 0u && sp > 0) {
                         uint2 g = pop();
@@ -885,7 +886,7 @@ k_trace_stats(const uint8_t *accel, const float4 *rays, uint32_t n, uint32_t ref
                 const InstRec ir = load_inst(tprims, rec);
                 const uint8_t *blas = reinterpret_cast<const uint8_t *>(ir.accel_ref);
                 const rt_accel_header *bh = reinterpret_cast<const rt_accel_header *>(blas);
-                if (((ir.cim >> 24) & 0xffu) == 0u || bh->prim_count == 0u) continue;
+                if (((ir.cim >> 24) & 0xffu) == 0u || !blas || bh->prim_count == 0u) continue;
                 if (sp + 3 > kInstDepth) {
                     fail(0x71000000u);
                     break;
